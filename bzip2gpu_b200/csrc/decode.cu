@@ -6,12 +6,10 @@
 //      block magic 0x314159265359 and the end-of-stream magic 0x177245385090;
 //      the host then follows the chain (a block starts where the previous one
 //      ended), so a magic that happens to appear inside a payload is ignored.
-//   2. k_dec_block: one warp per candidate block.  All 32 lanes walk the bit
-//      stream in lockstep (the same reads, so shared-memory tables are read as
-//      broadcasts): header (CRC, origPtr, symbol map, tables, selectors),
-//      Huffman symbols via an 8-bit lookup table with the canonical slow path
-//      for longer codes, RUNA/RUNB zero runs, and the inverse move-to-front
-//      32 MTF steps at a time across the warp.  Out: the BWT last column L.
+//   2. k_dec_head / _groups / _syms / _mscan / _emit: header and tables, the
+//      bit position of every 50-symbol group (the one serial chain, hopped 8
+//      codes at a time), the groups' symbols and the inverse move-to-front in
+//      parallel over chunks of 32 groups.  Out: the BWT last column L.
 //   3. k_dec_lf_hist / _scan / _rank: LF vector
 //      tt[C[L[i]] + rank(i)] = i << 8 | L[i] by a stable counting sort.
 //   4. k_dec_split / k_dec_walk / k_dec_chain: per block, the chain from
@@ -133,7 +131,7 @@ __global__ void k_dec_magic(const uint32_t *words, int64_t nwords, int64_t nbits
   }
 }
 
-// Per-block results of k_dec_block.
+// Per-block results of the entropy decode.
 struct DecBlock {
   int64_t start;    // bit position of the block magic
   int64_t end;      // bit position after the payload
@@ -141,19 +139,69 @@ struct DecBlock {
   int32_t orig_ptr;
   uint32_t crc;     // from the header
   int32_t status;
+  int32_t nchunks;  // chunks of symbols up to the end of the block
 };
 
-struct DecShared {
-  uint16_t lut[kDecMaxGroups][1 << kLutBits];  // (len << 9) | symbol; 0 = longer code
-  int32_t limit[kDecMaxGroups][kDecMaxCode + 2];
-  int32_t base[kDecMaxGroups][kDecMaxCode + 2];
-  uint16_t perm[kDecMaxGroups][kDecMaxAlpha];
-  uint8_t minlen[kDecMaxGroups];
-  uint8_t len[kDecMaxGroups][kDecMaxAlpha];
+// Entropy decode of one block, split so that only the group starts are a
+// serial chain (a code's length is known only once its start is):
+//   k_dec_head    header, selectors, code tables           (a CTA per block)
+//   k_dec_groups  bit position of every 50-symbol group    (a warp per block)
+//   k_dec_syms    the groups' symbols, a thread each, and the inverse
+//                 move-to-front of 32 groups (a chunk) from an unknown
+//                 starting list                            (a warp per chunk)
+//   k_dec_mscan   the chunks' starting lists and offsets   (a CTA per block)
+//   k_dec_emit    the last column                          (a warp per chunk)
+constexpr int kHeadThreads = 256;
+constexpr int kChunkGroups = 32;
+constexpr int kChunkSyms = kChunkGroups * kGroupSize;  // 1600
+constexpr int kMaxChunks = (kDecMaxSel + kChunkGroups - 1) / kChunkGroups;
+constexpr int kSymWarps = 4;
+
+// Per-block tables.  lj[t][n]: the largest 32-bit window (the stream's next
+// bits, left-justified) that starts with a code of at most n bits, for n in
+// [mn, mx]; a window's code length is the smallest such n.
+struct DecTab {
+  int64_t pay;  // bit position of the first symbol
+  int32_t status, nuse, ng, nsel, orig_ptr;
+  uint32_t crc;
+  int32_t ngv;  // groups whose start is known
+  uint8_t mn[kDecMaxGroups], mx[kDecMaxGroups];
+  uint32_t lj[kDecMaxGroups][kDecMaxCode + 4];
+  int32_t base[kDecMaxGroups][kDecMaxCode + 4];  // code - base = index into perm
+  uint16_t lut[kDecMaxGroups][1 << kLutBits];    // (len << 9) | symbol; 0 = longer code
+  uint16_t perm[kDecMaxGroups][kDecMaxAlpha + 6];
   uint8_t seq2unseq[256];
-  uint8_t list[2][256];  // MTF list before / after a batch of steps
-  uint32_t used[8];      // list positions a batch read
 };
+static_assert(sizeof(DecTab) % 8 == 0, "DecTab rows in an array");
+
+// What a chunk's symbols amount to, before the run digits carried into it and
+// its starting list are known.
+struct ChunkInfo {
+  int32_t nsym;   // symbols before the end of block, a bad code or the chunk's end
+  int32_t eob;    // 1: the end-of-block symbol follows them
+  int32_t bad;    // 1: a bad code follows them
+  int32_t lead;   // run digits before the first other symbol
+  int32_t trail;  // run digits after the last other symbol (nsym if there is none)
+  uint32_t end;   // eob: bits from the block's magic to the end of its payload
+  int64_t lead_sum, rest_sum;  // bytes of the leading run digits (counted from digit 0) and of the rest
+  int64_t off;    // offset of the chunk's bytes in the last column
+  int32_t q0;     // run digits just before the chunk
+  int32_t pad;
+};
+
+// A block's scratch until its LF vector is built, in that vector's memory.
+struct SymScratch {
+  uint16_t rec[kMaxChunks * kChunkSyms];
+  uint8_t list[kMaxChunks][256];  // end permutation, then starting list, of each chunk
+  ChunkInfo info[kMaxChunks];
+};
+static_assert(sizeof(SymScratch) <= (size_t)kDecCap * 4, "symbols fit the LF vector's memory");
+__device__ __forceinline__ SymScratch &sym_scratch(uint32_t *tt, int bi, int cap) {
+  return *reinterpret_cast<SymScratch *>(tt + (size_t)bi * cap);
+}
+// A record: the symbol's position in the chunk's starting list (bits 0-7);
+// a run digit has bit 15, its value in bit 13 and its place in bits 8-12.
+constexpr uint32_t kRecRun = 0x8000u;
 
 // c copies of byte v at d (word stores between unaligned ends).
 __device__ __forceinline__ void fill_bytes(uint8_t *d, int c, uint8_t v) {
@@ -166,317 +214,724 @@ __device__ __forceinline__ void fill_bytes(uint8_t *d, int c, uint8_t v) {
   while (c-- > 0) *d++ = v;
 }
 
-// One warp per candidate.  sel: per-candidate selector scratch (kDecMaxSel).
-__global__ void __launch_bounds__(32) k_dec_block(const uint32_t *words, int64_t nwords,
-                                                  const int64_t *cand, int ncand,
-                                                  DecBlock *out, uint8_t *Lbuf,
-                                                  uint8_t *selbuf, int cap,
-                                                  const int32_t *order) {
-  __shared__ DecShared sh;
-  if ((int)blockIdx.x >= ncand) return;
-  const int bi = order[blockIdx.x];  // largest compressed blocks first
-  const int ln = threadIdx.x;
-  DecBlock r;
-  r.start = cand[bi];
-  r.end = r.start;
-  r.m = 0;
-  r.orig_ptr = -1;
-  r.crc = 0;
-  r.status = kDecOk;
-  uint8_t *L = Lbuf + (size_t)bi * cap;
+// 32 stream bits from bit position p (zeros past the end).
+__device__ __forceinline__ uint32_t bits_at(const uint32_t *words, int64_t nwords, int64_t p) {
+  const int64_t i = p >> 5;
+  const uint32_t a = i < nwords ? bswap32(words[i]) : 0u;
+  const uint32_t b = i + 1 < nwords ? bswap32(words[i + 1]) : 0u;
+  return __funnelshift_l(b, a, (int)(p & 31));
+}
+
+// Selector lists as six nibbles, nibble k = table at list position k.
+__device__ __forceinline__ uint32_t sel_front(uint32_t lst, int j) {
+  const uint32_t t = (lst >> (4 * j)) & 0xFu;
+  const uint32_t low = (1u << (4 * j)) - 1u;
+  return (lst & ~((low << 4) | 0xFu)) | ((lst & low) << 4) | t;
+}
+// The list a after the moves that take the identity list to b.
+__device__ __forceinline__ uint32_t sel_then(uint32_t a, uint32_t b) {
+  uint32_t r = 0;
+#pragma unroll
+  for (int k = 0; k < kDecMaxGroups; k++)
+    r |= ((a >> (4 * ((b >> (4 * k)) & 0xFu))) & 0xFu) << (4 * k);
+  return r;
+}
+
+// Header, selectors and tables of a candidate block.
+// Selectors are unary codes: selector k ends at the k-th zero bit, so each
+// thread takes 32 bits, a scan of zero counts says which selectors end in
+// them, and the ones before a zero are its move-to-front index.  The index
+// sequence moves a six-entry list; each thread runs its share from the
+// identity list, a scan of those permutations gives every share's starting
+// list.  The delta-coded lengths are a serial chain (one thread).
+__global__ void __launch_bounds__(kHeadThreads) k_dec_head(const uint32_t *words, int64_t nwords,
+                                                           const int64_t *cand, DecTab *tabs,
+                                                           uint8_t *selbuf) {
+  __shared__ uint8_t sj[kDecMaxSel + 2];
+  __shared__ uint8_t len[kDecMaxGroups][kDecMaxAlpha + 6];
+  __shared__ int scratch[40];
+  __shared__ uint32_t wperm[kHeadThreads / 32];
+  __shared__ int64_t s_end;
+  __shared__ int s_status;
+  const int bi = blockIdx.x;
+  const int ln = lane_id(), w = warp_id();
+  DecTab &tab = tabs[bi];
   uint8_t *sel = selbuf + (size_t)bi * kDecMaxSel;
+  int status = kDecOk;
   BitReader br;
-  br.init(words, nwords, r.start + 48);
-  r.crc = br.get(32);
+  br.init(words, nwords, cand[bi] + 48);
+  const uint32_t crc = br.get(32);
   const uint32_t randomised = br.get(1);
-  r.orig_ptr = (int32_t)br.get(24);
-  // symbol map
+  const int orig_ptr = (int)br.get(24);
   const uint32_t used16 = br.get(16);
   int nuse = 0;
   for (int i = 0; i < 16; i++) {
     if ((used16 >> (15 - i)) & 1u) {
       const uint32_t bits = br.get(16);
-      for (int j = 0; j < 16; j++)
-        if ((bits >> (15 - j)) & 1u) {
-          if (ln == 0) sh.seq2unseq[nuse] = (uint8_t)(i * 16 + j);
-          nuse++;
-        }
+      if (threadIdx.x < 16 && ((bits >> (15 - threadIdx.x)) & 1u))
+        tab.seq2unseq[nuse + __popc(bits >> (16 - threadIdx.x))] = (uint8_t)(i * 16 + threadIdx.x);
+      nuse += __popc(bits);
     }
   }
   const int alpha = nuse + 2;
   const int ng = (int)br.get(3);
   const int nsel = (int)br.get(15);
-  if (randomised || nuse == 0 || ng < 2 || ng > 6 || nsel < 1 || nsel > kDecMaxSel) {
-    r.status = kDecBadHeader;
+  if (randomised || nuse == 0 || ng < 2 || ng > 6 || nsel < 1 || nsel > kDecMaxSel)
+    status = kDecBadHeader;
+  if (threadIdx.x == 0) {
+    s_status = status;
+    s_end = 0;
   }
-  // selectors: unary-coded MTF indices over 0..ng-1
-  if (r.status == kDecOk) {
-    uint32_t lst = 0x543210u;  // nibble k = table at list position k
-    for (int i = 0; i < nsel && r.status == kDecOk; i++) {
-      int j = 0;
-      while (br.get(1)) {
-        if (++j >= ng) {
-          r.status = kDecBadHeader;
+  __syncthreads();
+  if (status == kDecOk) {
+    const int64_t p0 = br.pos();
+    int done = 0;  // selectors ended so far
+    // a valid code has at most ng bits; a longer one ends the search
+    for (int r = 0; done < nsel && r < kDecMaxGroups * nsel; r += 32 * kHeadThreads) {
+      const int64_t p = p0 + r + 32 * (int64_t)threadIdx.x;
+      const uint32_t x = bits_at(words, nwords, p);
+      // the ones just before this thread's bits (none before the selectors)
+      const uint32_t before = p > p0 ? bits_at(words, nwords, p - 32) : 0u;
+      int ones = __ffs(~before) - 1;
+      if (ones < 0) ones = 32;
+      int tot;
+      int k = done + block_excl_sum(__popc(~x), scratch, &tot);
+      uint32_t z = ~x;
+      int at = -ones;  // where the current unary code began
+      while (z && k < nsel) {
+        const int q = __clz(z);
+        const int j = q - at;
+        if (j >= ng) s_status = kDecBadHeader;
+        sj[k] = (uint8_t)j;
+        if (k == nsel - 1) s_end = p + q + 1;
+        k++;
+        at = q + 1;
+        z &= ~(0x80000000u >> q);
+      }
+      done += tot;
+    }
+    if (done < nsel) s_status = kDecBadHeader;
+    __syncthreads();
+    status = s_status;
+  }
+  if (status == kDecOk) {
+    const int per = (nsel + kHeadThreads - 1) / kHeadThreads;
+    const int a = min(nsel, (int)threadIdx.x * per), e = min(nsel, a + per);
+    uint32_t mine = 0x543210u;
+    for (int i = a; i < e; i++) mine = sel_front(mine, sj[i]);
+    uint32_t inc = mine;  // moves of this and the earlier lanes
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
+      if (ln >= d) inc = sel_then(o, inc);
+    }
+    if (ln == 31) wperm[w] = inc;
+    uint32_t lst = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (ln == 0) lst = 0x543210u;
+    __syncthreads();
+    uint32_t pre = 0x543210u;
+    for (int q = 0; q < w; q++) pre = sel_then(pre, wperm[q]);
+    lst = sel_then(pre, lst);
+    for (int i = a; i < e; i++) {
+      lst = sel_front(lst, sj[i]);
+      sel[i] = (uint8_t)(lst & 0xFu);
+    }
+    // code lengths: 5-bit start, then per symbol 1x (x=0: +1, x=1: -1), 0 ends
+    if (threadIdx.x == 0) {
+      br.init(words, nwords, s_end);
+      int st = kDecOk;
+      for (int t = 0; t < ng && st == kDecOk; t++) {
+        int cur = (int)br.get(5);
+        for (int v = 0; v < alpha; v++) {
+          uint32_t x = br.peek32();
+          int used = 0, steps = 0;
+          for (;;) {
+            if (cur < 1 || cur > kDecMaxCode || ++steps > 64) {
+              st = kDecBadTables;
+              break;
+            }
+            if (!(x >> 31)) {
+              used++;
+              break;
+            }
+            cur += (x & 0x40000000u) ? -1 : 1;
+            x <<= 2;
+            used += 2;
+            if (used >= 30) {
+              br.skip(used);
+              used = 0;
+              x = br.peek32();
+            }
+          }
+          if (st != kDecOk) break;
+          br.skip(used);
+          len[t][v] = (uint8_t)cur;
+        }
+      }
+      s_status = st;
+      tab.pay = br.pos();
+    }
+    __syncthreads();
+    status = s_status;
+  }
+  if (status == kDecOk && w < ng) {
+    // canonical codes, a warp per table: the symbols of each length in symbol
+    // order take consecutive codes (lane l holds symbols l, l + 32, ...)
+    constexpr int kSlots = (kDecMaxAlpha + 31) / 32;
+    int lv[kSlots];
+    int mn = 32, mx = 0;
+#pragma unroll
+    for (int q = 0; q < kSlots; q++) {
+      const int v = 32 * q + ln;
+      lv[q] = v < alpha ? (int)len[w][v] : -1;
+      if (v < alpha) {
+        mn = min(mn, lv[q]);
+        mx = max(mx, lv[q]);
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    const unsigned below = (1u << ln) - 1u;
+    int idx = 0;
+    uint32_t code = 0;
+    for (int l = mn; l <= mx; l++) {
+      const int first = idx;
+#pragma unroll
+      for (int q = 0; q < kSlots; q++) {
+        const bool hit = lv[q] == l;
+        const unsigned bal = __ballot_sync(0xffffffffu, hit);
+        if (hit) tab.perm[w][idx + __popc(bal & below)] = (uint16_t)(32 * q + ln);
+        idx += __popc(bal);
+      }
+      // codes of length l: [code, code + idx - first)
+      const uint64_t end = (uint64_t)code + (uint32_t)(idx - first);
+      if (ln == 0) {
+        tab.base[w][l] = (int32_t)code - first;
+        tab.lj[w][l] = (end << (32 - l)) > 0xFFFFFFFFull ? 0xFFFFFFFFu
+                                                         : (uint32_t)(end << (32 - l)) - 1u;
+      }
+      code = (uint32_t)end << 1;
+    }
+    if (ln == 0) {
+      tab.mn[w] = (uint8_t)mn;
+      tab.mx[w] = (uint8_t)mx;
+    }
+    __syncwarp();
+    for (int p = ln; p < (1 << kLutBits); p += 32) {
+      const uint32_t x = (uint32_t)p << (32 - kLutBits);
+      uint16_t e = 0;
+      for (int l = mn; l <= min(mx, kLutBits); l++) {
+        if (x <= tab.lj[w][l]) {
+          const int i = (int)(x >> (32 - l)) - tab.base[w][l];
+          if (i >= 0 && i < alpha) e = (uint16_t)((l << 9) | tab.perm[w][i]);
           break;
         }
       }
-      if (r.status != kDecOk) break;
-      const uint32_t t = (lst >> (4 * j)) & 0xFu;
-      // move to front: nibbles below j shift up one
-      const uint32_t low = (1u << (4 * j)) - 1u;
-      lst = (lst & ~((low << 4) | 0xFu)) | ((lst & low) << 4) | t;
-      if (ln == 0) sel[i] = (uint8_t)t;
+      tab.lut[w][p] = e;
     }
   }
-  // code lengths: 5-bit start, then per symbol 1x (x=0: +1, x=1: -1), 0 ends
-  if (r.status == kDecOk) {
-    for (int t = 0; t < ng && r.status == kDecOk; t++) {
-      int cur = (int)br.get(5);
-      for (int v = 0; v < alpha; v++) {
-        int steps = 0;
-        for (;;) {
-          if (cur < 1 || cur > kDecMaxCode || ++steps > 64) {
-            r.status = kDecBadTables;
-            break;
+  if (threadIdx.x == 0) {
+    tab.status = status;
+    tab.nuse = nuse;
+    tab.ng = ng;
+    tab.nsel = nsel;
+    tab.orig_ptr = orig_ptr;
+    tab.crc = crc;
+    tab.ngv = 0;
+  }
+}
+
+// Bit position of every group, one warp per block.  The chain over a group's
+// 50 codes is cut short: for a window of bit positions from the group's start
+// all code lengths are looked up at once (32 positions per step), the map
+// "position -> position after one code" is squared three times in shared
+// memory (after 2, 4, 8 codes), and the group is six 8-code hops and one
+// 2-code hop.  The window is as wide as the table's last group was, plus a
+// quarter, and a group that leaves it goes on in another.  The chain bounds
+// it: 16 ms for a 900,000-byte block (4,800 groups), where one code after
+// another, with the move-to-front in the same warp, took 50 ms.
+constexpr int kWinSteps = 16;
+constexpr int kWin = 32 * kWinSteps;
+constexpr int kLenBits = 10;
+constexpr int kRing = 256;
+constexpr uint32_t kNoHop = 0x8000u;   // the map leaves the window on its way
+constexpr uint32_t kDeadCode = 0xFFFFu;  // no code starts here
+
+__global__ void __launch_bounds__(32) k_dec_groups(const uint32_t *words, int64_t nwords,
+                                                   const int64_t *cand, DecTab *tabs,
+                                                   const uint8_t *selbuf, uint32_t *gstart,
+                                                   const int32_t *order) {
+  __shared__ uint8_t llen[kDecMaxGroups][1 << kLenBits];
+  __shared__ uint32_t lj[kDecMaxGroups][kDecMaxCode + 4];
+  __shared__ uint16_t s1[kWin], s2[kWin], s8[kWin];
+  __shared__ uint32_t ring[kRing];
+  const unsigned full = 0xffffffffu;
+  const int bi = order[blockIdx.x];  // largest compressed blocks first
+  const int ln = threadIdx.x;
+  DecTab &tab = tabs[bi];
+  if (tab.status != kDecOk) return;
+  const int ng = tab.ng, nsel = tab.nsel;
+  for (int t = 0; t < ng; t++)
+    if (ln < kDecMaxCode + 4) lj[t][ln] = tab.lj[t][ln];
+  const int my_mn = ln < ng ? tab.mn[ln] : 0, my_mx = ln < ng ? tab.mx[ln] : 0;
+  __syncwarp();
+  for (int t = 0; t < ng; t++) {
+    const int mn = __shfl_sync(full, my_mn, t), mx = __shfl_sync(full, my_mx, t);
+    for (int p = ln; p < (1 << kLenBits); p += 32) {
+      const uint32_t x = (uint32_t)p << (32 - kLenBits);
+      int n = 0;
+      for (int l = min(mx, kLenBits); l >= mn; l--)
+        if (x <= lj[t][l]) n = l;
+      llen[t][p] = (uint8_t)n;
+    }
+  }
+  const uint8_t *sel = selbuf + (size_t)bi * kDecMaxSel;
+  uint32_t *gs = gstart + (size_t)bi * kDecMaxSel;
+  const int64_t start = cand[bi];
+  const int64_t wbase = start >> 5;  // word indices below are relative to it
+  const uint32_t *W = words + wbase;
+  const int64_t navail = nwords - wbase;
+  uint32_t p = (uint32_t)(tab.pay - (wbase << 5));
+  const uint32_t bias = (uint32_t)(start & 31);
+  // ring of byte-swapped words: [hi - kRing, hi) present, the next 128 in pf
+  uint32_t hi = p >> 5;
+  uint32_t pf[4];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int64_t i = (int64_t)hi + 32 * k + ln;
+      pf[k] = i < navail ? W[i] : 0u;
+    }
+  };
+  fetch();
+  int last_bits = kWin;  // lane t: bits of table t's last group
+  uint32_t my_start = 0;
+  int my_sel = 0;
+  int g = 0;
+  bool dead = false;
+  for (; g < nsel && !dead; g++) {
+    if ((g & 31) == 0) my_sel = g + ln < nsel ? sel[g + ln] : 0;
+    if (ln == (g & 31)) my_start = p - bias;
+    const int t = __shfl_sync(full, my_sel, g & 31);
+    const int mn = __shfl_sync(full, my_mn, t), mx = __shfl_sync(full, my_mx, t);
+    const int lb = __shfl_sync(full, last_bits, t);
+    const uint8_t *lt = llen[t];
+    const uint32_t *ljt = lj[t];
+    const uint32_t p_begin = p;
+    int rem = kGroupSize;
+    int J = min(kWinSteps, max(4, (lb + (lb >> 2) + 63) >> 5));
+    while (rem > 0 && !dead) {
+      const uint32_t i0 = p >> 5;
+      while (hi < i0 + kWinSteps + 4) {  // at most twice: i0 advances by less than 128 words
+#pragma unroll
+        for (int k = 0; k < 4; k++) ring[(hi + 32 * k + ln) & (kRing - 1)] = bswap32(pf[k]);
+        hi += 128;
+        fetch();
+      }
+      __syncwarp();
+      const int ew = 32 * J;  // window width
+      const int o0 = (int)(p & 31) + ln;
+      const uint32_t c = i0 + (o0 >> 5);
+      const int sh = o0 & 31;
+      uint32_t cur[kWinSteps];
+      uint32_t wa = ring[c & (kRing - 1)];
+#pragma unroll
+      for (int j = 0; j < kWinSteps; j++) {
+        if (j < J) {
+          const uint32_t wb = ring[(c + j + 1) & (kRing - 1)];
+          const uint32_t x = __funnelshift_l(wb, wa, sh);
+          wa = wb;
+          int n = lt[x >> (32 - kLenBits)];
+          if (n == 0) {
+            n = max(mn, kLenBits + 1);
+            while (n <= mx && x > ljt[n]) n++;
+            if (n > mx) n = 0;
           }
-          if (!br.get(1)) break;
-          cur += br.get(1) ? -1 : 1;
+          const int o = 32 * j + ln;
+          cur[j] = n ? (uint32_t)(o + n) : kDeadCode;
+          s1[o] = (uint16_t)cur[j];
         }
-        if (r.status != kDecOk) break;
-        if (ln == 0) sh.len[t][v] = (uint8_t)cur;
       }
+      __syncwarp();
+      auto square = [&](const uint16_t *from, uint16_t *to) {
+#pragma unroll
+        for (int j = 0; j < kWinSteps; j++)
+          if (j < J) cur[j] = cur[j] < (uint32_t)ew ? (uint32_t)from[cur[j]] : kNoHop;
+        if (from == to) __syncwarp();
+#pragma unroll
+        for (int j = 0; j < kWinSteps; j++)
+          if (j < J) to[32 * j + ln] = (uint16_t)cur[j];
+        __syncwarp();
+      };
+      square(s1, s2);
+      square(s2, s8);  // after 4 codes
+      square(s8, s8);  // after 8
+      uint32_t at = 0;
+      while (rem >= 8 && at < (uint32_t)ew) {
+        const uint32_t v = s8[at];
+        if (v >= kNoHop) break;
+        at = v;
+        rem -= 8;
+      }
+      while (rem >= 2 && at < (uint32_t)ew) {
+        const uint32_t v = s2[at];
+        if (v >= kNoHop) break;
+        at = v;
+        rem -= 2;
+      }
+      while (rem >= 1 && at < (uint32_t)ew) {
+        const uint32_t v = s1[at];
+        if (v >= kNoHop) {
+          dead = true;
+          break;
+        }
+        at = v;
+        rem--;
+      }
+      p += at;
+      __syncwarp();
+    }
+    if (ln == t) last_bits = (int)(p - p_begin);
+    if ((g & 31) == 31 || g + 1 == nsel || dead) {
+      const int gb = g & ~31;
+      if (gb + ln <= g) gs[gb + ln] = my_start;
     }
   }
-  __syncwarp();
-  // canonical decoding tables: for each length, the symbols of that length in
-  // symbol order get consecutive codes; limit[n] = largest code of length n,
-  // base[n] turns a length-n code into an index into perm.
-  if (r.status == kDecOk) {
-    for (int t = 0; t < ng; t++) {
-      int mn = 32, mx = 0;
-      for (int v = 0; v < alpha; v++) {
-        mn = min(mn, (int)sh.len[t][v]);
-        mx = max(mx, (int)sh.len[t][v]);
-      }
-      if (ln == 0) {
-        sh.minlen[t] = (uint8_t)mn;
-        int pp = 0;
-        for (int l = mn; l <= mx; l++)
-          for (int v = 0; v < alpha; v++)
-            if (sh.len[t][v] == l) sh.perm[t][pp++] = (uint16_t)v;
-        int count[kDecMaxCode + 2];
-        for (int l = 0; l <= kDecMaxCode + 1; l++) count[l] = 0;
-        for (int v = 0; v < alpha; v++) count[sh.len[t][v]]++;
-        int code = 0, idx = 0;
-        for (int l = 0; l <= kDecMaxCode + 1; l++) {
-          sh.limit[t][l] = -1;
-          sh.base[t][l] = 0;
+  if (ln == 0) tab.ngv = g;
+}
+
+// Symbols and local move-to-front of a chunk of 32 groups, one warp each.
+// Lane l decodes group l's codes into shared memory.  The inverse
+// move-to-front then runs over the chunk from the identity list (so a
+// symbol's value is a position in the chunk's starting list), 32 symbols at
+// a time across the warp:
+//  * lane t walks its index back through the batch's earlier steps s: a
+//    step moved the entry at v_s to the front, so position p after it was
+//    p - 1 before it when 1 <= p <= v_s, and p == 0 is step s's own output
+//    (a run digit repeats the front entry: index 0, no move);
+//  * lanes that reach position 0 point at that step's lane, the others read
+//    the list as it was before the batch; pointer jumping settles pointers;
+//  * the new list: the batch's distinct outputs, most recent first, then
+//    the untouched entries in their old order (equal outputs found by
+//    ballots).
+__global__ void __launch_bounds__(32 * kSymWarps)
+    k_dec_syms(const uint32_t *words, int64_t nwords, const int64_t *cand, const DecTab *tabs,
+               const uint8_t *selbuf, const uint32_t *gstart, uint32_t *tt, int cap) {
+  __shared__ uint16_t lut[kDecMaxGroups][1 << kLutBits];
+  __shared__ uint32_t lj[kDecMaxGroups][kDecMaxCode + 4];
+  __shared__ int32_t base[kDecMaxGroups][kDecMaxCode + 4];
+  __shared__ uint16_t perm[kDecMaxGroups][kDecMaxAlpha + 6];
+  __shared__ uint16_t sy[kSymWarps][kChunkSyms];
+  __shared__ uint8_t lists[kSymWarps][2][256];
+  __shared__ uint32_t used_s[kSymWarps][8];
+  const unsigned full = 0xffffffffu;
+  const int bi = blockIdx.y;
+  const DecTab &tab = tabs[bi];
+  if (tab.status != kDecOk) return;
+  const int ngv = tab.ngv;
+  const int c0 = blockIdx.x * kSymWarps;
+  if (c0 * kChunkGroups >= ngv) return;
+  const int ng = tab.ng, nuse = tab.nuse;
+  for (int i = threadIdx.x; i < ng * (1 << kLutBits); i += blockDim.x)
+    (&lut[0][0])[i] = (&tab.lut[0][0])[i];
+  for (int i = threadIdx.x; i < ng * (kDecMaxCode + 4); i += blockDim.x) {
+    (&lj[0][0])[i] = (&tab.lj[0][0])[i];
+    (&base[0][0])[i] = (&tab.base[0][0])[i];
+  }
+  for (int i = threadIdx.x; i < ng * (kDecMaxAlpha + 6); i += blockDim.x)
+    (&perm[0][0])[i] = (&tab.perm[0][0])[i];
+  __syncthreads();
+  const int ln = lane_id(), w = warp_id();
+  const int c = c0 + w;
+  if (c * kChunkGroups >= ngv) return;
+  SymScratch &out = sym_scratch(tt, bi, cap);
+  const int64_t start = cand[bi];
+  const int alpha = nuse + 2, eob = nuse + 1;
+  const int ngc = min(kChunkGroups, ngv - c * kChunkGroups);
+  int e_at = INT32_MAX, b_at = INT32_MAX;  // chunk index of this lane's end-of-block, bad code
+  uint32_t e_end = 0;
+  if (ln < ngc) {
+    const int g = c * kChunkGroups + ln;
+    const int t = selbuf[(size_t)bi * kDecMaxSel + g];
+    const int mn = tab.mn[t], mx = tab.mx[t];
+    BitReader br;
+    br.init(words, nwords, start + gstart[(size_t)bi * kDecMaxSel + g]);
+    uint16_t *dst = sy[w] + ln * kGroupSize;
+    for (int i = 0; i < kGroupSize; i++) {
+      const uint32_t x = br.peek32();
+      const uint32_t e = lut[t][x >> (32 - kLutBits)];
+      int sym;
+      if (e) {
+        br.skip((int)(e >> 9));
+        sym = (int)(e & 511u);
+      } else {
+        int n = max(mn, kLutBits + 1);
+        while (n <= mx && x > lj[t][n]) n++;
+        const int idx = n <= mx ? (int)(x >> (32 - n)) - base[t][n] : -1;
+        if (idx < 0 || idx >= alpha) {
+          b_at = ln * kGroupSize + i;
+          break;
         }
-        for (int l = mn; l <= mx; l++) {
-          // codes of length l: [code, code + count[l]), perm index idx ..
-          sh.base[t][l] = code - idx;
-          sh.limit[t][l] = code + count[l] - 1;
-          idx += count[l];
-          code = (code + count[l]) << 1;
-        }
+        br.skip(n);
+        sym = perm[t][idx];
       }
+      if (sym == eob) {
+        e_at = ln * kGroupSize + i;
+        e_end = (uint32_t)(br.pos() - start);
+        break;
+      }
+      dst[i] = (uint16_t)sym;
     }
   }
+  const int eob_at = __reduce_min_sync(full, e_at), bad_at = __reduce_min_sync(full, b_at);
+  const int n = min(min(eob_at, bad_at), ngc * kGroupSize);
   __syncwarp();
-  if (r.status == kDecOk) {
-    // lookup tables: every kLutBits-bit prefix that starts a code of at most
-    // kLutBits bits
-    for (int t = 0; t < ng; t++) {
-      for (int p = ln; p < (1 << kLutBits); p += 32) {
-        uint16_t e = 0;
-        for (int l = sh.minlen[t]; l <= kLutBits; l++) {
-          const int code = p >> (kLutBits - l);
-          if (code <= sh.limit[t][l] && sh.limit[t][l] >= 0) {
-            const int idx = code - sh.base[t][l];
-            if (idx >= 0 && idx < alpha) e = (uint16_t)((l << 9) | sh.perm[t][idx]);
-            break;
-          }
-        }
-        sh.lut[t][p] = e;
-      }
-    }
-  }
-  __syncwarp();
-  // Huffman symbols -> RUNA/RUNB runs -> MTF steps, batched: lane q holds
-  // step q of the batch (v = MTF index, 0 for a zero run; bytes = 1, or the
-  // run length).  A full batch is resolved across the warp at once:
-  //  * lane t walks its index back through the batch's earlier steps s: a
-  //    step moved the entry at v_s to the front, so position p after it was
-  //    p - 1 before it when 1 <= p <= v_s, and p == 0 is step s's own output;
-  //  * lanes that reach position 0 point at that step's lane, the others read
-  //    the list as it was before the batch; pointer jumping settles pointers;
-  //  * the new list: the batch's distinct outputs, most recent first, then
-  //    the untouched entries in their old order (equal outputs found by
-  //    ballots).
-  for (int p = ln; p < 256; p += 32) sh.list[0][p] = (uint8_t)p;
+  uint8_t *lb = lists[w][0];
+  uint32_t *used = used_s[w];
+  for (int q = ln; q < 256; q += 32) lb[q] = (uint8_t)q;
   __syncwarp();
   int cur = 0;
-  int my_v = 0, my_n = 0, nst = 0;
-  int m = 0;     // bytes written by resolved batches
-  int pend = 0;  // bytes of the batch being filled
-  int64_t zrun = 0;
-  int zbit = 0;
-  const int eob = nuse + 1;
-  int gsel = 0, gleft = 0, tsel = 0;
-  auto resolve_batch = [&]() {
-    const unsigned full = 0xffffffffu;
-    const bool act = ln < nst;
-    int p = my_v, ptr = -1;
+  int run = 0;        // run digits just before the batch
+  bool lead = true;   // only run digits so far
+  int lead_cnt = 0;
+  int64_t lead_sum = 0, rest_sum = 0;
+  uint16_t *rec = out.rec + (size_t)c * kChunkSyms;
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    const int nb = min(32, n - i0);
+    const bool act = ln < nb;
+    const int sym = act ? sy[w][i0 + ln] : 0;
+    const bool dgt = act && sym <= 1;
+    const unsigned runs = __ballot_sync(full, dgt);
+    const unsigned others = __ballot_sync(full, act && !dgt);
+    const uint8_t *lst = lb + 256 * cur;
+    int val;
+    if (others == 0u) {
+      val = lst[0];
+    } else {
+      const int my_v = act && !dgt ? sym - 1 : 0;
+      int p = my_v, ptr = -1;
 #pragma unroll
-    for (int s = 30; s >= 0; --s) {
-      const int vs = __shfl_sync(full, my_v, s);
-      if (ln > s && ptr < 0) {
-        if (p == 0) ptr = s;
-        else if (p <= vs) p--;
+      for (int s = 30; s >= 0; --s) {
+        const int vs = __shfl_sync(full, my_v, s);
+        if (ln > s && ptr < 0) {
+          if (p == 0) ptr = s;
+          else if (p <= vs) p--;
+        }
       }
-    }
-    const uint8_t *lst = sh.list[cur];
-    const bool from_list = act && ptr < 0;
-    int val = from_list ? (int)lst[p] : -1;
+      const bool from_list = act && ptr < 0;
+      val = from_list ? (int)lst[p] : -1;
 #pragma unroll
-    for (int r2 = 0; r2 < 5; r2++) {
-      const int src = ptr >= 0 ? ptr : ln;
-      const int tv = __shfl_sync(full, val, src);
-      const int tp = __shfl_sync(full, ptr, src);
-      if (val < 0 && ptr >= 0) {
-        if (tv >= 0) val = tv;
-        else ptr = tp;
+      for (int r2 = 0; r2 < 5; r2++) {
+        const int src = ptr >= 0 ? ptr : ln;
+        const int tv = __shfl_sync(full, val, src);
+        const int tp = __shfl_sync(full, ptr, src);
+        if (val < 0 && ptr >= 0) {
+          if (tv >= 0) val = tv;
+          else ptr = tp;
+        }
       }
-    }
-    // active lanes with the same output: one ballot per bit of it
-    unsigned peers = __ballot_sync(full, act);
+      // active lanes with the same output: one ballot per bit of it
+      unsigned peers = __ballot_sync(full, act);
 #pragma unroll
-    for (int bit = 0; bit < 8; bit++) {
-      const bool on = act && ((val >> bit) & 1);
-      const unsigned bb = __ballot_sync(full, on);
-      peers &= on ? bb : ~bb;
-    }
-    const unsigned above = ~((2u << ln) - 1u);  // lanes after this one
-    const bool last = act && (peers & above) == 0u;
-    const unsigned lastm = __ballot_sync(full, last);
-    const int D = __popc(lastm);
-    if (ln < 8) sh.used[ln] = 0u;
-    __syncwarp();
-    if (from_list) atomicOr(&sh.used[p >> 5], 1u << (p & 31));
-    __syncwarp();
-    uint8_t *nx = sh.list[cur ^ 1];
-    if (last) nx[__popc(lastm & above)] = (uint8_t)val;
-    {
+      for (int bit = 0; bit < 8; bit++) {
+        const bool on = act && ((val >> bit) & 1);
+        const unsigned bb = __ballot_sync(full, on);
+        peers &= on ? bb : ~bb;
+      }
+      const unsigned above = ~((2u << ln) - 1u);  // lanes after this one
+      const bool last = act && (peers & above) == 0u;
+      const unsigned lastm = __ballot_sync(full, last);
+      const int D = __popc(lastm);
+      if (ln < 8) used[ln] = 0u;
+      __syncwarp();
+      if (from_list) atomicOr(&used[p >> 5], 1u << (p & 31));
+      __syncwarp();
+      uint8_t *nx = lb + 256 * (cur ^ 1);
+      if (last) nx[__popc(lastm & above)] = (uint8_t)val;
       const int q0 = 8 * ln;
       int below = 0;
-      for (int x = 0; x < (q0 >> 5); x++) below += __popc(sh.used[x]);
-      const uint32_t uw = sh.used[q0 >> 5];
+      for (int x = 0; x < (q0 >> 5); x++) below += __popc(used[x]);
+      const uint32_t uw = used[q0 >> 5];
       for (int j = 0; j < 8; j++) {
         const int q = q0 + j;
         if (q >= nuse) break;
         const uint32_t bit = 1u << (q & 31);
         if (!(uw & bit)) nx[D + q - below - __popc(uw & (bit - 1u))] = lst[q];
       }
+      cur ^= 1;
+      __syncwarp();
     }
-    // bytes: step t at m + (bytes of the earlier steps)
-    const int nb = act ? my_n : 0;
-    const int incl = warp_incl_sum(nb);
+    // a run digit's place: the digits just before it
+    const unsigned bm = others & ((1u << ln) - 1u);
+    const int q = bm ? ln - 32 + __clz(bm) : ln + run;
+    const int qc = min(q, 31);
+    if (act) rec[i0 + ln] = (uint16_t)(dgt ? kRecRun | (sym << 13) | (qc << 8) | val : val);
     if (act) {
-      const uint8_t c = sh.seq2unseq[val];
-      if (nb == 1) L[m + incl - 1] = c;
-      else fill_bytes(L + m + incl - nb, nb, c);
+      const int64_t bytes = dgt ? (int64_t)(sym + 1) << min(q, 40) : 1;
+      if (lead && bm == 0u && dgt) lead_sum += bytes;
+      else rest_sum += bytes;
     }
-    m += __shfl_sync(full, incl, 31);
-    cur ^= 1;
-    nst = 0;
-    pend = 0;
-    __syncwarp();
-  };
-  // queue one step (the caller has checked the capacity)
-  auto push_step = [&](int v, int bytes) {
-    if (ln == nst) {
-      my_v = v;
-      my_n = bytes;
+    if (lead) lead_cnt += others ? __ffs(others) - 1 : nb;
+    if (others) {
+      lead = false;
+      run = nb - 32 + __clz(others);
+    } else {
+      run += nb;
     }
-    nst++;
-    pend += bytes;
-    if (nst == 32) resolve_batch();
-  };
-  // Every iteration takes one symbol of a 50-symbol group and the groups are
-  // bounded by nsel, so the loop ends.
-  if (r.status == kDecOk) {
-    int tsel_next = sel[0];
-    const uint16_t *lut = sh.lut[0];
-    for (;;) {
-      if (gleft == 0) {
-        if (gsel >= nsel) {
-          r.status = kDecBadSymbol;
-          break;
-        }
-        tsel = tsel_next;
-        lut = sh.lut[tsel];
-        gsel++;
-        tsel_next = gsel < nsel ? sel[gsel] : 0;  // next group's table, loaded early
-        gleft = 50;
-      }
-      gleft--;
-      // one symbol with table tsel
-      int sym;
-      const uint32_t win = br.peek32();
-      const uint32_t e = lut[win >> (32 - kLutBits)];
-      if (e) {
-        br.skip((int)(e >> 9));
-        sym = (int)(e & 511u);
-      } else {
-        // longer than the table: the canonical limits from kLutBits + 1 bits
-        int n = max((int)sh.minlen[tsel], kLutBits + 1);
-        int code = (int)(win >> (32 - n));
-        while (n <= kDecMaxCode && code > sh.limit[tsel][n]) {
-          n++;
-          code = (int)(win >> (32 - n));
-        }
-        const int idx = n <= kDecMaxCode ? code - sh.base[tsel][n] : -1;
-        if (idx < 0 || idx >= alpha) {
-          r.status = kDecBadSymbol;
-          break;
-        }
-        br.skip(n);
-        sym = sh.perm[tsel][idx];
-      }
-      if (sym <= 1) {  // RUNA / RUNB: bijective base-2 digits, least significant first
-        if (zbit > 40) {
-          r.status = kDecTooLong;
-          break;
-        }
-        zrun += (int64_t)(sym + 1) << zbit;
-        zbit++;
-        continue;
-      }
-      // a pending zero run: copies of the list's front entry (no move)
-      if (zrun > 0) {
-        if (zrun > (int64_t)(cap - m - pend)) {
-          r.status = kDecTooLong;
-          break;
-        }
-        push_step(0, (int)zrun);
-        zrun = 0;
-        zbit = 0;
-      }
-      if (sym == eob) break;
-      // value v = sym - 1 >= 1: the entry at list position v moves to the front
-      const int v = sym - 1;
-      if (v >= nuse || m + pend >= cap) {
-        r.status = v >= nuse ? kDecBadSymbol : kDecTooLong;
-        break;
-      }
-      push_step(v, 1);
-    }
-    if (r.status == kDecOk && nst > 0) resolve_batch();
   }
-  if (r.status == kDecOk && (r.orig_ptr < 0 || r.orig_ptr >= m)) r.status = kDecBadOrigPtr;
-  r.m = m;
-  r.end = br.pos();
-  if (ln == 0) out[bi] = r;
+  for (int o = 16; o; o >>= 1) {
+    lead_sum += __shfl_xor_sync(full, lead_sum, o);
+    rest_sum += __shfl_xor_sync(full, rest_sum, o);
+  }
+  const uint8_t *lst = lb + 256 * cur;
+  for (int q = ln; q < 64; q += 32)
+    reinterpret_cast<uint32_t *>(out.list[c])[q] = reinterpret_cast<const uint32_t *>(lst)[q];
+  ChunkInfo &ci = out.info[c];
+  if (e_at == eob_at && e_at != INT32_MAX) ci.end = e_end;
+  if (ln == 0) {
+    ci.nsym = n;
+    ci.eob = eob_at != INT32_MAX && eob_at < bad_at;
+    ci.bad = bad_at < eob_at;
+    ci.lead = lead_cnt;
+    ci.trail = run;
+    ci.lead_sum = lead_sum;
+    ci.rest_sum = rest_sum;
+  }
+}
+
+// Per block: chunk offsets, starting lists, and the block's result.
+__global__ void __launch_bounds__(256) k_dec_mscan(const int64_t *cand, const DecTab *tabs,
+                                                   uint32_t *tt, int cap, DecBlock *res) {
+  __shared__ int64_t scratch[40];
+  __shared__ int s_last;
+  __shared__ uint8_t lst[2][256];
+  const int bi = blockIdx.x;
+  const DecTab &tab = tabs[bi];
+  DecBlock r;
+  r.start = cand[bi];
+  r.end = r.start;
+  r.m = 0;
+  r.orig_ptr = tab.orig_ptr;
+  r.crc = tab.crc;
+  r.status = tab.status;
+  r.nchunks = 0;
+  if (r.status != kDecOk) {
+    if (threadIdx.x == 0) res[bi] = r;
+    return;
+  }
+  SymScratch &sc = sym_scratch(tt, bi, cap);
+  const int nch = (tab.ngv + kChunkGroups - 1) / kChunkGroups;
+  if (threadIdx.x == 0) s_last = nch;
+  __syncthreads();
+  for (int c = threadIdx.x; c < nch; c += 256)
+    if (sc.info[c].eob || sc.info[c].bad) atomicMin(&s_last, c);
+  __syncthreads();
+  const int last = s_last;  // the chunk holding the end of the block (nch: none does)
+  if (last == nch || sc.info[last].bad) r.status = kDecBadSymbol;
+  const int nc = min(last + 1, nch);
+  // bytes per chunk and their offsets
+  int64_t total = 0;
+  for (int c0 = 0; c0 < nc; c0 += 256) {
+    const int c = c0 + threadIdx.x;
+    int64_t bytes = 0;
+    if (c < nc) {
+      // digits just before the chunk (a chunk of nothing else is an overlong run by itself)
+      const int q0 = c > 0 ? min(sc.info[c - 1].trail, 40) : 0;
+      sc.info[c].q0 = q0;
+      // more than 2^30 bytes, or a digit past place 20, is too long in any case
+      constexpr int64_t kHuge = (int64_t)1 << 30;
+      const int64_t ls = sc.info[c].lead_sum;
+      bytes = ls > 0 && (ls > kHuge || q0 > 20) ? kHuge : ls << min(q0, 20);
+      bytes = min(kHuge, bytes) + min(kHuge, sc.info[c].rest_sum);
+    }
+    int64_t tot;
+    const int64_t off = total + block_excl_sum(bytes, scratch, &tot);
+    if (c < nc) sc.info[c].off = off;
+    total += tot;
+  }
+  if (r.status == kDecOk && total > cap) r.status = kDecTooLong;
+  if (r.status == kDecOk) {
+    r.m = (int)total;
+    r.nchunks = nc;
+    r.end = r.start + sc.info[last].end;
+    if (r.orig_ptr < 0 || r.orig_ptr >= r.m) r.status = kDecBadOrigPtr;
+  }
+  if (threadIdx.x == 0) res[bi] = r;
+  if (r.status != kDecOk) return;
+  // starting lists, in bytes: chunk c + 1's entry k is chunk c's entry P_c[k]
+  const int k = threadIdx.x;
+  lst[0][k] = k < tab.nuse ? tab.seq2unseq[k] : 0;
+  __syncthreads();
+  int cur = 0;
+  constexpr int kAhead = 8;
+  for (int c0 = 0; c0 < nc; c0 += kAhead) {
+    uint8_t P[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; q++) P[q] = c0 + q < nc ? sc.list[c0 + q][k] : 0;
+#pragma unroll
+    for (int q = 0; q < kAhead; q++) {
+      if (c0 + q < nc) {
+        sc.list[c0 + q][k] = lst[cur][k];
+        lst[cur ^ 1][k] = lst[cur][P[q]];
+        __syncthreads();
+        cur ^= 1;
+      }
+    }
+  }
+}
+
+// The last column: a warp per chunk writes its symbols' bytes, long runs by
+// all its lanes.
+__global__ void __launch_bounds__(32 * kSymWarps)
+    k_dec_emit(const DecBlock *res, uint32_t *tt, uint8_t *Lbuf, int cap) {
+  __shared__ uint8_t lists[kSymWarps][256];
+  const unsigned full = 0xffffffffu;
+  const int bi = blockIdx.y;
+  if (res[bi].status != kDecOk) return;
+  const int ln = lane_id(), w = warp_id();
+  const int c = blockIdx.x * kSymWarps + w;
+  if (c >= res[bi].nchunks) return;
+  SymScratch &sc = sym_scratch(tt, bi, cap);
+  const ChunkInfo ci = sc.info[c];
+  int64_t off = ci.off;
+  for (int q = ln; q < 64; q += 32)
+    reinterpret_cast<uint32_t *>(lists[w])[q] = reinterpret_cast<const uint32_t *>(sc.list[c])[q];
+  __syncwarp();
+  uint8_t *L = Lbuf + (size_t)bi * cap;
+  const uint16_t *rec = sc.rec + (size_t)c * kChunkSyms;
+  for (int i0 = 0; i0 < ci.nsym; i0 += 32) {
+    const int i = i0 + ln;
+    const uint32_t r = i < ci.nsym ? rec[i] : 0u;
+    int nb = i < ci.nsym ? 1 : 0;
+    if (r & kRecRun) {
+      const int q = (int)((r >> 8) & 31u) + (i < ci.lead ? ci.q0 : 0);
+      nb = (int)(((r >> 13) & 1u) + 1u) << min(q, 28);
+    }
+    const uint8_t v = lists[w][r & 0xFFu];
+    const int inc = warp_incl_sum(nb);
+    const int64_t at = off + inc - nb;
+    if (nb == 1) L[at] = v;
+    else if (nb > 1 && nb <= 64) fill_bytes(L + at, nb, v);
+    unsigned big = __ballot_sync(full, nb > 64);
+    while (big) {
+      const int s = __ffs(big) - 1;
+      big &= big - 1u;
+      const int bn = __shfl_sync(full, nb, s);
+      const int64_t ba = __shfl_sync(full, at, s);
+      const uint32_t bv = 0x01010101u * __shfl_sync(full, (uint32_t)v, s);
+      uint8_t *d = L + ba;
+      const int head = min(bn, (int)((0u - (uint32_t)reinterpret_cast<uintptr_t>(d)) & 15u));
+      const int body = (bn - head) / 16;
+      if (ln < head) d[ln] = (uint8_t)bv;
+      for (int q = ln; q < body; q += 32)
+        reinterpret_cast<uint4 *>(d + head)[q] = make_uint4(bv, bv, bv, bv);
+      const int done = head + 16 * body;
+      if (done + ln < bn) d[done + ln] = (uint8_t)bv;
+    }
+    off += __shfl_sync(full, inc, 31);
+  }
 }
 
 // LF vector without serial ranks: T[C[L[i]] + rank(i)] = i << 8 | L[i], with
@@ -945,15 +1400,15 @@ struct MallocSink : DecSink {
 // (stream st).
 struct DecWork {
   std::mutex mu;
-  DevBuf words, blk, eos, cnt, cand, order, db, L, hist, sel, idx, tt, lens, off, crc, ctl, bad,
-      lanes;
+  DevBuf words, blk, eos, cnt, cand, order, db, tab, gstart, L, hist, sel, idx, tt, lens, off, crc,
+      ctl, bad, lanes;
   DevBuf out[2];
   cudaStream_t st = nullptr, cs = nullptr;
   cudaEvent_t written[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
   bool used[2] = {false, false};
   uint32_t *h_crc = nullptr;  // pinned
   size_t h_crc_cap = 0;
-  int resident = 0;  // k_dec_block warps resident on the whole device
+  int resident = 0;  // k_dec_groups warps resident on the whole device
 
   void init() {
     if (st) return;
@@ -966,12 +1421,12 @@ struct DecWork {
     int dev = 0, sms = 0, per_sm = 0;
     BZ_CUDA(cudaGetDevice(&dev));
     BZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dec_block, 32, 0));
+    BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dec_groups, 32, 0));
     resident = std::max(1, sms * per_sm);
   }
   size_t held() const {
     size_t s = 0;
-    for (const DevBuf *b : {&L, &hist, &tt, &sel, &ctl, &out[0], &out[1]}) s += b->cap;
+    for (const DevBuf *b : {&L, &hist, &tt, &sel, &tab, &gstart, &ctl, &out[0], &out[1]}) s += b->cap;
     return s;
   }
 };
@@ -988,9 +1443,10 @@ DecWork &dec_work() {
 }
 
 // Device bytes of one candidate slot: last column (later the RLE1 bytes), LF
-// vector, chunk histograms, selectors, walk control.
-constexpr size_t kSlotBytes = (size_t)kDecCap * 5 + (size_t)kLfChunks * 256 * 4 + kDecMaxSel +
-                              sizeof(WalkCtl) + sizeof(DecBlock) + 32 * 8 + 64;
+// vector (before it the symbols), chunk histograms, selectors and group
+// starts, tables, walk control.
+constexpr size_t kSlotBytes = (size_t)kDecCap * 5 + (size_t)kLfChunks * 256 * 4 + kDecMaxSel * 5 +
+                              sizeof(DecTab) + sizeof(WalkCtl) + sizeof(DecBlock) + 32 * 8 + 64;
 constexpr int kMaxBatch = 4096;
 
 bool is_header(const uint8_t *h) {
@@ -1039,7 +1495,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
   BZ_CUDA(cudaStreamSynchronize(st));
   std::sort(cands.begin(), cands.end());
   std::sort(eoss.begin(), eoss.end());
-  // batch: whole waves of resident k_dec_block warps where memory allows
+  // batch: whole waves of resident k_dec_groups warps where memory allows
   size_t freeb = 0, totb = 0;
   BZ_CUDA(cudaMemGetInfo(&freeb, &totb));
   int bmax = (int)std::min<size_t>(kMaxBatch, (freeb + w.held()) / 3 / kSlotBytes);
@@ -1058,6 +1514,8 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
   w.L.reserve((size_t)batch * cap);
   w.hist.reserve((size_t)batch * kLfChunks * 256 * 4);
   w.sel.reserve((size_t)batch * kDecMaxSel);
+  w.gstart.reserve((size_t)batch * kDecMaxSel * 4);
+  w.tab.reserve((size_t)batch * sizeof(DecTab));
   w.idx.reserve(4 * (size_t)batch);
   w.tt.reserve((size_t)batch * cap * 4);
   w.lens.reserve(8 * (size_t)batch);
@@ -1140,9 +1598,23 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return csize(a) > csize(b); });
     BZ_CUDA(cudaMemcpyAsync(w.order.p, order.data(), 4 * nc, cudaMemcpyHostToDevice, st));
-    k_dec_block<<<nc, 32, 0, st>>>(w.words.get<uint32_t>(), nwords, w.cand.get<int64_t>(), nc,
-                                   w.db.get<DecBlock>(), L, w.sel.get<uint8_t>(), cap,
-                                   w.order.get<int32_t>());
+    const uint32_t *wd = w.words.get<uint32_t>();
+    const int64_t *dcand = w.cand.get<int64_t>();
+    DecTab *dtab = w.tab.get<DecTab>();
+    const dim3 cgrid((kMaxChunks + kSymWarps - 1) / kSymWarps, nc);
+    k_dec_head<<<nc, kHeadThreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>());
+    BZ_LAUNCH_CHECK();
+    k_dec_groups<<<nc, 32, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>(),
+                                    w.gstart.get<uint32_t>(), w.order.get<int32_t>());
+    BZ_LAUNCH_CHECK();
+    k_dec_syms<<<cgrid, 32 * kSymWarps, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>(),
+                                                 w.gstart.get<uint32_t>(), w.tt.get<uint32_t>(),
+                                                 cap);
+    BZ_LAUNCH_CHECK();
+    k_dec_mscan<<<nc, 256, 0, st>>>(dcand, dtab, w.tt.get<uint32_t>(), cap, w.db.get<DecBlock>());
+    BZ_LAUNCH_CHECK();
+    k_dec_emit<<<cgrid, 32 * kSymWarps, 0, st>>>(w.db.get<DecBlock>(), w.tt.get<uint32_t>(), L,
+                                                 cap);
     BZ_LAUNCH_CHECK();
     BZ_CUDA(cudaMemcpyAsync(hdb.data(), w.db.p, sizeof(DecBlock) * nc, cudaMemcpyDeviceToHost,
                             st));
