@@ -443,49 +443,62 @@ __global__ void __launch_bounds__(kHeadThreads) k_dec_head(const uint32_t *words
   }
 }
 
-// Bit position of every group, one warp per block.  The chain over a group's
-// 50 codes is cut short: for a window of bit positions from the group's start
-// all code lengths are looked up at once (32 positions per step), the map
-// "position -> position after one code" is squared three times in shared
-// memory (after 2, 4, 8 codes), and the group is six 8-code hops and one
-// 2-code hop.  The window is as wide as the table's last group was, plus a
-// quarter, and a group that leaves it goes on in another.  The chain bounds
-// it: 16 ms for a 900,000-byte block (4,800 groups), where one code after
-// another, with the move-to-front in the same warp, took 50 ms.
-constexpr int kWinSteps = 16;
-constexpr int kWin = 32 * kWinSteps;
-constexpr int kLenBits = 10;
+// Bit position of every group, one CTA of NW warps per block.  The chain over
+// a group's 50 codes is cut short: for a window of bit positions from the
+// group's start all code lengths are looked up at once, the map "position ->
+// position after one code" is squared three times in shared memory (after 2,
+// 4, 8 codes), and the group is six 8-code hops and one 2-code hop.  The
+// window is as wide as the table's last group was, plus a quarter; a group
+// that leaves it goes on in another.  Positions are table indices, and three
+// kinds of entries map to themselves or out, so that hops need no tests:
+// kPadAt .. the 32 positions past the window (a hop that ends there is good,
+// a further one is not), kNoHop (the map leaves the window on its way) and
+// kDeadCode (no code starts here).
+// The latency of this chain bounds a call of few blocks.
+constexpr int kWin = 512;
+constexpr int kLenBits = 12;
 constexpr int kRing = 256;
-constexpr uint32_t kNoHop = 0x8000u;   // the map leaves the window on its way
-constexpr uint32_t kDeadCode = 0xFFFFu;  // no code starts here
+constexpr int kRingLoad = 128;  // words per refill
+constexpr uint32_t kNoHop = kWin + 32;
+constexpr uint32_t kDeadCode = kWin + 33;
+constexpr int kHops = kWin + 34;
 
-__global__ void __launch_bounds__(32) k_dec_groups(const uint32_t *words, int64_t nwords,
-                                                   const int64_t *cand, DecTab *tabs,
-                                                   const uint8_t *selbuf, uint32_t *gstart,
-                                                   const int32_t *order) {
+template <int NW>
+__global__ void __launch_bounds__(32 * NW)
+    k_dec_groups(const uint32_t *words, int64_t nwords, const int64_t *cand, DecTab *tabs,
+                 const uint8_t *selbuf, uint32_t *gstart, const int32_t *order) {
+  constexpr int NT = 32 * NW;
+  constexpr int kPer = kWin / NT;  // window positions per thread
+  static_assert(NT >= kRingLoad && kPer >= 1, "warps per block");
   __shared__ uint8_t llen[kDecMaxGroups][1 << kLenBits];
   __shared__ uint32_t lj[kDecMaxGroups][kDecMaxCode + 4];
-  __shared__ uint16_t s1[kWin], s2[kWin], s8[kWin];
+  __shared__ uint8_t mn_s[kDecMaxGroups + 2], mx_s[kDecMaxGroups + 2];
+  // two sets used in turn: a warp may still hop in one while others fill the next
+  __shared__ uint16_t s1[2][kHops], s2[2][kHops], s4[2][kHops], s8[2][kHops];
   __shared__ uint32_t ring[kRing];
   const unsigned full = 0xffffffffu;
   const int bi = order[blockIdx.x];  // largest compressed blocks first
-  const int ln = threadIdx.x;
+  const int tid = threadIdx.x, ln = lane_id();
   DecTab &tab = tabs[bi];
   if (tab.status != kDecOk) return;
   const int ng = tab.ng, nsel = tab.nsel;
-  for (int t = 0; t < ng; t++)
-    if (ln < kDecMaxCode + 4) lj[t][ln] = tab.lj[t][ln];
-  const int my_mn = ln < ng ? tab.mn[ln] : 0, my_mx = ln < ng ? tab.mx[ln] : 0;
-  __syncwarp();
-  for (int t = 0; t < ng; t++) {
-    const int mn = __shfl_sync(full, my_mn, t), mx = __shfl_sync(full, my_mx, t);
-    for (int p = ln; p < (1 << kLenBits); p += 32) {
-      const uint32_t x = (uint32_t)p << (32 - kLenBits);
-      int n = 0;
-      for (int l = min(mx, kLenBits); l >= mn; l--)
-        if (x <= lj[t][l]) n = l;
-      llen[t][p] = (uint8_t)n;
-    }
+  for (int i = tid; i < ng * (kDecMaxCode + 4); i += NT) (&lj[0][0])[i] = (&tab.lj[0][0])[i];
+  if (tid < ng) {
+    mn_s[tid] = tab.mn[tid];
+    mx_s[tid] = tab.mx[tid];
+  }
+  if (tid < 2) {
+    for (uint32_t q : {kNoHop, kDeadCode})
+      s1[tid][q] = s2[tid][q] = s4[tid][q] = s8[tid][q] = (uint16_t)q;
+  }
+  __syncthreads();
+  for (int i = tid; i < ng << kLenBits; i += NT) {
+    const int t = i >> kLenBits;
+    const uint32_t x = (uint32_t)(i & ((1 << kLenBits) - 1)) << (32 - kLenBits);
+    const int mn = mn_s[t], mx = min((int)mx_s[t], kLenBits);
+    int n = mn;
+    while (n <= mx && x > lj[t][n]) n++;
+    llen[t][i & ((1 << kLenBits) - 1)] = (uint8_t)(n <= mx ? n : 0);
   }
   const uint8_t *sel = selbuf + (size_t)bi * kDecMaxSel;
   uint32_t *gs = gstart + (size_t)bi * kDecMaxSel;
@@ -495,111 +508,126 @@ __global__ void __launch_bounds__(32) k_dec_groups(const uint32_t *words, int64_
   const int64_t navail = nwords - wbase;
   uint32_t p = (uint32_t)(tab.pay - (wbase << 5));
   const uint32_t bias = (uint32_t)(start & 31);
-  // ring of byte-swapped words: [hi - kRing, hi) present, the next 128 in pf
+  // ring of byte-swapped words: [hi - kRing, hi) present, the next ones in pf
   uint32_t hi = p >> 5;
-  uint32_t pf[4];
+  uint32_t pf = 0;
   auto fetch = [&]() {
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int64_t i = (int64_t)hi + 32 * k + ln;
-      pf[k] = i < navail ? W[i] : 0u;
-    }
+    const int64_t i = (int64_t)hi + tid;
+    if (tid < kRingLoad) pf = i < navail ? W[i] : 0u;
   };
   fetch();
   int last_bits = kWin;  // lane t: bits of table t's last group
   uint32_t my_start = 0;
-  int my_sel = 0;
-  int g = 0;
+  int my_sel = 0, next_sel = ln < nsel ? sel[ln] : 0;
+  int g = 0, set = 0;
   bool dead = false;
   for (; g < nsel && !dead; g++) {
-    if ((g & 31) == 0) my_sel = g + ln < nsel ? sel[g + ln] : 0;
+    if ((g & 31) == 0) {
+      my_sel = next_sel;
+      next_sel = g + 32 + ln < nsel ? sel[g + 32 + ln] : 0;
+    }
     if (ln == (g & 31)) my_start = p - bias;
     const int t = __shfl_sync(full, my_sel, g & 31);
-    const int mn = __shfl_sync(full, my_mn, t), mx = __shfl_sync(full, my_mx, t);
     const int lb = __shfl_sync(full, last_bits, t);
     const uint8_t *lt = llen[t];
-    const uint32_t *ljt = lj[t];
     const uint32_t p_begin = p;
     int rem = kGroupSize;
-    int J = min(kWinSteps, max(4, (lb + (lb >> 2) + 63) >> 5));
+    const int ew = min(kWin, ((lb + (lb >> 2) + 63) >> 5) << 5);  // window width
     while (rem > 0 && !dead) {
       const uint32_t i0 = p >> 5;
-      while (hi < i0 + kWinSteps + 4) {  // at most twice: i0 advances by less than 128 words
-#pragma unroll
-        for (int k = 0; k < 4; k++) ring[(hi + 32 * k + ln) & (kRing - 1)] = bswap32(pf[k]);
-        hi += 128;
-        fetch();
+      if (hi < i0 + kWin / 32 + 4) {  // i0 advances by less than kRingLoad words
+        do {
+          if (tid < kRingLoad) ring[(hi + tid) & (kRing - 1)] = bswap32(pf);
+          hi += kRingLoad;
+          fetch();
+        } while (hi < i0 + kWin / 32 + 4);
+        __syncthreads();
       }
-      __syncwarp();
-      const int ew = 32 * J;  // window width
-      const int o0 = (int)(p & 31) + ln;
+      set ^= 1;
+      uint16_t *a1 = s1[set], *a2 = s2[set], *a4 = s4[set], *a8 = s8[set];
+      if (tid < 32) a1[ew + tid] = a2[ew + tid] = a4[ew + tid] = a8[ew + tid] = (uint16_t)kNoHop;
+      const int o0 = (int)(p & 31) + tid;
       const uint32_t c = i0 + (o0 >> 5);
       const int sh = o0 & 31;
-      uint32_t cur[kWinSteps];
-      uint32_t wa = ring[c & (kRing - 1)];
+      uint32_t cur[kPer];
 #pragma unroll
-      for (int j = 0; j < kWinSteps; j++) {
-        if (j < J) {
-          const uint32_t wb = ring[(c + j + 1) & (kRing - 1)];
-          const uint32_t x = __funnelshift_l(wb, wa, sh);
-          wa = wb;
+      for (int j = 0; j < kPer; j++) {
+        const int o = NT * j + tid;
+        if (o < ew) {
+          const uint32_t x = __funnelshift_l(ring[(c + NW * j + 1) & (kRing - 1)],
+                                             ring[(c + NW * j) & (kRing - 1)], sh);
           int n = lt[x >> (32 - kLenBits)];
           if (n == 0) {
-            n = max(mn, kLenBits + 1);
-            while (n <= mx && x > ljt[n]) n++;
+            const int mx = mx_s[t];
+            n = max((int)mn_s[t], kLenBits + 1);
+            while (n <= mx && x > lj[t][n]) n++;
             if (n > mx) n = 0;
           }
-          const int o = 32 * j + ln;
           cur[j] = n ? (uint32_t)(o + n) : kDeadCode;
-          s1[o] = (uint16_t)cur[j];
+          a1[o] = (uint16_t)cur[j];
         }
       }
-      __syncwarp();
+      __syncthreads();
       auto square = [&](const uint16_t *from, uint16_t *to) {
 #pragma unroll
-        for (int j = 0; j < kWinSteps; j++)
-          if (j < J) cur[j] = cur[j] < (uint32_t)ew ? (uint32_t)from[cur[j]] : kNoHop;
-        if (from == to) __syncwarp();
-#pragma unroll
-        for (int j = 0; j < kWinSteps; j++)
-          if (j < J) to[32 * j + ln] = (uint16_t)cur[j];
-        __syncwarp();
-      };
-      square(s1, s2);
-      square(s2, s8);  // after 4 codes
-      square(s8, s8);  // after 8
-      uint32_t at = 0;
-      while (rem >= 8 && at < (uint32_t)ew) {
-        const uint32_t v = s8[at];
-        if (v >= kNoHop) break;
-        at = v;
-        rem -= 8;
-      }
-      while (rem >= 2 && at < (uint32_t)ew) {
-        const uint32_t v = s2[at];
-        if (v >= kNoHop) break;
-        at = v;
-        rem -= 2;
-      }
-      while (rem >= 1 && at < (uint32_t)ew) {
-        const uint32_t v = s1[at];
-        if (v >= kNoHop) {
-          dead = true;
-          break;
+        for (int j = 0; j < kPer; j++) {
+          if (NT * j + tid < ew) {
+            cur[j] = from[cur[j]];
+            to[NT * j + tid] = (uint16_t)cur[j];
+          }
         }
-        at = v;
-        rem--;
+        __syncthreads();
+      };
+      square(a1, a2);
+      square(a2, a4);
+      square(a4, a8);
+      uint32_t at = kNoHop;
+      if (rem == kGroupSize) {
+        at = 0;
+#pragma unroll
+        for (int q = 0; q < kGroupSize / 8; q++) at = a8[at];
+        at = a2[at];
+      }
+      if (at < kNoHop) {
+        rem = 0;
+      } else {  // out of the window on the way: as far as the window goes
+        at = 0;
+        while (rem >= 8 && a8[at] < kNoHop) {
+          at = a8[at];
+          rem -= 8;
+        }
+        while (rem >= 2 && a2[at] < kNoHop) {
+          at = a2[at];
+          rem -= 2;
+        }
+        while (rem >= 1 && at < (uint32_t)ew && !dead) {
+          const uint32_t v = a1[at];
+          if (v == kDeadCode) {
+            dead = true;
+          } else {
+            at = v;
+            rem--;
+          }
+        }
       }
       p += at;
-      __syncwarp();
     }
     if (ln == t) last_bits = (int)(p - p_begin);
-    if ((g & 31) == 31 || g + 1 == nsel || dead) {
+    if (tid < 32 && ((g & 31) == 31 || g + 1 == nsel || dead)) {
       const int gb = g & ~31;
       if (gb + ln <= g) gs[gb + ln] = my_start;
     }
   }
-  if (ln == 0) tab.ngv = g;
+  if (tid == 0) tab.ngv = g;
+}
+
+// Warps per block: eight where the blocks leave the GPU room (the chain's
+// latency is what counts), four where there are enough blocks to fill it.
+using GroupsKernel = decltype(&k_dec_groups<8>);
+inline GroupsKernel groups_kernel(int nblocks, int sms, int *threads) {
+  const bool few = nblocks <= 6 * sms;
+  *threads = few ? 256 : 128;
+  return few ? k_dec_groups<8> : k_dec_groups<4>;
 }
 
 // Symbols and local move-to-front of a chunk of 32 groups, one warp each.
@@ -1408,7 +1436,8 @@ struct DecWork {
   bool used[2] = {false, false};
   uint32_t *h_crc = nullptr;  // pinned
   size_t h_crc_cap = 0;
-  int resident = 0;  // k_dec_groups warps resident on the whole device
+  int sms = 0;
+  int resident = 0;  // k_dec_groups blocks resident on the whole device
 
   void init() {
     if (st) return;
@@ -1418,10 +1447,10 @@ struct DecWork {
       BZ_CUDA(cudaEventCreateWithFlags(&written[q], cudaEventDisableTiming));
       BZ_CUDA(cudaEventCreateWithFlags(&copied[q], cudaEventDisableTiming));
     }
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, per_sm = 0;
     BZ_CUDA(cudaGetDevice(&dev));
     BZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dec_groups, 32, 0));
+    BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dec_groups<4>, 128, 0));
     resident = std::max(1, sms * per_sm);
   }
   size_t held() const {
@@ -1495,7 +1524,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
   BZ_CUDA(cudaStreamSynchronize(st));
   std::sort(cands.begin(), cands.end());
   std::sort(eoss.begin(), eoss.end());
-  // batch: whole waves of resident k_dec_groups warps where memory allows
+  // batch: whole waves of resident k_dec_groups blocks where memory allows
   size_t freeb = 0, totb = 0;
   BZ_CUDA(cudaMemGetInfo(&freeb, &totb));
   int bmax = (int)std::min<size_t>(kMaxBatch, (freeb + w.held()) / 3 / kSlotBytes);
@@ -1604,7 +1633,9 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const dim3 cgrid((kMaxChunks + kSymWarps - 1) / kSymWarps, nc);
     k_dec_head<<<nc, kHeadThreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>());
     BZ_LAUNCH_CHECK();
-    k_dec_groups<<<nc, 32, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>(),
+    int gthreads = 0;
+    const GroupsKernel groups = groups_kernel(nc, w.sms, &gthreads);
+    groups<<<nc, gthreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>(),
                                     w.gstart.get<uint32_t>(), w.order.get<int32_t>());
     BZ_LAUNCH_CHECK();
     k_dec_syms<<<cgrid, 32 * kSymWarps, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>(),
