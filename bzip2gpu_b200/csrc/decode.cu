@@ -15,8 +15,8 @@
 //   4. k_dec_split / k_dec_walk / k_dec_chain: per block, the chain from
 //      origPtr gives the RLE1 bytes, cut at up to 2048 splitters that are
 //      walked in parallel.
-//   5. k_dec_unrle1_count / _write: per block, one warp expands the RLE1 runs
-//      (4 equal bytes then a count byte) from 32 segments at once; k_dec_crc
+//   5. k_dec_unrle1_count / _scan / _write expand the RLE1 runs (4 equal bytes
+//      then a count byte) from 32-byte segments at once; k_dec_crc
 //      computes each block's CRC over its output (4096-byte chunks combined
 //      over GF(2)), checked against the header.
 // Batches of blocks go through steps 2-5 while the previous batch's bytes are
@@ -1192,23 +1192,46 @@ __global__ void k_dec_repeat(const int32_t *idx, const DecBlock *db, const WalkC
 }
 
 
-// Inverse RLE1 (4 equal bytes are followed by a count of further copies), one
-// warp per block.  The block's RLE1 bytes are cut into 32 lane segments.  What
-// a segment produces depends only on the run state it starts in: 0 = no run
-// (block start, or just after a count byte), 1..3 = the byte before the
-// segment closes a run of that length, 4 = the next byte is a count.  The
-// count pass follows each segment from all five states at once until they
-// merge (typically within a few bytes: at a byte that differs from the one
-// before it), chains the lanes' state maps from state 0 across the warp and
-// keeps each lane's entry state and output offset; the write pass expands
-// every segment at its offset (runs with word stores), and k_dec_crc computes
-// the block CRCs over the output.
-constexpr int kUnrleWarps = 8;
+// Inverse RLE1 (4 equal bytes are followed by a count of further copies).
+// The block's RLE1 bytes are cut into segments of 32, one thread each, 256 to
+// a tile.  What a segment produces depends only on the run state it starts
+// in: 0 = no run (block start, or just after a count byte), 1..3 = the byte
+// before the segment closes a run of that length, 4 = the next byte is a
+// count.  A segment is followed from all five states at once until they merge
+// (typically within a few bytes: at a byte that differs from the one before
+// it); its map "state before -> state after, bytes written" is one of an
+// associative set, so scans over a tile's segments, and over a block's tiles,
+// give every segment its state and offset.  The write pass forms the maps of
+// its tile again instead of reading them back (they would be 20 bytes per 32).
+// One warp per block took 3.5 + 1.0 ms for a single block, the latency of
+// 7,500 bytes per lane one after another.
+constexpr int kSegBytes = 32;
+constexpr int kUnTile = 256 * kSegBytes;  // 8192
+constexpr int kUnTiles = (kDecCap + kUnTile - 1) / kUnTile;
+constexpr int kSegStride = kSegBytes + 4;  // in shared memory: lanes on different banks
 
-struct LaneStart {
-  int32_t state;
-  int32_t off;  // output offset of the segment within its block
+// state after (bits 29-31) and bytes written, for each state before
+struct RunMap {
+  uint32_t v[5];
 };
+constexpr uint32_t kRunBytes = (1u << 29) - 1u;
+
+__device__ __forceinline__ uint32_t pick5(uint32_t x, const uint32_t (&a)[5]) {
+  return x == 0 ? a[0] : x == 1 ? a[1] : x == 2 ? a[2] : x == 3 ? a[3] : a[4];
+}
+// f, then g
+__device__ __forceinline__ RunMap run_then(const RunMap &f, const RunMap &g) {
+  RunMap h;
+#pragma unroll
+  for (int q = 0; q < 5; q++) h.v[q] = pick5(f.v[q] >> 29, g.v) + (f.v[q] & kRunBytes);
+  return h;
+}
+__device__ __forceinline__ RunMap run_identity() {
+  RunMap h;
+#pragma unroll
+  for (int q = 0; q < 5; q++) h.v[q] = (uint32_t)q << 29;
+  return h;
+}
 
 __device__ __forceinline__ void rle1_step(int &r, int &n, int c, int p) {
   if (r == 4) {
@@ -1223,28 +1246,35 @@ __device__ __forceinline__ void rle1_step(int &r, int &n, int c, int p) {
   }
 }
 
-__device__ __forceinline__ int pick5(int x, int a0, int a1, int a2, int a3, int a4) {
-  return x == 0 ? a0 : x == 1 ? a1 : x == 2 ? a2 : x == 3 ? a3 : a4;
+// Loads the tile's bytes (thread t's segment at t * kSegStride) and returns
+// the bytes of this thread's segment; *prev: the byte before it (-1: none).
+__device__ __forceinline__ int load_segments(const uint8_t *R, int m, int tile, uint8_t *sb,
+                                             int *prev) {
+  const int t0 = tile * kUnTile;
+  const int len = min(kUnTile, m - t0);
+  for (int q = threadIdx.x; q < (len + 15) / 16; q += 256) {
+    const uint4 v = reinterpret_cast<const uint4 *>(R + t0)[q];  // rows are 16-byte aligned
+    uint32_t *d = reinterpret_cast<uint32_t *>(sb + (q >> 1) * kSegStride + (q & 1) * 16);
+    d[0] = v.x;
+    d[1] = v.y;
+    d[2] = v.z;
+    d[3] = v.w;
+  }
+  __syncthreads();
+  const int s0 = threadIdx.x * kSegBytes;
+  *prev = -1;
+  if (threadIdx.x > 0) *prev = sb[(threadIdx.x - 1) * kSegStride + kSegBytes - 1];
+  else if (t0 > 0) *prev = R[t0 - 1];
+  return max(0, min(kSegBytes, len - s0));
 }
 
-__global__ void __launch_bounds__(32 * kUnrleWarps)
-    k_dec_unrle1_count(const int32_t *idx, const DecBlock *db, const uint8_t *rle, int nacc,
-                       int cap, LaneStart *lanes, int64_t *lens) {
-  const int k = blockIdx.x * kUnrleWarps + (threadIdx.x >> 5);
-  const int ln = threadIdx.x & 31;
-  if (k >= nacc) return;  // the whole warp
-  const int bi = idx[k];
-  const int m = db[bi].m;
-  const uint8_t *R = rle + (size_t)bi * cap;
-  const int seg = (m + 31) / 32;
-  const int s0 = min(ln * seg, m), e0 = min(s0 + seg, m);
-  int p = s0 > 0 ? R[s0 - 1] : -1;
+__device__ __forceinline__ RunMap segment_map(const uint8_t *seg, int n, int p) {
   int r0 = 0, r1 = 1, r2 = 2, r3 = 3, r4 = 4;
   int n0 = 0, n1 = 0, n2 = 0, n3 = 0, n4 = 0;
-  int i = s0;
+  int i = 0;
   bool merged = false;
-  while (i < e0 && !merged) {
-    const int c = R[i++];
+  while (i < n && !merged) {
+    const int c = seg[i++];
     rle1_step(r0, n0, c, p);
     rle1_step(r1, n1, c, p);
     rle1_step(r2, n2, c, p);
@@ -1253,13 +1283,13 @@ __global__ void __launch_bounds__(32 * kUnrleWarps)
     p = c;
     merged = r0 == r1 && r0 == r2 && r0 == r3 && r0 == r4;
   }
-  int r = r0, nb = 0;
-  while (i < e0) {
-    const int c = R[i++];
-    rle1_step(r, nb, c, p);
-    p = c;
-  }
   if (merged) {
+    int r = r0, nb = 0;
+    while (i < n) {
+      const int c = seg[i++];
+      rle1_step(r, nb, c, p);
+      p = c;
+    }
     r0 = r1 = r2 = r3 = r4 = r;
     n0 += nb;
     n1 += nb;
@@ -1267,78 +1297,208 @@ __global__ void __launch_bounds__(32 * kUnrleWarps)
     n3 += nb;
     n4 += nb;
   }
-  int state = 0, off = 0, my_state = 0, my_off = 0;
-  for (int l = 0; l < 32; l++) {
-    if (ln == l) {
-      my_state = state;
-      my_off = off;
-    }
-    const int ro = __shfl_sync(0xffffffffu, pick5(state, r0, r1, r2, r3, r4), l);
-    const int no = __shfl_sync(0xffffffffu, pick5(state, n0, n1, n2, n3, n4), l);
-    state = ro;
-    off += no;
-  }
-  lanes[(size_t)k * 32 + ln] = LaneStart{my_state, my_off};
-  if (ln == 0) lens[k] = off;
+  RunMap h;
+  h.v[0] = ((uint32_t)r0 << 29) | (uint32_t)n0;
+  h.v[1] = ((uint32_t)r1 << 29) | (uint32_t)n1;
+  h.v[2] = ((uint32_t)r2 << 29) | (uint32_t)n2;
+  h.v[3] = ((uint32_t)r3 << 29) | (uint32_t)n3;
+  h.v[4] = ((uint32_t)r4 << 29) | (uint32_t)n4;
+  return h;
 }
 
-__global__ void __launch_bounds__(32 * kUnrleWarps)
-    k_dec_unrle1_write(const int32_t *idx, const DecBlock *db, const uint8_t *rle, int nacc,
-                       int cap, const LaneStart *lanes, const int64_t *off, uint8_t *out) {
-  const int k = blockIdx.x * kUnrleWarps + (threadIdx.x >> 5);
-  const int ln = threadIdx.x & 31;
-  if (k >= nacc) return;
+// Exclusive scan of the tile's maps (256 threads); *total: the tile's map.
+__device__ __forceinline__ RunMap scan_maps(RunMap mine, RunMap (&wm)[8], RunMap *total) {
+  const int ln = lane_id(), w = warp_id();
+  RunMap inc = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    RunMap o;
+#pragma unroll
+    for (int q = 0; q < 5; q++) o.v[q] = __shfl_up_sync(0xffffffffu, inc.v[q], d);
+    if (ln >= d) inc = run_then(o, inc);
+  }
+  if (ln == 31) wm[w] = inc;
+  RunMap ex;
+#pragma unroll
+  for (int q = 0; q < 5; q++) ex.v[q] = __shfl_up_sync(0xffffffffu, inc.v[q], 1);
+  if (ln == 0) ex = run_identity();
+  __syncthreads();
+  RunMap pre = run_identity();
+  for (int q = 0; q < w; q++) pre = run_then(pre, wm[q]);
+  if (total) *total = run_then(pre, wm[7]);  // meaningful in the last warp
+  return run_then(pre, ex);
+}
+
+// grid: (tile, block)
+__global__ void __launch_bounds__(256) k_dec_unrle1_count(const int32_t *idx, const DecBlock *db,
+                                                          const uint8_t *rle, int cap,
+                                                          RunMap *maps) {
+  __shared__ __align__(16) uint8_t sb[256 * kSegStride];
+  __shared__ RunMap wm[8];
+  const int k = blockIdx.y, tile = blockIdx.x;
   const int bi = idx[k];
   const int m = db[bi].m;
-  const uint8_t *R = rle + (size_t)bi * cap;
-  const int seg = (m + 31) / 32;
-  const int s0 = min(ln * seg, m), e0 = min(s0 + seg, m);
-  int p = s0 > 0 ? R[s0 - 1] : -1;
-  const LaneStart ls = lanes[(size_t)k * 32 + ln];
-  int r = ls.state;
-  uint8_t *O = out + off[k] + ls.off;
-  for (int i = s0; i < e0; i++) {
-    const int c = R[i];
+  if (tile * kUnTile >= m) return;
+  int prev;
+  const int n = load_segments(rle + (size_t)bi * cap, m, tile, sb, &prev);
+  RunMap total;
+  scan_maps(segment_map(sb + threadIdx.x * kSegStride, n, prev), wm, &total);
+  if (threadIdx.x == 255) maps[(size_t)k * kUnTiles + tile] = total;
+}
+
+// Per block: every tile's state and offset (map v[0] = state, v[1..2] = its
+// 64-bit offset) and the block's length.
+__global__ void __launch_bounds__(256) k_dec_unrle1_scan(const int32_t *idx, const DecBlock *db,
+                                                         RunMap *maps, int64_t *lens) {
+  __shared__ RunMap tm[kUnTiles];
+  const int k = blockIdx.x;
+  const int nt = (db[idx[k]].m + kUnTile - 1) / kUnTile;
+  RunMap *mp = maps + (size_t)k * kUnTiles;
+  for (int q = threadIdx.x; q < nt; q += 256) tm[q] = mp[q];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t state = 0;
+    int64_t off = 0;
+    for (int q = 0; q < nt; q++) {
+      const uint32_t e = pick5(state, tm[q].v);
+      tm[q].v[0] = state;
+      tm[q].v[1] = (uint32_t)off;
+      tm[q].v[2] = (uint32_t)(off >> 32);
+      state = e >> 29;
+      off += e & kRunBytes;
+    }
+    lens[k] = off;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < nt; q += 256) mp[q] = tm[q];
+}
+
+// Sequential byte writer: whole words where the thread owns them, bytes at
+// its two ends.
+struct ByteWriter {
+  uint8_t *o;     // next byte
+  uint8_t *lo;    // first byte
+  uint32_t acc;
+  __device__ __forceinline__ void init(uint8_t *p) {
+    o = lo = p;
+    acc = 0;
+  }
+  __device__ __forceinline__ void store_part(uint8_t *from) {  // bytes [from, o) of one word
+    for (uint8_t *q = from; q < o; q++)
+      *q = (uint8_t)(acc >> (8 * (int)(reinterpret_cast<uintptr_t>(q) & 3u)));
+  }
+  __device__ __forceinline__ void put(uint32_t c) {
+    const int sh = 8 * (int)(reinterpret_cast<uintptr_t>(o) & 3u);
+    acc = (sh ? acc : 0u) | (c << sh);
+    o++;
+    if (sh == 24) {
+      if (o - lo >= 4) *reinterpret_cast<uint32_t *>(o - 4) = acc;
+      else store_part(lo);
+    }
+  }
+  __device__ __forceinline__ void fill(uint32_t c, int n) {
+    while (n > 0 && (reinterpret_cast<uintptr_t>(o) & 3u)) {
+      put(c);
+      n--;
+    }
+    const uint32_t wv = 0x01010101u * c;
+    while (n >= 4 && (reinterpret_cast<uintptr_t>(o) & 15u)) {
+      *reinterpret_cast<uint32_t *>(o) = wv;
+      o += 4;
+      n -= 4;
+    }
+    for (; n >= 16; n -= 16, o += 16) *reinterpret_cast<uint4 *>(o) = make_uint4(wv, wv, wv, wv);
+    for (; n >= 4; n -= 4, o += 4) *reinterpret_cast<uint32_t *>(o) = wv;
+    while (n-- > 0) put(c);
+  }
+  __device__ __forceinline__ void finish() {
+    const int k = (int)(reinterpret_cast<uintptr_t>(o) & 3u);
+    if (k && o > lo) store_part(o - k > lo ? o - k : lo);
+  }
+};
+
+__global__ void __launch_bounds__(256) k_dec_unrle1_write(const int32_t *idx, const DecBlock *db,
+                                                          const uint8_t *rle, int cap,
+                                                          const RunMap *maps, const int64_t *off,
+                                                          uint8_t *out) {
+  __shared__ __align__(16) uint8_t sb[256 * kSegStride];
+  __shared__ RunMap wm[8];
+  const int k = blockIdx.y, tile = blockIdx.x;
+  const int bi = idx[k];
+  const int m = db[bi].m;
+  if (tile * kUnTile >= m) return;
+  int p;
+  const int n = load_segments(rle + (size_t)bi * cap, m, tile, sb, &p);
+  const uint8_t *seg = sb + threadIdx.x * kSegStride;
+  const RunMap ex = scan_maps(segment_map(seg, n, p), wm, nullptr);
+  const RunMap &tm = maps[(size_t)k * kUnTiles + tile];
+  const uint32_t e = pick5(tm.v[0], ex.v);
+  int r = (int)(e >> 29);
+  ByteWriter bw;
+  bw.init(out + off[k] + (((int64_t)tm.v[2] << 32) | tm.v[1]) + (e & kRunBytes));
+  for (int i = 0; i < n; i++) {
+    const int c = seg[i];
     if (r == 4) {
-      fill_bytes(O, c, (uint8_t)p);
-      O += c;
+      bw.fill((uint32_t)p, c);
       r = 0;
     } else {
       r = (r >= 1 && c == p) ? r + 1 : 1;
-      *O++ = (uint8_t)c;
+      bw.put((uint32_t)c);
     }
     p = c;
   }
+  bw.finish();
 }
 
-// Block CRCs of the expanded output, one thread block per block: 4096-byte
-// chunks staged in shared memory, thread l's 16 bytes give crc0 * x^(8*16*(255-l))
-// (the chunk right-aligned in 4096 bytes when shorter), the XOR is the
-// chunk's crc0, and the block's crc0 accumulates chunk by chunk.
+// Block CRCs of the expanded output.  kCrcParts CTAs share a block's
+// 4096-byte chunks; in a chunk thread l's 16 bytes give crc0 *
+// x^(8*16*(255-l)) (the chunk right-aligned in 4096 bytes when shorter), the
+// XOR is the chunk's crc0, a CTA's crc0 accumulates chunk by chunk and is
+// shifted past the bytes after its part.  crcs: all ones before (the format's
+// complement); the initial value's term comes with part 0.
+constexpr int kCrcParts = 32;
+
 __global__ void __launch_bounds__(256) k_dec_crc(const int64_t *lens, const int64_t *off,
                                                  const uint8_t *out, uint32_t *crcs) {
   __shared__ uint32_t tbl[256];
   __shared__ uint32_t red4[16];
-  __shared__ __align__(16) uint8_t chunk[4096];
   __shared__ uint32_t part[2][8];
+  const int k = blockIdx.y;
+  const int64_t n = lens[k];
+  const int64_t nch = (n + 4095) / 4096;
+  const int64_t per = (nch + kCrcParts - 1) / kCrcParts;
+  const int64_t b0 = (int64_t)blockIdx.x * per * 4096;
+  const int64_t b1 = b0 + per * 4096 < n ? b0 + per * 4096 : n;
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    atomicXor(&crcs[k], gf_mul(0xFFFFFFFFu, xpow8((uint64_t)n)));
+  if (b0 >= b1) return;
   crc_table_fill(tbl);
   red4_fill(red4);
-  const int k = blockIdx.x;
-  const int64_t n = lens[k];
+  __syncthreads();
   const uint8_t *src = out + off[k];
   uint32_t acc = 0;  // thread 0
   int it = 0;
-  for (int64_t base = 0; base < n; base += 4096, it++) {
-    const int len = n - base < 4096 ? (int)(n - base) : 4096;
-    const int pad = 4096 - len;
-    __syncthreads();  // chunk free
-    for (int i = threadIdx.x; i < 4096; i += 256) chunk[i] = i >= pad ? src[base + i - pad] : 0;
-    __syncthreads();
+  for (int64_t base = b0; base < b1; base += 4096, it++) {
+    const int len = b1 - base < 4096 ? (int)(b1 - base) : 4096;
+    const int at = 16 * (int)threadIdx.x - (4096 - len);  // this thread's first byte in the chunk
     uint32_t r = 0;
-    const uint4 v = *reinterpret_cast<const uint4 *>(chunk + 16 * threadIdx.x);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    if (at >= 0) {
+      // 16 bytes from any address: five aligned words (the buffer has slack)
+      const uintptr_t a = reinterpret_cast<uintptr_t>(src + base + at);
+      const uint32_t *wp = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+      const int sh = 8 * (int)(a & 3u);
+      uint32_t lo = wp[0];
 #pragma unroll
-    for (int q = 0; q < 16; q++) r = crc_byte(r, (w[q >> 2] >> (8 * (q & 3))) & 0xFFu, tbl);
+      for (int q = 0; q < 4; q++) {
+        const uint32_t hi = wp[q + 1];
+        const uint32_t x = __funnelshift_r(lo, hi, sh);
+        lo = hi;
+#pragma unroll
+        for (int z = 0; z < 4; z++) r = crc_byte(r, (x >> (8 * z)) & 0xFFu, tbl);
+      }
+    } else {
+      for (int q = -at; q < 16; q++) r = crc_byte(r, src[base + at + q], tbl);
+    }
     r = gf_mul_lane(r, threadIdx.x, red4);
     for (int o = 16; o; o >>= 1) r ^= __shfl_xor_sync(0xffffffffu, r, o);
     if ((threadIdx.x & 31) == 0) part[it & 1][threadIdx.x >> 5] = r;
@@ -1350,7 +1510,7 @@ __global__ void __launch_bounds__(256) k_dec_crc(const int64_t *lens, const int6
       acc = (acc ? gf_mul(acc, len == 4096 ? c_xpow[12] : xpow8((uint64_t)len)) : 0u) ^ c;
     }
   }
-  if (threadIdx.x == 0) crcs[k] = ~(gf_mul(0xFFFFFFFFu, xpow8((uint64_t)n)) ^ acc);
+  if (threadIdx.x == 0) atomicXor(&crcs[k], gf_mul(acc, xpow8((uint64_t)(n - b1))));
 }
 
 // Device buffer that only grows (contents are not kept).
@@ -1429,7 +1589,7 @@ struct MallocSink : DecSink {
 struct DecWork {
   std::mutex mu;
   DevBuf words, blk, eos, cnt, cand, order, db, tab, gstart, L, hist, sel, idx, tt, lens, off, crc,
-      ctl, bad, lanes;
+      ctl, bad, maps;
   DevBuf out[2];
   cudaStream_t st = nullptr, cs = nullptr;
   cudaEvent_t written[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
@@ -1475,7 +1635,8 @@ DecWork &dec_work() {
 // vector (before it the symbols), chunk histograms, selectors and group
 // starts, tables, walk control.
 constexpr size_t kSlotBytes = (size_t)kDecCap * 5 + (size_t)kLfChunks * 256 * 4 + kDecMaxSel * 5 +
-                              sizeof(DecTab) + sizeof(WalkCtl) + sizeof(DecBlock) + 32 * 8 + 64;
+                              sizeof(DecTab) + sizeof(WalkCtl) + sizeof(DecBlock) +
+                              sizeof(RunMap) * kUnTiles + 64;
 constexpr int kMaxBatch = 4096;
 
 bool is_header(const uint8_t *h) {
@@ -1552,7 +1713,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
   w.crc.reserve(4 * (size_t)batch);
   w.ctl.reserve(sizeof(WalkCtl) * (size_t)batch);
   w.bad.reserve(16);
-  w.lanes.reserve(sizeof(LaneStart) * 32 * (size_t)batch);
+  w.maps.reserve(sizeof(RunMap) * kUnTiles * (size_t)batch);
   if (w.h_crc_cap < (size_t)batch) {
     if (w.h_crc) BZ_CUDA(cudaFreeHost(w.h_crc));
     w.h_crc = nullptr;
@@ -1691,9 +1852,10 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     BZ_LAUNCH_CHECK();
     k_dec_repeat<<<dim3(16, na), 256, 0, st>>>(didx, ddb, w.ctl.get<WalkCtl>(), L, cap);
     BZ_LAUNCH_CHECK();
-    const unsigned ugrid = (unsigned)((na + kUnrleWarps - 1) / kUnrleWarps);
-    k_dec_unrle1_count<<<ugrid, 32 * kUnrleWarps, 0, st>>>(
-        didx, ddb, L, na, cap, w.lanes.get<LaneStart>(), w.lens.get<int64_t>());
+    const dim3 ugrid(kUnTiles, na);
+    k_dec_unrle1_count<<<ugrid, 256, 0, st>>>(didx, ddb, L, cap, w.maps.get<RunMap>());
+    BZ_LAUNCH_CHECK();
+    k_dec_unrle1_scan<<<na, 256, 0, st>>>(didx, ddb, w.maps.get<RunMap>(), w.lens.get<int64_t>());
     BZ_LAUNCH_CHECK();
     std::vector<int64_t> lens(na), offs(na);
     int hbad = 0;
@@ -1713,12 +1875,13 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     }
     w.out[slot].reserve((size_t)tot + 16);
     BZ_CUDA(cudaMemcpyAsync(w.off.p, offs.data(), 8 * na, cudaMemcpyHostToDevice, st));
-    k_dec_unrle1_write<<<ugrid, 32 * kUnrleWarps, 0, st>>>(
-        didx, ddb, L, na, cap, w.lanes.get<LaneStart>(), w.off.get<int64_t>(),
-        w.out[slot].get<uint8_t>());
+    k_dec_unrle1_write<<<ugrid, 256, 0, st>>>(didx, ddb, L, cap, w.maps.get<RunMap>(),
+                                              w.off.get<int64_t>(), w.out[slot].get<uint8_t>());
     BZ_LAUNCH_CHECK();
-    k_dec_crc<<<na, 256, 0, st>>>(w.lens.get<int64_t>(), w.off.get<int64_t>(),
-                                  w.out[slot].get<uint8_t>(), w.crc.get<uint32_t>());
+    BZ_CUDA(cudaMemsetAsync(w.crc.p, 0xFF, 4 * na, st));
+    k_dec_crc<<<dim3(kCrcParts, na), 256, 0, st>>>(w.lens.get<int64_t>(), w.off.get<int64_t>(),
+                                                   w.out[slot].get<uint8_t>(),
+                                                   w.crc.get<uint32_t>());
     BZ_LAUNCH_CHECK();
     BZ_CUDA(cudaMemcpyAsync(w.h_crc, w.crc.p, 4 * na, cudaMemcpyDeviceToHost, st));
     BZ_CUDA(cudaEventRecord(w.written[slot], st));
