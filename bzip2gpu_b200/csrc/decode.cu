@@ -12,9 +12,9 @@
 //      parallel over chunks of 32 groups.  Out: the BWT last column L.
 //   3. k_dec_lf_hist / _scan / _rank: LF vector
 //      tt[C[L[i]] + rank(i)] = i << 8 | L[i] by a stable counting sort.
-//   4. k_dec_split / k_dec_walk / k_dec_chain: per block, the chain from
-//      origPtr gives the RLE1 bytes, cut at up to 2048 splitters that are
-//      walked in parallel.
+//   4. k_dec_walk / k_dec_chain / k_dec_gather: per block, the chain from
+//      origPtr gives the RLE1 bytes, cut at every 64th or 128th position; the
+//      segments are walked in parallel and copied to their places.
 //   5. k_dec_unrle1_count / _scan / _write expand the RLE1 runs (4 equal bytes
 //      then a count byte) from 32-byte segments at once; k_dec_crc
 //      computes each block's CRC over its output (4096-byte chunks combined
@@ -962,6 +962,48 @@ __global__ void __launch_bounds__(32 * kSymWarps)
   }
 }
 
+// The RLE1 bytes of each block follow tt from origPtr:
+// T[j] = psi(j) << 8 | F[j], psi = LF^-1, and the text is F[origPtr],
+// F[psi(origPtr)], ...  One dependent load per byte, so the chain is cut at
+// every walk_step(m)-th position and at origPtr: a walker per cut follows the
+// chain to the next one, the segments are ordered along the chain from origPtr
+// by pointer jumping, and their bytes are copied to their place.  Segment
+// lengths are close to exponential, so the longest is about ln(walkers) times
+// the step.  A walker keeps its bytes in 64-byte chunks of a pool (its own
+// first one, then the block's next free ones), so the chain is walked once.
+// The step is as small as the ordering's shared memory allows: the walk is
+// bound by the latency of its longest segments, and the more walkers a block
+// has, the fewer blocks' T (4 bytes per RLE1 byte) are in use at a time, which
+// keeps them in L2.  Two walks of steps of 512 took 0.67 ms each for one block
+// and 4.7 ms each for 600 blocks.
+constexpr int kWalkChunk = 64;
+constexpr int kMaxWalkers = (kDecCap + 127) / 128 + 2;
+constexpr int kMaxWalkChunks = kMaxWalkers + kDecCap / kWalkChunk + 1;
+constexpr int kChainThreads = 1024;
+constexpr int kChainPer = (kMaxWalkers + kChainThreads - 1) / kChainThreads;
+constexpr int kNoWalker = 0xFFFF;
+static_assert(kMaxWalkers < (1 << 14) && kDecCap / kWalkChunk < (1 << 18), "chunk owner packing");
+
+__host__ __device__ __forceinline__ int walk_step(int m) { return m > kDecCap / 2 ? 128 : 64; }
+__device__ __forceinline__ int walker_count(int m, int orig) {
+  const int s = walk_step(m);
+  return (m + s - 1) / s + (orig % s != 0);
+}
+// The walker that starts at a cut.
+__device__ __forceinline__ int walker_at(int p, int m, int orig) {
+  const int s = walk_step(m);
+  return p % s == 0 ? p / s : (m + s - 1) / s;
+}
+
+struct WalkCtl {
+  int32_t cycle;     // bytes of the chain from origPtr before it closes (m if it does not)
+  int32_t nchunks;   // pool chunks taken
+  int32_t len[kMaxWalkers];     // segment length (steps to the next cut)
+  uint16_t next[kMaxWalkers];   // the walker there
+  int32_t off[kMaxWalkers];     // output offset, -1 when off the chain
+  uint32_t owner[kMaxWalkChunks];  // chunk: walker | its place among the walker's << 14
+};
+
 // LF vector without serial ranks: T[C[L[i]] + rank(i)] = i << 8 | L[i], with
 // rank(i) = #{j < i : L[j] == L[i]} (then for j = LF(i), psi(j) = i and
 // F[j] = L[i]).  A stable counting sort by the byte: per 4096-entry chunk a
@@ -991,10 +1033,12 @@ __global__ void __launch_bounds__(256) k_dec_lf_hist(const int32_t *idx, const D
 // Per block (thread = byte value): H[chunk][c] becomes the position of the
 // chunk's first c in F order.
 __global__ void __launch_bounds__(256) k_dec_lf_scan(const int32_t *idx, const DecBlock *db,
-                                                     int32_t *H) {
+                                                     int32_t *H, WalkCtl *ctl) {
   __shared__ int scratch[40];
   const int k = blockIdx.x;
   const int m = db[idx[k]].m;
+  // every walker owns the pool chunk of its number; the next ones are free
+  if (threadIdx.x == 0) ctl[k].nchunks = walker_count(m, db[idx[k]].orig_ptr);
   const int nch = (m + kLfChunk - 1) / kLfChunk;
   int32_t *h = H + (size_t)k * kLfChunks * 256 + threadIdx.x;
   int tot = 0;
@@ -1050,133 +1094,128 @@ __global__ void __launch_bounds__(256) k_dec_lf_rank(const int32_t *idx, const D
   }
 }
 
-// The RLE1 bytes of each block follow tt from origPtr:
-// T[j] = psi(j) << 8 | F[j], psi = LF^-1, and the text is F[origPtr],
-// F[psi(origPtr)], ...  One dependent load per byte, so the chain is cut at
-// S splitters per block (origPtr and evenly spaced positions, marked in bit
-// 31 of their T entry, which the walk loads anyway): every walker counts the
-// steps to the next marked position, the segments are ordered along the chain
-// from origPtr, and the walkers walk again writing their segment at its
-// offset.  Segment lengths along the chain are close to exponential, so the
-// longest is about ln(S) times the mean (m / S, about 512 here).  A periodic
-// block (its cycle closes before m bytes) repeats that one cycle.
-constexpr int kMaxWalkers = 2048;
-constexpr int kWalkSpan = 512;
-constexpr uint32_t kMark = 0x80000000u;
-constexpr uint32_t kPsiMask = 0x7FFFFF00u;
-
-struct WalkCtl {
-  int32_t nw;        // splitters
-  int32_t cycle;     // bytes of the chain from origPtr before it closes (m if it does not)
-  int32_t pos[kMaxWalkers];   // sorted splitter positions
-  int32_t len[kMaxWalkers];   // segment length (steps to the next splitter)
-  int32_t next[kMaxWalkers];  // index of the splitter reached
-  int32_t off[kMaxWalkers];   // output offset, -1 when off the chain
-};
-
-// Splitter positions (one thread) and their marks in T (all threads).
-__global__ void k_dec_split(const int32_t *idx, const DecBlock *db, WalkCtl *ctl, uint32_t *tt,
-                            int cap) {
-  const int k = blockIdx.x;
-  const DecBlock b = db[idx[k]];
-  WalkCtl &c = ctl[k];
-  uint32_t *T = tt + (size_t)k * cap;
-  const int m = b.m;
-  if (threadIdx.x == 0) {
-    const int S = max(1, min(kMaxWalkers, m / kWalkSpan));
-    int n = 0;
-    bool placed = false;
-    for (int t = 1; t <= S; t++) {
-      const int j = t < S ? (int)((int64_t)t * m / S) : m;  // t == S: sentinel
-      if (!placed && b.orig_ptr <= j) {
-        c.pos[n++] = b.orig_ptr;
-        placed = true;
-      }
-      if (t < S && j != b.orig_ptr && j < m) c.pos[n++] = j;
-    }
-    if (!placed) c.pos[n++] = b.orig_ptr;
-    c.nw = n;
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < c.nw; q += blockDim.x) {
-    const int p = c.pos[q];
-    if (p >= 0 && p < m) T[p] |= kMark;
-  }
-}
-
-__device__ __forceinline__ int splitter_index(const WalkCtl &c, int p) {
-  int lo = 0, hi = c.nw - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (c.pos[mid] < p) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// write == 0: segment lengths and successors; write != 0: the segment bytes.
-__global__ void k_dec_walk(const int32_t *idx, const DecBlock *db, const uint32_t *tt,
-                           WalkCtl *ctl, uint8_t *rle, int cap, int write) {
+__global__ void __launch_bounds__(128) k_dec_walk(const int32_t *idx, const DecBlock *db,
+                                                  const uint32_t *tt, WalkCtl *ctl, uint8_t *pool,
+                                                  int cap) {
   const int k = blockIdx.y;
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   WalkCtl &c = ctl[k];
-  if (w >= c.nw) return;
-  const int m = db[idx[k]].m;
+  const DecBlock b = db[idx[k]];
+  const int m = b.m, orig = b.orig_ptr;
+  if (w >= walker_count(m, orig)) return;
   const uint32_t *T = tt + (size_t)k * cap;
-  uint8_t *R = rle + (size_t)idx[k] * cap;
-  if (write && c.off[w] < 0) return;
-  uint32_t p = (uint32_t)c.pos[w];
+  uint8_t *P = pool + (size_t)k * kMaxWalkChunks * kWalkChunk;
+  const int step = walk_step(m);  // a power of two
+  int p = w * step < m ? w * step : orig;
+  uint32_t *chunk = reinterpret_cast<uint32_t *>(P + (size_t)w * kWalkChunk);
+  c.owner[w] = (uint32_t)w;
   int n = 0;
-  const int o = write ? c.off[w] : 0;
-  const int lim = write ? c.len[w] : m;
-  bool at_mark = false;
+  uint32_t acc = 0;
+  // T is a permutation, so segments are disjoint and a walk ends within m steps
   for (;;) {
-    if (p >= (uint32_t)m || n >= lim || o + n >= m) break;
     const uint32_t e = T[p];
-    if (n > 0 && (e & kMark)) {
-      at_mark = true;
-      break;
-    }
-    if (write) R[o + n] = (uint8_t)(e & 0xFFu);
+    acc |= (e & 0xFFu) << (8 * (n & 3));
     n++;
-    p = (e & kPsiMask) >> 8;
+    p = (int)(e >> 8);
+    const bool end = (p & (step - 1)) == 0 || p == orig || n >= m;
+    if ((n & 3) == 0 || end) {
+      chunk[((n - 1) & (kWalkChunk - 1)) >> 2] = acc;
+      acc = 0;
+    }
+    if (end) break;
+    if ((n & (kWalkChunk - 1)) == 0) {
+      const int q = atomicAdd(&c.nchunks, 1);
+      c.owner[q] = (uint32_t)w | (uint32_t)(n / kWalkChunk) << 14;
+      chunk = reinterpret_cast<uint32_t *>(P + (size_t)q * kWalkChunk);
+    }
   }
-  if (!write) {
-    c.len[w] = n;
-    c.next[w] = at_mark ? splitter_index(c, (int)p) : -1;
-  }
+  c.len[w] = n;
+  c.next[w] = (uint16_t)walker_at(p, m, orig);
 }
 
-// Per block: segment offsets along the chain from origPtr (one thread walks
-// the segments, held in shared memory).
-__global__ void __launch_bounds__(256) k_dec_chain(const int32_t *idx, const DecBlock *db,
-                                                   WalkCtl *ctl, int *bad) {
-  __shared__ int32_t len[kMaxWalkers], nxt[kMaxWalkers], off[kMaxWalkers];
+// Per block: segment offsets along the chain from origPtr.  The chain is
+// opened before origPtr's walker; pointer jumping sums the lengths from each
+// walker to the end (walkers of other cycles never reach it).
+constexpr size_t kChainSmem = (size_t)kMaxWalkers * 6 + 16;
+
+__global__ void __launch_bounds__(kChainThreads) k_dec_chain(const int32_t *idx,
+                                                             const DecBlock *db, WalkCtl *ctl,
+                                                             int *bad) {
+  extern __shared__ uint32_t chain_smem[];
+  uint32_t *sum = chain_smem;
+  uint16_t *nxt = reinterpret_cast<uint16_t *>(sum + kMaxWalkers);
   const int k = blockIdx.x;
   const DecBlock b = db[idx[k]];
   WalkCtl &c = ctl[k];
-  const int nw = c.nw;
-  for (int q = threadIdx.x; q < nw; q += blockDim.x) {
-    len[q] = c.len[q];
-    nxt[q] = c.next[q];
-    off[q] = -1;
+  const int nw = walker_count(b.m, b.orig_ptr);
+  const int w0 = walker_at(b.orig_ptr, b.m, b.orig_ptr);
+  for (int q = threadIdx.x; q < nw; q += kChainThreads) {
+    sum[q] = (uint32_t)c.len[q];
+    const int x = c.next[q];
+    nxt[q] = (uint16_t)(x == w0 ? kNoWalker : x);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int w0 = splitter_index(c, b.orig_ptr);
-    int w = w0, o = 0;
-    for (int steps = 0; steps <= nw; steps++) {
-      if (w < 0 || w >= nw || off[w] >= 0) break;
-      off[w] = o;
-      o += len[w];
-      if (o >= b.m) break;
-      w = nxt[w];
+  for (int span = 1; span < nw; span <<= 1) {
+    uint32_t s[kChainPer];
+    uint16_t x[kChainPer];
+#pragma unroll
+    for (int j = 0; j < kChainPer; j++) {
+      const int q = threadIdx.x + j * kChainThreads;
+      if (q < nw) {
+        x[j] = nxt[q];
+        s[j] = sum[q];
+        if (x[j] != kNoWalker) {
+          s[j] += sum[x[j]];
+          x[j] = nxt[x[j]];
+        }
+      }
     }
-    c.cycle = min(o, b.m);
-    if (c.cycle <= 0 || b.m % c.cycle != 0) atomicOr(bad, 1);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kChainPer; j++) {
+      const int q = threadIdx.x + j * kChainThreads;
+      if (q < nw) {
+        sum[q] = s[j];
+        nxt[q] = x[j];
+      }
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int q = threadIdx.x; q < nw; q += blockDim.x) c.off[q] = off[q];
+  const uint32_t total = sum[w0];
+  for (int q = threadIdx.x; q < nw; q += kChainThreads)
+    c.off[q] = nxt[q] == kNoWalker ? (int32_t)(total - sum[q]) : -1;
+  if (threadIdx.x == 0) {
+    const int cyc = (int)min(total, (uint32_t)b.m);
+    c.cycle = cyc;
+    if (cyc <= 0 || b.m % cyc != 0 || total > (uint32_t)b.m) atomicOr(bad, 1);
+  }
+}
+
+// The walkers' chunks to their places: 16 threads per chunk, 4 bytes each.
+constexpr int kGatherChunks = 128;  // per CTA
+
+__global__ void __launch_bounds__(256) k_dec_gather(const int32_t *idx, const DecBlock *db,
+                                                    const WalkCtl *ctl, const uint8_t *pool,
+                                                    uint8_t *rle, int cap) {
+  const int k = blockIdx.y;
+  const WalkCtl &c = ctl[k];
+  const int bi = idx[k];
+  const int m = db[bi].m;
+  const int nq = min(c.nchunks, kMaxWalkChunks);
+  const uint8_t *P = pool + (size_t)k * kMaxWalkChunks * kWalkChunk;
+  uint8_t *R = rle + (size_t)bi * cap;
+  const int l = 4 * (threadIdx.x & 15);
+  const int q1 = min(nq, ((int)blockIdx.x + 1) * kGatherChunks);
+  for (int q = blockIdx.x * kGatherChunks + (threadIdx.x >> 4); q < q1; q += 16) {
+    const uint32_t ow = c.owner[q];
+    const int w = (int)(ow & 0x3FFFu), at = (int)(ow >> 14) * kWalkChunk + l;
+    const int off = c.off[w], n = c.len[w] - at;
+    if (off < 0 || n <= 0) continue;
+    const uint32_t v = *reinterpret_cast<const uint32_t *>(P + (size_t)q * kWalkChunk + l);
+#pragma unroll
+    for (int z = 0; z < 4; z++)
+      if (z < n && off + at + z < m) R[off + at + z] = (uint8_t)(v >> (8 * z));
+  }
 }
 
 // A periodic block: the first `cycle` bytes repeated to m.
@@ -1589,7 +1628,7 @@ struct MallocSink : DecSink {
 struct DecWork {
   std::mutex mu;
   DevBuf words, blk, eos, cnt, cand, order, db, tab, gstart, L, hist, sel, idx, tt, lens, off, crc,
-      ctl, bad, maps;
+      ctl, pool, bad, maps;
   DevBuf out[2];
   cudaStream_t st = nullptr, cs = nullptr;
   cudaEvent_t written[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
@@ -1610,12 +1649,14 @@ struct DecWork {
     int dev = 0, per_sm = 0;
     BZ_CUDA(cudaGetDevice(&dev));
     BZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    BZ_CUDA(cudaFuncSetAttribute(k_dec_chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kChainSmem));
     BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dec_groups<4>, 128, 0));
     resident = std::max(1, sms * per_sm);
   }
   size_t held() const {
     size_t s = 0;
-    for (const DevBuf *b : {&L, &hist, &tt, &sel, &tab, &gstart, &ctl, &out[0], &out[1]}) s += b->cap;
+    for (const DevBuf *b : {&L, &hist, &tt, &sel, &tab, &gstart, &ctl, &pool, &out[0], &out[1]}) s += b->cap;
     return s;
   }
 };
@@ -1633,9 +1674,10 @@ DecWork &dec_work() {
 
 // Device bytes of one candidate slot: last column (later the RLE1 bytes), LF
 // vector (before it the symbols), chunk histograms, selectors and group
-// starts, tables, walk control.
+// starts, tables, walk control and pool.
 constexpr size_t kSlotBytes = (size_t)kDecCap * 5 + (size_t)kLfChunks * 256 * 4 + kDecMaxSel * 5 +
                               sizeof(DecTab) + sizeof(WalkCtl) + sizeof(DecBlock) +
+                              (size_t)kMaxWalkChunks * kWalkChunk +
                               sizeof(RunMap) * kUnTiles + 64;
 constexpr int kMaxBatch = 4096;
 
@@ -1712,6 +1754,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
   w.off.reserve(8 * (size_t)batch);
   w.crc.reserve(4 * (size_t)batch);
   w.ctl.reserve(sizeof(WalkCtl) * (size_t)batch);
+  w.pool.reserve((size_t)kMaxWalkChunks * kWalkChunk * (size_t)batch);
   w.bad.reserve(16);
   w.maps.reserve(sizeof(RunMap) * kUnTiles * (size_t)batch);
   if (w.h_crc_cap < (size_t)batch) {
@@ -1833,22 +1876,20 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const dim3 lgrid(kLfChunks, na);
     k_dec_lf_hist<<<lgrid, 256, 0, st>>>(didx, ddb, L, w.hist.get<int32_t>(), cap);
     BZ_LAUNCH_CHECK();
-    k_dec_lf_scan<<<na, 256, 0, st>>>(didx, ddb, w.hist.get<int32_t>());
+    WalkCtl *dctl = w.ctl.get<WalkCtl>();
+    k_dec_lf_scan<<<na, 256, 0, st>>>(didx, ddb, w.hist.get<int32_t>(), dctl);
     BZ_LAUNCH_CHECK();
     k_dec_lf_rank<<<lgrid, 256, 0, st>>>(didx, ddb, L, w.hist.get<int32_t>(),
                                          w.tt.get<uint32_t>(), cap);
     BZ_LAUNCH_CHECK();
-    k_dec_split<<<na, 256, 0, st>>>(didx, ddb, w.ctl.get<WalkCtl>(), w.tt.get<uint32_t>(), cap);
-    BZ_LAUNCH_CHECK();
-    const dim3 wgrid(kMaxWalkers / 64, na);
-    k_dec_walk<<<wgrid, 64, 0, st>>>(didx, ddb, w.tt.get<uint32_t>(), w.ctl.get<WalkCtl>(), L,
-                                     cap, 0);
+    k_dec_walk<<<dim3((kMaxWalkers + 127) / 128, na), 128, 0, st>>>(
+        didx, ddb, w.tt.get<uint32_t>(), dctl, w.pool.get<uint8_t>(), cap);
     BZ_LAUNCH_CHECK();
     BZ_CUDA(cudaMemsetAsync(w.bad.p, 0, 4, st));
-    k_dec_chain<<<na, 256, 0, st>>>(didx, ddb, w.ctl.get<WalkCtl>(), w.bad.get<int>());
+    k_dec_chain<<<na, kChainThreads, kChainSmem, st>>>(didx, ddb, dctl, w.bad.get<int>());
     BZ_LAUNCH_CHECK();
-    k_dec_walk<<<wgrid, 64, 0, st>>>(didx, ddb, w.tt.get<uint32_t>(), w.ctl.get<WalkCtl>(), L,
-                                     cap, 1);
+    k_dec_gather<<<dim3((kMaxWalkChunks + kGatherChunks - 1) / kGatherChunks, na), 256, 0, st>>>(
+        didx, ddb, dctl, w.pool.get<uint8_t>(), L, cap);
     BZ_LAUNCH_CHECK();
     k_dec_repeat<<<dim3(16, na), 256, 0, st>>>(didx, ddb, w.ctl.get<WalkCtl>(), L, cap);
     BZ_LAUNCH_CHECK();
