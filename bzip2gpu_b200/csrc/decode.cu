@@ -109,22 +109,32 @@ struct BitReader {
   __device__ __forceinline__ int64_t pos() const { return (wnext - 3) * 32 + bo; }
 };
 
+// A thread tests the 32 bit positions of a word: the first 32 bits of both
+// magics by one funnel shift and two compares, the other 16 on a match (64-bit
+// shifts and compares of all 48 bits took 8 times the instructions).
 __global__ void k_dec_magic(const uint32_t *words, int64_t nwords, int64_t nbits,
                             int64_t *blk, int *nblk, int64_t *eos, int *neos, int cap) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nwords) return;
-  const uint64_t a = bswap32(words[i]);
-  const uint64_t b = i + 1 < nwords ? bswap32(words[i + 1]) : 0u;
-  const uint64_t c = i + 2 < nwords ? bswap32(words[i + 2]) : 0u;
-  const uint64_t hi = (a << 32) | b;  // bits 32i .. 32i + 63
+  const uint32_t a = bswap32(words[i]);
+  const uint32_t b = i + 1 < nwords ? bswap32(words[i + 1]) : 0u;
+  uint32_t hits = 0;
+#pragma unroll
   for (int s = 0; s < 32; s++) {
+    const uint32_t v = __funnelshift_l(b, a, s);
+    if (v == 0x31415926u || v == 0x17724538u) hits |= 1u << s;
+  }
+  while (hits) {
+    const int s = __ffs(hits) - 1;
+    hits &= hits - 1u;
     const int64_t p = i * 32 + s;
     if (p + 48 > nbits) break;
-    const uint64_t v = ((hi << s) | (s ? (c >> (32 - s)) : 0)) >> 16;  // 48 bits at p
-    if (v == 0x314159265359ull) {
+    const uint32_t c = i + 2 < nwords ? bswap32(words[i + 2]) : 0u;
+    const uint32_t v = __funnelshift_l(b, a, s), low = __funnelshift_l(c, b, s) >> 16;
+    if (v == 0x31415926u && low == 0x5359u) {
       const int k = atomicAdd(nblk, 1);
       if (k < cap) blk[k] = p;
-    } else if (v == 0x177245385090ull) {
+    } else if (v == 0x17724538u && low == 0x5090u) {
       const int k = atomicAdd(neos, 1);
       if (k < cap) eos[k] = p;
     }
@@ -638,7 +648,8 @@ inline GroupsKernel groups_kernel(int nblocks, int sms, int *threads) {
 //  * lane t walks its index back through the batch's earlier steps s: a
 //    step moved the entry at v_s to the front, so position p after it was
 //    p - 1 before it when 1 <= p <= v_s, and p == 0 is step s's own output
-//    (a run digit repeats the front entry: index 0, no move);
+//    (a run digit repeats the front entry: index 0, no move; 5 instructions
+//    per step and 32 symbols);
 //  * lanes that reach position 0 point at that step's lane, the others read
 //    the list as it was before the batch; pointer jumping settles pointers;
 //  * the new list: the batch's distinct outputs, most recent first, then
@@ -734,22 +745,30 @@ __global__ void __launch_bounds__(32 * kSymWarps)
     const unsigned runs = __ballot_sync(full, dgt);
     const unsigned others = __ballot_sync(full, act && !dgt);
     const uint8_t *lst = lb + 256 * cur;
-    int val;
+    int rv;  // the symbol's position in the chunk's starting list
     if (others == 0u) {
-      val = lst[0];
+      rv = lst[0];
     } else {
       const int my_v = act && !dgt ? sym - 1 : 0;
-      int p = my_v, ptr = -1;
+      // p: the position before step ln - d of what this step puts out.  Once
+      // at 0 it stays there; it then is the output of the step before the one
+      // that last moved it (a run digit: of the step before itself).
+      int p = my_v, moved = 0;
 #pragma unroll
-      for (int s = 30; s >= 0; --s) {
-        const int vs = __shfl_sync(full, my_v, s);
-        if (ln > s && ptr < 0) {
-          if (p == 0) ptr = s;
-          else if (p <= vs) p--;
+      for (int d = 1; d < 32; d++) {
+        uint32_t vs;
+        int in;
+        asm volatile("{ .reg .pred q; shfl.sync.up.b32 %0|q, %2, %3, 0, 0xffffffff; selp.s32 %1, 1, 0, q; }"
+            : "=r"(vs), "=r"(in)
+            : "r"(my_v), "r"(d));
+        if (in && (uint32_t)(p - 1) < vs) {
+          p--;
+          moved = d;
         }
       }
+      int ptr = p == 0 ? ln - moved - 1 : -1;  // below 0: no step before, the list's front
       const bool from_list = act && ptr < 0;
-      val = from_list ? (int)lst[p] : -1;
+      int val = from_list ? (int)lst[p] : -1;
 #pragma unroll
       for (int r2 = 0; r2 < 5; r2++) {
         const int src = ptr >= 0 ? ptr : ln;
@@ -789,13 +808,14 @@ __global__ void __launch_bounds__(32 * kSymWarps)
         if (!(uw & bit)) nx[D + q - below - __popc(uw & (bit - 1u))] = lst[q];
       }
       cur ^= 1;
+      rv = val;
       __syncwarp();
     }
     // a run digit's place: the digits just before it
     const unsigned bm = others & ((1u << ln) - 1u);
     const int q = bm ? ln - 32 + __clz(bm) : ln + run;
     const int qc = min(q, 31);
-    if (act) rec[i0 + ln] = (uint16_t)(dgt ? kRecRun | (sym << 13) | (qc << 8) | val : val);
+    if (act) rec[i0 + ln] = (uint16_t)(dgt ? kRecRun | (sym << 13) | (qc << 8) | rv : rv);
     if (act) {
       const int64_t bytes = dgt ? (int64_t)(sym + 1) << min(q, 40) : 1;
       if (lead && bm == 0u && dgt) lead_sum += bytes;
