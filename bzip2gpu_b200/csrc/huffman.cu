@@ -165,14 +165,178 @@ __global__ void __launch_bounds__(kGroupTile) k_huff_select(SlabDev d, int which
 // its alphabet size, so the lanes' heaps have equal sizes at every step and
 // stay in step), so the warp issues about one heap's instructions for all
 // six.  Heap entries carry their node's weight in the high half (weight << 32
-// | node), so a sift step reads a sibling pair with one 16-byte shared load;
-// comparisons use the weight half only, with the reference's strict '<', so
-// ties resolve exactly as there.  All lanes then walk the parent links for
-// the code lengths, table by table.
-constexpr int kHeapN = kMaxAlpha + 2;
+// | node); comparisons use the weight half only, with the reference's strict
+// '<', so ties resolve exactly as there: every step leaves the heap in the
+// reference's state.
+// The chain of heap steps is the kernel's time, so a step is made short.  A
+// sift down always follows the lighter children; which child is lighter is
+// kept as one bit per inner node in registers, so the path is seven
+// shift-and-adds, its entries are then loaded and compared all at once (the
+// weights along a path do not fall, so the entries that move up are those not
+// heavier than the moved one), and the entries that moved are written with the
+// path's new bits.  A sift up knows its path from the start.  Slots past the
+// heap hold an infinite weight, so neither tests the heap's size.  One entry
+// after another, a launch took 307 us for 258 symbols.
+// All lanes then walk the parent links for the code lengths, six tables at a
+// time.
+constexpr int kHeapRow = 266;  // entries per table: 16-byte rows, lanes on different banks
 constexpr int kNodeN = kMaxAlpha * 2;
+constexpr uint32_t kInfWeight = 0xFFFFFFFEu;  // one more still fits 32 bits
 
 __device__ __forceinline__ uint32_t hw(uint64_t e) { return (uint32_t)(e >> 32); }
+
+__device__ __forceinline__ uint64_t pick(bool c, uint64_t x, uint64_t y) { return c ? x : y; }
+
+// Removes the top of a heap of n entries (n is the same for all lanes, n <
+// 2^(L + 1)); light: bit k set when entry 2k + 1 is lighter than entry 2k.
+// Free of branches: entries of the path that do not change are written again.
+// The path goes by the lighter children, so a node's bit flips exactly when
+// the path's new entry below it is no longer the one to take: heavier than its
+// sibling, or as heavy and on the right.
+template <int L>
+__device__ __forceinline__ uint64_t heap_pop(uint64_t *heap, uint32_t (&light)[4], int n) {
+  const uint64_t top = heap[1], tmp = heap[n];
+  heap[n] = (uint64_t)kInfWeight << 32;
+  {
+    const uint32_t off = ~(1u << ((n >> 1) & 31));  // the parent's left child is the lighter one
+    const int w = n >> 6;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (q == 0 || (q == 1 && L > 5) || (q > 1 && L > 6)) light[q] &= w == q ? off : ~0u;
+  }
+  uint32_t node[L + 1], right[L];
+  uint64_t ch[L];   // the path's entries
+  uint32_t sib[L];  // their siblings' weights
+  node[0] = 1;
+#pragma unroll
+  for (int l = 0; l < L; l++) {
+    const uint32_t v = node[l];
+    // level l: nodes 2^l .. 2^(l + 1) - 1
+    const uint32_t w = l < 5 ? light[0] : l == 5 ? light[1] : (v & 32u ? light[3] : light[2]);
+    right[l] = (w >> (v & 31)) & 1u;
+    node[l + 1] = 2 * v + right[l];
+    ch[l] = heap[node[l + 1]];
+    sib[l] = reinterpret_cast<const uint32_t *>(heap)[2 * (node[l + 1] ^ 1u) + 1];
+  }
+  const uint32_t tw = hw(tmp);
+  uint64_t nv = 0;
+  bool here = true;
+#pragma unroll
+  for (int l = 0; l <= L; l++) {
+    const bool up = l < L && hw(ch[l < L ? l : 0]) <= tw;
+    nv = pick(up, ch[l < L ? l : 0], pick(here, tmp, ch[l > 0 ? l - 1 : 0]));
+    here = up;
+    heap[node[l]] = nv;
+    if (l > 0) {
+      const bool flip = hw(nv) + right[l - 1] > sib[l - 1];
+      const uint32_t bit = flip ? 1u << (node[l - 1] & 31) : 0u;
+      if (l - 1 < 5) {
+        light[0] ^= bit;
+      } else if (l - 1 == 5) {
+        light[1] ^= bit;
+      } else {
+        light[2] ^= node[l - 1] & 32u ? 0u : bit;
+        light[3] ^= node[l - 1] & 32u ? bit : 0u;
+      }
+    }
+  }
+  return top;
+}
+
+// Adds e at slot z (the same for all lanes, z < 2^(L + 1)).  kBits: keep
+// `light` up to date.
+template <int L, bool kBits>
+__device__ __forceinline__ void heap_push(uint64_t *heap, uint32_t (&light)[4], int z, uint64_t e) {
+  uint64_t anc[L];
+  uint32_t sib[L];
+#pragma unroll
+  for (int l = 0; l < L; l++) {
+    anc[l] = heap[z >> (l + 1)];  // past the root: entry 0, weight 0
+    if (kBits) sib[l] = reinterpret_cast<const uint32_t *>(heap)[2 * ((z >> l) ^ 1) + 1];
+  }
+  const uint32_t ew = hw(e);
+  bool here = true;
+#pragma unroll
+  for (int l = 0; l <= L; l++) {
+    // slot z >> l's new entry
+    const bool down = l < L && ew < hw(anc[l < L ? l : 0]);
+    const uint64_t nv = pick(down, anc[l < L ? l : 0], pick(here, e, anc[l > 0 ? l - 1 : 0]));
+    here = down;
+    if ((z >> l) >= 1) heap[z >> l] = nv;
+    if (kBits && l < L) {
+      const bool odd = (z >> l) & 1;
+      const uint32_t x = odd ? hw(nv) : sib[l], y = odd ? sib[l] : hw(nv);
+      const int par = z >> (l + 1);
+      const uint32_t bit = par > 0 ? 1u << (par & 31) : 0u;
+      // a parent's word: slot z's by its number, further up by the level
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (q == 0 || (l == 0 && q == 1 && L > 5) || (l == 0 && q > 1 && L > 6) ||
+            (l == 1 && q == 1 && L > 6)) {
+          const uint32_t m = (par >> 5) == q ? bit : 0u;
+          light[q] = (light[q] & ~m) | (x < y ? m : 0u);
+        }
+      }
+    }
+  }
+}
+
+// Merges the two lightest nodes while the heap has more than `down_to`
+// entries.  Node numbers count up from n_nodes.
+__device__ __forceinline__ uint64_t merged(uint64_t p1, uint64_t p2, int node, int16_t *parent) {
+  const uint32_t w1 = hw(p1), w2 = hw(p2);
+  parent[(uint32_t)p1] = parent[(uint32_t)p2] = (int16_t)node;
+  parent[node] = -1;
+  const uint32_t d1 = w1 & 0xff, d2 = w2 & 0xff;
+  const uint32_t wn = ((w1 & 0xffffff00u) + (w2 & 0xffffff00u)) | (1 + (d1 > d2 ? d1 : d2));
+  return ((uint64_t)wn << 32) | (uint32_t)node;
+}
+
+template <int L>
+__device__ __forceinline__ void merge_down(uint64_t *heap, uint32_t (&light)[4], int16_t *parent,
+                                           int down_to, int &n, int &n_nodes) {
+#pragma unroll 1
+  while (n > down_to) {
+    const uint64_t p1 = heap_pop<L>(heap, light, n);
+    const uint64_t p2 = heap_pop<L>(heap, light, n - 1);
+    const uint64_t e = merged(p1, p2, ++n_nodes, parent);
+    heap_push<L, true>(heap, light, n - 1, e);
+    n--;
+  }
+}
+
+// The reference's steps one entry after another, for heaps of 256 entries and
+// more and for weights that may pass 32 bits.
+__device__ __forceinline__ uint64_t heap_pop_slow(uint64_t *heap, int n) {
+  const uint64_t top = heap[1], tmp = heap[n];
+  heap[n] = (uint64_t)kInfWeight << 32;
+  n--;
+  int zz = 1;
+  for (;;) {
+    int yy = zz << 1;
+    if (yy > n) break;
+    const ulonglong2 pr = *reinterpret_cast<const ulonglong2 *>(&heap[yy]);
+    uint64_t c = pr.x;
+    if (yy < n && hw(pr.y) < hw(pr.x)) {
+      yy++;
+      c = pr.y;
+    }
+    if (hw(tmp) < hw(c)) break;
+    heap[zz] = c;
+    zz = yy;
+  }
+  if (n > 0) heap[zz] = tmp;
+  return top;
+}
+__device__ __forceinline__ void heap_push_slow(uint64_t *heap, int z, uint64_t e) {
+  uint64_t up = heap[z >> 1];
+  while (hw(e) < hw(up)) {
+    heap[z] = up;
+    z >>= 1;
+    up = heap[z >> 1];
+  }
+  heap[z] = e;
+}
 
 // split (the learned form, grid.y = 2): y = 0 builds every block's tables
 // into len, y = 1 the learned blocks' plain-selector tables into len2.
@@ -180,7 +344,7 @@ __device__ __forceinline__ uint32_t hw(uint64_t e) { return (uint32_t)(e >> 32);
 // MLP's counts for learned blocks), y = 1 from the first plain pass's counts.
 // split == 2 (second build): y = 0 from rfreq, y = 1 from rfreq2.
 __global__ void __launch_bounds__(32) k_huff_lengths(SlabDev d, int which, int round, int split) {
-  __shared__ __align__(16) uint64_t heap_s[kMaxGroups][kHeapN + 2];
+  __shared__ __align__(16) uint64_t heap_s[kMaxGroups][kHeapRow];
   __shared__ int32_t leafw_s[kMaxGroups][kMaxAlpha + 1];
   __shared__ int16_t parent_s[kMaxGroups][kNodeN];
   const int b = blockIdx.x;
@@ -208,85 +372,85 @@ __global__ void __launch_bounds__(32) k_huff_lengths(SlabDev d, int which, int r
     }
   }
   __syncwarp();
+  const bool wide = d.s[b] >= (1 << 24) - 512;  // weights may pass 32 bits
   unsigned pending = (1u << ngrp) - 1u;  // tables whose lengths are not final yet
   while (pending) {
-    if ((pending >> ln) & 1u) {
-      uint64_t *heap = heap_s[ln];
+    for (int t = 0; t < ngrp; t++)
+      for (int i = ln; i < kHeapRow; i += 32) heap_s[t][i] = i ? (uint64_t)kInfWeight << 32 : 0ull;
+    __syncwarp();
+    const bool run = (pending >> ln) & 1u;
+    uint64_t *heap = heap_s[run ? ln : 0];
+    int16_t *parent = parent_s[run ? ln : 0];
+    int n = alpha, n_nodes = alpha;
+    uint32_t light[4] = {0, 0, 0, 0};
+    if (run) {
       const int32_t *leafw = leafw_s[ln];
-      int16_t *parent = parent_s[ln];
-      int n_nodes = alpha, n_heap = 0;
-      heap[0] = 0;  // sentinel: weight 0
       for (int i = 1; i <= alpha; i++) {
-        parent[i] = -1;
-        n_heap++;
         const uint64_t e = ((uint64_t)(uint32_t)leafw[i] << 32) | (uint32_t)i;
-        int zz = n_heap;
-        uint64_t up = heap[zz >> 1];
-        while (hw(e) < hw(up)) {
-          heap[zz] = up;
-          zz >>= 1;
-          up = heap[zz >> 1];
-        }
-        heap[zz] = e;
+        parent[i] = -1;
+        if (wide || i > 255) heap_push_slow(heap, i, e);
+        else if (i > 31) heap_push<7, false>(heap, light, i, e);
+        else heap_push<4, false>(heap, light, i, e);
       }
-      while (n_heap > 1) {
-        uint64_t pick[2];
-        for (int q = 0; q < 2; q++) {
-          pick[q] = heap[1];
-          const uint64_t tmp = heap[n_heap];
-          n_heap--;
-          int zz = 1;
-          for (;;) {
-            int yy = zz << 1;
-            if (yy > n_heap) break;
-            const ulonglong2 pr = *reinterpret_cast<const ulonglong2 *>(&heap[yy]);
-            uint64_t c = pr.x;
-            if (yy < n_heap && hw(pr.y) < hw(pr.x)) {
-              yy++;
-              c = pr.y;
-            }
-            if (hw(tmp) < hw(c)) break;
-            heap[zz] = c;
-            zz = yy;
-          }
-          heap[zz] = tmp;
-        }
-        const uint32_t w1 = hw(pick[0]), w2 = hw(pick[1]);
-        const int n1 = (int)(uint32_t)pick[0], n2 = (int)(uint32_t)pick[1];
-        n_nodes++;
-        parent[n1] = parent[n2] = (int16_t)n_nodes;
-        const uint32_t d1 = w1 & 0xff, d2 = w2 & 0xff;
-        const uint32_t wn = ((w1 & 0xffffff00u) + (w2 & 0xffffff00u)) | (1 + (d1 > d2 ? d1 : d2));
-        parent[n_nodes] = -1;
-        n_heap++;
-        const uint64_t e = ((uint64_t)wn << 32) | (uint32_t)n_nodes;
-        int zz = n_heap;
-        uint64_t up = heap[zz >> 1];
-        while (hw(e) < hw(up)) {
-          heap[zz] = up;
-          zz >>= 1;
-          up = heap[zz >> 1];
-        }
-        heap[zz] = e;
+      while (n > (wide ? 1 : 255)) {
+        const uint64_t p1 = heap_pop_slow(heap, n);
+        const uint64_t p2 = heap_pop_slow(heap, n - 1);
+        const uint64_t e = merged(p1, p2, ++n_nodes, parent);
+        heap_push_slow(heap, n - 1, e);
+        n--;
       }
     }
     __syncwarp();
-    unsigned redo = 0;
-    for (int t = 0; t < ngrp; t++) {
-      if (!((pending >> t) & 1u)) continue;
-      const int16_t *parent = parent_s[t];
-      uint8_t *len = len_base + ((size_t)b * kMaxGroups + t) * kMaxAlpha;
-      bool too_long = false;
-      for (int i = ln + 1; i <= alpha; i += 32) {
-        int j = 0, k = i;
-        while (parent[k] >= 0) {
-          k = parent[k];
-          j++;
+    if (!wide) {
+      // which children are lighter, all nodes at once (lane t keeps table t's)
+      for (int t = 0; t < ngrp; t++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const ulonglong2 pr = *reinterpret_cast<const ulonglong2 *>(&heap_s[t][2 * (32 * q + ln)]);
+          const unsigned m = __ballot_sync(0xffffffffu, hw(pr.y) < hw(pr.x));
+          if (ln == t) light[q] = m;
         }
-        len[i - 1] = (uint8_t)j;
-        too_long |= j > kMaxCodeLen;
       }
-      if (__any_sync(0xffffffffu, too_long)) {
+      if (run) {
+        merge_down<7>(heap, light, parent, 127, n, n_nodes);
+        merge_down<6>(heap, light, parent, 63, n, n_nodes);
+        merge_down<5>(heap, light, parent, 31, n, n_nodes);
+        merge_down<4>(heap, light, parent, 1, n, n_nodes);
+      }
+    }
+    __syncwarp();
+    bool too_long[kMaxGroups] = {};
+    for (int i = ln + 1; i <= alpha; i += 32) {
+      int j[kMaxGroups], k[kMaxGroups];
+#pragma unroll
+      for (int t = 0; t < kMaxGroups; t++) {
+        j[t] = 0;
+        k[t] = (pending >> t) & 1u ? (int)parent_s[t][i] : -1;
+      }
+      for (;;) {
+        bool more = false;
+#pragma unroll
+        for (int t = 0; t < kMaxGroups; t++) {
+          if (k[t] >= 0) {
+            j[t]++;
+            k[t] = parent_s[t][k[t]];
+            more = true;
+          }
+        }
+        if (!more) break;
+      }
+#pragma unroll
+      for (int t = 0; t < kMaxGroups; t++) {
+        if ((pending >> t) & 1u) {
+          len_base[((size_t)b * kMaxGroups + t) * kMaxAlpha + i - 1] = (uint8_t)j[t];
+          too_long[t] |= j[t] > kMaxCodeLen;
+        }
+      }
+    }
+    unsigned redo = 0;
+#pragma unroll
+    for (int t = 0; t < kMaxGroups; t++) {
+      if (__any_sync(0xffffffffu, too_long[t])) {
         redo |= 1u << t;
         for (int i = ln + 1; i <= alpha; i += 32) {
           int j = leafw_s[t][i] >> 8;
