@@ -14,6 +14,9 @@
 //      h -> 2h) keys them (head << kb) | ISA[(i + h) mod m] and re-sorts them
 //      stably; the k-th of them in sorted order goes to the k-th active SA
 //      position (groups are contiguous, so this sorts within each group).
+//      Groups of up to kGroupMax rotations need no radix sort: a block whose
+//      active groups are all that short sorts them one by one in shared memory
+//      (k_bwt_local), in the same rounds.
 //   4. A block stops when no rotation is active, when a round splits no group
 //      (the rest are equal rotations, already index-ascending), or when the
 //      prefix length reaches m.
@@ -102,8 +105,16 @@ __device__ __forceinline__ uint64_t text_item(const uint8_t *T, int m, int i) {
   return ((uint64_t)k << 32) | (uint32_t)i;
 }
 
+// The key buffers alternate with the passes that move anything: sort_ctl[0] is
+// the buffer before a sort, bit p of sort_ctl[1] says whether pass p moves
+// items (k_bwt_tile_list settles both at the end of a round).
+__device__ __forceinline__ int keys_before(const SlabDev &d, int pass) {
+  return (d.sort_ctl[0] ^ __popc(d.sort_ctl[1] & ((1 << pass) - 1))) & 1;
+}
+__device__ __forceinline__ int keys_now(const SlabDev &d) { return keys_before(d, 31); }
+
 template <int RB>
-__device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int force,
+__device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int force, int pass,
                                                  uint32_t *scratch);
 
 // gen != 0: the generating first pass (items from the text, see text_item;
@@ -113,7 +124,7 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
 // counts, so the pass needs no scan launch of its own.
 template <int RB>
 __global__ void __launch_bounds__(256) k_radix_hist(SlabDev d, int shift, const int32_t *list,
-                                                    int gen) {
+                                                    int gen, int pass) {
   constexpr int kN = 1 << RB;
   __shared__ uint32_t cnt[kN];
   const int t = tile_id(list);
@@ -122,7 +133,7 @@ __global__ void __launch_bounds__(256) k_radix_hist(SlabDev d, int shift, const 
   if (valid == 0) return;
   for (int i = threadIdx.x; i < kN; i += blockDim.x) cnt[i] = 0;
   __syncthreads();
-  const uint64_t *K = d.keys[d.sort_ctl[0]] + d.off[b] + lt;
+  const uint64_t *K = d.keys[keys_before(d, pass)] + d.off[b] + lt;
   const uint8_t *T = d.rle1 + d.off[b];
   const int m = d.m[b];
   if (gen) {
@@ -151,7 +162,7 @@ __global__ void __launch_bounds__(256) k_radix_hist(SlabDev d, int shift, const 
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  block_digit_scan<RB>(d, b, gen, scratch);
+  block_digit_scan<RB>(d, b, gen, pass, scratch);
   if (threadIdx.x == 0) d.blk_count[b] = 0;
 }
 
@@ -161,7 +172,7 @@ __global__ void __launch_bounds__(256) k_radix_hist(SlabDev d, int shift, const 
 // digit only, since it writes the items the later passes read.
 // Thread i handles the kD = 2^RB / 256 consecutive digits kD*i .. kD*i+kD-1.
 template <int RB>
-__device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int force,
+__device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int force, int pass,
                                                  uint32_t *scratch) {
   constexpr int kN = 1 << RB, kD = kN / 256;
   const int len = d.sort_len[b];
@@ -198,7 +209,7 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
   uint32_t tot;
   uint32_t base = block_excl_sum(sum, scratch, &tot);
   int trivial = __syncthreads_or(one);
-  if ((!trivial || force) && threadIdx.x == 0) atomicOr(&d.sort_ctl[1], 1);
+  if ((!trivial || force) && threadIdx.x == 0) atomicOr(&d.sort_ctl[1], 1 << pass);
 #pragma unroll
   for (int q = 0; q < kD; q++) {
     d.sort_base[(size_t)b * kN + kD * threadIdx.x + q] = (uint32_t)d.off[b] + base;
@@ -213,9 +224,9 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
 // All of a thread's loads are issued before the ranking starts.
 template <bool kVals, int RB>
 __global__ void __launch_bounds__(256, kVals ? 2 : 3)
-    k_radix_scatter(SlabDev d, int shift, int timed, const int32_t *list, int gen) {
+    k_radix_scatter(SlabDev d, int shift, int timed, const int32_t *list, int gen, int pass) {
   constexpr int kN = 1 << RB, kD = kN / 256;
-  if (!d.sort_ctl[1]) return;
+  if (!((d.sort_ctl[1] >> pass) & 1)) return;  // every block's items share this digit
   const int t = tile_id(list);
   int b, lt;
   const int valid = tile_valid(d, t, d.sort_len, &b, &lt);
@@ -227,7 +238,7 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   uint32_t *sv = reinterpret_cast<uint32_t *>(sk + kTile);
   uint32_t *wcnt = kVals ? sv + kTile : reinterpret_cast<uint32_t *>(sk + kTile);  // [warp][digit]
   uint32_t *goff = wcnt + kSortWarps * kN + kN;  // global digit base for this tile
-  const int cur = d.sort_ctl[0];
+  const int cur = keys_before(d, pass);
   const uint64_t *K = d.keys[cur] + d.off[b] + lt;
   const uint32_t *V = d.vals[cur] + d.off[b] + lt;
   const int w = warp_id(), ln = lane_id();
@@ -342,11 +353,6 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   }
 }
 
-__global__ void k_radix_flip(SlabDev d) {
-  if (d.sort_ctl[1]) d.sort_ctl[0] ^= 1;
-  d.sort_ctl[1] = 0;
-}
-
 // Stable sort of each block's elements by key bits [lo, hi), over `grid`
 // tiles (all tiles, or the listed ones).
 // gen: the first pass generates the packed first-sort items from the text.
@@ -357,9 +363,10 @@ void radix_passes(const SlabDev &d, int lo, int hi, int has_vals, cudaStream_t s
                   const int32_t *list, bool gen) {
   BZ_REQUIRE(RB == 8 || (!has_vals && !gen), kErrInternal, "wide digits are for packed rounds");
   const size_t smem = has_vals ? scatter_smem_vals<RB>() : scatter_smem_keys<RB>();
-  for (int shift = lo; shift < hi; shift += RB) {
+  int pass = 0;
+  for (int shift = lo; shift < hi; shift += RB, pass++) {
     const int g = gen && shift == lo;
-    k_radix_hist<RB><<<grid, 256, 0, st>>>(d, shift, list, g);
+    k_radix_hist<RB><<<grid, 256, 0, st>>>(d, shift, list, g, pass);
     BZ_LAUNCH_CHECK();
     int timed = -1;
     if (d.kt_on && *d.kt_n < kMaxTimedLaunches) {
@@ -369,16 +376,14 @@ void radix_passes(const SlabDev &d, int lo, int hi, int has_vals, cudaStream_t s
     }
     if constexpr (RB == 8) {
       if (has_vals)
-        k_radix_scatter<true, 8><<<grid, 256, smem, st>>>(d, shift, timed, list, 0);
+        k_radix_scatter<true, 8><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
       else
-        k_radix_scatter<false, 8><<<grid, 256, smem, st>>>(d, shift, timed, list, g);
+        k_radix_scatter<false, 8><<<grid, 256, smem, st>>>(d, shift, timed, list, g, pass);
     } else {
-      k_radix_scatter<false, RB><<<grid, 256, smem, st>>>(d, shift, timed, list, 0);
+      k_radix_scatter<false, RB><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
     }
     BZ_LAUNCH_CHECK();
     if (timed >= 0) BZ_CUDA(cudaEventRecord(d.kt_ev[2 * timed + 1], st));
-    k_radix_flip<<<1, 1, 0, st>>>(d);
-    BZ_LAUNCH_CHECK();
   }
 }
 
@@ -407,6 +412,7 @@ __global__ void k_bwt_init(SlabDev d) {
   d.ngroups[b] = -1;
   d.act_len[b] = 0;
   d.active_sum[b] = 0;
+  d.loc[b] = d.loc_act[b] = d.loc_heads[b] = d.loc_sing[b] = d.gmax[b] = 0;
   d.blk_count[b] = 0;  // the histogram tile counter: each pass resets it, and so does this
   for (int k = 0; k < 8; k++) d.pstat[b * 8 + k] = 0;
   if (m == 1) d.sa[d.off[b]] = 0;
@@ -416,11 +422,8 @@ __global__ void k_bwt_init(SlabDev d) {
 // stands for (round h runs while the partition has a non-singleton group and
 // the previous round split one), and the group count of the prefix before
 // the first sort's as the fixed-point reference of the first ranking.
-__global__ void k_bwt_prefix_account(SlabDev d, int nq) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.nblocks) return;
+__device__ void prefix_account(const SlabDev &d, int b, int nq) {
   const int m = d.m[b];
-  if (m <= 1) return;
   const int32_t *ps = d.pstat + b * 8;
   int64_t A = 0;
   bool stop = false;
@@ -490,7 +493,7 @@ __global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, Layout L, int init
   if (valid == 0) return;
   const int len = d.sort_len[b];
   const int64_t off = d.off[b];
-  const uint64_t *K = d.keys[d.sort_ctl[0]] + off;
+  const uint64_t *K = d.keys[keys_now(d)] + off;
   const int32_t *P = d.kpos[d.sort_ctl[3]] + off;
   const int w = warp_id(), ln = lane_id();
   int last = -1, heads = 0, sing = 0;
@@ -559,12 +562,30 @@ __global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, Layout L, int init
 // tile), compaction offsets of the active elements per warp span, and the
 // stop test: no active element left, no group split by this round (the rest
 // are equal rotations), or prefix >= m.
-__global__ void __launch_bounds__(256) k_bwt_rank_block(SlabDev d, int64_t prefix_len) {
+// nq > 0: after the first sort (prefix_account).  Blocks sorted group by group
+// (loc) are not ranked here.
+__device__ void block_round_end(const SlabDev &d, int b, int active, int heads, int singles,
+                                int64_t prefix_len) {
+  const int m = d.m[b];
+  const bool fin = active == 0 || heads == d.ngroups[b] || prefix_len >= m;
+  d.ngroups[b] = heads - singles;  // groups among the rotations still active
+  if (fin) {
+    d.done[b] = 1;
+    d.act_len[b] = 0;
+  } else {
+    d.act_len[b] = active;
+    atomicAdd(&d.sort_ctl[2], 1);
+    atomicAdd(&d.sort_ctl[6], active);
+    d.active_sum[b] += active;  // rotations entering the next round
+  }
+}
+
+__global__ void __launch_bounds__(256) k_bwt_rank_block(SlabDev d, int64_t prefix_len, int nq) {
   __shared__ int scratch[40];
   __shared__ int sx[256];
   const int b = blockIdx.x;
   const int len = d.sort_len[b];
-  if (len <= 0) return;
+  if (len <= 0 || d.loc[b]) return;
   const int nt = (len + kTile - 1) / kTile;
   const int t0 = (int)(d.off[b] / kTile);
   const int nw = nt * kSortWarps;
@@ -597,19 +618,8 @@ __global__ void __launch_bounds__(256) k_bwt_rank_block(SlabDev d, int64_t prefi
     singles += tot;
   }
   if (threadIdx.x == 0) {
-    const int m = d.m[b];
-    const bool fin = active == 0 || heads == d.ngroups[b] || prefix_len >= m;
-    d.ngroups[b] = heads - singles;  // groups among the rotations still active
-    if (fin) {
-      d.done[b] = 1;
-      d.act_len[b] = 0;
-    } else {
-      d.act_len[b] = active;
-      atomicAdd(&d.sort_ctl[2], 1);
-      atomicAdd(&d.sort_ctl[6], active);
-      atomicAdd(&d.sort_ctl[4], (active + kTile - 1) / kTile);
-      d.active_sum[b] += active;  // rotations entering the next round
-    }
+    if (nq > 0) prefix_account(d, b, nq);
+    block_round_end(d, b, active, heads, singles, prefix_len);
   }
 }
 
@@ -624,7 +634,7 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
   if (valid == 0) return;
   const int len = d.sort_len[b];
   const int64_t off = d.off[b];
-  const int cur = d.sort_ctl[0], pc = d.sort_ctl[3];
+  const int cur = keys_now(d), pc = d.sort_ctl[3];
   const uint64_t *K = d.keys[cur] + off;
   const uint32_t *V = d.vals[cur] + off;
   const int32_t *P = d.kpos[pc] + off;
@@ -639,6 +649,7 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
   int32_t *SA = d.sa + off;
   int32_t *IS = d.isa + off;
   const unsigned lt_mask = (1u << ln) - 1u;
+  int gmax = 0;  // largest active group that ends here
   // heads by a running max, writes, compaction
 #pragma unroll 4
   for (int i = 0; i < kTileItems; i++) {
@@ -646,7 +657,7 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
     const bool ok = e < valid;
     int pos = 0, hdpos = -1;
     uint32_t val = 0;
-    bool active = false;
+    bool active = false, last = false;
     if (ok) {
       const int k = lt + e;
       const uint64_t item = K[k];
@@ -657,10 +668,12 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
       val = L.packed ? (uint32_t)(item & ((1ull << L.low) - 1)) : V[k];
       if (hd) hdpos = pos;
       active = !(hd && tl);
+      last = tl && !hd;
     }
     const int head = max(carry, warp_incl_max(hdpos));
     carry = __shfl_sync(0xffffffffu, head, 31);
     const unsigned am = __ballot_sync(0xffffffffu, active);
+    if (last) gmax = max(gmax, pos - head + 1);
     if (ok) {
       SA[pos] = (int32_t)val;
       IS[val] = head;
@@ -677,38 +690,327 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
     }
     aoff += __popc(am);
   }
+  if (compact && L.packed) {
+    gmax = __reduce_max_sync(0xffffffffu, gmax);
+    if (ln == 0 && gmax > 0) atomicMax(&d.gmax[b], gmax);
+  }
 }
 
-// Next round: sort_len = active rotations; list the tiles that hold them.
-__global__ void k_bwt_tile_list(SlabDev d) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.nblocks) return;
-  const int len = d.act_len[b];
-  d.sort_len[b] = len;
-  if (len <= 0) return;
-  const int nt = (len + kTile - 1) / kTile;
-  const int at = atomicAdd(&d.sort_ctl[5], nt);
-  const int t0 = (int)(d.off[b] / kTile);
-  for (int k = 0; k < nt; k++) d.tile_list[at + k] = t0 + k;
+// Groups of at most kGroupMax rotations are sorted in shared memory: a CTA
+// takes the groups that start in its kGroupMax items (a half tile) of a block's
+// active list, so it holds at most kTile.
+constexpr int kGroupMax = kTile / 2;
+
+// Lists a block's tiles: half tiles when it is sorted group by group.  The
+// blocks' places are taken by a thread each, the entries written by a warp
+// each.  One CTA of 1024 threads; nblocks in passes of 1024.
+struct TileRuns {
+  int at[1024], n[1024], t0[1024];
+  int32_t *list[1024];
+};
+
+__device__ __forceinline__ void list_block(const SlabDev &d, TileRuns &r, int b, int len) {
+  const bool loc = d.loc[b];
+  const int unit = loc ? kGroupMax : kTile;
+  const int nt = (len + unit - 1) / unit;
+  r.at[threadIdx.x] = atomicAdd(&d.sort_ctl[loc ? 7 : 5], nt);
+  r.n[threadIdx.x] = nt;
+  r.t0[threadIdx.x] = (int)(d.off[b] / unit);
+  r.list[threadIdx.x] = loc ? d.loc_list : d.tile_list;
 }
 
-__global__ void k_bwt_flip(SlabDev d) {
-  d.sort_ctl[0] ^= 1;
-  d.sort_ctl[3] ^= 1;
+__device__ __forceinline__ void write_lists(const TileRuns &r, int nb) {
+  for (int q = warp_id(); q < nb; q += 32)
+    for (int k = lane_id(); k < r.n[q]; k += 32) r.list[q][r.at[q] + k] = r.t0[q] + k;
 }
 
-// Round keys for the compacted active rotations: add the rank of i+h.
-__global__ void __launch_bounds__(256) k_bwt_round_keys(SlabDev d, int h, int packed, int kb,
-                                                        const int32_t *list) {
-  const int t = tile_id(list);
-  const int b = d.tile_block[t];
+// Ends a round: blocks sorted group by group settle their counts, the key and
+// position buffers switch, sort_len = active rotations, and the next round's
+// tiles are listed: tiles of the blocks that go on by radix sort, half tiles of
+// those whose groups are all short.
+__global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefix_len, int packed) {
+  __shared__ TileRuns runs;
+  for (int b0 = 0; b0 < d.nblocks; b0 += 1024) {
+    const int b = b0 + threadIdx.x;
+    runs.n[threadIdx.x] = 0;
+    if (b < d.nblocks) {
+      if (d.loc[b] && d.sort_len[b] > 0) {
+        block_round_end(d, b, d.loc_act[b], d.loc_heads[b], d.loc_sing[b], prefix_len);
+        d.loc_act[b] = d.loc_heads[b] = d.loc_sing[b] = 0;
+        d.loc_cur[b] ^= 1;
+      }
+      const int len = d.act_len[b];
+      d.sort_len[b] = len;
+      if (len > 0) {
+        if (packed && !d.loc[b] && d.gmax[b] <= kGroupMax) {
+          d.loc[b] = 1;
+          d.loc_cur[b] = keys_now(d) ^ 1;
+        }
+        d.gmax[b] = 0;
+        list_block(d, runs, b, len);
+      }
+    }
+    __syncthreads();
+    write_lists(runs, min(1024, d.nblocks - b0));
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    d.sort_ctl[0] = keys_now(d) ^ 1;
+    d.sort_ctl[1] = 0;
+    d.sort_ctl[3] ^= 1;
+  }
+}
+
+// One round of the groups of a half tile.  Items are head << 2kb | rank << kb |
+// rotation; with the head replaced by the group's start in the tile (groups
+// stand in no order in the list) they are all different and sorting them by
+// value sorts every group by rank with ties in index order.  Each group is
+// sorted by itself: ranks within 8 items by counting the smaller ones, then
+// runs of 8, 16, .. merged, an item's place being its place in its run plus
+// the number of smaller items in the sibling run (binary search; what follows
+// a group's end is larger).  The new heads follow within the CTA, since an
+// item's SA position is its group's head plus its place in the group.  About 200 instructions per rotation where
+// the radix passes, ranking and compaction of a round took about 700.
+__global__ void __launch_bounds__(256, 3) k_bwt_local(SlabDev d, int kb) {
+  __shared__ uint64_t key[kTile + 8];
+  __shared__ int red[4][kSortWarps];
+  __shared__ int s_base;
+  const int h = d.loc_list[blockIdx.x];
+  const int b = d.tile_block[h >> 1];
   const int64_t off = d.off[b];
-  const int lt = (int)((int64_t)t * kTile - off);
+  const int s = (int)((int64_t)h * kGroupMax - off);  // first item of the half tile
   const int len = d.sort_len[b];
-  const int valid = min(kTile, len - lt);
+  const int cur = d.loc_cur[b];
+  const uint64_t *K = d.keys[cur] + off;
+  const int w = warp_id(), ln = lane_id();
+  const int avail = min(kTile, len - s);
+  const unsigned le_mask = 0xffffffffu >> (31 - ln);
+  // items, and the first groups starting in this half tile and after it
+  int first = INT32_MAX, after = avail;
+  const int hs = 2 * kb;
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = w * kWarpSpan + i * 32 + ln;
+    if (e < avail) {
+      const uint64_t x = K[s + e];
+      key[e] = x;
+      const bool st = s + e == 0 || (K[s + e - 1] >> hs) != (x >> hs);
+      if (st) {
+        if (e < kGroupMax) first = min(first, e);
+        else after = min(after, e);
+      }
+    }
+  }
+  if (threadIdx.x < 8) key[avail + threadIdx.x] = ~0ull;
+  first = __reduce_min_sync(0xffffffffu, first);
+  after = __reduce_min_sync(0xffffffffu, after);
+  if (ln == 0) {
+    red[0][w] = first;
+    red[1][w] = after;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kSortWarps; q++) {
+    first = min(first, red[0][q]);
+    after = min(after, red[1][q]);
+  }
+  if (first >= kGroupMax) return;  // one group from before covers the half tile
+  // [first, after): whole groups.  Each item's group start.
+  uint64_t mine[kTileItems];
+  uint32_t gs2[kTileItems / 2];  // two 16-bit positions per register
+  int carry = -1;
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = w * kWarpSpan + i * 32 + ln;
+    const bool in = e >= first && e < after;
+    mine[i] = in ? key[e] : ~0ull;
+    const bool st = in && (e == first || (key[e - 1] >> hs) != (mine[i] >> hs));
+    const unsigned bm = __ballot_sync(0xffffffffu, st) & le_mask;
+    const int g = bm ? e - ln + 31 - __clz(bm) : carry;
+    carry = __shfl_sync(0xffffffffu, g, 31);
+    if (i & 1) gs2[i >> 1] |= (uint32_t)(g & 0xffff) << 16;
+    else gs2[i >> 1] = (uint32_t)(g & 0xffff);
+  }
+  if (ln == 0) red[2][w] = carry;
+  __syncthreads();
+  int before = -1;  // last group start in the earlier warps
+  for (int q = 0; q < w; q++) before = max(before, red[2][q]);
+  auto group_start = [&](int i) {
+    const uint32_t g = (i & 1) ? gs2[i >> 1] >> 16 : gs2[i >> 1] & 0xffffu;
+    return g == 0xffffu ? before : (int)g;
+  };
+  int big = 0;  // the largest place of this warp's items in their groups
+  const uint64_t low = (1ull << hs) - 1;
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = w * kWarpSpan + i * 32 + ln;
+    if (e >= first && e < after) {
+      const int g = group_start(i);
+      big = max(big, e - g);
+      mine[i] = ((uint64_t)(uint32_t)g << hs) | (mine[i] & low);
+      key[e] = mine[i];
+    } else if (e >= after && e < avail) {
+      key[e] = ~0ull;
+    }
+  }
+  __syncthreads();
+  big = __reduce_max_sync(0xffffffffu, big);
+  if (ln == 0) red[3][w] = big;
+  // runs of 8
+  uint32_t to2[kTileItems / 2];
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = w * kWarpSpan + i * 32 + ln;
+    int to = 0;
+    if (e >= first && e < after) {
+      const int g = group_start(i);
+      const int c0 = g + ((e - g) & ~7);
+      to = c0;
+#pragma unroll
+      for (int q = 0; q < 8; q++) to += key[min(c0 + q, avail)] < mine[i];
+    }
+    if (i & 1) to2[i >> 1] |= (uint32_t)to << 16;
+    else to2[i >> 1] = (uint32_t)to;
+  }
+  __syncthreads();
+  int most = 0;
+#pragma unroll
+  for (int q = 0; q < kSortWarps; q++) most = max(most, red[3][q]);
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = w * kWarpSpan + i * 32 + ln;
+    const uint32_t to = (i & 1) ? to2[i >> 1] >> 16 : to2[i >> 1] & 0xffffu;
+    if (e >= first && e < after) key[to] = mine[i];
+  }
+  __syncthreads();
+  for (int run = 8; run <= most; run <<= 1) {  // some group has more than `run` items
+    // a warp whose groups end within its first run has nothing to move; one
+    // that holds a long group's beginning sees it through the sibling's head
+    bool moves = false;
+#pragma unroll
+    for (int i = 0; i < kTileItems; i++) {
+      const int e = w * kWarpSpan + i * 32 + ln;
+      int to = e;
+      if (e >= first && e < after) {
+        const uint64_t x = key[e];
+        mine[i] = x;
+        const int g = group_start(i);
+        const int r0 = g + ((e - g) & ~(run - 1));   // this run
+        const bool odd = (e - g) & run;
+        const int o0 = odd ? r0 - run : r0 + run;    // its sibling
+        if (o0 < after && (odd || (key[o0] >> hs) == (x >> hs))) {
+          int lo = o0, hi = min(o0 + run, after);
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key[mid] < x) lo = mid + 1;
+            else hi = mid;
+          }
+          to = e + (lo - o0) - (odd ? run : 0);
+          moves = true;
+        }
+      }
+      if (i & 1) to2[i >> 1] |= (uint32_t)to << 16;
+      else to2[i >> 1] = (uint32_t)to;
+    }
+    __syncthreads();
+    if (__any_sync(0xffffffffu, moves)) {
+#pragma unroll
+      for (int i = 0; i < kTileItems; i++) {
+        const int e = w * kWarpSpan + i * 32 + ln;
+        const uint32_t to = (i & 1) ? to2[i >> 1] >> 16 : to2[i >> 1] & 0xffffu;
+        if (e >= first && e < after && (int)to != e) key[to] = mine[i];
+      }
+    }
+    __syncthreads();
+  }
+  // new groups: head and rank alike
+  int32_t *SA = d.sa + off;
+  int32_t *IS = d.isa + off;
+  const uint64_t vmask = (1ull << kb) - 1;
+  carry = -1;
+  int heads = 0, sing = 0, act = 0;
+  uint32_t sg2[kTileItems / 2];
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = w * kWarpSpan + i * 32 + ln;
+    const bool in = e >= first && e < after;
+    const uint64_t x = in ? key[e] : ~0ull;
+    mine[i] = x;
+    const bool hd = in && (e == first || (key[e - 1] >> kb) != (x >> kb));
+    const bool tl = in && (e + 1 == after || (key[e + 1] >> kb) != (x >> kb));
+    const unsigned bm = __ballot_sync(0xffffffffu, hd);
+    const unsigned below = bm & le_mask;
+    const int g = below ? e - ln + 31 - __clz(below) : carry;
+    carry = __shfl_sync(0xffffffffu, g, 31);
+    if (i & 1) sg2[i >> 1] |= (uint32_t)(g & 0xffff) << 16;
+    else sg2[i >> 1] = (uint32_t)(g & 0xffff);
+    const unsigned sm = __ballot_sync(0xffffffffu, hd && tl);
+    const unsigned im = __ballot_sync(0xffffffffu, in);
+    heads += __popc(bm);
+    sing += __popc(sm);
+    act += __popc(im & ~sm);
+  }
+  if (ln == 0) {
+    red[0][w] = carry;
+    red[1][w] = act;
+    red[2][w] = heads;
+    red[3][w] = sing;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int a = 0, hh = 0, ss = 0;
+    for (int q = 0; q < kSortWarps; q++) {
+      const int v = red[1][q];
+      red[1][q] = a;
+      a += v;
+      hh += red[2][q];
+      ss += red[3][q];
+    }
+    s_base = a ? atomicAdd(&d.loc_act[b], a) : 0;
+    atomicAdd(&d.loc_heads[b], hh);
+    if (ss) atomicAdd(&d.loc_sing[b], ss);
+  }
+  __syncthreads();
+  int sbefore = -1;
+  for (int q = 0; q < w; q++) sbefore = max(sbefore, red[0][q]);
+  uint64_t *KO = d.keys[cur ^ 1] + off + s_base + red[1][w];
+  const unsigned lt_mask = le_mask >> 1;
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = w * kWarpSpan + i * 32 + ln;
+    const bool in = e >= first && e < after;
+    const uint64_t x = mine[i];
+    const int g = group_start(i);
+    const uint32_t sgv = (i & 1) ? sg2[i >> 1] >> 16 : sg2[i >> 1] & 0xffffu;
+    const int sg = sgv == 0xffffu ? sbefore : (int)sgv;
+    const int head = in ? (int)(K[s + e] >> hs) : 0;  // the list still holds the group here
+    const int nhead = head + (sg - g);
+    const uint32_t val = (uint32_t)(x & vmask);
+    const bool tl = in && (e + 1 == after || (key[e + 1] >> kb) != (x >> kb));
+    const bool active = in && !(sg == e && tl);
+    if (in) {
+      SA[head + (e - g)] = (int32_t)val;
+      if (nhead != head) IS[val] = nhead;
+    }
+    const unsigned am = __ballot_sync(0xffffffffu, active);
+    if (active) KO[__popc(am & lt_mask)] = ((uint64_t)(uint32_t)nhead << hs) | val;
+    KO += __popc(am);
+  }
+}
+
+// Round keys for the compacted active rotations: add the rank of i+h.  unit:
+// items per list entry (kTile, or kGroupMax for the blocks sorted by groups).
+__global__ void __launch_bounds__(256) k_bwt_round_keys(SlabDev d, int h, int packed, int kb,
+                                                        const int32_t *list, int unit) {
+  const int t = list[blockIdx.x];
+  const int b = d.tile_block[unit == kTile ? t : t >> 1];
+  const int64_t off = d.off[b];
+  const int lt = (int)((int64_t)t * unit - off);
+  const int len = d.sort_len[b];
+  const int valid = min(unit, len - lt);
   if (valid <= 0) return;
   const int m = d.m[b];
-  const int cur = d.sort_ctl[0];
+  const int cur = unit == kTile ? d.sort_ctl[0] : d.loc_cur[b];
   uint64_t *K = d.keys[cur] + off + lt;
   const uint32_t *V = d.vals[cur] + off + lt;
   const int32_t *IS = d.isa + off;
@@ -776,39 +1078,40 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
   }
   const int nq = packed ? 3 : 4;  // prefixes 1,2,4 (,8) bytes
   int64_t prefix = packed ? 4 : 8;
-  int grid = grid0;
+  int grid = grid0, lgrid = 0;
   const int32_t *list = list0;
   int r = 0;  // round being run (0: the first sort)
   for (int initial = 1;; initial = 0) {
     const Layout L = initial ? first : round;
     BZ_CUDA(cudaMemsetAsync(d.sort_ctl + 2, 0, sizeof(int32_t), st));
-    BZ_CUDA(cudaMemsetAsync(d.sort_ctl + 4, 0, 3 * sizeof(int32_t), st));
-    k_bwt_flags<<<grid, 256, 0, st>>>(d, L, initial, list, packed ? 32 : 64, initial ? nq : 0);
-    BZ_LAUNCH_CHECK();
-    if (initial) {
-      k_bwt_prefix_account<<<(d.nblocks + 127) / 128, 128, 0, st>>>(d, nq);
+    BZ_CUDA(cudaMemsetAsync(d.sort_ctl + 5, 0, 3 * sizeof(int32_t), st));
+    if (grid > 0) {
+      k_bwt_flags<<<grid, 256, 0, st>>>(d, L, initial, list, packed ? 32 : 64, initial ? nq : 0);
+      BZ_LAUNCH_CHECK();
+      k_bwt_rank_block<<<d.nblocks, 256, 0, st>>>(d, prefix, initial ? nq : 0);
+      BZ_LAUNCH_CHECK();
+      k_bwt_apply<<<grid, 256, 0, st>>>(d, L, initial, kb, list);
       BZ_LAUNCH_CHECK();
     }
-    k_bwt_rank_block<<<d.nblocks, 256, 0, st>>>(d, prefix);
-    BZ_LAUNCH_CHECK();
-    k_bwt_apply<<<grid, 256, 0, st>>>(d, L, initial, kb, list);
-    BZ_LAUNCH_CHECK();
-    k_bwt_flip<<<1, 1, 0, st>>>(d);
+    if (lgrid > 0) {
+      k_bwt_local<<<lgrid, 256, 0, st>>>(d, kb);
+      BZ_LAUNCH_CHECK();
+    }
+    k_bwt_tile_list<<<1, 1024, 0, st>>>(d, prefix, packed);
     BZ_LAUNCH_CHECK();
     if (rounds_timed) {
       BZ_CUDA(cudaEventRecord(d.rt_ev[2 * r + 1], st));
       *d.rt_n = r + 1;
     }
     if (prefix >= max_m) break;
-    k_bwt_tile_list<<<(d.nblocks + 127) / 128, 128, 0, st>>>(d);
-    BZ_LAUNCH_CHECK();
     BZ_CUDA(cudaMemcpyAsync(d.h_flags, d.sort_ctl + 2, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost,
                             st));
     BZ_CUDA(cudaStreamSynchronize(st));
     if (rounds_timed && initial)
       std::memcpy(&d.rt_act[0], d.h_flags + 6, sizeof(int64_t));  // sort_ctl[8..9]
     if (d.h_flags[0] == 0) break;
-    grid = d.h_flags[2];  // tiles holding active rotations
+    grid = d.h_flags[3];   // tiles holding active rotations
+    lgrid = d.h_flags[5];  // half tiles of the blocks sorted group by group
     list = d.tile_list;
     r++;
     if (rounds_timed && r >= kMaxRounds) rounds_timed = false;
@@ -816,8 +1119,15 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
       d.rt_act[r] = d.h_flags[4];  // rotations entering this round
       BZ_CUDA(cudaEventRecord(d.rt_ev[2 * r], st));
     }
-    k_bwt_round_keys<<<grid, 256, 0, st>>>(d, (int)prefix, packed, kb, list);
-    BZ_LAUNCH_CHECK();
+    // every block's keys before any block's ranks change
+    if (grid > 0) {
+      k_bwt_round_keys<<<grid, 256, 0, st>>>(d, (int)prefix, packed, kb, list, kTile);
+      BZ_LAUNCH_CHECK();
+    }
+    if (lgrid > 0) {
+      k_bwt_round_keys<<<lgrid, 256, 0, st>>>(d, (int)prefix, packed, kb, d.loc_list, kGroupMax);
+      BZ_LAUNCH_CHECK();
+    }
     if (packed)
       radix_sort(d, kb, 3 * kb, 0, st, grid, list);
     else

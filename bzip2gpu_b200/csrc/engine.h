@@ -94,6 +94,12 @@ struct SlabDev {
   int32_t *sort_len, *done, *ngroups;  // BWT control (ngroups: groups among active rotations)
   int32_t *act_len;                    // BWT: active rotations entering the next round
   int32_t *tile_list;                  // BWT: tiles holding active rotations [ntiles]
+  // BWT: blocks whose active groups are all short are sorted group by group in
+  // shared memory.  loc[b]: 1 for such a block; loc_cur: its current key
+  // buffer; loc_act, loc_heads, loc_sing: the running round's active
+  // rotations, groups and singletons; gmax: the largest active group after a
+  // radix round; loc_list: their half tiles [2 * ntiles].
+  int32_t *loc, *loc_cur, *loc_act, *loc_heads, *loc_sing, *gmax, *loc_list;
   // The tiles that hold data, listed in block order (a block's workspace is
   // sized for its worst-case RLE1 output, so most of its tiles can be empty):
   // element tiles of the m[b] RLE1 bytes, and group tiles of the
@@ -108,9 +114,10 @@ struct SlabDev {
   int32_t *pstat;                      // [nblocks * 8]: heads and singletons at prefix 1,2,4,8
   int64_t *hdr_bits, *pay_bits, *blk_start;
   // radix sort control
-  int32_t *sort_ctl;                   // [0]=cur key buffer, [1]=nontrivial flag,
+  int32_t *sort_ctl;                   // [0]=cur key buffer, [1]=passes that move items,
                                        // [2]=blocks still sorting, [3]=cur kpos buffer,
-                                       // [4]=tiles of the next round, [5]=tile list fill,
+                                       // [5]=tiles of the next round,
+                                       // [7]=half tiles of its group-sorted blocks,
                                        // [6]=rotations entering the next round,
                                        // [8..9]=u64 rotations the first sort's model charges
                                        // [10], [11]=tile-list counts, [12]=largest m
