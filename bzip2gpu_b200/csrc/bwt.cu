@@ -16,7 +16,7 @@
 //      position (groups are contiguous, so this sorts within each group).
 //      Groups of up to kGroupMax rotations need no radix sort: a block whose
 //      active groups are all that short sorts them one by one in shared memory
-//      (k_bwt_local), in the same rounds.
+//      (k_bwt_groups), in the same rounds.
 //   4. A block stops when no rotation is active, when a round splits no group
 //      (the rest are equal rotations, already index-ascending), or when the
 //      prefix length reaches m.
@@ -26,6 +26,7 @@
 // (item = prefix << 32 | i), rounds use item = head << 2kb | rank << kb | i.
 // Larger m keeps separate 64-bit keys and 32-bit rotations, with P = 8.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "engine.h"
@@ -47,17 +48,6 @@ constexpr size_t scatter_smem_keys() {
 template <int RB>
 constexpr size_t scatter_smem_vals() {
   return scatter_smem_keys<RB>() + (size_t)kTile * 4;
-}
-
-// How a sorted element is stored: packed (one item: key << low | rotation)
-// or as separate keys[] and vals[].
-struct Layout {
-  int packed;
-  int low;
-};
-
-__device__ __forceinline__ uint64_t key_of(const Layout L, uint64_t item) {
-  return L.packed ? item >> L.low : item;
 }
 
 // Tile of this CTA: blockIdx.x, or the blockIdx.x-th entry of a list of the
@@ -89,6 +79,21 @@ __device__ __forceinline__ unsigned digit_peers(int dg, bool ok) {
   }
   return peers;
 }
+
+// The RB bits of an item from bit `shift` on.  kHigh: a byte of the high word
+// (the first sort's 8-bit digits), one byte permutation.
+template <int RB, bool kHigh>
+struct Digit {
+  int sh;
+  bool high;
+  __device__ __forceinline__ explicit Digit(int shift)
+      : sh(kHigh ? 0x4440 + (shift - 32) / 8 : shift & 31), high(shift >= 32) {}
+  __device__ __forceinline__ int operator()(uint64_t item) const {
+    const uint32_t lo = (uint32_t)item, hi = (uint32_t)(item >> 32);
+    if (kHigh) return (int)__byte_perm(hi, 0, sh);
+    return (int)(__funnelshift_r(high ? hi : lo, high ? 0u : hi, sh) & ((1u << RB) - 1u));
+  }
+};
 
 // The first sort of the packed layout starts from index order, so its first
 // pass builds each tile's items itself from the block's text (read in order:
@@ -146,8 +151,9 @@ __global__ void __launch_bounds__(256) k_radix_hist(SlabDev d, int shift, const 
       atomicAdd(&cnt[T[j]], 1u);
     }
   } else {
-    for (int e = threadIdx.x; e < valid; e += blockDim.x)
-      atomicAdd(&cnt[(uint32_t)(K[e] >> shift) & (kN - 1)], 1u);
+    const Digit<RB, false> dig(shift);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < valid; e += blockDim.x) atomicAdd(&cnt[dig(K[e])], 1u);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kN; i += blockDim.x) d.tile_hist[(size_t)t * kN + i] = cnt[i];
@@ -222,7 +228,7 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
 // over the lanes with equal digits keeps the original order; the tile is sorted locally
 // in shared memory, then written so that equal digits go out contiguously.
 // All of a thread's loads are issued before the ranking starts.
-template <bool kVals, int RB>
+template <bool kVals, int RB, bool kHigh>
 __global__ void __launch_bounds__(256, kVals ? 2 : 3)
     k_radix_scatter(SlabDev d, int shift, int timed, const int32_t *list, int gen, int pass) {
   constexpr int kN = 1 << RB, kD = kN / 256;
@@ -242,10 +248,11 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   const uint64_t *K = d.keys[cur] + d.off[b] + lt;
   const uint32_t *V = d.vals[cur] + d.off[b] + lt;
   const int w = warp_id(), ln = lane_id();
+  const Digit<RB, kHigh> dig(shift);
 
   uint64_t key[kTileItems];
   uint32_t val[kTileItems];
-  if (!kVals && gen) {
+  if (kHigh && gen) {
     const uint8_t *T = d.rle1 + d.off[b];
     const int m = d.m[b];
 #pragma unroll
@@ -272,7 +279,7 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   for (int i = 0; i < kTileItems; i++) {
     const int e = w * kWarpSpan + i * 32 + ln;
     const bool ok = e < valid;
-    const int dg = ok ? (int)((key[i] >> shift) & (kN - 1)) : 0;
+    const int dg = dig(key[i]);
     const unsigned peers = digit_peers<RB>(dg, ok);
     const uint32_t before = ok ? wcnt[w * kN + dg] : 0;
     const uint32_t r = before + __popc(peers & lt_mask);
@@ -334,7 +341,7 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   for (int i = 0; i < kTileItems; i++) {
     const int e = w * kWarpSpan + i * 32 + ln;
     if (e < valid) {
-      const int dg = (int)((key[i] >> shift) & (kN - 1));
+      const int dg = dig(key[i]);
       const uint32_t r = (i & 1) ? rank2[i >> 1] >> 16 : rank2[i >> 1] & 0xffffu;
       const uint32_t pos = wcnt[w * kN + dg] + r;
       sk[pos] = key[i];
@@ -346,7 +353,7 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   uint32_t *VO = d.vals[cur ^ 1];
   for (int k = threadIdx.x; k < valid; k += blockDim.x) {
     const uint64_t kk = sk[k];
-    const int dg = (int)((kk >> shift) & (kN - 1));
+    const int dg = dig(kk);
     const uint32_t g = goff[dg] + (uint32_t)k;
     KO[g] = kk;
     if (kVals) VO[g] = sv[k];
@@ -376,11 +383,13 @@ void radix_passes(const SlabDev &d, int lo, int hi, int has_vals, cudaStream_t s
     }
     if constexpr (RB == 8) {
       if (has_vals)
-        k_radix_scatter<true, 8><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
+        k_radix_scatter<true, 8, false><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
+      else if (gen)
+        k_radix_scatter<false, 8, true><<<grid, 256, smem, st>>>(d, shift, timed, list, g, pass);
       else
-        k_radix_scatter<false, 8><<<grid, 256, smem, st>>>(d, shift, timed, list, g, pass);
+        k_radix_scatter<false, 8, false><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
     } else {
-      k_radix_scatter<false, RB><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
+      k_radix_scatter<false, RB, false><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
     }
     BZ_LAUNCH_CHECK();
     if (timed >= 0) BZ_CUDA(cudaEventRecord(d.kt_ev[2 * timed + 1], st));
@@ -477,16 +486,43 @@ __global__ void __launch_bounds__(256) k_bwt_keys0(SlabDev d, int packed) {
 // where the key changes; its head is the SA position of its first element.
 // Elements are read warp-striped (warp w owns [512w, 512w + 512), item i of
 // lane l is element 512w + 32i + l) so every load is coalesced.
-__device__ __forceinline__ uint64_t key_at(const uint64_t *K, int k) { return K[k]; }
 
-// Per tile: last head (SA position), head count, singleton count, active
-// (non-singleton) count.  After the first sort (nq > 0) it also counts, from
-// the same reads, the group heads and singletons of the prefix-1, -2 (-4, -8)
-// byte partitions (key_bits = 32 packed, 64 otherwise): pstat[b*8 + q] heads
-// and pstat[b*8 + 4 + q] singletons of prefix 2^q bytes.
-__global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, Layout L, int initial,
-                                                   const int32_t *list, int key_bits, int nq) {
-  __shared__ int red[4][kSortWarps];
+// Kinds of sorted elements: the first sort's packed items (prefix << 32 |
+// rotation), a round's packed items (head << 2kb | rank << kb | rotation),
+// separate keys.
+enum Kind { kPrefixItems, kRoundItems, kKeys };
+
+// Bytes (first sort) that elements k and k + 1 have in common at the front of
+// their keys; a round's keys only agree (1) or not (0).  kWhole: equal keys.
+template <int kKind>
+constexpr int kWhole = kKind == kPrefixItems ? 4 : kKind == kRoundItems ? 1 : 8;
+
+template <int kKind>
+__device__ __forceinline__ int common(const uint64_t *K, int k, int kb) {
+  if constexpr (kKind == kPrefixItems) {
+    const uint32_t *H = reinterpret_cast<const uint32_t *>(K) + 1;  // the items' high words
+    return __clz(H[2 * k] ^ H[2 * k + 2]) >> 3;
+  } else if constexpr (kKind == kRoundItems) {
+    return ((K[k] ^ K[k + 1]) >> kb) == 0;
+  } else {
+    return __clzll((long long)(K[k] ^ K[k + 1])) >> 3;
+  }
+}
+
+// Per tile: the group heads as a bit per element (head_bits), the last head
+// (SA position) and the active (non-singleton) count of each warp span, head
+// and singleton counts.  After the first sort it also counts the group heads
+// and singletons of the prefix-1, -2, -4 (, -8) byte partitions: pstat[b*8 + q]
+// heads and pstat[b*8 + 4 + q] singletons of prefix 2^q bytes.  An element
+// heads its group of prefix P when it has fewer than P bytes in common with
+// the one before it, and is alone when the one after it has too: one count of
+// leading zeros gives all partitions (separate compares of each took 142
+// instructions per element and warp).
+template <int kKind, bool kInitial>
+__global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, int kb, const int32_t *list) {
+  __shared__ int red[2][kSortWarps];
+  constexpr int kAll = kWhole<kKind>;
+  constexpr int kQ = !kInitial ? 0 : kKind == kPrefixItems ? 3 : 4;
   const int t = tile_id(list);
   int b, lt;
   const int valid = tile_valid(d, t, d.sort_len, &b, &lt);
@@ -494,64 +530,54 @@ __global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, Layout L, int init
   const int len = d.sort_len[b];
   const int64_t off = d.off[b];
   const uint64_t *K = d.keys[keys_now(d)] + off;
-  const int32_t *P = d.kpos[d.sort_ctl[3]] + off;
   const int w = warp_id(), ln = lane_id();
+  uint32_t *bits = d.head_bits + (size_t)t * (kTile / 32) + w * kTileItems;
   int last = -1, heads = 0, sing = 0;
   int pc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 4
   for (int i = 0; i < kTileItems; i++) {
     const int e = w * kWarpSpan + i * 32 + ln;
+    const int k = lt + e;
+    bool hd = false, alone = false;
     if (e < valid) {
-      const int k = lt + e;
-      const uint64_t key = key_of(L, K[k]);
-      const uint64_t kp = k > 0 ? key_of(L, K[k - 1]) : 0;
-      const uint64_t kn = k + 1 < len ? key_of(L, K[k + 1]) : 0;
-      const bool hd = k == 0 || key != kp;
-      if (hd) {
-        const bool tl = k + 1 == len || kn != key;
-        last = max(last, initial ? k : P[k]);
-        heads++;
-        sing += tl;
-      }
+      const int p = k > 0 ? common<kKind>(K, k - 1, kb) : -1;
+      const int n = k + 1 < len ? common<kKind>(K, k, kb) : -1;
+      const int pn = max(p, n);
+      hd = p < kAll;
+      alone = pn < kAll;
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (q < nq) {
-          const int sh = key_bits - 8 * (1 << q);
-          const uint64_t a = sh > 0 ? key >> sh : key;
-          const bool h2 = k == 0 || a != (sh > 0 ? kp >> sh : kp);
-          const bool t2 = k + 1 == len || a != (sh > 0 ? kn >> sh : kn);
-          pc[q] += h2;
-          pc[4 + q] += h2 && t2;
-        }
+      for (int q = 0; q < kQ; q++) {
+        pc[q] += p < (1 << q);
+        pc[4 + q] += pn < (1 << q);
       }
     }
+    const unsigned bm = __ballot_sync(0xffffffffu, hd);
+    sing += __popc(__ballot_sync(0xffffffffu, alone));
+    heads += __popc(bm);
+    if (bm) last = k - ln + 31 - __clz(bm);
+    if (ln == 0) bits[i] = bm;
   }
-  if (nq > 0) {
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      int v = pc[q];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int q = 0; q < 8; q++) {
+    if ((q & 3) < kQ) {
+      const int v = __reduce_add_sync(0xffffffffu, pc[q]);
       if (ln == 0 && v) atomicAdd(&d.pstat[b * 8 + q], v);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
-    heads += __shfl_xor_sync(0xffffffffu, heads, o);
-    sing += __shfl_xor_sync(0xffffffffu, sing, o);
-  }
   if (ln == 0) {
     const int wvalid = min(max(valid - w * kWarpSpan, 0), kWarpSpan);
-    d.warp_last[t * kSortWarps + w] = last;
+    d.warp_last[t * kSortWarps + w] =
+        kInitial || last < 0 ? last : (d.kpos[d.sort_ctl[3]] + off)[last];
     d.warp_act[t * kSortWarps + w] = wvalid - sing;  // elements in groups of size >= 2
-    red[1][w] = heads;
-    red[2][w] = sing;
+    red[0][w] = heads;
+    red[1][w] = sing;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     int h = 0, sg = 0;
     for (int q = 0; q < kSortWarps; q++) {
-      h += red[1][q];
-      sg += red[2][q];
+      h += red[0][q];
+      sg += red[1][q];
     }
     d.tile_b[t] = h;
     d.tile_c[t] = sg;
@@ -626,8 +652,10 @@ __global__ void __launch_bounds__(256) k_bwt_rank_block(SlabDev d, int64_t prefi
 // Write SA and ISA for the sorted elements, and compact the elements of
 // groups of size >= 2 (for blocks still sorting) into the other key/value/
 // position buffers, keyed by their new head (rank of i+h added next round).
-__global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int initial, int kb,
-                                                   const int32_t *list) {
+// Heads come from head_bits: an element's group starts at the last head up to
+// it, and ends where the next element is a head.
+template <int kKind, bool kInitial>
+__global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, int kb, const int32_t *list) {
   const int t = tile_id(list);
   int b, lt;
   const int valid = tile_valid(d, t, d.sort_len, &b, &lt);
@@ -640,6 +668,7 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
   const int32_t *P = d.kpos[pc] + off;
   const bool compact = d.done[b] == 0;
   const int w = warp_id(), ln = lane_id();
+  const uint32_t *bits = d.head_bits + (size_t)t * (kTile / 32) + w * kTileItems;
   // this warp span's head carry and compaction offset (k_bwt_rank_block)
   int carry = d.warp_last[t * kSortWarps + w];
   int aoff = d.warp_act[t * kSortWarps + w];
@@ -648,38 +677,47 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
   int32_t *PO = d.kpos[pc ^ 1] + off;
   int32_t *SA = d.sa + off;
   int32_t *IS = d.isa + off;
-  const unsigned lt_mask = (1u << ln) - 1u;
+  const unsigned lt_mask = (1u << ln) - 1u, le_mask = 0xffffffffu >> (31 - ln);
   int gmax = 0;  // largest active group that ends here
-  // heads by a running max, writes, compaction
+  uint32_t bm = bits[0];
 #pragma unroll 4
   for (int i = 0; i < kTileItems; i++) {
     const int e = w * kWarpSpan + i * 32 + ln;
+    const int k = lt + e;
     const bool ok = e < valid;
-    int pos = 0, hdpos = -1;
+    const uint32_t bn = bits[i + 1];  // past the tile: the block's next tile, or not used
+    int pos = k;
     uint32_t val = 0;
-    bool active = false, last = false;
     if (ok) {
-      const int k = lt + e;
-      const uint64_t item = K[k];
-      const uint64_t key = key_of(L, item);
-      const bool hd = k == 0 || key != key_of(L, K[k - 1]);
-      const bool tl = k + 1 == len || key_of(L, K[k + 1]) != key;
-      pos = initial ? k : P[k];
-      val = L.packed ? (uint32_t)(item & ((1ull << L.low) - 1)) : V[k];
-      if (hd) hdpos = pos;
-      active = !(hd && tl);
-      last = tl && !hd;
+      if (!kInitial) pos = P[k];
+      if (kKind == kPrefixItems) val = (uint32_t)K[k];
+      else if (kKind == kRoundItems) val = (uint32_t)(K[k] & ((1ull << kb) - 1));
+      else val = V[k];
     }
-    const int head = max(carry, warp_incl_max(hdpos));
-    carry = __shfl_sync(0xffffffffu, head, 31);
+    const bool hd = (bm >> ln) & 1u;
+    const bool tl = k + 1 == len || ((__funnelshift_r(bm, bn, 1) >> ln) & 1u);
+    const bool active = ok && !(hd && tl);
+    const uint32_t below = bm & le_mask;
+    int head, next;  // up to this element, and up to the row's end
+    if (kInitial) {
+      head = below ? k - ln + 31 - __clz(below) : carry;
+      next = bm ? k - ln + 31 - __clz(bm) : carry;
+    } else {
+      head = __shfl_sync(0xffffffffu, pos, below ? 31 - __clz(below) : 0);
+      next = __shfl_sync(0xffffffffu, pos, bm ? 31 - __clz(bm) : 0);
+      if (!below) head = carry;
+      if (!bm) next = carry;
+    }
+    carry = next;
+    bm = bn;
     const unsigned am = __ballot_sync(0xffffffffu, active);
-    if (last) gmax = max(gmax, pos - head + 1);
     if (ok) {
+      if (tl && !hd) gmax = max(gmax, pos - head + 1);
       SA[pos] = (int32_t)val;
       IS[val] = head;
       if (compact && active) {
         const int r = aoff + __popc(am & lt_mask);
-        if (L.packed) {
+        if (kKind != kKeys) {
           KO[r] = ((uint64_t)(uint32_t)head << (2 * kb)) | val;
         } else {
           KO[r] = (uint64_t)(uint32_t)head << kb;
@@ -690,7 +728,7 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, Layout L, int init
     }
     aoff += __popc(am);
   }
-  if (compact && L.packed) {
+  if (compact && kKind != kKeys) {
     gmax = __reduce_max_sync(0xffffffffu, gmax);
     if (ln == 0 && gmax > 0) atomicMax(&d.gmax[b], gmax);
   }
@@ -768,12 +806,15 @@ __global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefi
 // sorted by itself: ranks within 8 items by counting the smaller ones, then
 // runs of 8, 16, .. merged, an item's place being its place in its run plus
 // the number of smaller items in the sibling run (binary search; what follows
-// a group's end is larger).  The new heads follow within the CTA, since an
+// a group's end is larger).  A warp takes part up to its
+// longest group.  The new heads follow within the CTA, since an
 // item's SA position is its group's head plus its place in the group.  About 200 instructions per rotation where
 // the radix passes, ranking and compaction of a round took about 700.
-__global__ void __launch_bounds__(256, 3) k_bwt_local(SlabDev d, int kb) {
+__global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
   __shared__ uint64_t key[kTile + 8];
-  __shared__ int red[4][kSortWarps];
+  __shared__ uint16_t gsize[kTile];           // at a group's start
+  __shared__ uint32_t starts[kTile / 32 + 1];  // bit per item: a group starts here
+  __shared__ int red[3][kSortWarps];
   __shared__ int s_base;
   const int h = d.loc_list[blockIdx.x];
   const int b = d.tile_block[h >> 1];
@@ -785,163 +826,174 @@ __global__ void __launch_bounds__(256, 3) k_bwt_local(SlabDev d, int kb) {
   const int w = warp_id(), ln = lane_id();
   const int avail = min(kTile, len - s);
   const unsigned le_mask = 0xffffffffu >> (31 - ln);
-  // items, and the first groups starting in this half tile and after it
-  int first = INT32_MAX, after = avail;
-  const int hs = 2 * kb;
-#pragma unroll
-  for (int i = 0; i < kTileItems; i++) {
-    const int e = w * kWarpSpan + i * 32 + ln;
-    if (e < avail) {
-      const uint64_t x = K[s + e];
-      key[e] = x;
-      const bool st = s + e == 0 || (K[s + e - 1] >> hs) != (x >> hs);
-      if (st) {
-        if (e < kGroupMax) first = min(first, e);
-        else after = min(after, e);
-      }
-    }
-  }
-  if (threadIdx.x < 8) key[avail + threadIdx.x] = ~0ull;
-  first = __reduce_min_sync(0xffffffffu, first);
-  after = __reduce_min_sync(0xffffffffu, after);
-  if (ln == 0) {
-    red[0][w] = first;
-    red[1][w] = after;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < kSortWarps; q++) {
-    first = min(first, red[0][q]);
-    after = min(after, red[1][q]);
-  }
-  if (first >= kGroupMax) return;  // one group from before covers the half tile
-  // [first, after): whole groups.  Each item's group start.
+  const int hs = 2 * kb;  // bits of (rank, rotation)
+  const uint64_t low = (1ull << hs) - 1, vmask = (1ull << kb) - 1;
+  const int e0 = w * kWarpSpan + ln;  // item i of this thread: e0 + 32 i
   uint64_t mine[kTileItems];
-  uint32_t gs2[kTileItems / 2];  // two 16-bit positions per register
-  int carry = -1;
+  bool before_first = false;  // thread 0: the item before the half tile is of another group
 #pragma unroll
   for (int i = 0; i < kTileItems; i++) {
-    const int e = w * kWarpSpan + i * 32 + ln;
-    const bool in = e >= first && e < after;
-    mine[i] = in ? key[e] : ~0ull;
-    const bool st = in && (e == first || (key[e - 1] >> hs) != (mine[i] >> hs));
-    const unsigned bm = __ballot_sync(0xffffffffu, st) & le_mask;
-    const int g = bm ? e - ln + 31 - __clz(bm) : carry;
-    carry = __shfl_sync(0xffffffffu, g, 31);
+    const int e = e0 + 32 * i;
+    mine[i] = e < avail ? K[s + e] : ~0ull;
+    if (e < avail) key[e] = mine[i];
+  }
+  if (threadIdx.x == 0) before_first = s == 0 || (K[s - 1] >> hs) != (mine[0] >> hs);
+  __syncthreads();
+  // group starts: the first in each of this warp's rows, and the last so far
+  uint32_t gs2[kTileItems / 2];  // two 16-bit fields per register
+  int wfirst = INT32_MAX, carry = -1;
+#pragma unroll
+  for (int i = 0; i < kTileItems; i++) {
+    const int e = e0 + 32 * i;
+    bool st = false;
+    if (e < avail) {
+      if (e == 0) st = before_first;
+      else st = (key[e - 1] >> hs) != (mine[i] >> hs);
+    }
+    const unsigned bm = __ballot_sync(0xffffffffu, st);
+    if (ln == 0) starts[e >> 5] = bm;
+    if (bm && wfirst == INT32_MAX) wfirst = e - ln + __ffs(bm) - 1;
+    const unsigned below = bm & le_mask;
+    const int g = below ? e - ln + 31 - __clz(below) : carry;
+    carry = bm ? e - ln + 31 - __clz(bm) : carry;
     if (i & 1) gs2[i >> 1] |= (uint32_t)(g & 0xffff) << 16;
     else gs2[i >> 1] = (uint32_t)(g & 0xffff);
   }
-  if (ln == 0) red[2][w] = carry;
+  if (threadIdx.x == 0) starts[kTile / 32] = 0;
+  if (ln == 0) {
+    red[0][w] = wfirst;
+    red[1][w] = carry;
+  }
   __syncthreads();
-  int before = -1;  // last group start in the earlier warps
-  for (int q = 0; q < w; q++) before = max(before, red[2][q]);
-  auto group_start = [&](int i) {
-    const uint32_t g = (i & 1) ? gs2[i >> 1] >> 16 : gs2[i >> 1] & 0xffffu;
-    return g == 0xffffu ? before : (int)g;
-  };
-  int big = 0;  // the largest place of this warp's items in their groups
-  const uint64_t low = (1ull << hs) - 1;
+  int first = INT32_MAX, after = avail, before = -1;
+#pragma unroll
+  for (int q = 0; q < kSortWarps; q++) {
+    if (q < kSortWarps / 2) first = min(first, red[0][q]);
+    else after = min(after, red[0][q]);
+    if (q < w) before = max(before, red[1][q]);
+  }
+  if (first >= kGroupMax) return;  // one group from before covers the half tile
+  // [first, after): whole groups.  Keys with the group's start in front; a
+  // group's last item leaves its size at its start.
 #pragma unroll
   for (int i = 0; i < kTileItems; i++) {
-    const int e = w * kWarpSpan + i * 32 + ln;
+    const int e = e0 + 32 * i;
+    uint32_t g = (i & 1) ? gs2[i >> 1] >> 16 : gs2[i >> 1] & 0xffffu;
+    if (g == 0xffffu) g = (uint32_t)before & 0xffffu;
+    if (i & 1) gs2[i >> 1] = (gs2[i >> 1] & 0xffffu) | (g << 16);
+    else gs2[i >> 1] = (gs2[i >> 1] & 0xffff0000u) | g;
+    const uint32_t nx = __funnelshift_r(starts[e >> 5], starts[(e >> 5) + 1], 1);
     if (e >= first && e < after) {
-      const int g = group_start(i);
-      big = max(big, e - g);
-      mine[i] = ((uint64_t)(uint32_t)g << hs) | (mine[i] & low);
+      mine[i] = ((uint64_t)g << hs) | (mine[i] & low);
       key[e] = mine[i];
+      if (((nx >> ln) & 1u) || e + 1 == after) gsize[g] = (uint16_t)(e - (int)g + 1);
     } else if (e >= after && e < avail) {
       key[e] = ~0ull;
     }
   }
+  if (threadIdx.x < 8) key[avail + threadIdx.x] = ~0ull;
   __syncthreads();
-  big = __reduce_max_sync(0xffffffffu, big);
-  if (ln == 0) red[3][w] = big;
-  // runs of 8
-  uint32_t to2[kTileItems / 2];
-#pragma unroll
-  for (int i = 0; i < kTileItems; i++) {
-    const int e = w * kWarpSpan + i * 32 + ln;
-    int to = 0;
-    if (e >= first && e < after) {
-      const int g = group_start(i);
-      const int c0 = g + ((e - g) & ~7);
-      to = c0;
-#pragma unroll
-      for (int q = 0; q < 8; q++) to += key[min(c0 + q, avail)] < mine[i];
-    }
-    if (i & 1) to2[i >> 1] |= (uint32_t)to << 16;
-    else to2[i >> 1] = (uint32_t)to;
-  }
-  __syncthreads();
+  // the fields become start | log2 of the size, rounded up, << 12
   int most = 0;
 #pragma unroll
-  for (int q = 0; q < kSortWarps; q++) most = max(most, red[3][q]);
-#pragma unroll
   for (int i = 0; i < kTileItems; i++) {
-    const int e = w * kWarpSpan + i * 32 + ln;
-    const uint32_t to = (i & 1) ? to2[i >> 1] >> 16 : to2[i >> 1] & 0xffffu;
-    if (e >= first && e < after) key[to] = mine[i];
+    const int e = e0 + 32 * i;
+    const uint32_t g = (i & 1) ? gs2[i >> 1] >> 16 : gs2[i >> 1] & 0xffffu;
+    uint32_t lg = 0;
+    if (e >= first && e < after) lg = 32 - __clz((uint32_t)gsize[g] - 1u);
+    most = max(most, (int)lg);
+    if (i & 1) gs2[i >> 1] += lg << 28;
+    else gs2[i >> 1] += lg << 12;
   }
-  __syncthreads();
-  for (int run = 8; run <= most; run <<= 1) {  // some group has more than `run` items
-    // a warp whose groups end within its first run has nothing to move; one
-    // that holds a long group's beginning sees it through the sibling's head
-    bool moves = false;
+  most = __reduce_max_sync(0xffffffffu, most);  // this warp's longest group: up to 2^most
+  if (ln == 0) red[2][w] = most;
+  auto field = [&](int i) { return (i & 1) ? gs2[i >> 1] >> 16 : gs2[i >> 1] & 0xffffu; };
+  // runs of 8
+  uint32_t to2[kTileItems / 2];
+  if (most > 0) {
 #pragma unroll
     for (int i = 0; i < kTileItems; i++) {
-      const int e = w * kWarpSpan + i * 32 + ln;
+      const int e = e0 + 32 * i;
       int to = e;
       if (e >= first && e < after) {
-        const uint64_t x = key[e];
-        mine[i] = x;
-        const int g = group_start(i);
-        const int r0 = g + ((e - g) & ~(run - 1));   // this run
-        const bool odd = (e - g) & run;
-        const int o0 = odd ? r0 - run : r0 + run;    // its sibling
-        if (o0 < after && (odd || (key[o0] >> hs) == (x >> hs))) {
-          int lo = o0, hi = min(o0 + run, after);
+        const int g = field(i) & 0xfff;
+        to = g + ((e - g) & ~7);
+        const uint64_t *c = key + to;
+#pragma unroll
+        for (int q = 0; q < 8; q++) to += c[q] < mine[i];
+      }
+      if (i & 1) to2[i >> 1] |= (uint32_t)to << 16;
+      else to2[i >> 1] = (uint32_t)to;
+    }
+  }
+  __syncthreads();
+  int all = 0;
+#pragma unroll
+  for (int q = 0; q < kSortWarps; q++) all = max(all, red[2][q]);
+  if (most > 0) {
+#pragma unroll
+    for (int i = 0; i < kTileItems; i++) {
+      const int e = e0 + 32 * i;
+      const int to = (int)((i & 1) ? to2[i >> 1] >> 16 : to2[i >> 1] & 0xffffu);
+      if (e >= first && e < after && to != e) key[to] = mine[i];
+    }
+  }
+  __syncthreads();
+  for (int l = 3; l < all; l++) {  // some group has more than 2^l items
+    const int run = 1 << l;
+    if (most > l) {
+#pragma unroll
+      for (int i = 0; i < kTileItems; i++) {
+        const int e = e0 + 32 * i;
+        int to = e;
+        const uint32_t f = field(i);
+        if (e >= first && e < after && (int)(f >> 12) > l) {
+          const uint64_t x = key[e];
+          mine[i] = x;
+          const int at = e - (int)(f & 0xfffu);
+          const bool odd = at & run;
+          const int r0 = e - (at & (run - 1));          // this run
+          int lo = odd ? r0 - run : r0 + run;           // its sibling
+          to = odd ? e - run - lo : e - lo;
+          int hi = min(lo + run, after);
           while (lo < hi) {
             const int mid = (lo + hi) >> 1;
             if (key[mid] < x) lo = mid + 1;
             else hi = mid;
           }
-          to = e + (lo - o0) - (odd ? run : 0);
-          moves = true;
+          to += lo;
         }
+        if (i & 1) to2[i >> 1] |= (uint32_t)to << 16;
+        else to2[i >> 1] = (uint32_t)to;
       }
-      if (i & 1) to2[i >> 1] |= (uint32_t)to << 16;
-      else to2[i >> 1] = (uint32_t)to;
     }
     __syncthreads();
-    if (__any_sync(0xffffffffu, moves)) {
+    if (most > l) {
 #pragma unroll
       for (int i = 0; i < kTileItems; i++) {
-        const int e = w * kWarpSpan + i * 32 + ln;
-        const uint32_t to = (i & 1) ? to2[i >> 1] >> 16 : to2[i >> 1] & 0xffffu;
-        if (e >= first && e < after && (int)to != e) key[to] = mine[i];
+        const int e = e0 + 32 * i;
+        const int to = (int)((i & 1) ? to2[i >> 1] >> 16 : to2[i >> 1] & 0xffffu);
+        if (to != e) key[to] = mine[i];
       }
     }
     __syncthreads();
   }
-  // new groups: head and rank alike
-  int32_t *SA = d.sa + off;
-  int32_t *IS = d.isa + off;
-  const uint64_t vmask = (1ull << kb) - 1;
+  // new groups: group and rank alike
   carry = -1;
   int heads = 0, sing = 0, act = 0;
   uint32_t sg2[kTileItems / 2];
 #pragma unroll
   for (int i = 0; i < kTileItems; i++) {
-    const int e = w * kWarpSpan + i * 32 + ln;
+    const int e = e0 + 32 * i;
     const bool in = e >= first && e < after;
     const uint64_t x = in ? key[e] : ~0ull;
     mine[i] = x;
     const bool hd = in && (e == first || (key[e - 1] >> kb) != (x >> kb));
-    const bool tl = in && (e + 1 == after || (key[e + 1] >> kb) != (x >> kb));
+    const bool tl = in && (key[e + 1] >> kb) != (x >> kb);
     const unsigned bm = __ballot_sync(0xffffffffu, hd);
     const unsigned below = bm & le_mask;
     const int g = below ? e - ln + 31 - __clz(below) : carry;
-    carry = __shfl_sync(0xffffffffu, g, 31);
+    carry = bm ? e - ln + 31 - __clz(bm) : carry;
     if (i & 1) sg2[i >> 1] |= (uint32_t)(g & 0xffff) << 16;
     else sg2[i >> 1] = (uint32_t)(g & 0xffff);
     const unsigned sm = __ballot_sync(0xffffffffu, hd && tl);
@@ -953,8 +1005,7 @@ __global__ void __launch_bounds__(256, 3) k_bwt_local(SlabDev d, int kb) {
   if (ln == 0) {
     red[0][w] = carry;
     red[1][w] = act;
-    red[2][w] = heads;
-    red[3][w] = sing;
+    red[2][w] = heads | sing << 16;  // at most 512 each
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -963,8 +1014,8 @@ __global__ void __launch_bounds__(256, 3) k_bwt_local(SlabDev d, int kb) {
       const int v = red[1][q];
       red[1][q] = a;
       a += v;
-      hh += red[2][q];
-      ss += red[3][q];
+      hh += red[2][q] & 0xffff;
+      ss += red[2][q] >> 16;
     }
     s_base = a ? atomicAdd(&d.loc_act[b], a) : 0;
     atomicAdd(&d.loc_heads[b], hh);
@@ -973,20 +1024,22 @@ __global__ void __launch_bounds__(256, 3) k_bwt_local(SlabDev d, int kb) {
   __syncthreads();
   int sbefore = -1;
   for (int q = 0; q < w; q++) sbefore = max(sbefore, red[0][q]);
+  int32_t *SA = d.sa + off;
+  int32_t *IS = d.isa + off;
   uint64_t *KO = d.keys[cur ^ 1] + off + s_base + red[1][w];
   const unsigned lt_mask = le_mask >> 1;
 #pragma unroll
   for (int i = 0; i < kTileItems; i++) {
-    const int e = w * kWarpSpan + i * 32 + ln;
+    const int e = e0 + 32 * i;
     const bool in = e >= first && e < after;
     const uint64_t x = mine[i];
-    const int g = group_start(i);
     const uint32_t sgv = (i & 1) ? sg2[i >> 1] >> 16 : sg2[i >> 1] & 0xffffu;
     const int sg = sgv == 0xffffu ? sbefore : (int)sgv;
+    const int g = field(i) & 0xfff;
     const int head = in ? (int)(K[s + e] >> hs) : 0;  // the list still holds the group here
     const int nhead = head + (sg - g);
     const uint32_t val = (uint32_t)(x & vmask);
-    const bool tl = in && (e + 1 == after || (key[e + 1] >> kb) != (x >> kb));
+    const bool tl = in && (key[e + 1] >> kb) != (x >> kb);
     const bool active = in && !(sg == e && tl);
     if (in) {
       SA[head + (e - g)] = (int32_t)val;
@@ -1029,23 +1082,27 @@ __global__ void __launch_bounds__(256) k_bwt_round_keys(SlabDev d, int h, int pa
   }
 }
 
-bool smem_configured = false;
+// Shared memory above the default, once per device.
+void configure_smem() {
+  static std::atomic<uint64_t> configured{0};
+  int dev = 0;
+  BZ_CUDA(cudaGetDevice(&dev));
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (bit && (configured.load(std::memory_order_acquire) & bit)) return;
+  auto room = [](auto kernel, size_t bytes) {
+    BZ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  };
+  room(k_radix_scatter<true, 8, false>, scatter_smem_vals<8>());
+  room(k_radix_scatter<false, 8, true>, scatter_smem_keys<8>());
+  room(k_radix_scatter<false, 8, false>, scatter_smem_keys<8>());
+  room(k_radix_scatter<false, 9, false>, scatter_smem_keys<9>());
+  configured.fetch_or(bit, std::memory_order_release);
+}
 
 }  // namespace
 
 void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
-  if (!smem_configured) {
-    BZ_CUDA(cudaFuncSetAttribute(k_radix_scatter<true, 8>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)scatter_smem_vals<8>()));
-    BZ_CUDA(cudaFuncSetAttribute(k_radix_scatter<false, 8>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)scatter_smem_keys<8>()));
-    BZ_CUDA(cudaFuncSetAttribute(k_radix_scatter<false, 9>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)scatter_smem_keys<9>()));
-    smem_configured = true;
-  }
+  configure_smem();
   k_bwt_init<<<(d.nblocks + 127) / 128, 128, 0, st>>>(d);
   BZ_LAUNCH_CHECK();
   if (max_m <= 1) return;
@@ -1067,8 +1124,6 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
   const int grid0 = nlive > 0 ? nlive : d.ntiles;
   const int32_t *list0 = nlive > 0 ? d.vt_list : nullptr;
   // first sort: 4-byte prefixes in the high half of packed items, or 8-byte keys
-  const Layout first = {packed, packed ? 32 : 0};
-  const Layout round = {packed, packed ? kb : 0};
   if (packed) {
     radix_sort(d, 32, 64, 0, st, grid0, list0, true);
   } else {
@@ -1082,19 +1137,24 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
   const int32_t *list = list0;
   int r = 0;  // round being run (0: the first sort)
   for (int initial = 1;; initial = 0) {
-    const Layout L = initial ? first : round;
     BZ_CUDA(cudaMemsetAsync(d.sort_ctl + 2, 0, sizeof(int32_t), st));
     BZ_CUDA(cudaMemsetAsync(d.sort_ctl + 5, 0, 3 * sizeof(int32_t), st));
     if (grid > 0) {
-      k_bwt_flags<<<grid, 256, 0, st>>>(d, L, initial, list, packed ? 32 : 64, initial ? nq : 0);
-      BZ_LAUNCH_CHECK();
-      k_bwt_rank_block<<<d.nblocks, 256, 0, st>>>(d, prefix, initial ? nq : 0);
-      BZ_LAUNCH_CHECK();
-      k_bwt_apply<<<grid, 256, 0, st>>>(d, L, initial, kb, list);
-      BZ_LAUNCH_CHECK();
+      auto rank = [&](auto flags, auto apply) {
+        flags<<<grid, 256, 0, st>>>(d, kb, list);
+        BZ_LAUNCH_CHECK();
+        k_bwt_rank_block<<<d.nblocks, 256, 0, st>>>(d, prefix, initial ? nq : 0);
+        BZ_LAUNCH_CHECK();
+        apply<<<grid, 256, 0, st>>>(d, kb, list);
+        BZ_LAUNCH_CHECK();
+      };
+      if (packed && initial) rank(k_bwt_flags<kPrefixItems, true>, k_bwt_apply<kPrefixItems, true>);
+      else if (packed) rank(k_bwt_flags<kRoundItems, false>, k_bwt_apply<kRoundItems, false>);
+      else if (initial) rank(k_bwt_flags<kKeys, true>, k_bwt_apply<kKeys, true>);
+      else rank(k_bwt_flags<kKeys, false>, k_bwt_apply<kKeys, false>);
     }
     if (lgrid > 0) {
-      k_bwt_local<<<lgrid, 256, 0, st>>>(d, kb);
+      k_bwt_groups<<<lgrid, 256, 0, st>>>(d, kb);
       BZ_LAUNCH_CHECK();
     }
     k_bwt_tile_list<<<1, 1024, 0, st>>>(d, prefix, packed);

@@ -126,6 +126,7 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     dev.vg_list = (int32_t *)alloc(((int64_t)mgt + 1) * 4);
     dev.warp_last = (int32_t *)alloc(((int64_t)mt + 1) * (kTileThreads / 32) * 4);
     dev.warp_act = (int32_t *)alloc(((int64_t)mt + 1) * (kTileThreads / 32) * 4);
+    dev.head_bits = (uint32_t *)alloc(((int64_t)mt * (kTile / 32) + 1) * 4);
     dev.tile_hist = (uint32_t *)alloc((int64_t)mt * kMaxRadix * 4);
     dev.tile_last = (int32_t *)alloc((int64_t)mt * 256 * 4);
     dev.gt_bits = (uint32_t *)alloc(((int64_t)mgt + 1) * 4);

@@ -108,6 +108,8 @@ struct SlabDev {
   // the slab's largest m, known with [0]; [4..6]: staging.
   int32_t *vt_list, *vg_list;
   int *live;
+  uint32_t *head_bits;                 // BWT: a bit per sorted element: group heads
+                                       // [ntiles * 128 + 1]
   int32_t *warp_last, *warp_act;       // BWT: per 512-element warp span [ntiles * 8]: last
                                        // head, then its carry; active count, then offset
   int64_t *active_sum;                 // A: rotations in non-singleton groups, summed over rounds
