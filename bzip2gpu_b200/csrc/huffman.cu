@@ -80,18 +80,25 @@ __global__ void k_huff_init(SlabDev d, int learned_mode) {
   init_tables(d, b);
 }
 
-// One thread per 50-symbol group.  Costs of all tables are packed in 10-bit
+// One thread per 50-symbol group, its symbols in 25 registers (two 16-bit
+// loads per symbol and pass before).  Costs of all tables are packed in 10-bit
 // fields of one 64-bit word per symbol (50 * 17 < 1024), so a group's six
-// costs are one 64-bit sum.
+// costs are one 64-bit sum.  The frequent symbols (RUNA, RUNB and the first
+// MTF indices) are counted in byte fields of a register: shared-memory adds,
+// about 1.5 a cycle and SM, bound the rest.
 // grid.y == 2 (the learned form's second passes): y = 1 runs, for the
 // learned blocks, the plain selector's second pass over its first-pass
 // tables (len2) into sel2 / rfreq2, beside y = 0's pass over len.
 // list: the group tiles to run (blockIdx.x-th entry), or nullptr for all.
+constexpr int kSymRegs = kGroupSize / 2;
+constexpr int kPadSym = kMaxAlpha;       // fills the block's last group: costs and counts nothing
+constexpr int kFreqRow = kMaxAlpha + 2;
+
 __global__ void __launch_bounds__(kGroupTile) k_huff_select(SlabDev d, int which, int round,
                                                             const int32_t *list) {
-  __shared__ uint16_t sy[kGroupTile * kGroupSize];
-  __shared__ uint64_t plen[kMaxAlpha];
-  __shared__ int rf[kMaxGroups * kMaxAlpha];
+  __shared__ __align__(16) uint32_t sy[kGroupTile * kSymRegs];  // two symbols per word
+  __shared__ uint64_t plen[kMaxAlpha + 1];
+  __shared__ int rf[kMaxGroups * kFreqRow];
   const int gt = list ? list[blockIdx.x] : (int)blockIdx.x;
   const int b = d.gt_block[gt];
   const int g0 = d.gt_first[gt];
@@ -110,21 +117,33 @@ __global__ void __launch_bounds__(kGroupTile) k_huff_select(SlabDev d, int which
   const int sym0 = g0 * kGroupSize;
   const int nsym = min(s, (g0 + ng_here) * kGroupSize) - sym0;
   const uint8_t *len = len_src + (size_t)b * kMaxGroups * kMaxAlpha;
-  for (int i = threadIdx.x; i < nsym; i += blockDim.x) sy[i] = d.rle2[off + sym0 + i];
-  for (int v = threadIdx.x; v < kMaxAlpha; v += blockDim.x) {
+  // a tile's symbols start on a 16-byte boundary (off is a multiple of kTile,
+  // 128 groups are 12,800 bytes); the buffer has slack past a block's end
+  const uint4 *src = reinterpret_cast<const uint4 *>(d.rle2 + off + sym0);
+  for (int i = threadIdx.x; i < (nsym + 7) / 8; i += blockDim.x)
+    reinterpret_cast<uint4 *>(sy)[i] = src[i];
+  for (int v = threadIdx.x; v <= kMaxAlpha; v += blockDim.x) {
     uint64_t p = 0;
     if (v < alpha)
       for (int t = 0; t < ngrp; t++) p |= (uint64_t)len[t * kMaxAlpha + v] << (10 * t);
     plen[v] = p;
   }
-  for (int i = threadIdx.x; i < kMaxGroups * kMaxAlpha; i += blockDim.x) rf[i] = 0;
+  for (int i = threadIdx.x; i < kMaxGroups * kFreqRow; i += blockDim.x) rf[i] = 0;
   __syncthreads();
   const int g = threadIdx.x;
   if (g < ng_here) {
-    const int a = g * kGroupSize;
-    const int e = min(a + kGroupSize, nsym);
+    const int n = min(kGroupSize, nsym - g * kGroupSize);
+    uint32_t v2[kSymRegs];
     uint64_t cost = 0;
-    for (int i = a; i < e; i++) cost += plen[sy[i]];
+#pragma unroll
+    for (int i = 0; i < kSymRegs; i++) {
+      v2[i] = sy[g * kSymRegs + i];
+      if (n < kGroupSize) {
+        if (2 * i >= n) v2[i] = kPadSym | kPadSym << 16;
+        else if (2 * i + 1 >= n) v2[i] = (v2[i] & 0xffffu) | kPadSym << 16;
+      }
+      cost += plen[v2[i] & 0xffffu] + plen[v2[i] >> 16];
+    }
     uint32_t bc = 0xFFFFFFFFu;
     int bt = -1;
     for (int t = 0; t < ngrp; t++) {
@@ -135,29 +154,30 @@ __global__ void __launch_bounds__(kGroupTile) k_huff_select(SlabDev d, int which
       }
     }
     sel_dst[off / 32 + g0 + g] = (uint8_t)bt;
-    // RUNA, RUNB and MTF index 1 (symbols 0, 1, 2) make up most of a block's
-    // symbols: count them in registers, so that the threads of a warp do not
-    // all add to the same few counters one symbol at a time
-    int c0 = 0, c1 = 0, c2 = 0;
-    int *rft = rf + bt * kMaxAlpha;
-    for (int i = a; i < e; i++) {
-      const int v = sy[i];
-      if (v < 3) {
-        c0 += v == 0;
-        c1 += v == 1;
-        c2 += v == 2;
-      } else {
-        atomicAdd(&rft[v], 1);
+    uint64_t hot = 0;  // byte v: symbols v < 8 (at most 50)
+    int *rft = rf + bt * kFreqRow;
+#pragma unroll
+    for (int i = 0; i < kSymRegs; i++) {
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const uint32_t v = q ? v2[i] >> 16 : v2[i] & 0xffffu;
+        if (v < 8) hot += 1ull << (8 * v);
+        else atomicAdd(&rft[v], 1);
       }
     }
-    if (c0) atomicAdd(&rft[0], c0);
-    if (c1) atomicAdd(&rft[1], c1);
-    if (c2) atomicAdd(&rft[2], c2);
+#pragma unroll
+    for (int v = 0; v < 8; v++) {
+      const int c = (int)((hot >> (8 * v)) & 0xffu);
+      if (c) atomicAdd(&rft[v], c);
+    }
   }
   __syncthreads();
   int32_t *rfreq = rf_dst + (size_t)b * kMaxGroups * kMaxAlpha;
-  for (int i = threadIdx.x; i < ngrp * kMaxAlpha; i += blockDim.x)
-    if (rf[i]) atomicAdd(&rfreq[i], rf[i]);
+  for (int t = 0; t < ngrp; t++)
+    for (int v = threadIdx.x; v < alpha; v += blockDim.x) {
+      const int c = rf[t * kFreqRow + v];
+      if (c) atomicAdd(&rfreq[t * kMaxAlpha + v], c);
+    }
 }
 
 // bzip2's length-limited Huffman lengths (src/compression/huffman.cu:13-124),
