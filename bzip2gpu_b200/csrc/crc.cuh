@@ -128,6 +128,35 @@ struct ByteCrcTable {
 };
 __device__ const ByteCrcTable c_crc_byte{};
 
+// c_crc_word.v[k][b] = crc0 of the byte b followed by k zero bytes: four
+// independent lookups take a crc0 over a 4-byte word (slicing by 4).
+struct WordCrcTable {
+  uint32_t v[4][256];
+  constexpr WordCrcTable() : v() {
+    for (int i = 0; i < 256; ++i) {
+      uint32_t c = (uint32_t)i << 24;
+      for (int k = 0; k < 4; ++k) {
+        for (int z = 0; z < 8; z++) c = (c & 0x80000000u) ? (c << 1) ^ kPoly : (c << 1);
+        v[k][i] = c;
+      }
+    }
+  }
+};
+__device__ const WordCrcTable c_crc_word{};
+
+// tbl[k][b] = c_crc_word.v[k][b] (shared memory, 256 threads; the caller
+// synchronises)
+__device__ __forceinline__ void crc_word_table_fill(uint32_t (&tbl)[4][256]) {
+  reinterpret_cast<uint4 *>(&tbl[0][0])[threadIdx.x] =
+      reinterpret_cast<const uint4 *>(&c_crc_word.v[0][0])[threadIdx.x];
+}
+
+// crc0 of what r is the crc0 of, followed by the four bytes of w (memory order)
+__device__ __forceinline__ uint32_t crc_word(uint32_t r, uint32_t w, const uint32_t (&tbl)[4][256]) {
+  const uint32_t x = r ^ __byte_perm(w, 0, 0x0123);
+  return tbl[3][x >> 24] ^ tbl[2][(x >> 16) & 0xffu] ^ tbl[1][(x >> 8) & 0xffu] ^ tbl[0][x & 0xffu];
+}
+
 // tbl[b] = crc0 of the single byte b (shared memory; the caller synchronises)
 __device__ __forceinline__ void crc_table_fill(uint32_t *tbl) {
   for (int i = threadIdx.x; i < 256; i += blockDim.x) tbl[i] = c_crc_byte.v[i];

@@ -25,43 +25,63 @@ namespace bz2g {
 namespace {
 
 
-// Stage one raw tile into shared memory: sb[0..len) = bytes, *prev = byte
-// before the tile (or -1 at the block start).
-__device__ __forceinline__ int load_raw_tile(const SlabDev &d, int t, uint8_t *sb, int *blk,
-                                             int *start, int *n_out, int *prev) {
-  int b = d.rt_block[t];
-  int st = d.rt_start[t];
-  int n = d.raw_len[b];
-  int len = min(kRawTile, n - st);
-  const uint8_t *base = d.raw + d.raw_off[b] + st;
-  int nw = (len + 15) >> 4;
-  for (int w = threadIdx.x; w < nw; w += blockDim.x)
-    reinterpret_cast<uint4 *>(sb)[w] = reinterpret_cast<const uint4 *>(base)[w];
-  *prev = st > 0 ? (int)base[-1] : -1;
-  *blk = b;
-  *start = st;
-  *n_out = n;
-  return len;
+// A thread's 16 bytes of a raw tile (positions p0 .. p0 + 15 of the tile, p0 =
+// 16 * thread): the bytes as words, the mask of run starts among them (bit k:
+// byte k lies in the tile and differs from the byte before it; a block's first
+// byte is one), and how many lie in the tile.
+struct RawBytes {
+  uint32_t w[4];
+  uint32_t starts;
+  int p0, nv;
+  int b, st, n, len;  // block, tile start in the block, block and tile length
+  const uint8_t *base;
+};
+
+__device__ __forceinline__ RawBytes raw_bytes(const SlabDev &d, int t) {
+  RawBytes r;
+  r.b = d.rt_block[t];
+  r.st = d.rt_start[t];
+  r.n = d.raw_len[r.b];
+  r.len = min(kRawTile, r.n - r.st);
+  r.base = d.raw + d.raw_off[r.b] + r.st;
+  r.p0 = threadIdx.x * kTileItems;
+  r.nv = min(kTileItems, max(0, r.len - r.p0));
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (r.nv > 0) v = reinterpret_cast<const uint4 *>(r.base)[threadIdx.x];
+  r.w[0] = v.x;
+  r.w[1] = v.y;
+  r.w[2] = v.z;
+  r.w[3] = v.w;
+  // the byte before: the neighbour lane's last, or for lane 0 from memory
+  uint32_t prev = __shfl_up_sync(0xffffffffu, v.w, 1);
+  if (lane_id() == 0 && r.nv > 0 && r.st + r.p0 > 0) prev = (uint32_t)r.base[r.p0 - 1] << 24;
+  r.starts = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    // bytes that differ from the one before: the top bit of each such byte,
+    // the four bits gathered by one multiplication
+    const uint32_t x = r.w[i] ^ __funnelshift_l(prev, r.w[i], 8);
+    const uint32_t t8 = (((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x) & 0x80808080u;
+    r.starts |= ((t8 * 0x00204081u) >> 28) << (4 * i);
+    prev = r.w[i];
+  }
+  if (r.st + r.p0 == 0) r.starts |= 1u;
+  r.starts &= (1u << r.nv) - 1u;
+  return r;
 }
 
-// The thread's 16 bytes of the staged tile (positions p0 .. p0 + 15, with
-// p0 = 16 * thread, one 16-byte shared load) and the mask of run starts among
-// them: bit k is set when byte k lies in the tile and differs from the byte
-// before it (`prev` before the tile, -1 at a block start).
-__device__ __forceinline__ uint32_t tile_bytes(const uint8_t *sb, int p0, int len, int prev,
-                                               uint8_t (&c)[kTileItems]) {
-  const uint4 v = *reinterpret_cast<const uint4 *>(sb + p0);
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int k = 0; k < kTileItems; k++) c[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
-  int pv = p0 == 0 ? prev : (int)sb[p0 - 1];
-  uint32_t starts = 0;
-#pragma unroll
-  for (int k = 0; k < kTileItems; k++) {
-    if (p0 + k < len && (int)c[k] != pv) starts |= 1u << k;
-    pv = c[k];
-  }
-  return starts;
+// A thread's position in the run chunk of the cut (259 or 255).
+__device__ __forceinline__ int mod_cut(int x, int cut) {
+  return cut == 259 ? (int)((uint32_t)x % 259u) : (int)((uint32_t)x % (uint32_t)255);
+}
+
+// Last run start in the warp before this lane (-1: none) and, in *warp_last,
+// of the whole warp, from the lanes' own last starts ls (-1: none).
+__device__ __forceinline__ int start_before(int ls, unsigned have, int *warp_last) {
+  const unsigned below = have & ((1u << lane_id()) - 1u);
+  const int v = __shfl_sync(0xffffffffu, ls, below ? 31 - __clz(below) : 0);
+  *warp_last = have ? __shfl_sync(0xffffffffu, ls, 31 - __clz(have)) : -1;
+  return below ? v : -1;
 }
 
 // Output bytes of the positions [0, n) of a run (the per-position counts
@@ -107,91 +127,70 @@ __device__ __forceinline__ void rle1_emit_masks(uint32_t sm, int q0, int nv, int
 // Per raw tile: its first and last run start, its crc0, and its RLE1 output
 // bytes from its first run start on (the bytes before it continue a run from
 // an earlier tile; the per-block kernel adds their count in closed form).
+// Bound by instructions: neighbours come by shuffle, starts by word arithmetic
+// and ballots, the CRC four bytes at a time.
 __global__ void __launch_bounds__(256) k_rle1_scan_tiles(SlabDev d) {
-  __shared__ __align__(16) uint8_t sb[kRawTile + 16];
-  __shared__ uint32_t tbl[256];
+  __shared__ __align__(16) uint32_t tbl[4][256];
   __shared__ uint32_t red4[16];
-  __shared__ int red[2][9];
-  __shared__ int scratch[40];
-  __shared__ int wl[8];
+  __shared__ int wl[8], wf[8], wc[8];
+  __shared__ uint32_t wcrc[8];
   const int t = blockIdx.x;
-  int b, st, n, prev;
-  crc_table_fill(tbl);
+  const int w = warp_id(), ln = lane_id();
+  crc_word_table_fill(tbl);
   red4_fill(red4);
-  int len = load_raw_tile(d, t, sb, &b, &st, &n, &prev);
+  const RawBytes r = raw_bytes(d, t);
+  const uint32_t sm = r.starts;
+  const int pbase = r.st + r.p0;
+  const int ls = sm ? pbase + 31 - __clz(sm) : -1;
+  const int fs = sm ? pbase + __ffs(sm) - 1 : INT32_MAX;
+  const unsigned have = __ballot_sync(0xffffffffu, sm != 0);
+  int wlast;
+  int before = start_before(ls, have, &wlast);
+  const int wfirst = __shfl_sync(0xffffffffu, fs, have ? __ffs(have) - 1 : 0);
+  if (ln == 0) {
+    wl[w] = wlast;
+    wf[w] = wfirst;
+  }
   __syncthreads();
-
-  // run starts: first and last in this tile (block-local indices)
-  const int p0 = threadIdx.x * kTileItems;
-  uint8_t c[kTileItems];
-  const uint32_t sm = tile_bytes(sb, p0, len, prev, c);
-  int first = sm ? st + p0 + __ffs(sm) - 1 : INT32_MAX;
-  int last = sm ? st + p0 + 31 - __clz(sm) : -1;
-  // block min / max
-  for (int o = 16; o > 0; o >>= 1) {
-    first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-    last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
-  }
-  if (lane_id() == 0) {
-    red[0][warp_id()] = first;
-    red[1][warp_id()] = last;
-  }
-  {
-    // output bytes: each thread's bytes from the last run start before them
-    // in this tile (positions in the run modulo the cut); bytes before the
-    // tile's first run start are left to the per-block kernel
-    const int nv = min(kTileItems, max(0, len - p0));
-    const int ls = sm ? st + p0 + 31 - __clz(sm) : -1;
-    const int inc = block_incl_max(ls, scratch, -1);
-    int ex = __shfl_up_sync(0xffffffffu, inc, 1);
-    if (lane_id() == 31) wl[warp_id()] = inc;
-    __syncthreads();
-    if (lane_id() == 0) ex = warp_id() == 0 ? -1 : wl[warp_id() - 1];
-    const int cut = d.run_cut;
-    uint32_t em, em3;
-    rle1_emit_masks(sm, ex >= 0 ? (st + p0 - ex) % cut : 0, nv, cut, ex >= 0, &em, &em3);
-    const int cnt = __popc(em) + __popc(em3);
-    int total;
-    block_excl_sum(cnt, scratch, &total);
-    if (threadIdx.x == 0) d.tile_c[t] = total;
-  }
-
+  if (before < 0)
+    for (int q = 0; q < w; q++) before = max(before, wl[q]);
+  // output bytes: each thread's bytes from the last run start before them in
+  // this tile (positions in the run modulo the cut)
+  const int cut = d.run_cut;
+  uint32_t em, em3;
+  rle1_emit_masks(sm, before >= 0 ? mod_cut(pbase - before, cut) : 0, r.nv, cut, before >= 0, &em,
+                  &em3);
+  const int cnt = __reduce_add_sync(0xffffffffu, __popc(em) + __popc(em3));
   // crc0 of the tile, right-aligned into a virtual 4096-byte tile (leading
   // zeros leave a zero-init CRC unchanged): 16 bytes per thread, each
   // thread's crc0 moved to the tile's end by one multiplication, then XOR.
-  __shared__ uint32_t wcrc[8];
-  {
-    const int pad = kRawTile - len;
-    uint32_t r = 0;
-    const int v0 = threadIdx.x * 16;
-    if (pad == 0) {
+  uint32_t c = 0;
+  if (r.len == kRawTile) {
 #pragma unroll
-      for (int k = 0; k < kTileItems; k++) r = (r << 8) ^ tbl[(r >> 24) ^ c[k]];
-    } else {
-      for (int v = max(v0, pad); v < v0 + 16; v++) {
-        uint32_t byte = sb[v - pad];
-        r = (r << 8) ^ tbl[(r >> 24) ^ byte];
-      }
-    }
-    r = gf_mul_lane(r, threadIdx.x, red4);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) r ^= __shfl_xor_sync(0xffffffffu, r, o);
-    if (lane_id() == 0) wcrc[warp_id()] = r;
+    for (int i = 0; i < 4; i++) c = crc_word(c, r.w[i], tbl);
+  } else {
+    const int pad = kRawTile - r.len;
+    for (int v = max(r.p0, pad); v < r.p0 + kTileItems; v++) c = crc_byte(c, r.base[v - pad], tbl[0]);
+  }
+  c = __reduce_xor_sync(0xffffffffu, gf_mul_lane(c, threadIdx.x, red4));
+  if (ln == 0) {
+    wc[w] = cnt;
+    wcrc[w] = c;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t r = 0;
-    for (int w = 0; w < 8; w++) r ^= wcrc[w];
-    d.tile_d[t] = (int32_t)r;  // the tile's crc0 (shifted per block)
-  }
-  if (threadIdx.x == 0) {
-    int f = INT32_MAX, l = -1;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-      f = min(f, red[0][w]);
-      l = max(l, red[1][w]);
+    int f = INT32_MAX, l = -1, total = 0;
+    uint32_t x = 0;
+    for (int q = 0; q < 8; q++) {
+      f = min(f, wf[q]);
+      l = max(l, wl[q]);
+      total += wc[q];
+      x ^= wcrc[q];
     }
     d.tile_a[t] = f;  // first run start in tile
     d.tile_b[t] = l;  // last run start in tile
+    d.tile_c[t] = total;
+    d.tile_d[t] = (int32_t)x;  // the tile's crc0 (shifted per block)
   }
 }
 
@@ -265,66 +264,87 @@ __global__ void __launch_bounds__(256) k_rle1_block_carry(SlabDev d, const int *
   }
 }
 
+// Bound by instructions like the scan: a byte of output costs a test, a byte
+// store and an add, the copy out goes by words.
 __global__ void __launch_bounds__(256) k_rle1_write(SlabDev d) {
-  __shared__ __align__(16) uint8_t sb[kRawTile + 16];
-  __shared__ __align__(16) uint8_t so[kRawTile + kRawTile / 4 + 16];  // the tile's output
-  __shared__ int scratch[40];
-  __shared__ int wl[8], wf[8];
+  // the tile's output, at the alignment it has in the block
+  __shared__ __align__(16) uint8_t so[kRawTile + kRawTile / 4 + 16];
+  __shared__ int wl[8], wf[8], wc[8];
   const int t = blockIdx.x;
-  int b, st, n, prev;
-  int len = load_raw_tile(d, t, sb, &b, &st, &n, &prev);
+  const int w = warp_id(), ln = lane_id();
+  const RawBytes r = raw_bytes(d, t);
+  const uint32_t sm = r.starts;
+  const int pbase = r.st + r.p0;  // block-local position of byte 0
+  const int ls = sm ? pbase + 31 - __clz(sm) : -1;
+  const int fs = sm ? pbase + __ffs(sm) - 1 : INT32_MAX;
+  const unsigned have = __ballot_sync(0xffffffffu, sm != 0);
+  int wlast;
+  int before = start_before(ls, have, &wlast);
+  // first start after this lane in the warp, and in the whole warp
+  const unsigned above = have & ~((2u << ln) - 1u);
+  int after = __shfl_sync(0xffffffffu, fs, above ? __ffs(above) - 1 : 0);
+  if (!above) after = INT32_MAX;
+  const int wfirst = __shfl_sync(0xffffffffu, fs, have ? __ffs(have) - 1 : 0);
+  if (ln == 0) {
+    wl[w] = wlast;
+    wf[w] = wfirst;
+  }
   __syncthreads();
-  const int p0 = threadIdx.x * kTileItems;
-  uint8_t c[kTileItems];
-  const uint32_t sm = tile_bytes(sb, p0, len, prev, c);
-  const int nv = min(kTileItems, max(0, len - p0));
-  int ls = sm ? st + p0 + 31 - __clz(sm) : -1;
-  int fs = sm ? st + p0 + __ffs(sm) - 1 : INT32_MAX;
-  // exclusive max of last starts over earlier threads
-  int inc = warp_incl_max(ls);
-  int exw = __shfl_up_sync(0xffffffffu, inc, 1);
-  if (lane_id() == 31) wl[warp_id()] = inc;
-  // exclusive min of first starts over later threads
-  int incm = warp_incl_min_rev(fs);
-  int exm = __shfl_down_sync(0xffffffffu, incm, 1);
-  if (lane_id() == 0) wf[warp_id()] = incm;
-  __syncthreads();
-  int before = lane_id() == 0 ? -1 : exw;
-  for (int w = 0; w < (int)warp_id(); w++) before = max(before, wl[w]);
-  int after = lane_id() == 31 ? INT32_MAX : exm;
-  for (int w = warp_id() + 1; w < (int)(blockDim.x >> 5); w++) after = min(after, wf[w]);
-  before = max(before, d.tile_b[t]);
-  after = min(after, d.tile_a[t]);  // next start after the tile (or n)
-
+  if (before < 0) {
+    before = d.tile_b[t];  // the last start before the tile
+    for (int q = 0; q < w; q++) before = max(before, wl[q]);
+  }
+  if (after == INT32_MAX) {
+    after = d.tile_a[t];  // next start after the tile (or n)
+    for (int q = w + 1; q < 8; q++) after = min(after, wf[q]);
+  }
   // each byte's emits: its position in its chunk from the run start before
   // the thread (one division per thread), then bit masks
   const int cut = d.run_cut;
-  const int pbase = st + p0;  // block-local position of byte 0
   uint32_t em = 0, em3 = 0;
-  if (nv > 0)
-    rle1_emit_masks(sm, before >= 0 ? (pbase - before) % cut : 0, nv, cut, before >= 0, &em, &em3);
-  int tot;
-  const int o = block_excl_sum(__popc(em) + __popc(em3), scratch, &tot);
-  uint8_t *out = so + o;
+  if (r.nv > 0)
+    rle1_emit_masks(sm, before >= 0 ? mod_cut(pbase - before, cut) : 0, r.nv, cut, before >= 0, &em,
+                    &em3);
+  const int cnt = __popc(em) + __popc(em3);
+  const int inc = warp_incl_sum(cnt);
+  if (ln == 31) wc[w] = inc;
+  __syncthreads();
+  int o = inc - cnt, tot = 0;
 #pragma unroll
-  for (int k = 0; k < kTileItems; k++) {
-    if ((em >> k) & 1u) {
-      const uint32_t below = (1u << k) - 1u;
-      const int at = __popc(em & below) + __popc(em3 & below);
-      out[at] = c[k];
-      if ((em3 >> k) & 1u) {
-        // the chunk's length: from its start (3 bytes back) to the run's end
-        // or the cut, whichever comes first
-        const uint32_t rest = k + 1 < kTileItems ? sm >> (k + 1) : 0u;
-        const int run_end = rest ? pbase + k + __ffs(rest) : after;
-        out[at + 1] = (uint8_t)(min(cut, run_end - (pbase + k - 3)) - 4);
+  for (int q = 0; q < 8; q++) {
+    const int c = wc[q];
+    if (q < w) o += c;
+    tot += c;
+  }
+  uint8_t *dst = d.rle1 + d.off[r.b] + d.tile_c[t];
+  const int lead = (int)(reinterpret_cast<uintptr_t>(dst) & 3u);
+  if (__any_sync(0xffffffffu, em)) {
+    uint8_t *out = so + lead + o;
+#pragma unroll
+    for (int k = 0; k < kTileItems; k++) {
+      if ((em >> k) & 1u) {
+        *out++ = (uint8_t)(r.w[k >> 2] >> (8 * (k & 3)));
+        if ((em3 >> k) & 1u) {
+          // the chunk's length: from its start (3 bytes back) to the run's end
+          // or the cut, whichever comes first
+          const uint32_t rest = k + 1 < kTileItems ? sm >> (k + 1) : 0u;
+          const int run_end = rest ? pbase + k + __ffs(rest) : after;
+          *out++ = (uint8_t)(min(cut, run_end - (pbase + k - 3)) - 4);
+        }
       }
     }
   }
   __syncthreads();
-  // coalesced copy of the tile's output to its place in the block
-  uint8_t *dst = d.rle1 + d.off[b] + d.tile_c[t];
-  for (int i = threadIdx.x; i < tot; i += blockDim.x) dst[i] = so[i];
+  // the tile's output to its place in the block, by words where they are whole
+  dst -= lead;
+  const int end = lead + tot;
+  for (int i = 4 * threadIdx.x; i < end; i += 4 * 256) {
+    if (i >= lead && i + 4 <= end) {
+      *reinterpret_cast<uint32_t *>(dst + i) = *reinterpret_cast<const uint32_t *>(so + i);
+    } else {
+      for (int q = max(i, lead); q < min(i + 4, end); q++) dst[q] = so[q];
+    }
+  }
 }
 
 }  // namespace
