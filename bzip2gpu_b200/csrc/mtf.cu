@@ -55,11 +55,18 @@ __global__ void __launch_bounds__(256) k_mtf_block_scan(SlabDev d) {
   const int nt = (m + kTile - 1) / kTile;
   const int t0 = (int)(d.off[b] / kTile);
   int carry = -1;
-  for (int k = 0; k < nt; k++) {
-    size_t idx = (size_t)(t0 + k) * 256 + threadIdx.x;
-    int v = d.tile_last[idx];
-    d.tile_last[idx] = carry;
-    carry = max(carry, v);
+  // sixteen tiles' loads in flight at a time
+  constexpr int kU = 16;
+  int32_t *p = d.tile_last + (size_t)t0 * 256 + threadIdx.x;
+  for (int k0 = 0; k0 < nt; k0 += kU) {
+    int v[kU];
+#pragma unroll
+    for (int j = 0; j < kU; j++) v[j] = k0 + j < nt ? p[(size_t)(k0 + j) * 256] : -1;
+#pragma unroll
+    for (int j = 0; j < kU; j++) {
+      if (k0 + j < nt) p[(size_t)(k0 + j) * 256] = carry;
+      carry = max(carry, v[j]);
+    }
   }
   if (threadIdx.x == 0) {
     int n = 0;

@@ -24,56 +24,92 @@ __device__ __forceinline__ int tile_len(const SlabDev &d, int t, int *b, int *lt
 
 __device__ __forceinline__ int n_digits(int k) { return 31 - __clz(k + 1); }
 
-// Thread-blocked view of a tile: each thread owns kTileItems consecutive
-// positions and learns the previous / next non-zero around each of them.
-struct ZeroRuns {
-  int before, after;
-};
-
-// The thread's 16 MTF values (one 16-byte load; the buffer has slack past
-// a block's end, and values at or past `valid` are not used).
+// A thread's 16 MTF values (one 16-byte load; the buffer has slack past a
+// block's end): the mask of non-zero ones, how many lie in the tile, and the
+// non-zeros nearest before and after them in the tile (block positions; -1 and
+// INT32_MAX when there are none).
 struct Values16 {
   uint32_t w[4];
-  __device__ __forceinline__ int operator[](int k) const { return (w[k >> 2] >> (8 * (k & 3))) & 0xff; }
+  uint32_t nz;
+  int nv, pos;  // pos: block position of value 0
+  int before, after;
+  int wlast, wfirst;  // the warp's last and first non-zero
 };
-__device__ __forceinline__ void load_values(const uint8_t *V, int lt, int p0, int valid,
-                                            Values16 &v) {
-  uint4 w = make_uint4(0, 0, 0, 0);
-  if (p0 < valid) w = *reinterpret_cast<const uint4 *>(V + lt + p0);
-  v.w[0] = w.x;
-  v.w[1] = w.y;
-  v.w[2] = w.z;
-  v.w[3] = w.w;
+
+__device__ __forceinline__ Values16 values16(const uint8_t *V, int lt, int valid) {
+  Values16 v;
+  const int p0 = threadIdx.x * kTileItems;
+  v.nv = min(kTileItems, max(0, valid - p0));
+  v.pos = lt + p0;
+  uint4 x = make_uint4(0, 0, 0, 0);
+  if (v.nv > 0) x = *reinterpret_cast<const uint4 *>(V + lt + p0);
+  v.w[0] = x.x;
+  v.w[1] = x.y;
+  v.w[2] = x.z;
+  v.w[3] = x.w;
+  v.nz = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    // the top bit of each non-zero byte, gathered by one multiplication
+    const uint32_t t8 = (((v.w[i] & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v.w[i]) & 0x80808080u;
+    v.nz |= ((t8 * 0x00204081u) >> 28) << (4 * i);
+  }
+  v.nz &= (1u << v.nv) - 1u;
+  return v;
 }
 
-// carry: include the non-zeros of the other tiles (tile_b / tile_a after the
-// per-block kernel); without it, -1 / INT32_MAX when the tile has none.
-__device__ __forceinline__ ZeroRuns zero_run_bounds(const SlabDev &d, const Values16 &v,
-                                                    int t, int lt, int valid, int p0, int *wl,
-                                                    int *wf, bool carry = true) {
-  int ls = -1, fs = INT32_MAX;
-#pragma unroll
-  for (int k = kTileItems - 1; k >= 0; k--) {
-    if (p0 + k < valid && v[k] != 0) {
-      ls = max(ls, lt + p0 + k);
-      fs = lt + p0 + k;
+// The non-zeros around each thread's values, within the tile (256 threads).
+__device__ __forceinline__ void zero_bounds(Values16 &v, int *wl, int *wf) {
+  const unsigned full = 0xffffffffu;
+  const int ln = lane_id(), w = warp_id();
+  const int ls = v.nz ? v.pos + 31 - __clz(v.nz) : -1;
+  const int fs = v.nz ? v.pos + __ffs(v.nz) - 1 : INT32_MAX;
+  const unsigned have = __ballot_sync(full, v.nz != 0);
+  const unsigned below = have & ((1u << ln) - 1u), above = have & ~((2u << ln) - 1u);
+  v.before = __shfl_sync(full, ls, below ? 31 - __clz(below) : 0);
+  v.after = __shfl_sync(full, fs, above ? __ffs(above) - 1 : 0);
+  if (!below) v.before = -1;
+  if (!above) v.after = INT32_MAX;
+  v.wlast = have ? __shfl_sync(full, ls, 31 - __clz(have)) : -1;
+  v.wfirst = have ? __shfl_sync(full, fs, __ffs(have) - 1) : INT32_MAX;
+  if (ln == 0) {
+    wl[w] = v.wlast;
+    wf[w] = v.wfirst;
+  }
+  __syncthreads();
+  if (v.before < 0)
+    for (int q = 0; q < w; q++) v.before = max(v.before, wl[q]);
+  if (v.after == INT32_MAX)
+    for (int q = w + 1; q < 8; q++) v.after = min(v.after, wf[q]);
+}
+
+// The run digits among a thread's values, zero run by zero run: which zeros
+// emit one (bit mask), and the digits (bit mask).  A run of k zeros from zs on
+// emits digit q at zs + q for q < n_digits(k); digit q is bit q of k + 1.
+// kTileOnly: v's bounds are the tile's, and runs that may start before it
+// (before < 0) or end after it (after INT32_MAX) are left out.
+template <bool kTileOnly>
+__device__ __forceinline__ void run_digits(const Values16 &v, uint32_t *emit, uint32_t *digits) {
+  uint32_t z = ~v.nz & ((1u << v.nv) - 1u);
+  uint32_t em = 0, dg = 0;
+  while (z) {
+    const int a = __ffs(z) - 1;
+    const int n = __ffs(~(z >> a)) - 1;
+    const uint32_t span = ((1u << n) - 1u) << a;
+    z &= ~span;
+    const int end = a + n >= v.nv ? v.after : v.pos + a + n;
+    if (kTileOnly && ((a == 0 && v.before < 0) || end == INT32_MAX)) continue;
+    const int q = a == 0 ? v.pos - v.before - 1 : 0;  // the run's zeros before position a
+    const int k = end - (v.pos + a - q);
+    const int c = min(n_digits(k) - q, n);
+    if (c > 0) {
+      const uint32_t m = (1u << c) - 1u;
+      em |= m << a;
+      dg |= (((uint32_t)(k + 1) >> q) & m) << a;
     }
   }
-  int inc = warp_incl_max(ls);
-  int exw = __shfl_up_sync(0xffffffffu, inc, 1);
-  if (lane_id() == 31) wl[warp_id()] = inc;
-  int incm = warp_incl_min_rev(fs);
-  int exm = __shfl_down_sync(0xffffffffu, incm, 1);
-  if (lane_id() == 0) wf[warp_id()] = incm;
-  __syncthreads();
-  int before = lane_id() == 0 ? -1 : exw;
-  for (int w = 0; w < (int)warp_id(); w++) before = max(before, wl[w]);
-  int after = lane_id() == 31 ? INT32_MAX : exm;
-  for (int w = warp_id() + 1; w < (int)(blockDim.x >> 5); w++) after = min(after, wf[w]);
-  ZeroRuns r;
-  r.before = carry ? max(before, d.tile_b[t]) : before;
-  r.after = carry ? min(after, d.tile_a[t]) : after;
-  return r;
+  *emit = em;
+  *digits = dg;
 }
 
 // Per tile: first and last non-zero (tile_a, tile_b, and the first again in
@@ -82,55 +118,24 @@ __device__ __forceinline__ ZeroRuns zero_run_bounds(const SlabDev &d, const Valu
 // counted by the per-block kernel, which knows where they start and end.
 __global__ void __launch_bounds__(256) k_rle2_scan_tiles(SlabDev d, const int32_t *list) {
   const int t = list ? list[blockIdx.x] : (int)blockIdx.x;
-  __shared__ int scratch[40];
-  __shared__ int wl[8], wf[8];
-  __shared__ int red[2][8];
+  __shared__ int wl[8], wf[8], wc[8];
   int b, lt, m;
   int64_t off;
   int valid = tile_len(d, t, &b, &lt, &off, &m);
   if (valid <= 0) return;
-  const int p0 = threadIdx.x * kTileItems;
-  Values16 v;
-  load_values(d.mtf + off, lt, p0, valid, v);
-  ZeroRuns zr = zero_run_bounds(d, v, t, lt, valid, p0, wl, wf, false);
-  uint32_t nzm = 0;
-#pragma unroll
-  for (int k = 0; k < kTileItems; k++) nzm |= (p0 + k < valid && v[k] != 0) ? 1u << k : 0u;
-  int cnt = __popc(nzm);
-  int prev_nz = zr.before;
-#pragma unroll
-  for (int k = 0; k < kTileItems; k++) {
-    if (p0 + k < valid) {
-      if ((nzm >> k) & 1u) {
-        prev_nz = lt + p0 + k;
-      } else if (prev_nz >= 0) {
-        const uint32_t rest = k + 1 < kTileItems ? nzm >> (k + 1) : 0u;
-        const int end = rest ? lt + p0 + k + __ffs(rest) : zr.after;
-        if (end != INT32_MAX) {
-          const int zs = prev_nz + 1;
-          cnt += (lt + p0 + k - zs) < n_digits(end - zs) ? 1 : 0;
-        }
-      }
-    }
-  }
-  int tot;
-  block_excl_sum(cnt, scratch, &tot);
-  int first = nzm ? lt + p0 + __ffs(nzm) - 1 : INT32_MAX;
-  int last = nzm ? lt + p0 + 31 - __clz(nzm) : -1;
-  for (int o = 16; o > 0; o >>= 1) {
-    first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-    last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
-  }
-  if (lane_id() == 0) {
-    red[0][warp_id()] = first;
-    red[1][warp_id()] = last;
-  }
+  Values16 v = values16(d.mtf + off, lt, valid);
+  zero_bounds(v, wl, wf);
+  uint32_t em, dg;
+  run_digits<true>(v, &em, &dg);
+  const int cnt = __reduce_add_sync(0xffffffffu, __popc(v.nz) + __popc(em));
+  if (lane_id() == 0) wc[warp_id()] = cnt;
   __syncthreads();
   if (threadIdx.x == 0) {
-    int f = INT32_MAX, l = -1;
+    int f = INT32_MAX, l = -1, tot = 0;
     for (int w = 0; w < 8; w++) {
-      f = min(f, red[0][w]);
-      l = max(l, red[1][w]);
+      f = min(f, wf[w]);
+      l = max(l, wl[w]);
+      tot += wc[w];
     }
     d.tile_a[t] = f;
     d.tile_b[t] = l;
@@ -227,85 +232,71 @@ __global__ void __launch_bounds__(256) k_rle2_block_carry(SlabDev d) {
   }
 }
 
+// The tile's symbols are assembled in shared memory, at the alignment they have
+// in the block, and copied out by words.
 __global__ void __launch_bounds__(256) k_rle2_write(SlabDev d, const int32_t *list) {
   const int t = list ? list[blockIdx.x] : (int)blockIdx.x;
-  __shared__ int scratch[40];
-  __shared__ int wl[8], wf[8];
+  __shared__ int wl[8], wf[8], wc[8];
   __shared__ int hist[kMaxAlpha];
+  __shared__ __align__(16) uint16_t so[kTile + 8];
   int b, lt, m;
   int64_t off;
   int valid = tile_len(d, t, &b, &lt, &off, &m);
   if (valid <= 0) return;
   for (int i = threadIdx.x; i < kMaxAlpha; i += blockDim.x) hist[i] = 0;
-  const uint8_t *V = d.mtf + off;
-  const int p0 = threadIdx.x * kTileItems;
-  Values16 v;
-  load_values(V, lt, p0, valid, v);
-  ZeroRuns zr = zero_run_bounds(d, v, t, lt, valid, p0, wl, wf);
-  // non-zero values as a mask; the end of the zero run holding value k is
-  // the next non-zero after it
-  uint32_t nzm = 0;
+  Values16 v = values16(d.mtf + off, lt, valid);
+  zero_bounds(v, wl, wf);
+  v.before = max(v.before, d.tile_b[t]);
+  v.after = min(v.after, d.tile_a[t]);
+  uint32_t em, dg;
+  run_digits<false>(v, &em, &dg);
+  const int cnt = __popc(v.nz) + __popc(em);
+  const int inc = warp_incl_sum(cnt);
+  if (lane_id() == 31) wc[warp_id()] = inc;
+  __syncthreads();
+  int o = inc - cnt, tot = 0;
 #pragma unroll
-  for (int k = 0; k < kTileItems; k++) nzm |= (p0 + k < valid && v[k] != 0) ? 1u << k : 0u;
-  auto run_end = [&](int k) {
-    const uint32_t rest = k + 1 < kTileItems ? nzm >> (k + 1) : 0u;
-    return rest ? lt + p0 + k + __ffs(rest) : zr.after;
-  };
-  int cnt = 0;
-  {
-    int prev_nz = zr.before;
-#pragma unroll
-    for (int k = 0; k < kTileItems; k++) {
-      int e = p0 + k;
-      if (e < valid) {
-        if (v[k] != 0) {
-          cnt++;
-          prev_nz = lt + e;
-        } else {
-          int zs = prev_nz + 1;
-          cnt += (lt + e - zs) < n_digits(run_end(k) - zs) ? 1 : 0;
-        }
-      }
-    }
+  for (int q = 0; q < 8; q++) {
+    const int c = wc[q];
+    if (q < (int)warp_id()) o += c;
+    tot += c;
   }
-  int tot;
-  int o = block_excl_sum(cnt, scratch, &tot);
-  uint16_t *out = d.rle2 + off + d.tile_c[t] + o;
-  int prev_nz = zr.before;
-  // RUNA, RUNB and symbol 2 (MTF index 1) are most of the symbols: counted
-  // in registers, added to the tile's histogram once per thread
-  int h0 = 0, h1 = 0, h2 = 0;
+  const int64_t at = off + d.tile_c[t];
+  const int lead = (int)(at & 1);
+  uint16_t *out = so + lead + o;
+  // the frequent symbols are counted in registers (RUNA and RUNB by their
+  // masks, symbols 2 .. 7 in byte fields), added to the tile's histogram once
+  // per thread
+  const int h1 = __popc(dg & em), h0 = __popc(em) - h1;
+  uint64_t hot = 0;
+  const uint32_t any = v.nz | em;
 #pragma unroll
   for (int k = 0; k < kTileItems; k++) {
-    int e = p0 + k;
-    if (e < valid) {
-      const int x = v[k];
-      if (x != 0) {
-        *out++ = (uint16_t)(x + 1);
-        if (x == 1)
-          h2++;
-        else
-          atomicAdd(&hist[x + 1], 1);
-        prev_nz = lt + e;
-      } else {
-        int zs = prev_nz + 1;
-        int q = lt + e - zs;
-        int k2 = run_end(k) - zs;
-        if (q < n_digits(k2)) {
-          // digit q of the run length in bijective base 2 (RUNA = 0 for 1,
-          // RUNB = 1 for 2) is bit q of length + 1
-          const int dgt = ((k2 + 1) >> q) & 1;
-          *out++ = (uint16_t)dgt;
-          h0 += dgt == 0;
-          h1 += dgt == 1;
-        }
-      }
+    if ((any >> k) & 1u) {
+      const uint32_t x = (v.w[k >> 2] >> (8 * (k & 3))) & 0xffu;
+      const uint32_t sym = x ? x + 1 : (dg >> k) & 1u;
+      *out++ = (uint16_t)sym;
+      if (sym < 8) hot += 1ull << (8 * sym);
+      else atomicAdd(&hist[sym], 1);
     }
   }
   if (h0) atomicAdd(&hist[0], h0);
   if (h1) atomicAdd(&hist[1], h1);
-  if (h2) atomicAdd(&hist[2], h2);
+#pragma unroll
+  for (int q = 2; q < 8; q++) {
+    const int c = (int)((hot >> (8 * q)) & 0xffu);
+    if (c) atomicAdd(&hist[q], c);
+  }
   __syncthreads();
+  uint32_t *dst = reinterpret_cast<uint32_t *>(d.rle2 + at - lead);
+  const int end = lead + tot;
+  for (int i = threadIdx.x; 2 * i < end; i += 256) {
+    if (2 * i >= lead && 2 * i + 2 <= end) {
+      dst[i] = reinterpret_cast<const uint32_t *>(so)[i];
+    } else {
+      for (int q = max(2 * i, lead); q < min(2 * i + 2, end); q++) d.rle2[at - lead + q] = so[q];
+    }
+  }
   for (int i = threadIdx.x; i < kMaxAlpha; i += blockDim.x)
     if (hist[i]) atomicAdd(&d.freq[b * kMaxAlpha + i], hist[i]);
 }
