@@ -155,7 +155,8 @@ struct DecBlock {
 // Entropy decode of one block, split so that only the group starts are a
 // serial chain (a code's length is known only once its start is):
 //   k_dec_head    header, selectors, code tables           (a CTA per block)
-//   k_dec_groups  bit position of every 50-symbol group    (a warp per block)
+//   k_dec_groups  bit position of every 50-symbol group    (a CTA per block), or
+//   k_dec_lens, _jumps, _starts the same, for few blocks
 //   k_dec_syms    the groups' symbols, a thread each, and the inverse
 //                 move-to-front of 32 groups (a chunk) from an unknown
 //                 starting list                            (a warp per chunk)
@@ -174,7 +175,7 @@ struct DecTab {
   int64_t pay;  // bit position of the first symbol
   int32_t status, nuse, ng, nsel, orig_ptr;
   uint32_t crc;
-  int32_t ngv;  // groups whose start is known
+  int32_t ngv;  // groups whose start is known (-1: not yet looked for)
   uint8_t mn[kDecMaxGroups], mx[kDecMaxGroups];
   uint32_t lj[kDecMaxGroups][kDecMaxCode + 4];
   int32_t base[kDecMaxGroups][kDecMaxCode + 4];  // code - base = index into perm
@@ -245,6 +246,88 @@ __device__ __forceinline__ uint32_t sel_then(uint32_t a, uint32_t b) {
   for (int k = 0; k < kDecMaxGroups; k++)
     r |= ((a >> (4 * ((b >> (4 * k)) & 0xFu))) & 0xFu) << (4 * k);
   return r;
+}
+
+// A table's code lengths by one warp: a 5-bit start, then per symbol steps 1x
+// (x = 0: +1, x = 1: -1) and a 0.  A lane takes 32 bits; whether it starts
+// inside a step follows from the bits before it (a 0 always ends what it is
+// in; after ones only, their number decides), then scans over the lanes give
+// each one's symbol and length so far.  Every length on the way must lie in
+// 1 .. kDecMaxCode, and a symbol takes at most 63 steps.  p: the table's
+// first bit; moved past it.  (One thread bit by bit: 150 us for six tables.)
+__device__ int code_lengths(const uint32_t *words, int64_t nwords, int64_t &p, int alpha,
+                            uint8_t *len) {
+  const unsigned full = 0xffffffffu;
+  const int ln = lane_id();
+  int cur0 = (int)(bits_at(words, nwords, p) >> 27);
+  p += 5;
+  int64_t last_end = p;  // where the symbol being read began
+  int done = 0;
+  uint32_t inside = 0;   // the round starts inside a step
+  for (;;) {
+    const uint32_t x = bits_at(words, nwords, p + 32 * ln);
+    const int ones = x == full ? 32 : __ffs(~x) - 1;  // at the word's end
+    const unsigned broken = __ballot_sync(full, x != full);
+    const unsigned odd = __ballot_sync(full, ones & 1);
+    const unsigned below = broken & ((1u << ln) - 1u);
+    const uint32_t in = below ? (odd >> (31 - __clz(below))) & 1u : inside;
+    uint32_t s = in;
+    int ends = 0, sum = 0, end_at = -1;
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+      const bool one = (x >> (31 - i)) & 1u;
+      if (s) {
+        sum += one ? -1 : 1;
+        s = 0;
+      } else if (one) {
+        s = 1;
+      } else {
+        ends++;
+        end_at = i;
+      }
+    }
+    const int esum = warp_incl_sum(ends), dsum = warp_incl_sum(sum);
+    const unsigned has = __ballot_sync(full, ends > 0);
+    const unsigned hb = has & ((1u << ln) - 1u);
+    const int pe = __shfl_sync(full, 32 * ln + end_at + 1, hb ? 31 - __clz(hb) : 0);
+    int64_t began = hb ? p + pe : last_end;
+    int sym = done + esum - ends;
+    int cur = cur0 + dsum - sum;
+    bool bad = sym < alpha && (cur < 1 || cur > kDecMaxCode);
+    int fin = -1;
+    s = in;
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+      const bool one = (x >> (31 - i)) & 1u;
+      if (s) {
+        cur += one ? -1 : 1;
+        s = 0;
+        if (sym < alpha) bad |= cur < 1 || cur > kDecMaxCode;
+      } else if (one) {
+        s = 1;
+      } else {
+        if (sym < alpha) {
+          const int64_t at = p + 32 * ln + i;
+          bad |= at - began > 2 * 63;
+          began = at + 1;
+          len[sym] = (uint8_t)cur;
+          if (sym == alpha - 1) fin = i;
+        }
+        sym++;
+      }
+    }
+    if (__any_sync(full, bad) || !has) return kDecBadTables;
+    const unsigned fm = __ballot_sync(full, fin >= 0);
+    if (fm) {
+      p += __shfl_sync(full, 32 * ln + fin + 1, __ffs(fm) - 1);
+      return kDecOk;
+    }
+    done += __shfl_sync(full, esum, 31);
+    cur0 += __shfl_sync(full, dsum, 31);
+    last_end = p + __shfl_sync(full, 32 * ln + end_at + 1, 31 - __clz(has));
+    inside = __shfl_sync(full, s, 31);
+    p += 1024;
+  }
 }
 
 // Header, selectors and tables of a candidate block.
@@ -346,40 +429,14 @@ __global__ void __launch_bounds__(kHeadThreads) k_dec_head(const uint32_t *words
       lst = sel_front(lst, sj[i]);
       sel[i] = (uint8_t)(lst & 0xFu);
     }
-    // code lengths: 5-bit start, then per symbol 1x (x=0: +1, x=1: -1), 0 ends
-    if (threadIdx.x == 0) {
-      br.init(words, nwords, s_end);
+    if (w == 0) {
+      int64_t p = s_end;
       int st = kDecOk;
-      for (int t = 0; t < ng && st == kDecOk; t++) {
-        int cur = (int)br.get(5);
-        for (int v = 0; v < alpha; v++) {
-          uint32_t x = br.peek32();
-          int used = 0, steps = 0;
-          for (;;) {
-            if (cur < 1 || cur > kDecMaxCode || ++steps > 64) {
-              st = kDecBadTables;
-              break;
-            }
-            if (!(x >> 31)) {
-              used++;
-              break;
-            }
-            cur += (x & 0x40000000u) ? -1 : 1;
-            x <<= 2;
-            used += 2;
-            if (used >= 30) {
-              br.skip(used);
-              used = 0;
-              x = br.peek32();
-            }
-          }
-          if (st != kDecOk) break;
-          br.skip(used);
-          len[t][v] = (uint8_t)cur;
-        }
+      for (int t = 0; t < ng && st == kDecOk; t++) st = code_lengths(words, nwords, p, alpha, len[t]);
+      if (ln == 0) {
+        s_status = st;
+        tab.pay = p;
       }
-      s_status = st;
-      tab.pay = br.pos();
     }
     __syncthreads();
     status = s_status;
@@ -449,7 +506,7 @@ __global__ void __launch_bounds__(kHeadThreads) k_dec_head(const uint32_t *words
     tab.nsel = nsel;
     tab.orig_ptr = orig_ptr;
     tab.crc = crc;
-    tab.ngv = 0;
+    tab.ngv = -1;
   }
 }
 
@@ -490,7 +547,7 @@ __global__ void __launch_bounds__(32 * NW)
   const int bi = order[blockIdx.x];  // largest compressed blocks first
   const int tid = threadIdx.x, ln = lane_id();
   DecTab &tab = tabs[bi];
-  if (tab.status != kDecOk) return;
+  if (tab.status != kDecOk || tab.ngv >= 0) return;  // bad header, or done by k_dec_starts
   const int ng = tab.ng, nsel = tab.nsel;
   for (int i = tid; i < ng * (kDecMaxCode + 4); i += NT) (&lj[0][0])[i] = (&tab.lj[0][0])[i];
   if (tid < ng) {
@@ -629,6 +686,183 @@ __global__ void __launch_bounds__(32 * NW)
     }
   }
   if (tid == 0) tab.ngv = g;
+}
+
+// Few blocks: the jump over a whole group (50 codes) from every bit position
+// with every table, then the chain of group starts is one lookup per group.
+// k_dec_jumps covers kJumpTile positions of a block per CTA: code lengths of
+// the tile and a halo (50 codes take at most 1000 bits), the map squared five
+// times in shared memory, composed to 32 + 16 + 2 codes.  k_dec_starts streams
+// a block's tiles through four buffers and hops.  This takes about 36
+// instructions per position and table, a hundred times what the chain of
+// k_dec_groups needs, but nothing of it waits: 0.1 ms and 0.3 ms for one block,
+// where k_dec_groups takes 3.4 ms.  Positions are relative to the block's magic.
+constexpr int kJumpTile = 4096;
+constexpr int kJumpHalo = 1024;
+constexpr int kJumpAll = kJumpTile + kJumpHalo;
+constexpr int kJumpPer = kJumpAll / 256;             // positions per thread
+constexpr uint32_t kJumpOut = kJumpAll + 32;         // leaves the tile and halo
+constexpr uint32_t kJumpDead = kJumpAll + 33;        // no code starts here
+constexpr int kJumpSlots = kJumpAll + 34;
+constexpr uint32_t kDeadJump = 0xFFFFu;
+constexpr int kLensBytes = kDecMaxGroups << kLenBits;
+constexpr size_t kJumpSmem = (size_t)3 * kJumpSlots * 2 + (1 << kLenBits) + 64;
+constexpr int kStartStages = 4;  // tiles in flight: 48 KB each
+constexpr size_t kStartStage = (size_t)kDecMaxGroups * kJumpTile * 2;
+constexpr size_t kStartsSmem = kStartStages * kStartStage;
+// Compressed bits of a batch up to which the jumps are used: their work grows
+// with the bits of all blocks (about 17 us per 1.4 Mbit block), while
+// k_dec_groups takes the time of its longest block (3.4 ms for such a block)
+// until the blocks fill the GPU.
+constexpr int64_t kJumpMaxBits = 200 << 20;
+
+// Code length (0: longer than kLenBits, or none) by the next kLenBits bits.
+// grid: (table, block)
+__global__ void __launch_bounds__(256) k_dec_lens(const DecTab *tabs, uint8_t *lens) {
+  const int bi = blockIdx.y, t = blockIdx.x;
+  const DecTab &tab = tabs[bi];
+  if (tab.status != kDecOk || t >= tab.ng) return;
+  uint8_t *out = lens + (size_t)bi * kLensBytes + ((size_t)t << kLenBits);
+  const int mn = tab.mn[t], mx = min((int)tab.mx[t], kLenBits);
+  for (int p = threadIdx.x; p < (1 << kLenBits); p += 256) {
+    const uint32_t x = (uint32_t)p << (32 - kLenBits);
+    int n = mn;
+    while (n <= mx && x > tab.lj[t][n]) n++;
+    out[p] = (uint8_t)(n <= mx ? n : 0);
+  }
+}
+
+// jt0: first tile of each block among all blocks' (jt0[nc]: their number).
+// jumps: per tile, per table, kJumpTile advances, twice the bits (table bytes;
+// kDeadJump: none).
+__global__ void __launch_bounds__(256) k_dec_jumps(const uint32_t *words, int64_t nwords,
+                                                   const int64_t *cand, const DecTab *tabs,
+                                                   const uint8_t *lens, const int32_t *jt0,
+                                                   uint16_t *jumps) {
+  extern __shared__ __align__(16) uint8_t jsm[];
+  uint16_t *A = reinterpret_cast<uint16_t *>(jsm), *B = A + kJumpSlots, *C = B + kJumpSlots;
+  uint8_t *llen = reinterpret_cast<uint8_t *>(
+      (reinterpret_cast<uintptr_t>(C + kJumpSlots) + 15) & ~(uintptr_t)15);
+  __shared__ uint32_t bits[kJumpAll / 32 + 2];
+  __shared__ uint32_t lj[kDecMaxCode + 4];
+  const int bi = blockIdx.y;
+  const int tile = jt0[bi] + blockIdx.x;
+  if (tile >= jt0[bi + 1]) return;
+  const DecTab &tab = tabs[bi];
+  if (tab.status != kDecOk) return;
+  const int tid = threadIdx.x;
+  const int64_t p0 = cand[bi] + (int64_t)blockIdx.x * kJumpTile;
+  for (int q = tid; q < kJumpAll / 32 + 2; q += 256) bits[q] = bits_at(words, nwords, p0 + 32 * q);
+  if (tid < 34) {  // positions past the halo, and the two states, in all buffers
+    const uint32_t q = kJumpAll + tid;
+    const uint16_t v = (uint16_t)(q == kJumpDead ? kJumpDead : kJumpOut);
+    A[q] = B[q] = C[q] = v;
+  }
+  for (int t = 0; t < tab.ng; t++) {
+    __syncthreads();  // the previous table's gathers are done
+    const uint8_t *src = lens + (size_t)bi * kLensBytes + ((size_t)t << kLenBits);
+    reinterpret_cast<uint4 *>(llen)[tid] = reinterpret_cast<const uint4 *>(src)[tid];
+    if (tid < kDecMaxCode + 4) lj[tid] = tab.lj[t][tid];
+    const int mn = tab.mn[t], mx = tab.mx[t];
+    __syncthreads();
+    uint32_t cur[kJumpPer];
+#pragma unroll
+    for (int j = 0; j < kJumpPer; j++) {
+      const int o = 256 * j + tid;
+      const uint32_t x = __funnelshift_l(bits[(o >> 5) + 1], bits[o >> 5], o & 31);
+      int n = llen[x >> (32 - kLenBits)];
+      if (n == 0) {
+        n = max(mn, kLenBits + 1);
+        while (n <= mx && x > lj[n]) n++;
+        if (n > mx) n = 0;
+      }
+      cur[j] = n ? (uint32_t)(o + n) : kJumpDead;
+      A[o] = (uint16_t)cur[j];
+    }
+    __syncthreads();
+    auto square = [&](const uint16_t *from, uint16_t *to) {
+#pragma unroll
+      for (int j = 0; j < kJumpPer; j++) {
+        cur[j] = from[cur[j]];
+        to[256 * j + tid] = (uint16_t)cur[j];
+      }
+      __syncthreads();
+    };
+    square(A, B);  // 2 codes, kept
+    square(B, C);  // 4
+    square(C, A);  // 8
+    square(A, C);  // 16, kept
+    square(C, A);  // 32
+    uint16_t *out = jumps + ((size_t)tile * kDecMaxGroups + t) * kJumpTile;
+#pragma unroll
+    for (int j = 0; j < kJumpTile / 256; j++) {
+      const uint32_t v = B[C[cur[j]]];  // 50
+      const int o = 256 * j + tid;
+      out[o] = (uint16_t)(v < kJumpOut ? 2 * (v - o) : kDeadJump);
+    }
+  }
+}
+
+// Group starts of one block by its jumps: the tiles come through
+// kStartStages buffers, one thread hops.  A chain that leaves the tiles (a magic inside a payload cuts
+// a block's tiles short) leaves ngv -1: k_dec_groups then walks that block.
+__global__ void __launch_bounds__(256) k_dec_starts(DecTab *tabs, const uint8_t *selbuf,
+                                                    uint32_t *gstart, const int64_t *cand,
+                                                    const int32_t *jt0, const uint16_t *jumps) {
+  extern __shared__ __align__(16) uint8_t ssm[];
+  __shared__ uint8_t sel[kDecMaxSel + 6];
+  __shared__ int s_done;
+  const int bi = blockIdx.x, tid = threadIdx.x;
+  DecTab &tab = tabs[bi];
+  if (tab.status != kDecOk) return;
+  const int ng = tab.ng, nsel = tab.nsel;
+  const int t0 = jt0[bi], nt = jt0[bi + 1] - t0;
+  for (int q = tid; q < nsel; q += 256) sel[q] = selbuf[(size_t)bi * kDecMaxSel + q];
+  uint32_t *gs = gstart + (size_t)bi * kDecMaxSel;
+  const uint32_t first = (uint32_t)(tab.pay - cand[bi]);
+  if (tid == 0) s_done = 0;
+  const int vec = ng * kJumpTile * 2 / 16;  // 16-byte pieces of a tile's tables
+  auto load = [&](int k) {
+    if (k < nt) {
+      const uint4 *src = reinterpret_cast<const uint4 *>(
+          jumps + (size_t)(t0 + k) * kDecMaxGroups * kJumpTile);
+      uint4 *dst = reinterpret_cast<uint4 *>(ssm + (size_t)(k % kStartStages) * kStartStage);
+      for (int q = tid; q < vec; q += 256) {
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + q);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src + q));
+      }
+    }
+    asm volatile("cp.async.commit_group;");
+  };
+  const int k0 = (int)(first / kJumpTile);
+  for (int k = k0; k < k0 + kStartStages - 1; k++) load(k);
+  int g = 0;             // thread 0's place in the chain
+  uint32_t p = first;
+  for (int k = k0; k < nt; k++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStartStages - 2));
+    __syncthreads();  // tile k is here for all threads, the tile before it is done with
+    if (s_done) break;
+    load(k + kStartStages - 1);
+    if (tid == 0) {
+      // bytes of the tile's tables: a jump is one load and one add
+      const uint8_t *J = ssm + (size_t)(k % kStartStages) * kStartStage;
+      const uint32_t base = (uint32_t)k * kJumpTile;
+      uint32_t q = 2 * (p - base), at = sel[g] * (uint32_t)(2 * kJumpTile), v = 0;
+      while (q < 2 * kJumpTile && g < nsel) {
+        gs[g] = base + (q >> 1);
+        g++;
+        v = *reinterpret_cast<const uint16_t *>(J + at + q);
+        at = sel[g] * (uint32_t)(2 * kJumpTile);  // one byte past nsel is there, not used
+        q += v;
+      }
+      p = base + (q >> 1);
+      if (g >= nsel || v == kDeadJump) {
+        tab.ngv = g;  // a dead jump's group is the last with a known start
+        s_done = 1;
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;");
 }
 
 // Warps per block: eight where the blocks leave the GPU room (the chain's
@@ -1648,7 +1882,7 @@ struct MallocSink : DecSink {
 struct DecWork {
   std::mutex mu;
   DevBuf words, blk, eos, cnt, cand, order, db, tab, gstart, L, hist, sel, idx, tt, lens, off, crc,
-      ctl, pool, bad, maps;
+      ctl, pool, bad, maps, jumps, jt0, lutlen;
   DevBuf out[2];
   cudaStream_t st = nullptr, cs = nullptr;
   cudaEvent_t written[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
@@ -1669,6 +1903,10 @@ struct DecWork {
     int dev = 0, per_sm = 0;
     BZ_CUDA(cudaGetDevice(&dev));
     BZ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    BZ_CUDA(cudaFuncSetAttribute(k_dec_jumps, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kJumpSmem));
+    BZ_CUDA(cudaFuncSetAttribute(k_dec_starts, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kStartsSmem));
     BZ_CUDA(cudaFuncSetAttribute(k_dec_chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kChainSmem));
     BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dec_groups<4>, 128, 0));
@@ -1857,6 +2095,34 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const dim3 cgrid((kMaxChunks + kSymWarps - 1) / kSymWarps, nc);
     k_dec_head<<<nc, kHeadThreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>());
     BZ_LAUNCH_CHECK();
+    // few blocks: group starts by jump tables
+    std::vector<int32_t> jt0(nc + 1, 0);
+    int jmax = 0;
+    int64_t jbits = 0;
+    for (int q = 0; q < nc; q++) {
+      const int nt = (int)std::min<int64_t>(csize(q) / kJumpTile + 1, 1 << 20);
+      jbits += (int64_t)nt * kJumpTile;
+      jmax = std::max(jmax, nt);
+      jt0[q + 1] = (int32_t)std::min<int64_t>((int64_t)jt0[q] + nt, 1 << 30);
+    }
+    const size_t jbytes = (size_t)jbits * kDecMaxGroups * 2;
+    if (jbits <= kJumpMaxBits && jmax <= 65535 && (jbytes <= w.jumps.cap || jbytes <= freeb / 4)) {
+      w.jumps.reserve(jbytes);
+      w.jt0.reserve(4 * (size_t)(nc + 1));
+      w.lutlen.reserve((size_t)nc * kLensBytes);
+      BZ_CUDA(cudaMemcpyAsync(w.jt0.p, jt0.data(), 4 * (size_t)(nc + 1), cudaMemcpyHostToDevice, st));
+      k_dec_lens<<<dim3(kDecMaxGroups, nc), 256, 0, st>>>(dtab, w.lutlen.get<uint8_t>());
+      BZ_LAUNCH_CHECK();
+      k_dec_jumps<<<dim3(jmax, nc), 256, kJumpSmem, st>>>(wd, nwords, dcand, dtab,
+                                                          w.lutlen.get<uint8_t>(),
+                                                          w.jt0.get<int32_t>(),
+                                                          w.jumps.get<uint16_t>());
+      BZ_LAUNCH_CHECK();
+      k_dec_starts<<<nc, 256, kStartsSmem, st>>>(dtab, w.sel.get<uint8_t>(),
+                                                 w.gstart.get<uint32_t>(), dcand,
+                                                 w.jt0.get<int32_t>(), w.jumps.get<uint16_t>());
+      BZ_LAUNCH_CHECK();
+    }
     int gthreads = 0;
     const GroupsKernel groups = groups_kernel(nc, w.sms, &gthreads);
     groups<<<nc, gthreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>(),
