@@ -185,8 +185,8 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
   const int nt = (len + kTile - 1) / kTile;
   const int t0 = (int)(d.off[b] / kTile);
   uint32_t *H = d.tile_hist + (size_t)t0 * kN + kD * threadIdx.x;
-  // eight tiles' counts in flight at a time (the loads are independent)
-  constexpr int kU = 8;
+  // many tiles' counts in flight at a time (the loads are independent)
+  constexpr int kU = kD == 1 ? 20 : 8;
   uint32_t run[kD];
 #pragma unroll
   for (int q = 0; q < kD; q++) run[q] = 0;
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, int kb, const int3
   uint32_t *bits = d.head_bits + (size_t)t * (kTile / 32) + w * kTileItems;
   int last = -1, heads = 0, sing = 0;
   int pc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 4
+#pragma unroll 8
   for (int i = 0; i < kTileItems; i++) {
     const int e = w * kWarpSpan + i * 32 + ln;
     const int k = lt + e;

@@ -33,33 +33,59 @@ __device__ __forceinline__ bool serves(const SlabDev &d, int b, int which, int r
 
 // bzip2's initial tables (src/compression/huffman.cu:148-185): every length
 // 15, then table n_part - 1 gets length 0 over the next range of symbols
-// holding about remaining / n_part of the symbol count.  One warp.
-__device__ void init_tables(const SlabDev &d, int b) {
+// holding about remaining / n_part of the symbol count: it ends at the first
+// symbol where the counts from its start reach that share (alpha if none
+// does).  One warp: running counts in shared memory, a ballot per 32 symbols
+// finds each end (one thread adding up the counts took 32 us).
+constexpr int kFreqSlots = (kMaxAlpha + 31) / 32;  // 9
+
+__device__ void init_tables(const SlabDev &d, int b, int32_t *cum) {
+  const unsigned full = 0xffffffffu;
+  const int ln = lane_id();
   const int s = d.s[b];
   const int ng = d.n_groups[b];
   const int alpha = d.n_in_use[b] + 2;
   uint8_t *len = d.len + (size_t)b * kMaxGroups * kMaxAlpha;
-  for (int i = lane_id(); i < kMaxGroups * kMaxAlpha; i += 32) len[i] = 15;
+  const int32_t *freq = d.freq + (size_t)b * kMaxAlpha;
+  int f[kFreqSlots];
+#pragma unroll
+  for (int q = 0; q < kFreqSlots; q++) f[q] = 32 * q + ln < kMaxAlpha ? freq[32 * q + ln] : 0;
+  int run = 0;
+#pragma unroll
+  for (int q = 0; q < kFreqSlots; q++) {
+    const int inc = warp_incl_sum(f[q]);
+    f[q] = run + inc;  // counts of the symbols up to this one
+    cum[32 * q + ln] = f[q];
+    run += __shfl_sync(full, inc, 31);
+  }
+  for (int i = ln; i < kMaxGroups * kMaxAlpha; i += 32) len[i] = 15;
   __syncwarp();
-  if (lane_id() == 0) {
-    const int32_t *freq = d.freq + (size_t)b * kMaxAlpha;
-    int gs = 0, remaining = s;
-    for (int n_part = ng; n_part > 0; n_part--) {
-      int t_freq = remaining / n_part;
-      int ge = gs - 1, a_freq = 0;
-      while (a_freq < t_freq && ge < alpha) {
-        ge++;
-        a_freq += ge < kMaxAlpha ? freq[ge] : 0;
+  // counts of the symbols up to v (nothing past the alphabet's room)
+  auto upto = [&](int v) { return v < 0 ? 0 : cum[min(v, kMaxAlpha - 1)]; };
+  int gs = 0, remaining = s;
+  for (int n_part = ng; n_part > 0; n_part--) {
+    const int t_freq = remaining / n_part;
+    const int base = upto(gs - 1);
+    int ge = gs - 1;
+    if (t_freq > 0) {
+      ge = alpha;
+#pragma unroll
+      for (int q = kFreqSlots - 1; q >= 0; q--) {
+        const int v = 32 * q + ln;
+        const unsigned hit = __ballot_sync(full, v >= gs && v < alpha && f[q] - base >= t_freq);
+        if (hit) ge = 32 * q + __ffs(hit) - 1;
       }
-      if (ge > gs && n_part != ng && n_part != 1 && ((ng - n_part) % 2 == 1)) {
-        a_freq -= ge < kMaxAlpha ? freq[ge] : 0;
-        ge--;
-      }
-      uint8_t *row = len + (n_part - 1) * kMaxAlpha;
-      for (int v = 0; v < alpha; v++) row[v] = (v >= gs && v <= ge) ? 0 : 15;
-      gs = ge + 1;
-      remaining -= a_freq;
+      if (gs > alpha) ge = gs - 1;  // no symbol is left
     }
+    int a_freq = upto(ge) - base;
+    if (ge > gs && n_part != ng && n_part != 1 && ((ng - n_part) % 2 == 1)) {
+      a_freq = upto(ge - 1) - base;
+      ge--;
+    }
+    uint8_t *row = len + (n_part - 1) * kMaxAlpha;
+    for (int v = gs + ln; v <= min(ge, alpha - 1); v += 32) row[v] = 0;
+    gs = ge + 1;
+    remaining -= a_freq;
   }
   __syncwarp();
 }
@@ -67,6 +93,7 @@ __device__ void init_tables(const SlabDev &d, int b) {
 // learned_mode: blocks with six tables take the learned selector; the plain
 // blocks of the learned form have 2 passes left after the two shared ones.
 __global__ void k_huff_init(SlabDev d, int learned_mode) {
+  __shared__ int32_t cum[32 * kFreqSlots];
   const int b = blockIdx.x;
   const int s = d.s[b];
   const int ng = s < 200 ? 2 : s < 600 ? 3 : s < 1200 ? 4 : s < 2400 ? 5 : 6;
@@ -77,7 +104,7 @@ __global__ void k_huff_init(SlabDev d, int learned_mode) {
     d.plain_left[b] = kIters - 2;
   }
   __syncwarp();
-  init_tables(d, b);
+  init_tables(d, b, cum);
 }
 
 // One thread per 50-symbol group, its symbols in 25 registers (two 16-bit

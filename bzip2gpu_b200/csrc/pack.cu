@@ -58,15 +58,15 @@ __device__ __forceinline__ int sel_chunk(int nsel, int *a, int *e) {
   return per;
 }
 
-__device__ int64_t table_bits(const uint8_t *len, int alpha) {
-  int cur = len[0];
-  int64_t tb = 5;
-  for (int v = 0; v < alpha; v++) {
-    int tg = len[v];
-    tb += 2 * abs(tg - cur) + 1;
-    cur = tg;
+// Bits of a table's delta-coded lengths (5-bit start, 2 bits per unit of
+// change, 1 terminator bit per symbol), by one warp.
+__device__ int table_bits(const uint8_t *len, int alpha) {
+  int e = 0;
+  for (int v = lane_id(); v < alpha; v += 32) {
+    const int l = len[v];
+    e += 2 * abs(l - (v ? (int)len[v - 1] : l)) + 1;
   }
-  return tb;
+  return 5 + __reduce_add_sync(0xffffffffu, e);
 }
 
 __device__ int used_ranges(const uint32_t *pres) {
@@ -77,7 +77,8 @@ __device__ int used_ranges(const uint32_t *pres) {
 
 __global__ void __launch_bounds__(kHdrThreads) k_sel_mtf_hdr(SlabDev d) {
   __shared__ int scratch[40];
-  __shared__ int64_t tbits[kMaxGroups];
+  __shared__ int tbits[kMaxGroups];
+  __shared__ int wl[kHdrThreads / 32][kMaxGroups];
   const int b = blockIdx.x;
   const int ngrp = d.n_groups[b];
   const int nsel = d.n_sel[b];
@@ -95,50 +96,53 @@ __global__ void __launch_bounds__(kHdrThreads) k_sel_mtf_hdr(SlabDev d) {
     for (int t = 0; t < kMaxGroups; t++)
       if (v == t) last[t] = i;
   }
+  // the tables' last uses before this thread's chunk
   int prev[kMaxGroups];
 #pragma unroll
   for (int t = 0; t < kMaxGroups; t++) {
-    int inc = block_incl_max(last[t], scratch, -1);
-    int ex = __shfl_up_sync(0xffffffffu, inc, 1);
-    __shared__ int wl[kHdrThreads / 32];
-    if (lane_id() == 31) wl[warp_id()] = inc;
-    __syncthreads();
-    if (lane_id() == 0) ex = warp_id() == 0 ? -1 : wl[warp_id() - 1];
-    prev[t] = ex;
-    __syncthreads();
+    const int inc = warp_incl_max(last[t]);
+    prev[t] = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane_id() == 0) prev[t] = -1;
+    if (lane_id() == 31) wl[warp_id()][t] = inc;
   }
-  // starting list: used tables by last use (latest first), then unused ones
-  uint8_t pos[kMaxGroups];
-  {
-    int key[kMaxGroups];
-    for (int t = 0; t < ngrp; t++) key[t] = prev[t] >= 0 ? prev[t] : -1 - t;
-    for (int t = 0; t < ngrp; t++) {
-      int r = 0;
-      for (int u = 0; u < ngrp; u++) r += key[u] > key[t];
-      pos[r] = (uint8_t)t;
+  if ((int)warp_id() < ngrp) {
+    const int tb = table_bits(d.len + ((size_t)b * kMaxGroups + warp_id()) * kMaxAlpha, alpha);
+    if (lane_id() == 0) tbits[warp_id()] = tb;
+  }
+  __syncthreads();
+  for (int w = 0; w < (int)warp_id(); w++) {
+#pragma unroll
+    for (int t = 0; t < kMaxGroups; t++) prev[t] = max(prev[t], wl[w][t]);
+  }
+  // starting list, nibble r = table at position r: used tables by last use
+  // (latest first), then unused ones
+  uint32_t lst = 0;
+#pragma unroll
+  for (int t = 0; t < kMaxGroups; t++) {
+    const int key = prev[t] >= 0 ? prev[t] : -1 - t;
+    int r = 0;
+#pragma unroll
+    for (int u = 0; u < kMaxGroups; u++) {
+      const int ku = prev[u] >= 0 ? prev[u] : -1 - u;
+      r += u < ngrp && ku > key;
     }
+    if (t < ngrp) lst |= (uint32_t)t << (4 * r);
   }
+  // positions past the last table hold a value no selector has
+  for (int r = ngrp; r < 8; r++) lst |= 15u << (4 * r);
   int unary = 0;
   for (int i = a; i < e; i++) {
-    const uint8_t v = sel[i];
-    int j = 0;
-    uint8_t tmp = pos[0];
-    while (v != tmp) {
-      j++;
-      uint8_t t2 = tmp;
-      tmp = pos[j];
-      pos[j] = t2;
-    }
-    pos[0] = tmp;
+    const uint32_t v = sel[i];
+    // the lowest zero nibble of x is v's position
+    const uint32_t x = lst ^ (v * 0x11111111u);
+    const int j = (__ffs((x - 0x11111111u) & ~x & 0x88888888u) - 1) >> 2;
+    const uint32_t low = (1u << (4 * j)) - 1u;
+    lst = (lst & ~((low << 4) | 0xFu)) | ((lst & low) << 4) | v;
     smtf[i] = (uint8_t)j;
     unary += j + 1;
   }
   int total_unary;
   block_excl_sum(unary, scratch, &total_unary);
-  if ((int)threadIdx.x < ngrp)
-    tbits[threadIdx.x] =
-        table_bits(d.len + ((size_t)b * kMaxGroups + threadIdx.x) * kMaxAlpha, alpha);
-  __syncthreads();
   if (threadIdx.x == 0) {
     int64_t tb = 0;
     for (int t = 0; t < ngrp; t++) tb += tbits[t];
@@ -194,22 +198,27 @@ __global__ void __launch_bounds__(256) k_pay_block(SlabDev d) {
   if (threadIdx.x == 0) d.pay_bits[b] = carry;
 }
 
-__global__ void k_block_starts(SlabDev d, int64_t slab_start) {
-  if (threadIdx.x != 0) return;
+__global__ void __launch_bounds__(256) k_block_starts(SlabDev d, int64_t slab_start) {
+  __shared__ int64_t scratch[40];
   int64_t run = slab_start;
-  for (int b = 0; b < d.nblocks; b++) {
-    d.blk_start[b] = run;
-    run += d.hdr_bits[b] + d.pay_bits[b];
+  for (int b0 = 0; b0 < d.nblocks; b0 += 256) {
+    const int b = b0 + threadIdx.x;
+    const int64_t bits = b < d.nblocks ? d.hdr_bits[b] + d.pay_bits[b] : 0;
+    int64_t tot;
+    const int64_t at = run + block_excl_sum(bits, scratch, &tot);
+    if (b < d.nblocks) d.blk_start[b] = at;
+    run += tot;
   }
 }
 
 // Block header at its stream position (src/compression/compress.cu:290-353).
 // Thread 0 writes the fixed fields; every thread writes the unary selector
-// codes of its chunk at an offset from a block scan; threads t < nGroups
-// write table t's delta-coded lengths.
+// codes of its chunk at an offset from a block scan; warp t < nGroups writes
+// table t's delta-coded lengths, a symbol per lane at offsets from warp scans
+// (a thread per table took 60 us).
 __global__ void __launch_bounds__(kHdrThreads) k_write_header(SlabDev d, int64_t w0) {
   __shared__ int scratch[40];
-  __shared__ int64_t tbits[kMaxGroups];
+  __shared__ int tbits[kMaxGroups];
   const int b = blockIdx.x;
   const int ngrp = d.n_groups[b];
   const int nsel = d.n_sel[b];
@@ -258,32 +267,41 @@ __global__ void __launch_bounds__(kHdrThreads) k_write_header(SlabDev d, int64_t
     }
     w.flush();
   }
-  if ((int)threadIdx.x < ngrp)
-    tbits[threadIdx.x] =
-        table_bits(d.len + ((size_t)b * kMaxGroups + threadIdx.x) * kMaxAlpha, alpha);
+  const int t = warp_id(), ln = lane_id();
+  if (t < ngrp) {
+    const int tb = table_bits(d.len + ((size_t)b * kMaxGroups + t) * kMaxAlpha, alpha);
+    if (ln == 0) tbits[t] = tb;
+  }
   __syncthreads();
-  if ((int)threadIdx.x < ngrp) {
-    const int t = threadIdx.x;
+  if (t < ngrp) {
     int64_t at = base + fixed + total;
     for (int u = 0; u < t; u++) at += tbits[u];
     const uint8_t *len = d.len + ((size_t)b * kMaxGroups + t) * kMaxAlpha;
-    BitSink w;
-    w.init(d.out, at);
-    int cur = len[0];
-    w.put((uint32_t)cur, 5);
-    for (int v = 0; v < alpha; v++) {
-      const int tg = len[v];
-      while (cur < tg) {
-        w.put(2, 2);
-        cur++;
+    // nb <= 33 bits at stream bit p: at most two words
+    auto place = [&](int64_t p, uint64_t v, int nb) {
+      const uint64_t x = v << (64 - (int)(p & 31) - nb);
+      const uint32_t hi = (uint32_t)(x >> 32), lo = (uint32_t)x;
+      if (hi) atomicOr(d.out + (p >> 5), bswap32(hi));
+      if (lo) atomicOr(d.out + (p >> 5) + 1, bswap32(lo));
+    };
+    if (ln == 0) place(at, len[0], 5);
+    at += 5;
+    for (int v0 = 0; v0 < alpha; v0 += 32) {
+      const int v = v0 + ln;
+      int nb = 0;
+      uint64_t code = 0;
+      if (v < alpha) {
+        const int l = len[v], k = l - (v ? (int)len[v - 1] : l);
+        // |k| steps of 10 (longer) or 11 (shorter), then a 0
+        const int n2 = 2 * abs(k);
+        const uint64_t ones = (1ull << n2) - 1ull;
+        code = (k > 0 ? ones & 0xAAAAAAAAAAAAAAAAull : ones) << 1;
+        nb = n2 + 1;
       }
-      while (cur > tg) {
-        w.put(3, 2);
-        cur--;
-      }
-      w.put(0, 1);
+      const int inc = warp_incl_sum(nb);
+      if (code) place(at + inc - nb, code, nb);
+      at += __shfl_sync(0xffffffffu, inc, 31);
     }
-    w.flush();
   }
 }
 
@@ -379,7 +397,7 @@ void stage_sizes_payload_only(const SlabDev &d, cudaStream_t st) {
 void stage_place(const SlabDev &d, int64_t slab_start_bit, int64_t w0, int64_t nwords,
                  cudaStream_t st) {
   BZ_CUDA(cudaMemsetAsync(d.out, 0, sizeof(uint32_t) * nwords, st));
-  k_block_starts<<<1, 32, 0, st>>>(d, slab_start_bit);
+  k_block_starts<<<1, 256, 0, st>>>(d, slab_start_bit);
   BZ_LAUNCH_CHECK();
   k_write_header<<<d.nblocks, kHdrThreads, 0, st>>>(d, w0);
   BZ_LAUNCH_CHECK();
