@@ -735,36 +735,42 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, int kb, const int3
 }
 
 // Groups of at most kGroupMax rotations are sorted in shared memory: a CTA
-// takes the groups that start in its kGroupMax items (a half tile) of a block's
-// active list, so it holds at most kTile.
-constexpr int kGroupMax = kTile / 2;
+// takes the groups that start in a unit of `step` items of a block's active
+// list, and holds kTile, so a step is what the block's longest group leaves of
+// that (2048 for every block took a CTA for half of what it can hold).  Longer
+// groups would leave steps that mostly reload what other CTAs hold.
+constexpr int kMinStep = 512;
+constexpr int kGroupMax = kTile - kMinStep;
+__device__ __forceinline__ int group_step(int gmax) { return (kTile - gmax) & ~31; }
 
-// Lists a block's tiles: half tiles when it is sorted group by group.  The
+// Lists a block's tiles, or its units when it is sorted group by group.  The
 // blocks' places are taken by a thread each, the entries written by a warp
 // each.  One CTA of 1024 threads; nblocks in passes of 1024.
 struct TileRuns {
-  int at[1024], n[1024], t0[1024];
+  int at[1024], n[1024], first[1024], step[1024];
   int32_t *list[1024];
 };
 
 __device__ __forceinline__ void list_block(const SlabDev &d, TileRuns &r, int b, int len) {
   const bool loc = d.loc[b];
-  const int unit = loc ? kGroupMax : kTile;
+  const int unit = loc ? d.loc_step[b] : kTile;  // entries: tiles, or items / 32
   const int nt = (len + unit - 1) / unit;
   r.at[threadIdx.x] = atomicAdd(&d.sort_ctl[loc ? 7 : 5], nt);
   r.n[threadIdx.x] = nt;
-  r.t0[threadIdx.x] = (int)(d.off[b] / unit);
+  r.first[threadIdx.x] = (int)(d.off[b] / (loc ? 32 : kTile));
+  r.step[threadIdx.x] = loc ? unit / 32 : 1;
   r.list[threadIdx.x] = loc ? d.loc_list : d.tile_list;
 }
 
 __device__ __forceinline__ void write_lists(const TileRuns &r, int nb) {
   for (int q = warp_id(); q < nb; q += 32)
-    for (int k = lane_id(); k < r.n[q]; k += 32) r.list[q][r.at[q] + k] = r.t0[q] + k;
+    for (int k = lane_id(); k < r.n[q]; k += 32)
+      r.list[q][r.at[q] + k] = r.first[q] + k * r.step[q];
 }
 
 // Ends a round: blocks sorted group by group settle their counts, the key and
 // position buffers switch, sort_len = active rotations, and the next round's
-// tiles are listed: tiles of the blocks that go on by radix sort, half tiles of
+// tiles are listed: tiles of the blocks that go on by radix sort, units of
 // those whose groups are all short.
 __global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefix_len, int packed) {
   __shared__ TileRuns runs;
@@ -784,6 +790,7 @@ __global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefi
           d.loc[b] = 1;
           d.loc_cur[b] = keys_now(d) ^ 1;
         }
+        d.loc_step[b] = group_step(d.gmax[b]);
         d.gmax[b] = 0;
         list_block(d, runs, b, len);
       }
@@ -799,7 +806,7 @@ __global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefi
   }
 }
 
-// One round of the groups of a half tile.  Items are head << 2kb | rank << kb |
+// One round of the groups of a unit.  Items are head << 2kb | rank << kb |
 // rotation; with the head replaced by the group's start in the tile (groups
 // stand in no order in the list) they are all different and sorting them by
 // value sorts every group by rank with ties in index order.  Each group is
@@ -816,10 +823,11 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
   __shared__ uint32_t starts[kTile / 32 + 1];  // bit per item: a group starts here
   __shared__ int red[3][kSortWarps];
   __shared__ int s_base;
-  const int h = d.loc_list[blockIdx.x];
-  const int b = d.tile_block[h >> 1];
+  const int64_t u = (int64_t)d.loc_list[blockIdx.x] * 32;  // the unit's first item
+  const int b = d.tile_block[u / kTile];
   const int64_t off = d.off[b];
-  const int s = (int)((int64_t)h * kGroupMax - off);  // first item of the half tile
+  const int s = (int)(u - off);
+  const int step = d.loc_step[b];
   const int len = d.sort_len[b];
   const int cur = d.loc_cur[b];
   const uint64_t *K = d.keys[cur] + off;
@@ -830,7 +838,7 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
   const uint64_t low = (1ull << hs) - 1, vmask = (1ull << kb) - 1;
   const int e0 = w * kWarpSpan + ln;  // item i of this thread: e0 + 32 i
   uint64_t mine[kTileItems];
-  bool before_first = false;  // thread 0: the item before the half tile is of another group
+  bool before_first = false;  // thread 0: the item before the unit is of another group
 #pragma unroll
   for (int i = 0; i < kTileItems; i++) {
     const int e = e0 + 32 * i;
@@ -841,7 +849,7 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
   __syncthreads();
   // group starts: the first in each of this warp's rows, and the last so far
   uint32_t gs2[kTileItems / 2];  // two 16-bit fields per register
-  int wfirst = INT32_MAX, carry = -1;
+  int wfirst = INT32_MAX, wafter = INT32_MAX, carry = -1;
 #pragma unroll
   for (int i = 0; i < kTileItems; i++) {
     const int e = e0 + 32 * i;
@@ -852,7 +860,10 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
     }
     const unsigned bm = __ballot_sync(0xffffffffu, st);
     if (ln == 0) starts[e >> 5] = bm;
-    if (bm && wfirst == INT32_MAX) wfirst = e - ln + __ffs(bm) - 1;
+    if (bm) {  // a row lies in the unit or after it
+      if (e - ln < step) wfirst = min(wfirst, e - ln + __ffs(bm) - 1);
+      else wafter = min(wafter, e - ln + __ffs(bm) - 1);
+    }
     const unsigned below = bm & le_mask;
     const int g = below ? e - ln + 31 - __clz(below) : carry;
     carry = bm ? e - ln + 31 - __clz(bm) : carry;
@@ -863,16 +874,17 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
   if (ln == 0) {
     red[0][w] = wfirst;
     red[1][w] = carry;
+    red[2][w] = wafter;
   }
   __syncthreads();
   int first = INT32_MAX, after = avail, before = -1;
 #pragma unroll
   for (int q = 0; q < kSortWarps; q++) {
-    if (q < kSortWarps / 2) first = min(first, red[0][q]);
-    else after = min(after, red[0][q]);
+    first = min(first, red[0][q]);
+    after = min(after, red[2][q]);
     if (q < w) before = max(before, red[1][q]);
   }
-  if (first >= kGroupMax) return;  // one group from before covers the half tile
+  if (first == INT32_MAX) return;  // one group from before covers the unit
   // [first, after): whole groups.  Keys with the group's start in front; a
   // group's last item leaves its size at its start.
 #pragma unroll
@@ -1028,6 +1040,7 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
   int32_t *IS = d.isa + off;
   uint64_t *KO = d.keys[cur ^ 1] + off + s_base + red[1][w];
   const unsigned lt_mask = le_mask >> 1;
+  int gmax = 0;  // the longest group that goes on
 #pragma unroll
   for (int i = 0; i < kTileItems; i++) {
     const int e = e0 + 32 * i;
@@ -1048,22 +1061,26 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
     const unsigned am = __ballot_sync(0xffffffffu, active);
     if (active) KO[__popc(am & lt_mask)] = ((uint64_t)(uint32_t)nhead << hs) | val;
     KO += __popc(am);
+    if (tl && sg != e) gmax = max(gmax, e - sg + 1);
   }
+  gmax = __reduce_max_sync(0xffffffffu, gmax);
+  if (ln == 0 && gmax > 0) atomicMax(&d.gmax[b], gmax);
 }
 
-// Round keys for the compacted active rotations: add the rank of i+h.  unit:
-// items per list entry (kTile, or kGroupMax for the blocks sorted by groups).
+// Round keys for the compacted active rotations: add the rank of i+h.  loc: the
+// list holds units of the blocks sorted group by group, else tiles.
 __global__ void __launch_bounds__(256) k_bwt_round_keys(SlabDev d, int h, int packed, int kb,
-                                                        const int32_t *list, int unit) {
+                                                        const int32_t *list, int loc) {
   const int t = list[blockIdx.x];
-  const int b = d.tile_block[unit == kTile ? t : t >> 1];
+  const int64_t u = (int64_t)t * (loc ? 32 : kTile);
+  const int b = d.tile_block[u / kTile];
   const int64_t off = d.off[b];
-  const int lt = (int)((int64_t)t * unit - off);
+  const int lt = (int)(u - off);
   const int len = d.sort_len[b];
-  const int valid = min(unit, len - lt);
+  const int valid = min(loc ? d.loc_step[b] : kTile, len - lt);
   if (valid <= 0) return;
   const int m = d.m[b];
-  const int cur = unit == kTile ? d.sort_ctl[0] : d.loc_cur[b];
+  const int cur = loc ? d.loc_cur[b] : d.sort_ctl[0];
   uint64_t *K = d.keys[cur] + off + lt;
   const uint32_t *V = d.vals[cur] + off + lt;
   const int32_t *IS = d.isa + off;
@@ -1171,7 +1188,7 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
       std::memcpy(&d.rt_act[0], d.h_flags + 6, sizeof(int64_t));  // sort_ctl[8..9]
     if (d.h_flags[0] == 0) break;
     grid = d.h_flags[3];   // tiles holding active rotations
-    lgrid = d.h_flags[5];  // half tiles of the blocks sorted group by group
+    lgrid = d.h_flags[5];  // units of the blocks sorted group by group
     list = d.tile_list;
     r++;
     if (rounds_timed && r >= kMaxRounds) rounds_timed = false;
@@ -1181,11 +1198,11 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
     }
     // every block's keys before any block's ranks change
     if (grid > 0) {
-      k_bwt_round_keys<<<grid, 256, 0, st>>>(d, (int)prefix, packed, kb, list, kTile);
+      k_bwt_round_keys<<<grid, 256, 0, st>>>(d, (int)prefix, packed, kb, list, 0);
       BZ_LAUNCH_CHECK();
     }
     if (lgrid > 0) {
-      k_bwt_round_keys<<<lgrid, 256, 0, st>>>(d, (int)prefix, packed, kb, d.loc_list, kGroupMax);
+      k_bwt_round_keys<<<lgrid, 256, 0, st>>>(d, (int)prefix, packed, kb, d.loc_list, 1);
       BZ_LAUNCH_CHECK();
     }
     if (packed)

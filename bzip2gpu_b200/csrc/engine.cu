@@ -121,7 +121,7 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     dev.tile_c = (int32_t *)alloc(T * 4);
     dev.tile_d = (int32_t *)alloc(T * 4);
     dev.tile_list = (int32_t *)alloc(T * 4);
-    dev.loc_list = (int32_t *)alloc(2 * T * 4);
+    dev.loc_list = (int32_t *)alloc(8 * T * 4);
     dev.vt_list = (int32_t *)alloc(T * 4);
     dev.vg_list = (int32_t *)alloc(((int64_t)mgt + 1) * 4);
     dev.warp_last = (int32_t *)alloc(((int64_t)mt + 1) * (kTileThreads / 32) * 4);
@@ -157,7 +157,7 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     dev.ngroups = (int32_t *)alloc(B * 4);
     dev.act_len = (int32_t *)alloc(B * 4);
     for (int32_t **a : {&dev.loc, &dev.loc_cur, &dev.loc_act, &dev.loc_heads, &dev.loc_sing,
-                        &dev.gmax})
+                        &dev.gmax, &dev.loc_step})
       *a = (int32_t *)alloc(B * 4);
     dev.active_sum = (int64_t *)alloc(B * 8);
     dev.pstat = (int32_t *)alloc(B * 8 * 4);

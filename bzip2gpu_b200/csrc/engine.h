@@ -98,8 +98,9 @@ struct SlabDev {
   // shared memory.  loc[b]: 1 for such a block; loc_cur: its current key
   // buffer; loc_act, loc_heads, loc_sing: the running round's active
   // rotations, groups and singletons; gmax: the largest active group after a
-  // radix round; loc_list: their half tiles [2 * ntiles].
-  int32_t *loc, *loc_cur, *loc_act, *loc_heads, *loc_sing, *gmax, *loc_list;
+  // round; loc_step: items per work unit; loc_list: the units, by their first
+  // item / 32 [8 * ntiles].
+  int32_t *loc, *loc_cur, *loc_act, *loc_heads, *loc_sing, *gmax, *loc_step, *loc_list;
   // The tiles that hold data, listed in block order (a block's workspace is
   // sized for its worst-case RLE1 output, so most of its tiles can be empty):
   // element tiles of the m[b] RLE1 bytes, and group tiles of the
@@ -119,7 +120,7 @@ struct SlabDev {
   int32_t *sort_ctl;                   // [0]=cur key buffer, [1]=passes that move items,
                                        // [2]=blocks still sorting, [3]=cur kpos buffer,
                                        // [5]=tiles of the next round,
-                                       // [7]=half tiles of its group-sorted blocks,
+                                       // [7]=units of its group-sorted blocks,
                                        // [6]=rotations entering the next round,
                                        // [8..9]=u64 rotations the first sort's model charges
                                        // [10], [11]=tile-list counts, [12]=largest m

@@ -1,6 +1,6 @@
 """The BWT's group sort at its edges: groups of equal 4-byte prefixes around
-the run lengths of its merges (8, 16, ..), around a half tile (2048, above
-which a block goes on by radix sort) and across tiles; long repeats (many
+the run lengths of its merges (8, 16, ..), around the longest that fit a tile with
+a step of 512 (3584, above which a block goes on by radix sort) and across tiles; long repeats (many
 rounds), equal rotations, and blocks of both kinds in one slab.  The suffix
 array equals the oracle's exactly; streams equal the oracle's byte for byte."""
 import numpy as np
@@ -29,7 +29,7 @@ def _check(torch, a):
     assert np.array_equal(B.bwt(d).cpu().numpy(), oracle.bwt(a))
 
 
-@pytest.mark.parametrize("k", [2, 7, 8, 9, 15, 16, 17, 63, 64, 65, 1023, 1025, 2047, 2048, 2049,
+@pytest.mark.parametrize("k", [2, 7, 8, 9, 15, 16, 17, 63, 64, 65, 1023, 1025, 2047, 2048, 2049, 3583, 3584, 3585,
                                4095, 4097, 9000])
 def test_group_sizes(torch_cuda, k):
     _check(torch_cuda, _groups([k, 3, 1, 5], k))
@@ -38,7 +38,7 @@ def test_group_sizes(torch_cuda, k):
 def test_many_groups_across_tiles(torch_cuda):
     rng = np.random.default_rng(3)
     _check(torch_cuda, _groups(rng.integers(1, 300, 300).tolist(), 4))
-    _check(torch_cuda, _groups([2048, 2047, 2, 2048, 1, 2046, 3], 5))
+    _check(torch_cuda, _groups([2048, 2047, 2, 2048, 1, 2046, 3, 3584], 5))
 
 
 @pytest.mark.parametrize("period,copies", [(1, 5000), (2, 4100), (17, 2048), (17, 2049),
