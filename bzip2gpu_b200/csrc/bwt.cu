@@ -128,7 +128,7 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
 // a fence that publishes the counts) runs the block's scan over its tiles'
 // counts, so the pass needs no scan launch of its own.
 template <int RB>
-__global__ void __launch_bounds__(256) k_radix_hist(SlabDev d, int shift, const int32_t *list,
+__global__ void __launch_bounds__(256, 8) k_radix_hist(SlabDev d, int shift, const int32_t *list,
                                                     int gen, int pass) {
   constexpr int kN = 1 << RB;
   __shared__ uint32_t cnt[kN];
@@ -186,7 +186,7 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
   const int t0 = (int)(d.off[b] / kTile);
   uint32_t *H = d.tile_hist + (size_t)t0 * kN + kD * threadIdx.x;
   // many tiles' counts in flight at a time (the loads are independent)
-  constexpr int kU = kD == 1 ? 20 : 8;
+  constexpr int kU = kD == 1 ? 16 : 8;
   uint32_t run[kD];
 #pragma unroll
   for (int q = 0; q < kD; q++) run[q] = 0;
