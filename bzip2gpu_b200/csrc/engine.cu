@@ -143,6 +143,7 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     dev.freq = (int32_t *)alloc(B * kMaxAlpha * 4);
     dev.len = (uint8_t *)alloc(B * kMaxGroups * kMaxAlpha);
     dev.code = (int32_t *)alloc(B * kMaxGroups * kMaxAlpha * 4);
+    dev.len_code = (uint32_t *)alloc(B * kLenCode * 4);
     dev.rfreq = (int32_t *)alloc(B * kMaxGroups * kMaxAlpha * 4);
     dev.learned = (int32_t *)alloc(B * 4);
     dev.rfreq_m = (int32_t *)alloc(B * kMaxGroups * kMaxAlpha * 4);

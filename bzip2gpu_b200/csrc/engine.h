@@ -49,6 +49,7 @@ struct SlabPlan {
 };
 
 constexpr int kGroupTile = 128;  // 50-symbol groups per group tile
+constexpr int kLenCode = (kMaxGroups * kMaxAlpha + 3) / 4 * 4;  // 16-byte multiples
 constexpr int kMaxRadix = 512;   // widest radix sort digit (9 bits)
 
 // Device pointers of one slab, passed to kernels by value.
@@ -81,6 +82,7 @@ struct SlabDev {
   int32_t *freq;                       // [nblocks * 258]
   uint8_t *len;                        // [nblocks * 6 * 258]
   int32_t *code;                       // [nblocks * 6 * 258]
+  uint32_t *len_code;                  // [nblocks * kLenCode]: len << 24 | code, in rows of 258
   int32_t *rfreq;                      // [nblocks * 6 * 258]
   int32_t *learned;                    // [nblocks]: table selection by the learned selector
   int32_t *rfreq_m;                    // [nblocks * 6 * 258]: the MLP's per-table counts

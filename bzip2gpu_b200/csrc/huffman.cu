@@ -533,19 +533,25 @@ __device__ int64_t predicted_bits(const SlabDev &d, int b, const uint8_t *len_ba
 
 // Learned form, after the second passes: a learned block whose predicted
 // size exceeds that of the plain selector's first two passes takes the
-// plain two-pass selection (sel2, len2) instead.
-__global__ void k_huff_judge(SlabDev d) {
+// plain two-pass selection (sel2, len2) instead.  A warp for each prediction,
+// the CTA for the copy (by one warp it took 77 us a slab).
+__global__ void __launch_bounds__(256) k_huff_judge(SlabDev d) {
+  __shared__ int64_t bits[2];
   const int b = blockIdx.x;
   if (!d.learned[b]) return;
-  const int64_t el = predicted_bits(d, b, d.len, d.rfreq);
-  const int64_t ep = predicted_bits(d, b, d.len2, d.rfreq2);
-  if (el <= ep) return;
+  const int w = warp_id();
+  if (w < 2) {
+    const int64_t e = predicted_bits(d, b, w ? d.len2 : d.len, w ? d.rfreq2 : d.rfreq);
+    if (lane_id() == 0) bits[w] = e;
+  }
+  __syncthreads();
+  if (bits[0] <= bits[1]) return;
   const size_t tb = (size_t)b * kMaxGroups * kMaxAlpha;
-  for (int i = lane_id(); i < kMaxGroups * kMaxAlpha; i += 32) d.len[tb + i] = d.len2[tb + i];
+  for (int i = threadIdx.x; i < kMaxGroups * kMaxAlpha; i += 256) d.len[tb + i] = d.len2[tb + i];
   const int64_t s0 = d.off[b] / 32;
   const int nsel = d.n_sel[b];
-  for (int g = lane_id(); g < nsel; g += 32) d.sel[s0 + g] = d.sel2[s0 + g];
-  if (lane_id() == 0) {
+  for (int g = threadIdx.x; g < nsel; g += 256) d.sel[s0 + g] = d.sel2[s0 + g];
+  if (threadIdx.x == 0) {
     d.learned[b] = 0;
     d.plain_left[b] = 0;
   }
@@ -566,6 +572,7 @@ __global__ void __launch_bounds__(kMaxGroups * 32) k_huff_codes(SlabDev d) {
   const int alpha = d.n_in_use[b] + 2;
   const uint8_t *len = d.len + ((size_t)b * kMaxGroups + t) * kMaxAlpha;
   int32_t *code = d.code + ((size_t)b * kMaxGroups + t) * kMaxAlpha;
+  uint32_t *both = d.len_code + (size_t)b * kLenCode + t * kMaxAlpha;  // for the payload
   int lv[kCodeSlots];
   int mn = 32, mx = 0;
 #pragma unroll
@@ -588,7 +595,11 @@ __global__ void __launch_bounds__(kMaxGroups * 32) k_huff_codes(SlabDev d) {
     for (int q = 0; q < kCodeSlots; q++) {
       const bool hit = lv[q] == l;
       const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      if (hit) code[32 * q + ln] = vec + __popc(bal & below);
+      if (hit) {
+        const int c = vec + __popc(bal & below);
+        code[32 * q + ln] = c;
+        both[32 * q + ln] = (uint32_t)l << 24 | (uint32_t)c;
+      }
       vec += __popc(bal);
     }
     vec <<= 1;
@@ -657,7 +668,7 @@ void stage_huffman(const SlabDev &d, cudaStream_t st, const uint8_t *learned, in
     }
     k_huff_lengths<<<dim3(d.nblocks, 2), 32, 0, st>>>(d, kAll, 0, 2);
     BZ_LAUNCH_CHECK();
-    k_huff_judge<<<d.nblocks, 32, 0, st>>>(d);
+    k_huff_judge<<<d.nblocks, 256, 0, st>>>(d);
     BZ_LAUNCH_CHECK();
     // plain blocks (fewer than six tables) finish their four passes
     for (int r = 0; r < kIters - 2; r++) {

@@ -151,9 +151,25 @@ __global__ void __launch_bounds__(kHdrThreads) k_sel_mtf_hdr(SlabDev d) {
   }
 }
 
+// A group tile's symbols, two per word, by 16-byte loads (a tile starts on a
+// 16-byte boundary: off is a multiple of kTile, 128 groups are 12,800 bytes;
+// the buffer has slack past a block's end).  Group g's are at 25 g: threads
+// reading their own groups meet on no bank.
+constexpr int kSymWords = kGroupSize / 2;
+__device__ __forceinline__ void load_groups(const SlabDev &d, int64_t off, int g0, int s,
+                                            uint32_t *sy) {
+  const int sym0 = g0 * kGroupSize;
+  const int n = min(s - sym0, kGroupTile * kGroupSize);
+  const uint4 *src = reinterpret_cast<const uint4 *>(d.rle2 + off + sym0);
+  for (int i = threadIdx.x; i < (n + 7) / 8; i += kGroupTile)
+    reinterpret_cast<uint4 *>(sy)[i] = src[i];
+}
+
 // Payload bits per 50-symbol group; exclusive offsets within the group tile.
 __global__ void __launch_bounds__(kGroupTile) k_pay_bits(SlabDev d, const int32_t *list) {
   __shared__ uint32_t scratch[8];
+  __shared__ __align__(16) uint32_t sy[kGroupTile * kSymWords];
+  __shared__ __align__(4) uint8_t len[kMaxGroups * kMaxAlpha];
   const int gt = list ? list[blockIdx.x] : (int)blockIdx.x;
   const int b = d.gt_block[gt];
   const int g0 = d.gt_first[gt];
@@ -164,13 +180,23 @@ __global__ void __launch_bounds__(kGroupTile) k_pay_bits(SlabDev d, const int32_
   }
   const int s = d.s[b];
   const int64_t off = d.off[b];
+  load_groups(d, off, g0, s, sy);
+  static_assert(kMaxGroups * kMaxAlpha % 4 == 0, "a block's lengths are whole words");
+  for (int i = threadIdx.x; i < kMaxGroups * kMaxAlpha / 4; i += kGroupTile)
+    reinterpret_cast<uint32_t *>(len)[i] =
+        reinterpret_cast<const uint32_t *>(d.len + (size_t)b * kMaxGroups * kMaxAlpha)[i];
+  __syncthreads();
   const int g = g0 + threadIdx.x;
   uint32_t bits = 0;
   if (g < nsel) {
-    const int t = d.sel[off / 32 + g];
-    const uint8_t *len = d.len + ((size_t)b * kMaxGroups + t) * kMaxAlpha;
-    const int a = g * kGroupSize, e = min(a + kGroupSize, s);
-    for (int i = a; i < e; i++) bits += len[d.rle2[off + i]];
+    const uint8_t *lt = len + d.sel[off / 32 + g] * kMaxAlpha;
+    const uint32_t *my = sy + threadIdx.x * kSymWords;
+    const int n = min(kGroupSize, s - g * kGroupSize);
+    for (int i = 0; i < n / 2; i++) {
+      const uint32_t v = my[i];
+      bits += lt[v & 0xffffu] + lt[v >> 16];
+    }
+    if (n & 1) bits += lt[my[n / 2] & 0xffffu];
   }
   uint32_t tot;
   uint32_t ex = block_excl_sum(bits, scratch, &tot);
@@ -305,28 +331,78 @@ __global__ void __launch_bounds__(kHdrThreads) k_write_header(SlabDev d, int64_t
   }
 }
 
-// Payload: one thread per 50-symbol group.
+// Payload: one thread per 50-symbol group.  The tile's bits are assembled in
+// shared memory (a thread's first and last word shared with its neighbours,
+// the ones between its own) and copied out by whole words; only a tile's first
+// and last word meet other tiles' bits (1 GiB: 0.88 ms with every word or-ed
+// into device memory).
+constexpr int kTileWords = kGroupTile * kGroupSize * kMaxCodeLen / 32 + 2;
+
 __global__ void __launch_bounds__(kGroupTile) k_write_payload(SlabDev d, int64_t w0, const int32_t *list) {
+  __shared__ __align__(16) uint32_t sy[kGroupTile * kSymWords];
+  __shared__ __align__(16) uint32_t tab[kLenCode];  // len << 24 | code
+  __shared__ uint32_t ob[kTileWords];
+  __shared__ uint32_t s_bits;
   const int gt = list ? list[blockIdx.x] : (int)blockIdx.x;
   const int b = d.gt_block[gt];
   const int g0 = d.gt_first[gt];
   const int nsel = d.n_sel[b];
-  const int g = g0 + threadIdx.x;
-  if (g >= nsel) return;
+  if (g0 >= nsel) return;
   const int s = d.s[b];
   const int64_t off = d.off[b];
-  const int t = d.sel[off / 32 + g];
-  const uint8_t *len = d.len + ((size_t)b * kMaxGroups + t) * kMaxAlpha;
-  const int32_t *code = d.code + ((size_t)b * kMaxGroups + t) * kMaxAlpha;
-  int64_t bit = d.blk_start[b] + d.hdr_bits[b] + d.gt_bits[gt] + d.grp_bits[off / 32 + g];
-  BitSink w;
-  w.init(d.out, bit - w0 * 32);
-  const int a = g * kGroupSize, e = min(a + kGroupSize, s);
-  for (int i = a; i < e; i++) {
-    int v = d.rle2[off + i];
-    w.put((uint32_t)code[v], len[v]);
+  const int ng = min(kGroupTile, nsel - g0);
+  const int64_t start = d.blk_start[b] + d.hdr_bits[b] + d.gt_bits[gt] - w0 * 32;
+  const uint32_t lead = (uint32_t)(start & 31);
+  load_groups(d, off, g0, s, sy);
+  for (int i = threadIdx.x; i < kLenCode / 4; i += kGroupTile)
+    reinterpret_cast<uint4 *>(tab)[i] =
+        reinterpret_cast<const uint4 *>(d.len_code + (size_t)b * kLenCode)[i];
+  // the last group's offset bounds the words
+  const uint32_t most = lead + d.grp_bits[off / 32 + g0 + ng - 1] + kGroupSize * kMaxCodeLen;
+  for (int i = threadIdx.x; i < min((int)(most / 32 + 1), kTileWords); i += kGroupTile) ob[i] = 0;
+  __syncthreads();
+  const int g = g0 + threadIdx.x;
+  if (g < nsel) {
+    const uint32_t *tt = tab + d.sel[off / 32 + g] * kMaxAlpha;
+    const uint32_t *my = sy + threadIdx.x * kSymWords;
+    const int ns = min(kGroupSize, s - g * kGroupSize);
+    uint32_t bit = lead + d.grp_bits[off / 32 + g];
+    uint32_t word = bit >> 5;
+    int n = (int)(bit & 31);
+    bool mine = n == 0;  // no other thread's bits in this word
+    uint64_t acc = 0;
+    auto put = [&](uint32_t sym) {
+      const uint32_t e = tt[sym];
+      const int nb = (int)(e >> 24);
+      acc = (acc << nb) | (e & 0xffffffu);
+      n += nb;
+      bit += nb;
+      if (n >= 32) {
+        const uint32_t w = (uint32_t)(acc >> (n - 32));
+        if (mine) ob[word] = w;
+        else atomicOr(&ob[word], w);
+        mine = true;
+        word++;
+        n -= 32;
+      }
+    };
+    for (int i = 0; i < ns / 2; i++) {
+      const uint32_t v = my[i];
+      put(v & 0xffffu);
+      put(v >> 16);
+    }
+    if (ns & 1) put(my[ns / 2] & 0xffffu);
+    if (n > 0) atomicOr(&ob[word], (uint32_t)(acc << (32 - n)));
+    if ((int)threadIdx.x == ng - 1) s_bits = bit;
   }
-  w.flush();
+  __syncthreads();
+  const int nw = (int)((s_bits + 31) / 32);
+  uint32_t *out = d.out + (start >> 5);
+  for (int i = threadIdx.x; i < nw; i += kGroupTile) {
+    const uint32_t v = bswap32(ob[i]);
+    if (i == 0 || i == nw - 1) atomicOr(out + i, v);
+    else out[i] = v;
+  }
 }
 
 // Payload only, in the reference's word layout (word w = stream bits
@@ -424,7 +500,9 @@ void stage_place_arena(const SlabDev &d, uint32_t *arena, int64_t w0, int64_t nw
 
 // Copy each block's bits (word-aligned in the arena) to its bit position in
 // the output streams; the output is zeroed, and the first and last word of a
-// block are OR-ed in because neighbours share them.
+// block are OR-ed in because neighbours share them.  kSpliceParts CTAs share a
+// block's words (one CTA per block left the longest blocks to run alone).
+constexpr int kSpliceParts = 8;
 __global__ void __launch_bounds__(256) k_splice(const int64_t *src_addr, const int64_t *dst_bit,
                                                 const int64_t *nbits, uint32_t *out) {
   const int b = blockIdx.x;
@@ -434,7 +512,7 @@ __global__ void __launch_bounds__(256) k_splice(const int64_t *src_addr, const i
   const uint32_t *src = reinterpret_cast<const uint32_t *>(src_addr[b]);
   const int64_t srcw = (L + 31) >> 5;
   const int64_t w_first = D >> 5, w_last = (D + L - 1) >> 5;
-  for (int64_t w = w_first + threadIdx.x; w <= w_last; w += blockDim.x) {
+  for (int64_t w = w_first + blockIdx.y * 256 + threadIdx.x; w <= w_last; w += 256 * kSpliceParts) {
     const int64_t s = w * 32 - D;  // source bit of this word's first bit
     const int64_t a = s >= 0 ? s >> 5 : -1;
     const int sh = (int)(s - a * 32);
@@ -452,7 +530,7 @@ __global__ void __launch_bounds__(256) k_splice(const int64_t *src_addr, const i
 void launch_splice(const int64_t *src_addr, const int64_t *dst_bit, const int64_t *nbits,
                    int nblocks, uint32_t *out, cudaStream_t st) {
   if (nblocks <= 0) return;
-  k_splice<<<nblocks, 256, 0, st>>>(src_addr, dst_bit, nbits, out);
+  k_splice<<<dim3(nblocks, kSpliceParts), 256, 0, st>>>(src_addr, dst_bit, nbits, out);
   BZ_LAUNCH_CHECK();
 }
 
