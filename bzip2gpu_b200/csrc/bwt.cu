@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 
 #include "engine.h"
 
@@ -492,20 +493,24 @@ __global__ void __launch_bounds__(256) k_bwt_keys0(SlabDev d, int packed) {
 // separate keys.
 enum Kind { kPrefixItems, kRoundItems, kKeys };
 
-// Bytes (first sort) that elements k and k + 1 have in common at the front of
-// their keys; a round's keys only agree (1) or not (0).  kWhole: equal keys.
+// How elements k and k + 1 differ: 0 for equal keys, else a number whose
+// highest set byte says how many leading bytes they share (first sort; a
+// round's keys only differ or not).  kFirstByte: from here on, the first byte
+// differs; the first element has all the others before it differ like that.
 template <int kKind>
-constexpr int kWhole = kKind == kPrefixItems ? 4 : kKind == kRoundItems ? 1 : 8;
+using Diff = std::conditional_t<kKind == kKeys, uint64_t, uint32_t>;
+template <int kKind>
+constexpr Diff<kKind> kFirstByte = Diff<kKind>(1) << (8 * (sizeof(Diff<kKind>) - 1));
 
 template <int kKind>
-__device__ __forceinline__ int common(const uint64_t *K, int k, int kb) {
+__device__ __forceinline__ Diff<kKind> difference(const uint64_t *K, int k, int kb) {
   if constexpr (kKind == kPrefixItems) {
     const uint32_t *H = reinterpret_cast<const uint32_t *>(K) + 1;  // the items' high words
-    return __clz(H[2 * k] ^ H[2 * k + 2]) >> 3;
+    return H[2 * k] ^ H[2 * k + 2];
   } else if constexpr (kKind == kRoundItems) {
-    return ((K[k] ^ K[k + 1]) >> kb) == 0;
+    return ((K[k] ^ K[k + 1]) >> kb) != 0;
   } else {
-    return __clzll((long long)(K[k] ^ K[k + 1])) >> 3;
+    return K[k] ^ K[k + 1];
   }
 }
 
@@ -514,14 +519,13 @@ __device__ __forceinline__ int common(const uint64_t *K, int k, int kb) {
 // and singleton counts.  After the first sort it also counts the group heads
 // and singletons of the prefix-1, -2, -4 (, -8) byte partitions: pstat[b*8 + q]
 // heads and pstat[b*8 + 4 + q] singletons of prefix 2^q bytes.  An element
-// heads its group of prefix P when it has fewer than P bytes in common with
-// the one before it, and is alone when the one after it has too: one count of
-// leading zeros gives all partitions (separate compares of each took 142
-// instructions per element and warp).
+// heads its group of prefix P when its first P bytes differ from those before
+// it, i.e. when the difference reaches the P-th byte, and is alone when the
+// one after it differs so too: two differences give all partitions (separate
+// compares of each took 142 instructions per element and warp).
 template <int kKind, bool kInitial>
 __global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, int kb, const int32_t *list) {
   __shared__ int red[2][kSortWarps];
-  constexpr int kAll = kWhole<kKind>;
   constexpr int kQ = !kInitial ? 0 : kKind == kPrefixItems ? 3 : 4;
   const int t = tile_id(list);
   int b, lt;
@@ -540,15 +544,16 @@ __global__ void __launch_bounds__(256) k_bwt_flags(SlabDev d, int kb, const int3
     const int k = lt + e;
     bool hd = false, alone = false;
     if (e < valid) {
-      const int p = k > 0 ? common<kKind>(K, k - 1, kb) : -1;
-      const int n = k + 1 < len ? common<kKind>(K, k, kb) : -1;
-      const int pn = max(p, n);
-      hd = p < kAll;
-      alone = pn < kAll;
+      const Diff<kKind> p = k > 0 ? difference<kKind>(K, k - 1, kb) : ~Diff<kKind>(0);
+      const Diff<kKind> n = k + 1 < len ? difference<kKind>(K, k, kb) : ~Diff<kKind>(0);
+      const Diff<kKind> pn = min(p, n);
+      hd = p != 0;
+      alone = pn != 0;
 #pragma unroll
       for (int q = 0; q < kQ; q++) {
-        pc[q] += p < (1 << q);
-        pc[4 + q] += pn < (1 << q);
+        const Diff<kKind> at = kFirstByte<kKind> >> (8 * ((1 << q) - 1));
+        pc[q] += p >= at;
+        pc[4 + q] += pn >= at;
       }
     }
     const unsigned bm = __ballot_sync(0xffffffffu, hd);

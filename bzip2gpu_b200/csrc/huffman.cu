@@ -216,91 +216,68 @@ __global__ void __launch_bounds__(kGroupTile) k_huff_select(SlabDev d, int which
 // '<', so ties resolve exactly as there: every step leaves the heap in the
 // reference's state.
 // The chain of heap steps is the kernel's time, so a step is made short.  A
-// sift down always follows the lighter children; which child is lighter is
-// kept as one bit per inner node in registers, so the path is seven
-// shift-and-adds, its entries are then loaded and compared all at once (the
-// weights along a path do not fall, so the entries that move up are those not
-// heavier than the moved one), and the entries that moved are written with the
-// path's new bits.  A sift up knows its path from the start.  Slots past the
-// heap hold an infinite weight, so neither tests the heap's size.  One entry
-// after another, a launch took 307 us for 258 symbols.
+// sift down always follows the lighter children, so the path to the bottom is
+// found first, two levels per load, then its entries are compared and written
+// all at once (the weights along a path do not fall, so the entries that move up
+// are those not heavier than the moved one).  A sift up knows its path from the
+// start.  Slots past the heap hold an infinite weight, so neither tests the
+// heap's size.  One entry after another, a launch took 295 us for 258 symbols;
+// this way 144 us, at about 340 instructions per merge.
 // All lanes then walk the parent links for the code lengths, six tables at a
 // time.
 constexpr int kHeapRow = 266;  // entries per table: 16-byte rows, lanes on different banks
 constexpr int kNodeN = kMaxAlpha * 2;
-constexpr uint32_t kInfWeight = 0xFFFFFFFEu;  // one more still fits 32 bits
+constexpr uint32_t kInfWeight = 0xFFFFFFFFu;
 
 __device__ __forceinline__ uint32_t hw(uint64_t e) { return (uint32_t)(e >> 32); }
 
 __device__ __forceinline__ uint64_t pick(bool c, uint64_t x, uint64_t y) { return c ? x : y; }
 
 // Removes the top of a heap of n entries (n is the same for all lanes, n <
-// 2^(L + 1)); light: bit k set when entry 2k + 1 is lighter than entry 2k.
-// Free of branches: entries of the path that do not change are written again.
-// The path goes by the lighter children, so a node's bit flips exactly when
-// the path's new entry below it is no longer the one to take: heavier than its
-// sibling, or as heavy and on the right.
+// 2^(L + 1)).  Two levels per step: a node's children and all its
+// grandchildren are loaded at once, so the path to the bottom by the lighter
+// children takes half as many waits.  Free of branches: entries of the path that
+// do not change are written again.
 template <int L>
-__device__ __forceinline__ uint64_t heap_pop(uint64_t *heap, uint32_t (&light)[4], int n) {
+__device__ __forceinline__ uint64_t heap_pop(uint64_t *heap, int n) {
   const uint64_t top = heap[1], tmp = heap[n];
   heap[n] = (uint64_t)kInfWeight << 32;
-  {
-    const uint32_t off = ~(1u << ((n >> 1) & 31));  // the parent's left child is the lighter one
-    const int w = n >> 6;
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (q == 0 || (q == 1 && L > 5) || (q > 1 && L > 6)) light[q] &= w == q ? off : ~0u;
-  }
-  uint32_t node[L + 1], right[L];
-  uint64_t ch[L];   // the path's entries
-  uint32_t sib[L];  // their siblings' weights
+  uint32_t node[L + 1];
+  uint64_t ch[L];  // the path's entries
   node[0] = 1;
+  auto pair = [&](uint32_t at) { return *reinterpret_cast<const ulonglong2 *>(&heap[at]); };
 #pragma unroll
-  for (int l = 0; l < L; l++) {
+  for (int l = 0; l < L; l += 2) {
     const uint32_t v = node[l];
-    // level l: nodes 2^l .. 2^(l + 1) - 1
-    const uint32_t w = l < 5 ? light[0] : l == 5 ? light[1] : (v & 32u ? light[3] : light[2]);
-    right[l] = (w >> (v & 31)) & 1u;
-    node[l + 1] = 2 * v + right[l];
-    ch[l] = heap[node[l + 1]];
-    sib[l] = reinterpret_cast<const uint32_t *>(heap)[2 * (node[l + 1] ^ 1u) + 1];
+    const ulonglong2 c = pair(2 * v);
+    const bool r = hw(c.y) < hw(c.x);
+    ch[l] = pick(r, c.y, c.x);
+    node[l + 1] = 2 * v + r;
+    if (l + 1 < L) {
+      const ulonglong2 x = pair(4 * v), y = pair(4 * v + 2);
+      const bool rx = hw(x.y) < hw(x.x), ry = hw(y.y) < hw(y.x);
+      const uint64_t mx = pick(rx, x.y, x.x), my = pick(ry, y.y, y.x);
+      ch[l + 1 < L ? l + 1 : l] = pick(r, my, mx);
+      node[l + 2 <= L ? l + 2 : L] = 2 * node[l + 1] + (r ? ry : rx);
+    }
   }
   const uint32_t tw = hw(tmp);
-  uint64_t nv = 0;
   bool here = true;
 #pragma unroll
   for (int l = 0; l <= L; l++) {
     const bool up = l < L && hw(ch[l < L ? l : 0]) <= tw;
-    nv = pick(up, ch[l < L ? l : 0], pick(here, tmp, ch[l > 0 ? l - 1 : 0]));
+    heap[node[l]] = pick(up, ch[l < L ? l : 0], pick(here, tmp, ch[l > 0 ? l - 1 : 0]));
     here = up;
-    heap[node[l]] = nv;
-    if (l > 0) {
-      const bool flip = hw(nv) + right[l - 1] > sib[l - 1];
-      const uint32_t bit = flip ? 1u << (node[l - 1] & 31) : 0u;
-      if (l - 1 < 5) {
-        light[0] ^= bit;
-      } else if (l - 1 == 5) {
-        light[1] ^= bit;
-      } else {
-        light[2] ^= node[l - 1] & 32u ? 0u : bit;
-        light[3] ^= node[l - 1] & 32u ? bit : 0u;
-      }
-    }
   }
   return top;
 }
 
-// Adds e at slot z (the same for all lanes, z < 2^(L + 1)).  kBits: keep
-// `light` up to date.
-template <int L, bool kBits>
-__device__ __forceinline__ void heap_push(uint64_t *heap, uint32_t (&light)[4], int z, uint64_t e) {
+// Adds e at slot z (the same for all lanes, z < 2^(L + 1)).
+template <int L>
+__device__ __forceinline__ void heap_push(uint64_t *heap, int z, uint64_t e) {
   uint64_t anc[L];
-  uint32_t sib[L];
 #pragma unroll
-  for (int l = 0; l < L; l++) {
-    anc[l] = heap[z >> (l + 1)];  // past the root: entry 0, weight 0
-    if (kBits) sib[l] = reinterpret_cast<const uint32_t *>(heap)[2 * ((z >> l) ^ 1) + 1];
-  }
+  for (int l = 0; l < L; l++) anc[l] = heap[z >> (l + 1)];  // past the root: entry 0, weight 0
   const uint32_t ew = hw(e);
   bool here = true;
 #pragma unroll
@@ -310,21 +287,6 @@ __device__ __forceinline__ void heap_push(uint64_t *heap, uint32_t (&light)[4], 
     const uint64_t nv = pick(down, anc[l < L ? l : 0], pick(here, e, anc[l > 0 ? l - 1 : 0]));
     here = down;
     if ((z >> l) >= 1) heap[z >> l] = nv;
-    if (kBits && l < L) {
-      const bool odd = (z >> l) & 1;
-      const uint32_t x = odd ? hw(nv) : sib[l], y = odd ? sib[l] : hw(nv);
-      const int par = z >> (l + 1);
-      const uint32_t bit = par > 0 ? 1u << (par & 31) : 0u;
-      // a parent's word: slot z's by its number, further up by the level
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (q == 0 || (l == 0 && q == 1 && L > 5) || (l == 0 && q > 1 && L > 6) ||
-            (l == 1 && q == 1 && L > 6)) {
-          const uint32_t m = (par >> 5) == q ? bit : 0u;
-          light[q] = (light[q] & ~m) | (x < y ? m : 0u);
-        }
-      }
-    }
   }
 }
 
@@ -340,14 +302,14 @@ __device__ __forceinline__ uint64_t merged(uint64_t p1, uint64_t p2, int node, i
 }
 
 template <int L>
-__device__ __forceinline__ void merge_down(uint64_t *heap, uint32_t (&light)[4], int16_t *parent,
-                                           int down_to, int &n, int &n_nodes) {
+__device__ __forceinline__ void merge_down(uint64_t *heap, int16_t *parent, int down_to, int &n,
+                                           int &n_nodes) {
 #pragma unroll 1
   while (n > down_to) {
-    const uint64_t p1 = heap_pop<L>(heap, light, n);
-    const uint64_t p2 = heap_pop<L>(heap, light, n - 1);
+    const uint64_t p1 = heap_pop<L>(heap, n);
+    const uint64_t p2 = heap_pop<L>(heap, n - 1);
     const uint64_t e = merged(p1, p2, ++n_nodes, parent);
-    heap_push<L, true>(heap, light, n - 1, e);
+    heap_push<L>(heap, n - 1, e);
     n--;
   }
 }
@@ -429,15 +391,15 @@ __global__ void __launch_bounds__(32) k_huff_lengths(SlabDev d, int which, int r
     uint64_t *heap = heap_s[run ? ln : 0];
     int16_t *parent = parent_s[run ? ln : 0];
     int n = alpha, n_nodes = alpha;
-    uint32_t light[4] = {0, 0, 0, 0};
     if (run) {
       const int32_t *leafw = leafw_s[ln];
       for (int i = 1; i <= alpha; i++) {
         const uint64_t e = ((uint64_t)(uint32_t)leafw[i] << 32) | (uint32_t)i;
         parent[i] = -1;
         if (wide || i > 255) heap_push_slow(heap, i, e);
-        else if (i > 31) heap_push<7, false>(heap, light, i, e);
-        else heap_push<4, false>(heap, light, i, e);
+        else if (i > 127) heap_push<7>(heap, i, e);
+        else if (i > 31) heap_push<6>(heap, i, e);
+        else heap_push<4>(heap, i, e);
       }
       while (n > (wide ? 1 : 255)) {
         const uint64_t p1 = heap_pop_slow(heap, n);
@@ -448,22 +410,12 @@ __global__ void __launch_bounds__(32) k_huff_lengths(SlabDev d, int which, int r
       }
     }
     __syncwarp();
-    if (!wide) {
-      // which children are lighter, all nodes at once (lane t keeps table t's)
-      for (int t = 0; t < ngrp; t++) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const ulonglong2 pr = *reinterpret_cast<const ulonglong2 *>(&heap_s[t][2 * (32 * q + ln)]);
-          const unsigned m = __ballot_sync(0xffffffffu, hw(pr.y) < hw(pr.x));
-          if (ln == t) light[q] = m;
-        }
-      }
-      if (run) {
-        merge_down<7>(heap, light, parent, 127, n, n_nodes);
-        merge_down<6>(heap, light, parent, 63, n, n_nodes);
-        merge_down<5>(heap, light, parent, 31, n, n_nodes);
-        merge_down<4>(heap, light, parent, 1, n, n_nodes);
-      }
+    if (run && !wide) {
+      merge_down<7>(heap, parent, 127, n, n_nodes);
+      merge_down<6>(heap, parent, 63, n, n_nodes);
+      merge_down<5>(heap, parent, 31, n, n_nodes);
+      merge_down<4>(heap, parent, 15, n, n_nodes);
+      merge_down<3>(heap, parent, 1, n, n_nodes);
     }
     __syncwarp();
     bool too_long[kMaxGroups] = {};

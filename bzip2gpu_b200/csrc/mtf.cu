@@ -30,13 +30,26 @@ __global__ void __launch_bounds__(256) k_mtf_last(SlabDev d, const int32_t *list
   const uint8_t *T = d.rle1 + off;
   const int32_t *SA = d.sa + off;
   uint8_t *L = d.last + off;
-  for (int e = threadIdx.x; e < valid; e += blockDim.x) {
-    int j = lt + e;
-    int i = SA[j];
-    if (i == 0) d.orig_ptr[b] = j;
-    uint8_t c = T[i == 0 ? m - 1 : i - 1];
-    L[j] = c;
-    atomicMax(&lastpos[c], j);
+  // The last column comes in runs, and a run's last position is what counts: a
+  // lane whose neighbour holds the same symbol leaves the shared-memory maximum
+  // to it.
+  int sa[kTileItems];
+#pragma unroll
+  for (int k = 0; k < kTileItems; k++) {
+    const int e = 256 * k + (int)threadIdx.x;
+    sa[k] = e < valid ? SA[lt + e] : -1;
+  }
+#pragma unroll
+  for (int k = 0; k < kTileItems; k++) {
+    const int j = lt + 256 * k + (int)threadIdx.x;
+    int c = 256;
+    if (sa[k] >= 0) {
+      if (sa[k] == 0) d.orig_ptr[b] = j;
+      c = T[sa[k] == 0 ? m - 1 : sa[k] - 1];
+      L[j] = (uint8_t)c;
+    }
+    const int next = __shfl_down_sync(0xffffffffu, c, 1);
+    if (c < 256 && (c != next || lane_id() == 31)) atomicMax(&lastpos[c], j);
   }
   __syncthreads();
   // thread k stands for symbol k: the symbols present in the tile are those
