@@ -39,7 +39,7 @@ namespace {
 constexpr int kSortWarps = kTileThreads / 32;  // 8
 constexpr int kWarpSpan = kTile / kSortWarps;   // elements per warp in a tile (512)
 // Digits of the doubling rounds' sorts may be 9 bits wide (fewer passes over
-// the 2kb key bits); the tile and block digit tables (tile_hist, sort_base)
+// the 2kb key bits); the tile and group digit tables (tile_hist, scan_base)
 // are sized for kMaxRadix digits.  Shared memory of the scatter: the tile's
 // keys (and values), per-warp digit counts, two digit tables.
 template <int RB>
@@ -119,115 +119,194 @@ __device__ __forceinline__ int keys_before(const SlabDev &d, int pass) {
 }
 __device__ __forceinline__ int keys_now(const SlabDev &d) { return keys_before(d, 31); }
 
+// Packed items leave the value buffers free; vals[0] holds the digit of each
+// item for the coming pass, written by the pass before it (by k_bwt_round_keys
+// for a round's first), so that the histogram reads 1 or 2 bytes per item
+// instead of 8.
 template <int RB>
-__device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int force, int pass,
-                                                 uint32_t *scratch);
+using DigitT = std::conditional_t<RB == 8, uint8_t, uint16_t>;
+template <int RB>
+__device__ __forceinline__ DigitT<RB> *next_digits(const SlabDev &d) {
+  return reinterpret_cast<DigitT<RB> *>(d.vals[0]);
+}
+
+template <int RB>
+__device__ __forceinline__ void digit_scan(const SlabDev &d, int t, int force, int pass,
+                                           uint32_t *scratch);
+// The group of a block's tile t: kScanTiles tiles, of this block only.
+__device__ __forceinline__ int scan_group(int t, int b) { return t / kScanTiles + b; }
 
 // gen != 0: the generating first pass (items from the text, see text_item;
 // 8-bit digits).  RB: digit width, tile_hist holds 2^RB counts per tile.
-// The last tile of a block to finish its counts (a per-block counter, after
-// a fence that publishes the counts) runs the block's scan over its tiles'
-// counts, so the pass needs no scan launch of its own.
-// Bound by the latency of its loads, not by the counting (DRAM 51 %, LSU 35 %):
-// a thread's 16 loads are all issued first, and of a digit that is a byte of
-// the items only that byte is loaded.  1 GiB of text, 16 launches: 2.30 -> 1.76 ms
-// (32 registers, 8 CTAs per SM; with 40 registers and 6 CTAs 1.87).
+// The last tile of a group to finish its counts (a counter, after a fence that
+// publishes the counts) runs the scan over the group's counts (digit_scan), so
+// the pass needs no scan launch of its own.
+// Bound by the latency of a tile's chain of loads, counts, fence and counter
+// (4 to 5 us whatever the bytes): a CTA takes kHistTiles entries of the list, two
+// warps each, a thread's loads are 16 bytes of digits, all issued before the
+// counting.  Reading the items (8 bytes each) a tile per CTA took 1.76 + 0.92 ms
+// (8- and 9-bit digits) for 1 GiB of text and 6.3 ms for 64 MiB of long repeats;
+// now 0.92 + 0.50 and 3.5, for 0.4 ms more in the scatter of the first and 0.5
+// of the second.
+constexpr int kHistTiles = 4;
+
+// Counts the digits of 16 loaded bytes that lie in [from, to) of the chunk.
 template <int RB>
-__global__ void __launch_bounds__(256, 8) k_radix_hist(SlabDev d, int shift, const int32_t *list,
-                                                       int gen, int pass) {
-  constexpr int kN = 1 << RB;
-  __shared__ uint32_t cnt[kN];
-  const int t = tile_id(list);
-  int b, lt;
-  int valid = tile_valid(d, t, d.sort_len, &b, &lt);
-  if (valid == 0) return;
-  for (int i = threadIdx.x; i < kN; i += blockDim.x) cnt[i] = 0;
-  __syncthreads();
-  const uint64_t *K = d.keys[keys_before(d, pass)] + d.off[b] + lt;
-  const uint8_t *T = d.rle1 + d.off[b];
-  const int m = d.m[b];
-  // all of a thread's loads before the first count: their latency is this
-  // kernel's time
-  uint32_t dg[kTileItems];
-  if (gen) {
-    // digit bits [shift, shift + 8) of the item are byte 3 - (shift - 32) / 8
-    // of the rotation's 4-byte prefix
-    const int q = 3 - (shift - 32) / 8;
-#pragma unroll
-    for (int i = 0; i < kTileItems; i++) {
-      int j = lt + 256 * i + (int)threadIdx.x + q;
-      while (j >= m) j -= m;
-      dg[i] = T[j];
-    }
-  } else if (RB == 8 && (shift & 7) == 0) {
-    // a byte of the items
-    const uint8_t *B = reinterpret_cast<const uint8_t *>(K) + shift / 8;
-#pragma unroll
-    for (int i = 0; i < kTileItems; i++) {
-      const int e = 256 * i + threadIdx.x;
-      dg[i] = e < valid ? B[8 * e] : 0;
-    }
-  } else {
-    const Digit<RB, false> dig(shift);
-#pragma unroll
-    for (int i = 0; i < kTileItems; i++) {
-      const int e = 256 * i + threadIdx.x;
-      dg[i] = e < valid ? dig(K[e]) : 0;
-    }
+__device__ __forceinline__ void count_chunk(uint32_t *cnt, const uint4 &v, int from, int to) {
+  constexpr int kPer = 16 / (int)sizeof(DigitT<RB>);
+  const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+  // sorted items come in long runs of equal digits: one count for all
+  if (from <= 0 && to >= kPer && v.x == v.y && v.x == v.z && v.x == v.w &&
+      v.x == __funnelshift_l(v.x, v.x, RB == 8 ? 8 : 16)) {
+    atomicAdd(&cnt[RB == 8 ? v.x & 255u : v.x & 0xffffu], (uint32_t)kPer);
+    return;
   }
 #pragma unroll
-  for (int i = 0; i < kTileItems; i++)
-    if (256 * i + (int)threadIdx.x < valid) atomicAdd(&cnt[dg[i]], 1u);
-  __syncthreads();
-  for (int i = threadIdx.x; i < kN; i += blockDim.x) d.tile_hist[(size_t)t * kN + i] = cnt[i];
-  __threadfence();
-  __syncthreads();
-  __shared__ int s_last;
-  __shared__ uint32_t scratch[40];
-  if (threadIdx.x == 0) {
-    const int nt = (d.sort_len[b] + kTile - 1) / kTile;
-    s_last = atomicAdd(&d.blk_count[b], 1) == nt - 1;
+  for (int i = 0; i < kPer; i++) {
+    const uint32_t q = RB == 8 ? __byte_perm(x[i / 4], 0, 0x4440 + i % 4)
+                               : __byte_perm(x[i / 2 % 4], 0, i & 1 ? 0x4432 : 0x4410);
+    if (i >= from && i < to) atomicAdd(&cnt[q], 1u);
   }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  block_digit_scan<RB>(d, b, gen, pass, scratch);
-  if (threadIdx.x == 0) d.blk_count[b] = 0;
 }
 
-// Per block: turn tile digit counts into each tile's count of the digit in
-// the block's earlier tiles (one pass), and the digit's base in the block.
-// force != 0 (the generating pass): the pass runs even if every tile holds one
-// digit only, since it writes the items the later passes read.
-// Thread i handles the kD = 2^RB / 256 consecutive digits kD*i .. kD*i+kD-1.
 template <int RB>
-__device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int force, int pass,
-                                                 uint32_t *scratch) {
-  constexpr int kN = 1 << RB, kD = kN / 256;
-  const int len = d.sort_len[b];
-  const int nt = (len + kTile - 1) / kTile;
-  const int t0 = (int)(d.off[b] / kTile);
-  uint32_t *H = d.tile_hist + (size_t)t0 * kN + kD * threadIdx.x;
-  // many tiles' counts in flight at a time (the loads are independent)
-  constexpr int kU = kD == 1 ? 16 : 8;
-  uint32_t run[kD];
+__global__ void __launch_bounds__(256, 6) k_radix_hist(SlabDev d, int shift, const int32_t *list,
+                                                       int ntiles, int gen, int packed, int pass) {
+  constexpr int kN = 1 << RB, kThreads = 256 / kHistTiles;
+  __shared__ uint32_t counts[kHistTiles][kN];
+  __shared__ int s_last[kHistTiles];  // this tile, where it was the last of its group, or -1
+  __shared__ uint32_t scratch[40];
+  const int p = threadIdx.x / kThreads, u = threadIdx.x % kThreads;
+  uint32_t *cnt = counts[p];
+  const int entry = blockIdx.x * kHistTiles + p;
+  int t = 0, b = 0, lt = 0, valid = 0;
+  if (entry < ntiles) {
+    t = list ? list[entry] : entry;
+    valid = tile_valid(d, t, d.sort_len, &b, &lt);
+  }
+  for (int i = u; i < kN; i += kThreads) cnt[i] = 0;
+  if (u == 0) s_last[p] = -1;
+  __syncthreads();
+  // the pass before wrote this one's digits if it ran
+  const bool ready = packed && !gen && (pass == 0 || ((d.sort_ctl[1] >> (pass - 1)) & 1));
+  if (valid > 0 && (ready || gen)) {
+    // gen: digit bits [shift, shift + 8) of the item are byte q of the
+    // rotation's 4-byte prefix: the tile's text from q on, and the q bytes after it
+    const int q = gen ? 3 - (shift - 32) / 8 : 0;
+    const uint8_t *T = d.rle1 + d.off[b];
+    const uint4 *D = gen ? reinterpret_cast<const uint4 *>(T + lt)
+                         : reinterpret_cast<const uint4 *>(next_digits<RB>(d) + d.off[b] + lt);
+    constexpr int kPer = 16 / (int)sizeof(DigitT<RB>);
+    constexpr int kLoads = 4;
 #pragma unroll
-  for (int q = 0; q < kD; q++) run[q] = 0;
-  for (int k0 = 0; k0 < nt; k0 += kU) {
+    for (int e0 = 0; e0 < kTile; e0 += kLoads * kThreads * kPer) {
+      uint4 v[kLoads];
+#pragma unroll
+      for (int i = 0; i < kLoads; i++) {
+        const int c = e0 / kPer + i * kThreads + u;
+        if (c * kPer < valid) v[i] = D[c];
+      }
+#pragma unroll
+      for (int i = 0; i < kLoads; i++) {
+        const int e = e0 + (i * kThreads + u) * kPer;
+        if (e < valid) count_chunk<RB>(cnt, v[i], q - e, valid - e);
+      }
+    }
+    if (u < min(q, valid)) {
+      // (of a tile shorter than q, the whole window lies past its end)
+      const int m = d.m[b];
+      int j = lt + max(valid, q) + u;
+      while (j >= m) j -= m;
+      atomicAdd(&cnt[T[j]], 1u);
+    }
+  } else if (valid > 0) {
+    const uint64_t *K = d.keys[keys_before(d, pass)] + d.off[b] + lt;
+    const Digit<RB, false> dig(shift);
+#pragma unroll 8
+    for (int e = u; e < valid; e += kThreads) atomicAdd(&cnt[dig(K[e])], 1u);
+  }
+  __syncthreads();
+  if (valid > 0)
+    for (int i = u; i < kN; i += kThreads) d.tile_hist[(size_t)t * kN + i] = cnt[i];
+  __threadfence();
+  __syncthreads();
+  if (u == 0 && valid > 0) {
+    const int t0 = t - lt / kTile, nt = (d.sort_len[b] + kTile - 1) / kTile;
+    const int tiles = min(t0 + nt, (t | (kScanTiles - 1)) + 1) - max(t0, t & -kScanTiles);
+    if (atomicAdd(&d.scan_count[scan_group(t, b)], 1) == tiles - 1) s_last[p] = t;
+  }
+  __syncthreads();
+  for (int k = 0; k < kHistTiles; k++)
+    if (s_last[k] >= 0) digit_scan<RB>(d, s_last[k], gen, pass, scratch);
+}
+
+// Adds n rows of digit counts to `run`, and (kWrite) replaces each row by what
+// `run` was before it.  Thread i handles the kD = 2^RB / 256 consecutive digits
+// kD*i .. kD*i+kD-1; a row's loads are independent, kU are in flight.
+template <int RB, bool kWrite>
+__device__ __forceinline__ void scan_rows(uint32_t *rows, int n, uint32_t *run) {
+  constexpr int kN = 1 << RB, kD = kN / 256;
+  constexpr int kU = kD == 1 ? 16 : 8;
+  uint32_t *H = rows + kD * threadIdx.x;
+  for (int k0 = 0; k0 < n; k0 += kU) {
 #pragma unroll
     for (int q = 0; q < kD; q++) {
       uint32_t h[kU];
 #pragma unroll
-      for (int j = 0; j < kU; j++) h[j] = k0 + j < nt ? __ldcg(&H[(size_t)(k0 + j) * kN + q]) : 0u;
+      for (int j = 0; j < kU; j++) h[j] = k0 + j < n ? __ldcg(&H[(size_t)(k0 + j) * kN + q]) : 0u;
 #pragma unroll
       for (int j = 0; j < kU; j++) {
-        if (k0 + j < nt) H[(size_t)(k0 + j) * kN + q] = run[q];
+        if (kWrite && k0 + j < n) H[(size_t)(k0 + j) * kN + q] = run[q];
         run[q] += h[j];
       }
     }
   }
-  // the digit's base in the block (exclusive sum over digits of the block's
-  // counts), added by the scatter to each tile's count before it
+}
+
+// By the CTA that counted the last tile of a group of kScanTiles tiles: each
+// tile's count of a digit becomes that of the group's earlier tiles.  The last
+// group of a block turns the groups' sums into where the digit's items of each
+// group go (scan_base).  One CTA per block over all the block's tiles took 10
+// to 25 us at the end of a launch (64 MiB of long repeats, 186 launches: 4.0 ms,
+// in groups 3.5).
+// force != 0 (the generating pass): the pass runs even if every tile holds one
+// digit only, since it writes the items the later passes read.
+template <int RB>
+__device__ __forceinline__ void digit_scan(const SlabDev &d, int t, int force, int pass,
+                                           uint32_t *scratch) {
+  constexpr int kN = 1 << RB, kD = kN / 256;
+  __shared__ int s_end;
+  const int b = d.tile_block[t];
+  const int len = d.sort_len[b];
+  const int t0 = (int)(d.off[b] / kTile), t1 = t0 + (len + kTile - 1) / kTile;
+  const int first = max(t0, t & -kScanTiles), g0 = scan_group(t0, b);
+  const int g = scan_group(t, b) - g0, ng = scan_group(t1 - 1, b) - g0 + 1;
+  uint32_t run[kD];
+#pragma unroll
+  for (int q = 0; q < kD; q++) run[q] = 0;
+  __threadfence();
+  scan_rows<RB, true>(d.tile_hist + (size_t)first * kN,
+                      min(t1, (t | (kScanTiles - 1)) + 1) - first, run);
+  uint32_t *base_rows = d.scan_base + (size_t)g0 * kN;
+  uint32_t *SB = base_rows + kD * threadIdx.x;
+  if (threadIdx.x == 0) d.scan_count[g0 + g] = 0;
+  if (ng > 1) {
+#pragma unroll
+    for (int q = 0; q < kD; q++) SB[(size_t)g * kN + q] = run[q];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_end = atomicAdd(&d.blk_count[b], 1) == ng - 1;
+      if (s_end) d.blk_count[b] = 0;
+    }
+    __syncthreads();
+    if (!s_end) return;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < kD; q++) run[q] = 0;
+    scan_rows<RB, false>(base_rows, ng, run);
+  }
+  // the digits' bases (exclusive sum over the digits of the block's counts)
   uint32_t sum = 0;
   bool one = false;
 #pragma unroll
@@ -236,13 +315,20 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
     one |= run[q] == (uint32_t)len;
   }
   uint32_t tot;
-  uint32_t base = block_excl_sum(sum, scratch, &tot);
+  uint32_t base = (uint32_t)d.off[b] + block_excl_sum(sum, scratch, &tot);
   int trivial = __syncthreads_or(one);
   if ((!trivial || force) && threadIdx.x == 0) atomicOr(&d.sort_ctl[1], 1 << pass);
 #pragma unroll
   for (int q = 0; q < kD; q++) {
-    d.sort_base[(size_t)b * kN + kD * threadIdx.x + q] = (uint32_t)d.off[b] + base;
-    base += run[q];
+    const uint32_t c = run[q];
+    run[q] = base;
+    base += c;
+  }
+  if (ng > 1) {
+    scan_rows<RB, true>(base_rows, ng, run);
+  } else {
+#pragma unroll
+    for (int q = 0; q < kD; q++) SB[q] = run[q];
   }
 }
 
@@ -253,7 +339,8 @@ __device__ __forceinline__ void block_digit_scan(const SlabDev &d, int b, int fo
 // All of a thread's loads are issued before the ranking starts.
 template <bool kVals, int RB, bool kHigh>
 __global__ void __launch_bounds__(256, kVals ? 2 : 3)
-    k_radix_scatter(SlabDev d, int shift, int timed, const int32_t *list, int gen, int pass) {
+    k_radix_scatter(SlabDev d, int shift, int next, int timed, const int32_t *list, int gen,
+                    int pass) {
   constexpr int kN = 1 << RB, kD = kN / 256;
   if (!((d.sort_ctl[1] >> pass) & 1)) return;  // every block's items share this digit
   const int t = tile_id(list);
@@ -316,6 +403,7 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   }
   __syncthreads();
   {
+    const uint32_t *SB = d.scan_base + (size_t)scan_group(t, b) * kN;
     // per digit: its local base (exclusive scan over digits of the tile's
     // counts); each warp's count becomes that warp's local start for the
     // digit, and the digit's global base becomes (global - local) base, so
@@ -333,7 +421,7 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
         wcnt[ww * kN + dg] = at;
         at += c;
       }
-      goff[dg] = d.tile_hist[(size_t)t * kN + dg] + d.sort_base[(size_t)b * kN + dg] - lb;
+      goff[dg] = d.tile_hist[(size_t)t * kN + dg] + SB[dg] - lb;
     } else {
       // thread i: the kD consecutive digits kD*i ..
       uint32_t run[kD], sum = 0;
@@ -354,7 +442,7 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
           wcnt[ww * kN + dg] = at;
           at += c;
         }
-        goff[dg] = d.tile_hist[(size_t)t * kN + dg] + d.sort_base[(size_t)b * kN + dg] - lb;
+        goff[dg] = d.tile_hist[(size_t)t * kN + dg] + SB[dg] - lb;
         lb += run[q];
       }
     }
@@ -374,12 +462,15 @@ __global__ void __launch_bounds__(256, kVals ? 2 : 3)
   __syncthreads();
   uint64_t *KO = d.keys[cur ^ 1];
   uint32_t *VO = d.vals[cur ^ 1];
+  DigitT<RB> *DO = next_digits<RB>(d);
+  const Digit<RB, kHigh> ndig(next);
   for (int k = threadIdx.x; k < valid; k += blockDim.x) {
     const uint64_t kk = sk[k];
     const int dg = dig(kk);
     const uint32_t g = goff[dg] + (uint32_t)k;
     KO[g] = kk;
     if (kVals) VO[g] = sv[k];
+    if (!kVals && next >= 0) DO[g] = (DigitT<RB>)ndig(kk);
   }
 }
 
@@ -396,37 +487,41 @@ void radix_passes(const SlabDev &d, int lo, int hi, int has_vals, cudaStream_t s
   int pass = 0;
   for (int shift = lo; shift < hi; shift += RB, pass++) {
     const int g = gen && shift == lo;
-    k_radix_hist<RB><<<grid, 256, 0, st>>>(d, shift, list, g, pass);
+    const int next = shift + RB < hi ? shift + RB : -1;
+    k_radix_hist<RB><<<(grid + kHistTiles - 1) / kHistTiles, 256, 0, st>>>(d, shift, list, grid, g,
+                                                                          !has_vals, pass);
     BZ_LAUNCH_CHECK();
     int timed = -1;
     if (d.kt_on && *d.kt_n < kMaxTimedLaunches) {
       timed = (*d.kt_n)++;
-      d.kt_bpe[timed] = has_vals ? 24 : g ? 9 : 16;  // the generating pass reads text bytes
+      // the generating pass reads text bytes; the next pass's digits are written too
+      d.kt_bpe[timed] = has_vals ? 24 : (g ? 9 : 16) + (next >= 0 ? (int)sizeof(DigitT<RB>) : 0);
       BZ_CUDA(cudaEventRecord(d.kt_ev[2 * timed], st));
     }
     if constexpr (RB == 8) {
       if (has_vals)
-        k_radix_scatter<true, 8, false><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
+        k_radix_scatter<true, 8, false><<<grid, 256, smem, st>>>(d, shift, next, timed, list, 0, pass);
       else if (gen)
-        k_radix_scatter<false, 8, true><<<grid, 256, smem, st>>>(d, shift, timed, list, g, pass);
+        k_radix_scatter<false, 8, true><<<grid, 256, smem, st>>>(d, shift, next, timed, list, g, pass);
       else
-        k_radix_scatter<false, 8, false><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
+        k_radix_scatter<false, 8, false><<<grid, 256, smem, st>>>(d, shift, next, timed, list, 0, pass);
     } else {
-      k_radix_scatter<false, RB, false><<<grid, 256, smem, st>>>(d, shift, timed, list, 0, pass);
+      k_radix_scatter<false, RB, false><<<grid, 256, smem, st>>>(d, shift, next, timed, list, 0, pass);
     }
     BZ_LAUNCH_CHECK();
     if (timed >= 0) BZ_CUDA(cudaEventRecord(d.kt_ev[2 * timed + 1], st));
   }
 }
 
+// 9-bit digits where they take fewer passes than 8-bit ones (10-bit
+// digits also save a pass for 19- and 20-bit rank fields, but their
+// 4x digit tables made the deep rounds of long blocks slower)
+bool wide_digits(int bits) { return (bits + 8) / 9 < (bits + 7) / 8; }
+
 void radix_sort(const SlabDev &d, int lo, int hi, int has_vals, cudaStream_t st, int grid,
                 const int32_t *list, bool gen = false) {
   if (grid <= 0) return;
-  // 9-bit digits where they take fewer passes than 8-bit ones (10-bit
-  // digits also save a pass for 19- and 20-bit rank fields, but their
-  // 4x digit tables made the deep rounds of long blocks slower)
-  const int bits = hi - lo;
-  if (!has_vals && !gen && (bits + 8) / 9 < (bits + 7) / 8)
+  if (!has_vals && !gen && wide_digits(hi - lo))
     radix_passes<9>(d, lo, hi, has_vals, st, grid, list, gen);
   else
     radix_passes<8>(d, lo, hi, has_vals, st, grid, list, gen);
@@ -445,7 +540,10 @@ __global__ void k_bwt_init(SlabDev d) {
   d.act_len[b] = 0;
   d.active_sum[b] = 0;
   d.loc[b] = d.loc_act[b] = d.loc_heads[b] = d.loc_sing[b] = d.gmax[b] = 0;
-  d.blk_count[b] = 0;  // the histogram tile counter: each pass resets it, and so does this
+  // the histogram's counters: each pass resets them, and so does this
+  d.blk_count[b] = 0;
+  const int t0 = (int)(d.off[b] / kTile), t1 = t0 + (m + kTile - 1) / kTile;
+  for (int g = scan_group(t0, b); m > 0 && g <= scan_group(t1 - 1, b); g++) d.scan_count[g] = 0;
   for (int k = 0; k < 8; k++) d.pstat[b * 8 + k] = 0;
   if (m == 1) d.sa[d.off[b]] = 0;
 }
@@ -1126,7 +1224,7 @@ __global__ void __launch_bounds__(256, 3) k_bwt_groups(SlabDev d, int kb) {
 // Round keys for the compacted active rotations: add the rank of i+h.  loc: the
 // list holds units of the blocks sorted group by group, else tiles.
 __global__ void __launch_bounds__(256) k_bwt_round_keys(SlabDev d, int h, int packed, int kb,
-                                                        const int32_t *list, int loc) {
+                                                        const int32_t *list, int loc, int wide) {
   const int t = list[blockIdx.x];
   const int64_t u = (int64_t)t * (loc ? 32 : kTile);
   const int b = d.tile_block[u / kTile];
@@ -1146,7 +1244,11 @@ __global__ void __launch_bounds__(256) k_bwt_round_keys(SlabDev d, int h, int pa
       const uint64_t item = K[e];
       int i2 = (int)(item & mask) + h;
       if (i2 >= m) i2 -= m;
-      K[e] = item | ((uint64_t)(uint32_t)IS[i2] << kb);
+      const uint32_t r = (uint32_t)IS[i2];
+      K[e] = item | ((uint64_t)r << kb);
+      // the first pass's digit, the low bits of the rank
+      if (!loc && wide) next_digits<9>(d)[off + lt + e] = r & 511u;
+      if (!loc && !wide) next_digits<8>(d)[off + lt + e] = (uint8_t)r;
     } else {
       int i2 = (int)V[e] + h;
       if (i2 >= m) i2 -= m;
@@ -1189,6 +1291,7 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
   int kb = 1;
   while ((1ll << kb) <= (int64_t)max_m) kb++;
   const int packed = 3 * kb <= 64;
+  const int wide = wide_digits(2 * kb);  // the rounds' digits
   bool rounds_timed = d.kt_on && d.rt_ev != nullptr;
   if (rounds_timed) {
     d.rt_act[0] = 0;
@@ -1254,11 +1357,11 @@ void stage_bwt(const SlabDev &d, int max_m, cudaStream_t st) {
     }
     // every block's keys before any block's ranks change
     if (grid > 0) {
-      k_bwt_round_keys<<<grid, 256, 0, st>>>(d, (int)prefix, packed, kb, list, 0);
+      k_bwt_round_keys<<<grid, 256, 0, st>>>(d, (int)prefix, packed, kb, list, 0, wide);
       BZ_LAUNCH_CHECK();
     }
     if (lgrid > 0) {
-      k_bwt_round_keys<<<lgrid, 256, 0, st>>>(d, (int)prefix, packed, kb, d.loc_list, 1);
+      k_bwt_round_keys<<<lgrid, 256, 0, st>>>(d, (int)prefix, packed, kb, d.loc_list, 1, 0);
       BZ_LAUNCH_CHECK();
     }
     if (packed)

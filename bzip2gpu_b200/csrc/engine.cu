@@ -166,7 +166,10 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     dev.pay_bits = (int64_t *)alloc(B * 8);
     dev.blk_start = (int64_t *)alloc(B * 8);
     dev.sort_ctl = (int32_t *)alloc(64);
-    dev.sort_base = (uint32_t *)alloc(B * kMaxRadix * 4);
+    const int64_t G = mt / kScanTiles + B;  // groups: t / kScanTiles + b of a block's tiles t
+    dev.scan_base = (uint32_t *)alloc(G * kMaxRadix * 4);
+    dev.scan_count = (int32_t *)alloc(G * 4);
+    BZ_CUDA(cudaMemset(dev.scan_count, 0, G * 4));
     dev.blk_count = (int32_t *)alloc(B * 4);
     BZ_CUDA(cudaMemset(dev.blk_count, 0, B * 4));
     dev.stream = (uint64_t *)alloc(64);

@@ -51,6 +51,7 @@ struct SlabPlan {
 constexpr int kGroupTile = 128;  // 50-symbol groups per group tile
 constexpr int kLenCode = (kMaxGroups * kMaxAlpha + 3) / 4 * 4;  // 16-byte multiples
 constexpr int kMaxRadix = 512;   // widest radix sort digit (9 bits)
+constexpr int kScanTiles = 16;   // tiles whose digit counts one CTA scans
 
 // Device pointers of one slab, passed to kernels by value.
 struct SlabDev {
@@ -71,8 +72,9 @@ struct SlabDev {
   // per-tile scratch
   int32_t *tile_a, *tile_b, *tile_c, *tile_d;  // [ntiles] or [n_raw_tiles]
   uint32_t *tile_hist;                 // [ntiles * kMaxRadix]: radix sort tile digit counts
-  uint32_t *sort_base;                 // [nblocks * kMaxRadix]: radix sort digit bases
-  int32_t *blk_count;                  // [nblocks]: radix sort tiles counted (reset by the last)
+  uint32_t *scan_base;                 // [groups * kMaxRadix]: digit bases of kScanTiles tiles
+  int32_t *scan_count, *blk_count;     // [groups], [nblocks]: radix sort tiles and groups
+                                       // counted (reset by the last)
   int32_t *tile_last;                  // [ntiles * 256]
   uint32_t *gt_bits;                   // [n_group_tiles]
   uint32_t *grp_bits;                  // per group, at sel layout
