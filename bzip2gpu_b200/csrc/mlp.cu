@@ -3,7 +3,8 @@
 // Inference (k_mlp_select): one persistent CTA per SM walks the slab's group
 // tiles (128 groups of 50 symbols each).  Per tile:
 //   warps 0-3  build the 128 x 272 count matrix in shared memory (the MMA's A
-//              operand), then run the epilogues: TMEM -> registers,
+//              operand), start the loads of the next tile's symbols, then run
+//              the epilogues: TMEM -> registers,
 //              scale / bias / ReLU, bf16 back into shared memory as the next
 //              layer's A operand; finally the masked argmax, the selector and
 //              the chosen table's symbol counts;
@@ -16,6 +17,12 @@
 //              layout, so one chunk is one contiguous copy).
 // mbarriers link the roles; every wait is bounded (tc::mbar_wait) and a
 // time-out ends the kernel with an error word instead of a hang.
+// Bound by the serial chain of a tile: counts, epilogues and symbol counts by 128
+// threads, with 4 us of weight copies and MMAs between them.  So every step keeps
+// several accesses in flight: 16-byte symbol loads a tile ahead, four counts
+// read before one is written, the next 32 accumulator columns loaded while
+// 32 are converted, eight copies of the symbol counts (equal symbols meet in
+// shared-memory atomics).  32 MiB of input, about 9 % issue: 253 -> 167 us.
 //
 // Training (k_gemm): a general C = A * B^T with bf16 operands read through
 // arbitrary strides (so transposed operands need no copies), staged by all
@@ -91,12 +98,16 @@ constexpr int kSW3 = kSRing + kStages * kChunkBytes;             // 135,168
 constexpr int kSBias = kSW3 + kW3Bytes;                          // 143,360
 constexpr int kSSym = kSBias + kBiasBytes;                       // 145,472
 constexpr int kSRf = kSSym + kGroupTile * kGroupSize * 2;        // 158,272
-constexpr int kSBar = kSRf + kMaxGroups * kMaxAlpha * 4;         // 164,464
+constexpr int kRfCopies = 8;  // by lane, so that equal symbols meet less often
+constexpr int kSBar = kSRf + kRfCopies * kMaxGroups * kMaxAlpha * 4;  // 207,808
 constexpr int kNBars = 2 * kStages + 8;
 constexpr int kSMisc = kSBar + kNBars * 8;
 constexpr int kSelSmem = kSMisc + 16;
-static_assert(kSRing % 16 == 0 && kSW3 % 16 == 0 && kSBias % 16 == 0 && kSSym % 16 == 0,
-              "bulk copy destinations must be 16-byte aligned");
+static_assert(kSRing % 16 == 0 && kSW3 % 16 == 0 && kSBias % 16 == 0 && kSSym % 16 == 0 &&
+                  kSRf % 16 == 0,
+              "bulk copy destinations and vector accesses must be 16-byte aligned");
+static_assert(kGroupTile * kGroupSize * 2 % 16 == 0, "a tile's symbols start on 16 bytes");
+static_assert(kGroupSize % 2 == 0, "a group's symbols start on 4 bytes");
 static_assert(kSBar % 8 == 0, "mbarriers are 8-byte aligned");
 static_assert(kSelSmem <= 227 * 1024, "shared memory");
 
@@ -134,22 +145,65 @@ __device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
 
 // 32 accumulator columns of one row -> scale, bias, ReLU -> bf16 -> the
 // row's slice of the next layer's A operand (kt = 256).
-__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], float scale,
-                                               const float *bias, uint8_t *act, int row,
-                                               int col0) {
+__device__ __forceinline__ void epilogue_chunk(uint32_t (&r)[32], float scale, const float *bias,
+                                               uint8_t *act, int row, int col0) {
+#pragma unroll
+  for (int c = 0; c < 32; c++) asm volatile("" : "+r"(r[c]));  // not before the wait for them
+  const float4 *b4 = reinterpret_cast<const float4 *>(bias + col0);
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     uint32_t w[4];
 #pragma unroll
-    for (int h = 0; h < 4; h++) {
-      const int c = q * 8 + h * 2;
-      const float a = fmaxf(fmaf(u2f(r[c]), scale, bias[col0 + c]), 0.f);
-      const float b = fmaxf(fmaf(u2f(r[c + 1]), scale, bias[col0 + c + 1]), 0.f);
-      w[h] = pack_bf16x2(a, b);
+    for (int h = 0; h < 2; h++) {
+      const int c = q * 8 + h * 4;
+      const float4 o = b4[c / 4];
+      const float v0 = fmaxf(fmaf(u2f(r[c]), scale, o.x), 0.f);
+      const float v1 = fmaxf(fmaf(u2f(r[c + 1]), scale, o.y), 0.f);
+      const float v2 = fmaxf(fmaf(u2f(r[c + 2]), scale, o.z), 0.f);
+      const float v3 = fmaxf(fmaf(u2f(r[c + 3]), scale, o.w), 0.f);
+      w[2 * h] = pack_bf16x2(v0, v1);
+      w[2 * h + 1] = pack_bf16x2(v2, v3);
     }
     *reinterpret_cast<uint4 *>(act + kmajor_off(row, col0 + q * 8, kHid)) =
         make_uint4(w[0], w[1], w[2], w[3]);
   }
+}
+
+// A hidden layer's 256 columns; the next chunk's load from tensor memory runs
+// while one is converted.
+__device__ __forceinline__ void epilogue(uint32_t tmem, float scale, const float *bias,
+                                         uint8_t *act, int row) {
+  uint32_t ra[32], rb[32];
+  BZ_TMEM_LD32(tmem, ra);
+#pragma unroll
+  for (int c = 0; c < kHid / 32; c += 2) {
+    tmem_wait_ld();
+    BZ_TMEM_LD32(tmem + (c + 1) * 32, rb);
+    epilogue_chunk(ra, scale, bias, act, row, c * 32);
+    tmem_wait_ld();
+    if (c + 2 < kHid / 32) BZ_TMEM_LD32(tmem + (c + 2) * 32, ra);
+    epilogue_chunk(rb, scale, bias, act, row, (c + 1) * 32);
+  }
+}
+
+// Adds the kQ symbols v to row's counts.  All counts are loaded before any is
+// stored; a symbol that occurs again counts those before it, and its later store
+// is the one that stays.
+template <int kQ>
+__device__ __forceinline__ void count_symbols(uint8_t *act, int row, const int (&v)[kQ]) {
+  bf16 *at[kQ];
+  float c[kQ];
+#pragma unroll
+  for (int q = 0; q < kQ; q++) {
+    // symbols are < nInUse + 2 <= 258
+    at[q] = reinterpret_cast<bf16 *>(act + kmajor_off(row, v[q] < kIn ? v[q] : 0, kInPad));
+    c[q] = bf2f(*at[q]) + 1.0f;
+#pragma unroll
+    for (int p = 0; p < q; p++) c[q] += v[p] == v[q] ? 1.0f : 0.0f;
+  }
+#pragma unroll
+  for (int q = 0; q < kQ; q++)
+    if (v[q] < kIn) *at[q] = __float2bfloat16(c[q]);
 }
 
 // wait_ns bounds every wait of the kernel.  withhold != 0 (the failure-path
@@ -278,57 +332,74 @@ __global__ void __launch_bounds__(kSelThreads, 1)
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
     bool stop = compute_any(!mbar_wait(wbar, 0, abort_s, err, 4, wait_ns));
     uint32_t it = 0;
-    for (int gt = blockIdx.x; gt < d.n_group_tiles && !stop; gt += gridDim.x) {
-      int b, g0, nh;
-      if (!tile_active(d, gt, &b, &g0, &nh)) continue;
+    // The next tile's place and symbols (whole 16-byte pieces, the rest one by
+    // one) are loaded while the current tile's layers run.
+    constexpr int kPieces = kGroupTile * kGroupSize / 8;
+    constexpr int kPer = (kPieces + kComputeThreads - 1) / kComputeThreads;
+    uint4 piece[kPer];
+    uint16_t rest = 0;
+    int gt = blockIdx.x, b = 0, g0 = 0, nh = 0, nsym = 0;
+    int64_t off = 0;
+    auto fetch = [&]() {
+      while (gt < d.n_group_tiles && !tile_active(d, gt, &b, &g0, &nh)) gt += gridDim.x;
+      if (gt >= d.n_group_tiles) return;
+      off = d.off[b];
+      nsym = min(d.s[b], (g0 + nh) * kGroupSize) - g0 * kGroupSize;
+      const uint16_t *src = d.rle2 + off + g0 * kGroupSize;
+#pragma unroll
+      for (int q = 0; q < kPer; q++)
+        if (q * kComputeThreads + tid < nsym / 8)
+          piece[q] = reinterpret_cast<const uint4 *>(src)[q * kComputeThreads + tid];
+      if (tid < nsym % 8) rest = src[nsym / 8 * 8 + tid];
+    };
+    fetch();
+    while (gt < d.n_group_tiles && !stop) {
       const uint32_t ph = it & 1;
-      const int64_t off = d.off[b];
-      const int sym0 = g0 * kGroupSize;
-      const int nsym = min(d.s[b], (g0 + nh) * kGroupSize) - sym0;
-      const uint16_t *src = d.rle2 + off + sym0;
-      for (int i = tid; i < nsym; i += kComputeThreads) sym[i] = src[i];
+      const int tile = gt, block = b, n = nsym;
+      uint8_t *sel = d.sel + off / 32 + g0;
+#pragma unroll
+      for (int q = 0; q < kPer; q++)
+        if (q * kComputeThreads + tid < n / 8)
+          reinterpret_cast<uint4 *>(sym)[q * kComputeThreads + tid] = piece[q];
+      if (tid < n % 8) sym[n / 8 * 8 + tid] = rest;
       const uint4 z = make_uint4(0, 0, 0, 0);
       for (int i = tid; i < kGroupTile * kInPad * 2 / 16; i += kComputeThreads)
         reinterpret_cast<uint4 *>(act)[i] = z;
-      for (int i = tid; i < kMaxGroups * kMaxAlpha; i += kComputeThreads) rf[i] = 0;
+      for (int i = tid; i < kRfCopies * kMaxGroups * kMaxAlpha / 4; i += kComputeThreads)
+        reinterpret_cast<uint4 *>(rf)[i] = z;
       compute_any(false);
       // counts of this thread's group: row tid of the A operand
-      const int ga = tid * kGroupSize, ge = min(ga + kGroupSize, nsym);
+      const int ga = tid * kGroupSize, ge = min(ga + kGroupSize, n);
       float inv = 0.f;
       if (ga < ge) {
-        for (int i = ga; i < ge; i++) {
-          const int v = sym[i];
-          if (v >= kIn) continue;  // symbols are < nInUse + 2 <= 258
-          bf16 *p = reinterpret_cast<bf16 *>(act + kmajor_off(tid, v, kInPad));
-          *p = __float2bfloat16(bf2f(*p) + 1.0f);
+        int i = ga;
+        for (; i + 4 <= ge; i += 4) {
+          const uint32_t *w = reinterpret_cast<const uint32_t *>(sym + i);
+          const int v[4] = {(int)(w[0] & 0xffffu), (int)(w[0] >> 16), (int)(w[1] & 0xffffu),
+                            (int)(w[1] >> 16)};
+          count_symbols<4>(act, tid, v);
+        }
+        for (; i < ge; i++) {
+          const int v[1] = {sym[i]};
+          count_symbols<1>(act, tid, v);
         }
         inv = 1.0f / (float)(ge - ga);
       }
       fence_async_smem();
       mbar_arrive(xbar);
+      gt += gridDim.x;
+      fetch();
       // layer 1: scale by 1/size, bias, ReLU -> H1 (kt = 256) over the counts
       if ((stop = compute_any(!mbar_wait(d1bar, ph, abort_s, err, 4, wait_ns)))) break;
       fence_after_sync();
-#pragma unroll 1
-      for (int c = 0; c < kHid / 32; c++) {
-        uint32_t r[32];
-        BZ_TMEM_LD32(tbase + lane_base + c * 32, r);
-        tmem_wait_ld();
-        epilogue_chunk(r, inv, b1, act, tid, c * 32);
-      }
+      epilogue(tbase + lane_base, inv, b1, act, tid);
       fence_async_smem();
       fence_before_sync();
       mbar_arrive(h1bar);
       // layer 2: bias, ReLU -> H2
       if ((stop = compute_any(!mbar_wait(d2bar, ph, abort_s, err, 4, wait_ns)))) break;
       fence_after_sync();
-#pragma unroll 1
-      for (int c = 0; c < kHid / 32; c++) {
-        uint32_t r[32];
-        BZ_TMEM_LD32(tbase + kHid + lane_base + c * 32, r);
-        tmem_wait_ld();
-        epilogue_chunk(r, 1.0f, b2, act, tid, c * 32);
-      }
+      epilogue(tbase + kHid + lane_base, 1.0f, b2, act, tid);
       fence_async_smem();
       fence_before_sync();
       mbar_arrive(h2bar);
@@ -347,19 +418,25 @@ __global__ void __launch_bounds__(kSelThreads, 1)
       for (int t = 1; t < kOut; t++)
         if (lg[t] > lg[best]) best = t;
       if (ga < ge) {
-        d.sel[off / 32 + g0 + tid] = (uint8_t)best;
+        sel[tid] = (uint8_t)best;
+        int *mine = rf + (lane % kRfCopies * kMaxGroups + best) * kMaxAlpha;
+#pragma unroll 10
         for (int i = ga; i < ge; i++)
-          if (sym[i] < kMaxAlpha) atomicAdd(&rf[best * kMaxAlpha + sym[i]], 1);
+          if (sym[i] < kMaxAlpha) atomicAdd(&mine[sym[i]], 1);
         if (logits) {
-          float *o = logits + ((int64_t)gt * kGroupTile + tid) * 8;
+          float *o = logits + ((int64_t)tile * kGroupTile + tid) * 8;
 #pragma unroll
           for (int t = 0; t < kOut; t++) o[t] = lg[t];
         }
       }
       compute_any(false);
-      int32_t *rfreq = rfreq_out + (size_t)b * kMaxGroups * kMaxAlpha;
-      for (int i = tid; i < kMaxGroups * kMaxAlpha; i += kComputeThreads)
-        if (rf[i]) atomicAdd(&rfreq[i], rf[i]);
+      int32_t *rfreq = rfreq_out + (size_t)block * kMaxGroups * kMaxAlpha;
+      for (int i = tid; i < kMaxGroups * kMaxAlpha; i += kComputeThreads) {
+        int sum = 0;
+#pragma unroll
+        for (int q = 0; q < kRfCopies; q++) sum += rf[q * kMaxGroups * kMaxAlpha + i];
+        if (sum) atomicAdd(&rfreq[i], sum);
+      }
       compute_any(false);
       it++;
     }

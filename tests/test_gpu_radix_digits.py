@@ -1,7 +1,7 @@
 """The radix sort's digit counts at their edges: blocks of a few bytes (shorter
 than the 3 bytes the first pass looks ahead), of one tile of 4096 more or less,
 of one group of 16 tiles more or less, blocks whose groups start anywhere in a
-slab, 8- and 9-bit digits, and digits that all items share, so that a pass is
+slab, 8- and 9-bit digits, separate keys and values (over 2^21 rotations), and digits that all items share, so that a pass is
 left out and the next counts the items themselves.  Suffix arrays and streams
 equal the oracle's exactly."""
 import numpy as np
@@ -24,7 +24,8 @@ def _text(m, symbols, seed):
 
 
 @pytest.mark.parametrize("m", [2, 3, 4, 15, 16, 17, 4093, 4094, 4095, 4096, 4097, 4098, 4099, 4100,
-                               65535, 65536, 65537, 65539, 131072, 131073, 200003, 263000, 600001])
+                               65535, 65536, 65537, 65539, 131072, 131073, 200003, 263000, 600001,
+                               (1 << 21) + 5])
 def test_sizes(torch_cuda, m):
     for symbols in (1, 2, 251):
         a = _text(m, symbols, m)
