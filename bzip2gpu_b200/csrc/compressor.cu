@@ -306,16 +306,14 @@ void Compressor::run(const uint8_t *const *ptrs, const int *lens, int nblocks, i
       const int slabs = std::max(1, std::min(nw * rounds, nblocks / kMinSlabBlocks));
       per_slab = std::min(per_slab, std::max(1, (nblocks + slabs - 1) / slabs));
     }
-    // room for per_slab blocks; with an RLE1 cap a block's raw bytes may exceed
-    // max_block_bytes and take the raw room of several
-    int want = std::min(per_slab, nblocks);
+    // room for min(nblocks, slab_blocks) blocks, whatever per_slab is, so that
+    // calls of other sizes find it; with an RLE1 cap a block's raw bytes may
+    // exceed max_block_bytes and take the raw room of several
+    int want = nblocks;
     if (cfg_.m_cap > 0) {
       const int64_t per = align_up(std::max<int64_t>(cfg_.max_block_bytes, 1), 16);
-      for (int b0 = 0; b0 < nblocks; b0 += per_slab) {
-        int64_t raw = 0;
-        for (int b = b0; b < std::min(nblocks, b0 + per_slab); b++) raw += align_up(lens[b], 16);
-        want = (int)std::max<int64_t>(want, std::min<int64_t>(cfg_.slab_blocks, (raw + per - 1) / per));
-      }
+      for (int b = 0; b < nblocks; b++)
+        want = (int)std::max<int64_t>(want, (lens[b] + per - 1) / per);
     }
     reserve(want);
   }
@@ -619,11 +617,14 @@ void Compressor::compress_batch(const Item *items, int count, bool on_device, By
                    [&](int a, int b) { return blks[a].len > blks[b].len; });
   // slabs over the queue: a slab takes up to the tuned block count for its
   // longest (first) block, fewer where the workspace's capacities end, and no
-  // more than a worker's share of the bytes (as in run(): 128 inputs in one
-  // slab 9.9 ms, split over the workers 9.2 ms)
+  // more than a worker's share of the bytes, down to the bytes of kMinSlabBlocks
+  // full blocks (as in run()).  128 inputs, 120 MB: one slab 9.9 ms, split over
+  // the workers 9.2 ms; 43 inputs, 8 MB: 1.72 and 1.65 ms, but 1.78 and 3.96 ms
+  // in the first call after the program has page-locked memory
   reserve(nb);
+  const int64_t least = kMinSlabBlocks * std::max<int64_t>(cfg_.max_block_bytes, 1);
   const int64_t share = std::max<int64_t>(
-      1, ntot / std::max(1, std::min((int)workers_.size(), nb / kMinSlabBlocks)));
+      1, ntot / std::max<int64_t>(1, std::min<int64_t>((int64_t)workers_.size(), ntot / least)));
   const Workspace &ws0 = *workers_[0]->ws;
   std::vector<int> slab_at{0};
   {

@@ -8,7 +8,8 @@
 //      ended), so a magic that happens to appear inside a payload is ignored.
 //   2. k_dec_head / _groups / _syms / _mscan / _emit: header and tables, the
 //      bit position of every 50-symbol group (the one serial chain, hopped 8
-//      codes at a time), the groups' symbols and the inverse move-to-front in
+//      codes at a time; for few blocks a group at a time, from the jumps of
+//      k_dec_lens / _jumps / _starts), the groups' symbols and the inverse move-to-front in
 //      parallel over chunks of 32 groups.  Out: the BWT last column L.
 //   3. k_dec_lf_hist / _scan / _rank: LF vector
 //      tt[C[L[i]] + rank(i)] = i << 8 | L[i] by a stable counting sort.
