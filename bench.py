@@ -311,10 +311,10 @@ def run_stress(args):
                           "bwt_rounds": rows}))
 
 
-# DRAM bytes per algorithmic byte of k_radix_scatter: (255.06 + 203.20) MB /
-# 494.13 MB in an ncu capture of the second pass of the first sort over a
-# 128-block slab (profiles/k_radix_scatter_ncu_full_256MiB.md)
-TRAFFIC_PER_ALGO_BYTE = (255.06 + 203.20) / 494.13
+# DRAM bytes per algorithmic byte of k_radix_scatter: (255.64 + 233.39) MB /
+# 525.01 MB in an ncu capture of the second pass of the first sort over a
+# 128-block slab (profiles/k_radix_scatter_ncu_256MiB.md)
+TRAFFIC_PER_ALGO_BYTE = (255.64 + 233.39) / 525.01
 
 
 def main():
@@ -514,14 +514,14 @@ def main():
     sc_ms = stats["scatter_ms"]
     sc_gbs = stats["scatter_bytes"] / (sc_ms / 1e3) / 1e9 if sc_ms > 0 else 0.0
     # DRAM traffic per launch, scaled from one ncu capture of the scatter
-    # (profiles/k_radix_scatter_ncu_full_256MiB.md: 0.927 DRAM bytes per
+    # (profiles/k_radix_scatter_ncu_256MiB.md: 0.931 DRAM bytes per
     # algorithmic byte) by this launch's algorithmic bytes
     per_launch = stats["scatter_bytes"] / max(stats["scatter_launches"], 1)
     traffic = int(per_launch * TRAFFIC_PER_ALGO_BYTE)
     roof = {"bound": "hbm", "achieved": round(sc_gbs, 1), "peak": peak, "unit": "GB/s",
             "frac": round(sc_gbs / peak, 4), "traffic": traffic,
             "traffic_source": "ncu dram bytes of a first-sort scatter pass (256 MiB stream, "
-                              "128-block slab), 0.927 per algorithmic byte, scaled to this launch",
+                              "128-block slab), 0.931 per algorithmic byte, scaled to this launch",
             "kernel": "k_radix_scatter (BWT radix sort scatter)",
             "launches_per_step": int(stats["scatter_launches"]),
             "avg_launch_us": round(1e3 * sc_ms / max(stats["scatter_launches"], 1), 1),
