@@ -129,8 +129,9 @@ struct ByteCrcTable {
 __device__ const ByteCrcTable c_crc_byte{};
 
 // c_crc_word.v[k][b] = crc0 of the byte b followed by k zero bytes: four
-// independent lookups take a crc0 over a 4-byte word (slicing by 4).
-struct WordCrcTable {
+// independent lookups take a crc0 over a 4-byte word (slicing by 4).  On a
+// 16-byte boundary: crc_word_table_fill copies it by uint4.
+struct alignas(16) WordCrcTable {
   uint32_t v[4][256];
   constexpr WordCrcTable() : v() {
     for (int i = 0; i < 256; ++i) {
@@ -145,8 +146,9 @@ struct WordCrcTable {
 __device__ const WordCrcTable c_crc_word{};
 
 // tbl[k][b] = c_crc_word.v[k][b] (shared memory, 256 threads; the caller
-// synchronises)
+// synchronises; tbl on a 16-byte boundary too)
 __device__ __forceinline__ void crc_word_table_fill(uint32_t (&tbl)[4][256]) {
+  static_assert(alignof(WordCrcTable) % alignof(uint4) == 0, "copied by uint4");
   reinterpret_cast<uint4 *>(&tbl[0][0])[threadIdx.x] =
       reinterpret_cast<const uint4 *>(&c_crc_word.v[0][0])[threadIdx.x];
 }
