@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(32 * kSymWarps)
   __shared__ int32_t base[kDecMaxGroups][kDecMaxCode + 4];
   __shared__ uint16_t perm[kDecMaxGroups][kDecMaxAlpha + 6];
   __shared__ uint16_t sy[kSymWarps][kChunkSyms];
-  __shared__ uint8_t lists[kSymWarps][2][256];
+  __shared__ __align__(4) uint8_t lists[kSymWarps][2][256];
   __shared__ uint32_t used_s[kSymWarps][8];
   const unsigned full = 0xffffffffu;
   const int bi = blockIdx.y;
@@ -1169,7 +1169,7 @@ __global__ void __launch_bounds__(256) k_dec_mscan(const int64_t *cand, const De
 // all its lanes.
 __global__ void __launch_bounds__(32 * kSymWarps)
     k_dec_emit(const DecBlock *res, uint32_t *tt, uint8_t *Lbuf, int cap) {
-  __shared__ uint8_t lists[kSymWarps][256];
+  __shared__ __align__(4) uint8_t lists[kSymWarps][256];
   const unsigned full = 0xffffffffu;
   const int bi = blockIdx.y;
   if (res[bi].status != kDecOk) return;

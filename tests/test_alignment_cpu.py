@@ -28,3 +28,34 @@ def test_tables_read_by_wider_words_are_aligned(name):
     src = _source(name)
     for word, table in re.findall(r"reinterpret_cast<const (\w+) \*>\(&(c_\w+)\.", src):
         assert _table_alignment(src, table) >= WIDE[word], (name, table, word)
+
+
+def _shared_arrays(src):
+    """name -> the smallest alignment among its __shared__ declarations."""
+    res = {}
+    for align, kind, names in re.findall(
+            r"__shared__ (?:__align__\((\d+)\) )?(\w+) ([^;]+);", src):
+        own = {"uint8_t": 1, "uint16_t": 2, "int16_t": 2, "uint64_t": 8, "int64_t": 8}.get(kind, 4)
+        for v in re.findall(r"(\w+)\s*\[", re.sub(r"\[[^\]]*\]", "[", names)):
+            res[v] = min(res.get(v, 1 << 10), max(own, int(align or 0)))
+    return res
+
+
+# shared arrays that kernels reach by wider words through another pointer or a
+# function: (file, array, bytes)
+THROUGH = [("decode.cu", "lists", 4),  # k_dec_syms: lst; k_dec_emit: lists[w]
+           ("decode.cu", "sb", 4),     # load_segments
+           ("rle1.cu", "tbl", 16),     # crc_word_table_fill
+           ("mtf.cu", "tab", 4), ("pack.cu", "sy", 16), ("huffman.cu", "heap_s", 16)]
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu")))
+def test_shared_arrays_read_by_wider_words_are_aligned(name):
+    src = _source(name)
+    for v, n in [(v, n) for f, v, n in THROUGH if f == name]:
+        assert _shared_arrays(src)[v] >= n, (name, v, n)
+    for part in re.split(r"__global__|__device__", src):  # function by function
+        arrays = _shared_arrays(part)
+        for word, v in re.findall(r"reinterpret_cast<(?:const )?(\w+) \*>\(&?(\w+)", part):
+            if v in arrays and word in WIDE:
+                assert arrays[v] >= WIDE[word], (name, v, word)
