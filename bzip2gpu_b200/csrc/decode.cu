@@ -812,7 +812,6 @@ __global__ void __launch_bounds__(256) k_dec_starts(DecTab *tabs, const uint8_t 
                                                     const int32_t *jt0, const uint16_t *jumps) {
   extern __shared__ __align__(16) uint8_t ssm[];
   __shared__ uint8_t sel[kDecMaxSel + 6];
-  __shared__ int s_done;
   const int bi = blockIdx.x, tid = threadIdx.x;
   DecTab &tab = tabs[bi];
   if (tab.status != kDecOk) return;
@@ -821,7 +820,6 @@ __global__ void __launch_bounds__(256) k_dec_starts(DecTab *tabs, const uint8_t 
   for (int q = tid; q < nsel; q += 256) sel[q] = selbuf[(size_t)bi * kDecMaxSel + q];
   uint32_t *gs = gstart + (size_t)bi * kDecMaxSel;
   const uint32_t first = (uint32_t)(tab.pay - cand[bi]);
-  if (tid == 0) s_done = 0;
   const int vec = ng * kJumpTile * 2 / 16;  // 16-byte pieces of a tile's tables
   auto load = [&](int k) {
     if (k < nt) {
@@ -839,10 +837,13 @@ __global__ void __launch_bounds__(256) k_dec_starts(DecTab *tabs, const uint8_t 
   for (int k = k0; k < k0 + kStartStages - 1; k++) load(k);
   int g = 0;             // thread 0's place in the chain
   uint32_t p = first;
+  bool done = false;     // thread 0: the chain has ended
   for (int k = k0; k < nt; k++) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kStartStages - 2));
-    __syncthreads();  // tile k is here for all threads, the tile before it is done with
-    if (s_done) break;
+    // tile k is here for all threads, the tile before it is done with, and all
+    // leave together (a flag in shared memory could be set by the next hop while
+    // a slower warp still reads it)
+    if (__syncthreads_or(done)) break;
     load(k + kStartStages - 1);
     if (tid == 0) {
       // bytes of the tile's tables: a jump is one load and one add
@@ -859,7 +860,7 @@ __global__ void __launch_bounds__(256) k_dec_starts(DecTab *tabs, const uint8_t 
       p = base + (q >> 1);
       if (g >= nsel || v == kDeadJump) {
         tab.ngv = g;  // a dead jump's group is the last with a known start
-        s_done = 1;
+        done = true;
       }
     }
   }
