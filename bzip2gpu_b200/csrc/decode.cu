@@ -867,11 +867,24 @@ __global__ void __launch_bounds__(256) k_dec_starts(DecTab *tabs, const uint8_t 
   asm volatile("cp.async.wait_group 0;");
 }
 
+// How group starts are found: by the rules below, or (BZ2G_DECODE_STARTS =
+// jumps, chains8, chains4) always by the jumps where their scratch fits, or by
+// k_dec_groups with 8 or 4 warps per block.  The decoded bytes are the same.
+enum class Starts { kByRule, kJumps, kChains8, kChains4 };
+Starts starts_choice() {
+  const char *e = std::getenv("BZ2G_DECODE_STARTS");
+  if (!e) return Starts::kByRule;
+  if (!std::strcmp(e, "jumps")) return Starts::kJumps;
+  if (!std::strcmp(e, "chains8")) return Starts::kChains8;
+  if (!std::strcmp(e, "chains4")) return Starts::kChains4;
+  return Starts::kByRule;
+}
+
 // Warps per block: eight where the blocks leave the GPU room (the chain's
 // latency is what counts), four where there are enough blocks to fill it.
 using GroupsKernel = decltype(&k_dec_groups<8>);
-inline GroupsKernel groups_kernel(int nblocks, int sms, int *threads) {
-  const bool few = nblocks <= 6 * sms;
+inline GroupsKernel groups_kernel(int nblocks, int sms, Starts how, int *threads) {
+  const bool few = how == Starts::kChains8 || (how != Starts::kChains4 && nblocks <= 6 * sms);
   *threads = few ? 256 : 128;
   return few ? k_dec_groups<8> : k_dec_groups<4>;
 }
@@ -1998,6 +2011,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const int v = std::atoi(e);
     if (v > 0) bmax = std::min(bmax, v);
   }
+  const Starts starts = starts_choice();
   const int batch = (int)std::min<size_t>(bmax, std::max<size_t>(cands.size(), 1));
   const int cap = kDecCap;
   w.cand.reserve(8 * (size_t)batch);
@@ -2108,7 +2122,8 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
       jt0[q + 1] = (int32_t)std::min<int64_t>((int64_t)jt0[q] + nt, 1 << 30);
     }
     const size_t jbytes = (size_t)jbits * kDecMaxGroups * 2;
-    if (jbits <= kJumpMaxBits && jmax <= 65535 && (jbytes <= w.jumps.cap || jbytes <= freeb / 4)) {
+    const bool few = jbits <= kJumpMaxBits;
+    if ((starts == Starts::kByRule ? few : starts == Starts::kJumps) && jmax <= 65535 && (jbytes <= w.jumps.cap || jbytes <= freeb / 4)) {
       w.jumps.reserve(jbytes);
       w.jt0.reserve(4 * (size_t)(nc + 1));
       w.lutlen.reserve((size_t)nc * kLensBytes);
@@ -2126,7 +2141,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
       BZ_LAUNCH_CHECK();
     }
     int gthreads = 0;
-    const GroupsKernel groups = groups_kernel(nc, w.sms, &gthreads);
+    const GroupsKernel groups = groups_kernel(nc, w.sms, starts, &gthreads);
     groups<<<nc, gthreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>(),
                                     w.gstart.get<uint32_t>(), w.order.get<int32_t>());
     BZ_LAUNCH_CHECK();
