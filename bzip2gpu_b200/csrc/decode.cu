@@ -38,6 +38,7 @@
 #include "common.cuh"
 #include "compressor.h"
 #include "crc.cuh"
+#include "decode_plan.h"
 
 namespace bz2g {
 
@@ -48,11 +49,8 @@ namespace {
 constexpr int kDecMaxGroups = 6;
 constexpr int kDecMaxAlpha = 258;
 constexpr int kDecMaxCode = 20;
-constexpr int kDecMaxSel = 18002;
 constexpr int kLutBits = 8;
-// Per-block capacity of the last column (the reference's 900,000-byte raw
-// blocks can exceed 900,000 RLE1 bytes by up to a quarter).
-constexpr int kDecCap = 1200000;
+static_assert(kDecGroupSyms == kGroupSize, "symbols per group");
 
 enum DecStatus {
   kDecOk = 0,
@@ -164,10 +162,7 @@ struct DecBlock {
 //   k_dec_mscan   the chunks' starting lists and offsets   (a CTA per block)
 //   k_dec_emit    the last column                          (a warp per chunk)
 constexpr int kHeadThreads = 256;
-constexpr int kChunkGroups = 32;
 constexpr int kChunkSyms = kChunkGroups * kGroupSize;  // 1600
-constexpr int kMaxChunks = (kDecMaxSel + kChunkGroups - 1) / kChunkGroups;
-constexpr int kSymWarps = 4;
 
 // Per-block tables.  lj[t][n]: the largest 32-bit window (the stream's next
 // bits, left-justified) that starts with a code of at most n bits, for n in
@@ -919,8 +914,7 @@ __global__ void __launch_bounds__(32 * kSymWarps)
   const DecTab &tab = tabs[bi];
   if (tab.status != kDecOk) return;
   const int ngv = tab.ngv;
-  const int c0 = blockIdx.x * kSymWarps;
-  if (c0 * kChunkGroups >= ngv) return;
+  if ((int)blockIdx.x * kSymWarps * kChunkGroups >= ngv) return;
   const int ng = tab.ng, nuse = tab.nuse;
   for (int i = threadIdx.x; i < ng * (1 << kLutBits); i += blockDim.x)
     (&lut[0][0])[i] = (&tab.lut[0][0])[i];
@@ -932,169 +926,171 @@ __global__ void __launch_bounds__(32 * kSymWarps)
     (&perm[0][0])[i] = (&tab.perm[0][0])[i];
   __syncthreads();
   const int ln = lane_id(), w = warp_id();
-  const int c = c0 + w;
-  if (c * kChunkGroups >= ngv) return;
   SymScratch &out = sym_scratch(tt, bi, cap);
   const int64_t start = cand[bi];
   const int alpha = nuse + 2, eob = nuse + 1;
-  const int ngc = min(kChunkGroups, ngv - c * kChunkGroups);
-  int e_at = INT32_MAX, b_at = INT32_MAX;  // chunk index of this lane's end-of-block, bad code
-  uint32_t e_end = 0;
-  if (ln < ngc) {
-    const int g = c * kChunkGroups + ln;
-    const int t = selbuf[(size_t)bi * kDecMaxSel + g];
-    const int mn = tab.mn[t], mx = tab.mx[t];
-    BitReader br;
-    br.init(words, nwords, start + gstart[(size_t)bi * kDecMaxSel + g]);
-    uint16_t *dst = sy[w] + ln * kGroupSize;
-    for (int i = 0; i < kGroupSize; i++) {
-      const uint32_t x = br.peek32();
-      const uint32_t e = lut[t][x >> (32 - kLutBits)];
-      int sym;
-      if (e) {
-        br.skip((int)(e >> 9));
-        sym = (int)(e & 511u);
-      } else {
-        int n = max(mn, kLutBits + 1);
-        while (n <= mx && x > lj[t][n]) n++;
-        const int idx = n <= mx ? (int)(x >> (32 - n)) - base[t][n] : -1;
-        if (idx < 0 || idx >= alpha) {
-          b_at = ln * kGroupSize + i;
+  const int stride = gridDim.x * kSymWarps;
+  for (int c = (int)blockIdx.x * kSymWarps + w; c * kChunkGroups < ngv; c += stride) {
+    const int ngc = min(kChunkGroups, ngv - c * kChunkGroups);
+    int e_at = INT32_MAX, b_at = INT32_MAX;  // chunk index of this lane's end-of-block, bad code
+    uint32_t e_end = 0;
+    if (ln < ngc) {
+      const int g = c * kChunkGroups + ln;
+      const int t = selbuf[(size_t)bi * kDecMaxSel + g];
+      const int mn = tab.mn[t], mx = tab.mx[t];
+      BitReader br;
+      br.init(words, nwords, start + gstart[(size_t)bi * kDecMaxSel + g]);
+      uint16_t *dst = sy[w] + ln * kGroupSize;
+      for (int i = 0; i < kGroupSize; i++) {
+        const uint32_t x = br.peek32();
+        const uint32_t e = lut[t][x >> (32 - kLutBits)];
+        int sym;
+        if (e) {
+          br.skip((int)(e >> 9));
+          sym = (int)(e & 511u);
+        } else {
+          int n = max(mn, kLutBits + 1);
+          while (n <= mx && x > lj[t][n]) n++;
+          const int idx = n <= mx ? (int)(x >> (32 - n)) - base[t][n] : -1;
+          if (idx < 0 || idx >= alpha) {
+            b_at = ln * kGroupSize + i;
+            break;
+          }
+          br.skip(n);
+          sym = perm[t][idx];
+        }
+        if (sym == eob) {
+          e_at = ln * kGroupSize + i;
+          e_end = (uint32_t)(br.pos() - start);
           break;
         }
-        br.skip(n);
-        sym = perm[t][idx];
+        dst[i] = (uint16_t)sym;
       }
-      if (sym == eob) {
-        e_at = ln * kGroupSize + i;
-        e_end = (uint32_t)(br.pos() - start);
-        break;
-      }
-      dst[i] = (uint16_t)sym;
     }
-  }
-  const int eob_at = __reduce_min_sync(full, e_at), bad_at = __reduce_min_sync(full, b_at);
-  const int n = min(min(eob_at, bad_at), ngc * kGroupSize);
-  __syncwarp();
-  uint8_t *lb = lists[w][0];
-  uint32_t *used = used_s[w];
-  for (int q = ln; q < 256; q += 32) lb[q] = (uint8_t)q;
-  __syncwarp();
-  int cur = 0;
-  int run = 0;        // run digits just before the batch
-  bool lead = true;   // only run digits so far
-  int lead_cnt = 0;
-  int64_t lead_sum = 0, rest_sum = 0;
-  uint16_t *rec = out.rec + (size_t)c * kChunkSyms;
-  for (int i0 = 0; i0 < n; i0 += 32) {
-    const int nb = min(32, n - i0);
-    const bool act = ln < nb;
-    const int sym = act ? sy[w][i0 + ln] : 0;
-    const bool dgt = act && sym <= 1;
-    const unsigned runs = __ballot_sync(full, dgt);
-    const unsigned others = __ballot_sync(full, act && !dgt);
+    const int eob_at = __reduce_min_sync(full, e_at), bad_at = __reduce_min_sync(full, b_at);
+    const int n = min(min(eob_at, bad_at), ngc * kGroupSize);
+    __syncwarp();
+    uint8_t *lb = lists[w][0];
+    uint32_t *used = used_s[w];
+    for (int q = ln; q < 256; q += 32) lb[q] = (uint8_t)q;
+    __syncwarp();
+    int cur = 0;
+    int run = 0;        // run digits just before the batch
+    bool lead = true;   // only run digits so far
+    int lead_cnt = 0;
+    int64_t lead_sum = 0, rest_sum = 0;
+    uint16_t *rec = out.rec + (size_t)c * kChunkSyms;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int nb = min(32, n - i0);
+      const bool act = ln < nb;
+      const int sym = act ? sy[w][i0 + ln] : 0;
+      const bool dgt = act && sym <= 1;
+      const unsigned runs = __ballot_sync(full, dgt);
+      const unsigned others = __ballot_sync(full, act && !dgt);
+      const uint8_t *lst = lb + 256 * cur;
+      int rv;  // the symbol's position in the chunk's starting list
+      if (others == 0u) {
+        rv = lst[0];
+      } else {
+        const int my_v = act && !dgt ? sym - 1 : 0;
+        // p: the position before step ln - d of what this step puts out.  Once
+        // at 0 it stays there; it then is the output of the step before the one
+        // that last moved it (a run digit: of the step before itself).
+        int p = my_v, moved = 0;
+  #pragma unroll
+        for (int d = 1; d < 32; d++) {
+          uint32_t vs;
+          int in;
+          asm volatile("{ .reg .pred q; shfl.sync.up.b32 %0|q, %2, %3, 0, 0xffffffff; selp.s32 %1, 1, 0, q; }"
+              : "=r"(vs), "=r"(in)
+              : "r"(my_v), "r"(d));
+          if (in && (uint32_t)(p - 1) < vs) {
+            p--;
+            moved = d;
+          }
+        }
+        int ptr = p == 0 ? ln - moved - 1 : -1;  // below 0: no step before, the list's front
+        const bool from_list = act && ptr < 0;
+        int val = from_list ? (int)lst[p] : -1;
+  #pragma unroll
+        for (int r2 = 0; r2 < 5; r2++) {
+          const int src = ptr >= 0 ? ptr : ln;
+          const int tv = __shfl_sync(full, val, src);
+          const int tp = __shfl_sync(full, ptr, src);
+          if (val < 0 && ptr >= 0) {
+            if (tv >= 0) val = tv;
+            else ptr = tp;
+          }
+        }
+        // active lanes with the same output: one ballot per bit of it
+        unsigned peers = __ballot_sync(full, act);
+  #pragma unroll
+        for (int bit = 0; bit < 8; bit++) {
+          const bool on = act && ((val >> bit) & 1);
+          const unsigned bb = __ballot_sync(full, on);
+          peers &= on ? bb : ~bb;
+        }
+        const unsigned above = ~((2u << ln) - 1u);  // lanes after this one
+        const bool last = act && (peers & above) == 0u;
+        const unsigned lastm = __ballot_sync(full, last);
+        const int D = __popc(lastm);
+        if (ln < 8) used[ln] = 0u;
+        __syncwarp();
+        if (from_list) atomicOr(&used[p >> 5], 1u << (p & 31));
+        __syncwarp();
+        uint8_t *nx = lb + 256 * (cur ^ 1);
+        if (last) nx[__popc(lastm & above)] = (uint8_t)val;
+        const int q0 = 8 * ln;
+        int below = 0;
+        for (int x = 0; x < (q0 >> 5); x++) below += __popc(used[x]);
+        const uint32_t uw = used[q0 >> 5];
+        for (int j = 0; j < 8; j++) {
+          const int q = q0 + j;
+          if (q >= nuse) break;
+          const uint32_t bit = 1u << (q & 31);
+          if (!(uw & bit)) nx[D + q - below - __popc(uw & (bit - 1u))] = lst[q];
+        }
+        cur ^= 1;
+        rv = val;
+        __syncwarp();
+      }
+      // a run digit's place: the digits just before it
+      const unsigned bm = others & ((1u << ln) - 1u);
+      const int q = bm ? ln - 32 + __clz(bm) : ln + run;
+      const int qc = min(q, 31);
+      if (act) rec[i0 + ln] = (uint16_t)(dgt ? kRecRun | (sym << 13) | (qc << 8) | rv : rv);
+      if (act) {
+        const int64_t bytes = dgt ? (int64_t)(sym + 1) << min(q, 40) : 1;
+        if (lead && bm == 0u && dgt) lead_sum += bytes;
+        else rest_sum += bytes;
+      }
+      if (lead) lead_cnt += others ? __ffs(others) - 1 : nb;
+      if (others) {
+        lead = false;
+        run = nb - 32 + __clz(others);
+      } else {
+        run += nb;
+      }
+    }
+    for (int o = 16; o; o >>= 1) {
+      lead_sum += __shfl_xor_sync(full, lead_sum, o);
+      rest_sum += __shfl_xor_sync(full, rest_sum, o);
+    }
     const uint8_t *lst = lb + 256 * cur;
-    int rv;  // the symbol's position in the chunk's starting list
-    if (others == 0u) {
-      rv = lst[0];
-    } else {
-      const int my_v = act && !dgt ? sym - 1 : 0;
-      // p: the position before step ln - d of what this step puts out.  Once
-      // at 0 it stays there; it then is the output of the step before the one
-      // that last moved it (a run digit: of the step before itself).
-      int p = my_v, moved = 0;
-#pragma unroll
-      for (int d = 1; d < 32; d++) {
-        uint32_t vs;
-        int in;
-        asm volatile("{ .reg .pred q; shfl.sync.up.b32 %0|q, %2, %3, 0, 0xffffffff; selp.s32 %1, 1, 0, q; }"
-            : "=r"(vs), "=r"(in)
-            : "r"(my_v), "r"(d));
-        if (in && (uint32_t)(p - 1) < vs) {
-          p--;
-          moved = d;
-        }
-      }
-      int ptr = p == 0 ? ln - moved - 1 : -1;  // below 0: no step before, the list's front
-      const bool from_list = act && ptr < 0;
-      int val = from_list ? (int)lst[p] : -1;
-#pragma unroll
-      for (int r2 = 0; r2 < 5; r2++) {
-        const int src = ptr >= 0 ? ptr : ln;
-        const int tv = __shfl_sync(full, val, src);
-        const int tp = __shfl_sync(full, ptr, src);
-        if (val < 0 && ptr >= 0) {
-          if (tv >= 0) val = tv;
-          else ptr = tp;
-        }
-      }
-      // active lanes with the same output: one ballot per bit of it
-      unsigned peers = __ballot_sync(full, act);
-#pragma unroll
-      for (int bit = 0; bit < 8; bit++) {
-        const bool on = act && ((val >> bit) & 1);
-        const unsigned bb = __ballot_sync(full, on);
-        peers &= on ? bb : ~bb;
-      }
-      const unsigned above = ~((2u << ln) - 1u);  // lanes after this one
-      const bool last = act && (peers & above) == 0u;
-      const unsigned lastm = __ballot_sync(full, last);
-      const int D = __popc(lastm);
-      if (ln < 8) used[ln] = 0u;
-      __syncwarp();
-      if (from_list) atomicOr(&used[p >> 5], 1u << (p & 31));
-      __syncwarp();
-      uint8_t *nx = lb + 256 * (cur ^ 1);
-      if (last) nx[__popc(lastm & above)] = (uint8_t)val;
-      const int q0 = 8 * ln;
-      int below = 0;
-      for (int x = 0; x < (q0 >> 5); x++) below += __popc(used[x]);
-      const uint32_t uw = used[q0 >> 5];
-      for (int j = 0; j < 8; j++) {
-        const int q = q0 + j;
-        if (q >= nuse) break;
-        const uint32_t bit = 1u << (q & 31);
-        if (!(uw & bit)) nx[D + q - below - __popc(uw & (bit - 1u))] = lst[q];
-      }
-      cur ^= 1;
-      rv = val;
-      __syncwarp();
+    for (int q = ln; q < 64; q += 32)
+      reinterpret_cast<uint32_t *>(out.list[c])[q] = reinterpret_cast<const uint32_t *>(lst)[q];
+    ChunkInfo &ci = out.info[c];
+    if (e_at == eob_at && e_at != INT32_MAX) ci.end = e_end;
+    if (ln == 0) {
+      ci.nsym = n;
+      ci.eob = eob_at != INT32_MAX && eob_at < bad_at;
+      ci.bad = bad_at < eob_at;
+      ci.lead = lead_cnt;
+      ci.trail = run;
+      ci.lead_sum = lead_sum;
+      ci.rest_sum = rest_sum;
     }
-    // a run digit's place: the digits just before it
-    const unsigned bm = others & ((1u << ln) - 1u);
-    const int q = bm ? ln - 32 + __clz(bm) : ln + run;
-    const int qc = min(q, 31);
-    if (act) rec[i0 + ln] = (uint16_t)(dgt ? kRecRun | (sym << 13) | (qc << 8) | rv : rv);
-    if (act) {
-      const int64_t bytes = dgt ? (int64_t)(sym + 1) << min(q, 40) : 1;
-      if (lead && bm == 0u && dgt) lead_sum += bytes;
-      else rest_sum += bytes;
-    }
-    if (lead) lead_cnt += others ? __ffs(others) - 1 : nb;
-    if (others) {
-      lead = false;
-      run = nb - 32 + __clz(others);
-    } else {
-      run += nb;
-    }
-  }
-  for (int o = 16; o; o >>= 1) {
-    lead_sum += __shfl_xor_sync(full, lead_sum, o);
-    rest_sum += __shfl_xor_sync(full, rest_sum, o);
-  }
-  const uint8_t *lst = lb + 256 * cur;
-  for (int q = ln; q < 64; q += 32)
-    reinterpret_cast<uint32_t *>(out.list[c])[q] = reinterpret_cast<const uint32_t *>(lst)[q];
-  ChunkInfo &ci = out.info[c];
-  if (e_at == eob_at && e_at != INT32_MAX) ci.end = e_end;
-  if (ln == 0) {
-    ci.nsym = n;
-    ci.eob = eob_at != INT32_MAX && eob_at < bad_at;
-    ci.bad = bad_at < eob_at;
-    ci.lead = lead_cnt;
-    ci.trail = run;
-    ci.lead_sum = lead_sum;
-    ci.rest_sum = rest_sum;
+    __syncwarp();  // the warp's shared memory is free for the next chunk
   }
 }
 
@@ -1188,46 +1184,48 @@ __global__ void __launch_bounds__(32 * kSymWarps)
   const int bi = blockIdx.y;
   if (res[bi].status != kDecOk) return;
   const int ln = lane_id(), w = warp_id();
-  const int c = blockIdx.x * kSymWarps + w;
-  if (c >= res[bi].nchunks) return;
+  const int nch = res[bi].nchunks;
   SymScratch &sc = sym_scratch(tt, bi, cap);
-  const ChunkInfo ci = sc.info[c];
-  int64_t off = ci.off;
-  for (int q = ln; q < 64; q += 32)
-    reinterpret_cast<uint32_t *>(lists[w])[q] = reinterpret_cast<const uint32_t *>(sc.list[c])[q];
-  __syncwarp();
   uint8_t *L = Lbuf + (size_t)bi * cap;
-  const uint16_t *rec = sc.rec + (size_t)c * kChunkSyms;
-  for (int i0 = 0; i0 < ci.nsym; i0 += 32) {
-    const int i = i0 + ln;
-    const uint32_t r = i < ci.nsym ? rec[i] : 0u;
-    int nb = i < ci.nsym ? 1 : 0;
-    if (r & kRecRun) {
-      const int q = (int)((r >> 8) & 31u) + (i < ci.lead ? ci.q0 : 0);
-      nb = (int)(((r >> 13) & 1u) + 1u) << min(q, 28);
+  for (int c = (int)blockIdx.x * kSymWarps + w; c < nch; c += gridDim.x * kSymWarps) {
+    const ChunkInfo ci = sc.info[c];
+    int64_t off = ci.off;
+    for (int q = ln; q < 64; q += 32)
+      reinterpret_cast<uint32_t *>(lists[w])[q] = reinterpret_cast<const uint32_t *>(sc.list[c])[q];
+    __syncwarp();
+    const uint16_t *rec = sc.rec + (size_t)c * kChunkSyms;
+    for (int i0 = 0; i0 < ci.nsym; i0 += 32) {
+      const int i = i0 + ln;
+      const uint32_t r = i < ci.nsym ? rec[i] : 0u;
+      int nb = i < ci.nsym ? 1 : 0;
+      if (r & kRecRun) {
+        const int q = (int)((r >> 8) & 31u) + (i < ci.lead ? ci.q0 : 0);
+        nb = (int)(((r >> 13) & 1u) + 1u) << min(q, 28);
+      }
+      const uint8_t v = lists[w][r & 0xFFu];
+      const int inc = warp_incl_sum(nb);
+      const int64_t at = off + inc - nb;
+      if (nb == 1) L[at] = v;
+      else if (nb > 1 && nb <= 64) fill_bytes(L + at, nb, v);
+      unsigned big = __ballot_sync(full, nb > 64);
+      while (big) {
+        const int s = __ffs(big) - 1;
+        big &= big - 1u;
+        const int bn = __shfl_sync(full, nb, s);
+        const int64_t ba = __shfl_sync(full, at, s);
+        const uint32_t bv = 0x01010101u * __shfl_sync(full, (uint32_t)v, s);
+        uint8_t *d = L + ba;
+        const int head = min(bn, (int)((0u - (uint32_t)reinterpret_cast<uintptr_t>(d)) & 15u));
+        const int body = (bn - head) / 16;
+        if (ln < head) d[ln] = (uint8_t)bv;
+        for (int q = ln; q < body; q += 32)
+          reinterpret_cast<uint4 *>(d + head)[q] = make_uint4(bv, bv, bv, bv);
+        const int done = head + 16 * body;
+        if (done + ln < bn) d[done + ln] = (uint8_t)bv;
+      }
+      off += __shfl_sync(full, inc, 31);
     }
-    const uint8_t v = lists[w][r & 0xFFu];
-    const int inc = warp_incl_sum(nb);
-    const int64_t at = off + inc - nb;
-    if (nb == 1) L[at] = v;
-    else if (nb > 1 && nb <= 64) fill_bytes(L + at, nb, v);
-    unsigned big = __ballot_sync(full, nb > 64);
-    while (big) {
-      const int s = __ffs(big) - 1;
-      big &= big - 1u;
-      const int bn = __shfl_sync(full, nb, s);
-      const int64_t ba = __shfl_sync(full, at, s);
-      const uint32_t bv = 0x01010101u * __shfl_sync(full, (uint32_t)v, s);
-      uint8_t *d = L + ba;
-      const int head = min(bn, (int)((0u - (uint32_t)reinterpret_cast<uintptr_t>(d)) & 15u));
-      const int body = (bn - head) / 16;
-      if (ln < head) d[ln] = (uint8_t)bv;
-      for (int q = ln; q < body; q += 32)
-        reinterpret_cast<uint4 *>(d + head)[q] = make_uint4(bv, bv, bv, bv);
-      const int done = head + 16 * body;
-      if (done + ln < bn) d[done + ln] = (uint8_t)bv;
-    }
-    off += __shfl_sync(full, inc, 31);
+    __syncwarp();  // the list is free for the next chunk
   }
 }
 
@@ -1245,7 +1243,6 @@ __global__ void __launch_bounds__(32 * kSymWarps)
 // has, the fewer blocks' T (4 bytes per RLE1 byte) are in use at a time, which
 // keeps them in L2.  Two walks of steps of 512 took 0.67 ms each for one block
 // and 4.7 ms each for 600 blocks.
-constexpr int kWalkChunk = 64;
 constexpr int kMaxWalkers = (kDecCap + 127) / 128 + 2;
 constexpr int kMaxWalkChunks = kMaxWalkers + kDecCap / kWalkChunk + 1;
 constexpr int kChainThreads = 1024;
@@ -1253,11 +1250,6 @@ constexpr int kChainPer = (kMaxWalkers + kChainThreads - 1) / kChainThreads;
 constexpr int kNoWalker = 0xFFFF;
 static_assert(kMaxWalkers < (1 << 14) && kDecCap / kWalkChunk < (1 << 18), "chunk owner packing");
 
-__host__ __device__ __forceinline__ int walk_step(int m) { return m > kDecCap / 2 ? 128 : 64; }
-__device__ __forceinline__ int walker_count(int m, int orig) {
-  const int s = walk_step(m);
-  return (m + s - 1) / s + (orig % s != 0);
-}
 // The walker that starts at a cut.
 __device__ __forceinline__ int walker_at(int p, int m, int orig) {
   const int s = walk_step(m);
@@ -1279,7 +1271,6 @@ struct WalkCtl {
 // histogram, per block a scan over chunks (each chunk's start per byte value,
 // C included), then per chunk the ranks of 256 entries at a time: equal bytes
 // in a warp by ballots, earlier warps by shared counts.
-constexpr int kLfChunk = 4096;
 constexpr int kLfChunks = (kDecCap + kLfChunk - 1) / kLfChunk;
 
 __global__ void __launch_bounds__(256) k_dec_lf_hist(const int32_t *idx, const DecBlock *db,
@@ -1363,9 +1354,9 @@ __global__ void __launch_bounds__(256) k_dec_lf_rank(const int32_t *idx, const D
   }
 }
 
-__global__ void __launch_bounds__(128) k_dec_walk(const int32_t *idx, const DecBlock *db,
-                                                  const uint32_t *tt, WalkCtl *ctl, uint8_t *pool,
-                                                  int cap) {
+__global__ void __launch_bounds__(kWalkThreads) k_dec_walk(const int32_t *idx, const DecBlock *db,
+                                                           const uint32_t *tt, WalkCtl *ctl,
+                                                           uint8_t *pool, int cap) {
   const int k = blockIdx.y;
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   WalkCtl &c = ctl[k];
@@ -1461,8 +1452,6 @@ __global__ void __launch_bounds__(kChainThreads) k_dec_chain(const int32_t *idx,
 }
 
 // The walkers' chunks to their places: 16 threads per chunk, 4 bytes each.
-constexpr int kGatherChunks = 128;  // per CTA
-
 __global__ void __launch_bounds__(256) k_dec_gather(const int32_t *idx, const DecBlock *db,
                                                     const WalkCtl *ctl, const uint8_t *pool,
                                                     uint8_t *rle, int cap) {
@@ -1514,7 +1503,7 @@ __global__ void k_dec_repeat(const int32_t *idx, const DecBlock *db, const WalkC
 // One warp per block took 3.5 + 1.0 ms for a single block, the latency of
 // 7,500 bytes per lane one after another.
 constexpr int kSegBytes = 32;
-constexpr int kUnTile = 256 * kSegBytes;  // 8192
+static_assert(kUnTile == 256 * kSegBytes, "a thread per segment");
 constexpr int kUnTiles = (kDecCap + kUnTile - 1) / kUnTile;
 constexpr int kSegStride = kSegBytes + 4;  // in shared memory: lanes on different banks
 
@@ -1758,14 +1747,12 @@ __global__ void __launch_bounds__(256) k_dec_unrle1_write(const int32_t *idx, co
   bw.finish();
 }
 
-// Block CRCs of the expanded output.  kCrcParts CTAs share a block's
+// Block CRCs of the expanded output.  gridDim.x CTAs share a block's
 // 4096-byte chunks; in a chunk thread l's 16 bytes give crc0 *
 // x^(8*16*(255-l)) (the chunk right-aligned in 4096 bytes when shorter), the
 // XOR is the chunk's crc0, a CTA's crc0 accumulates chunk by chunk and is
 // shifted past the bytes after its part.  crcs: all ones before (the format's
 // complement); the initial value's term comes with part 0.
-constexpr int kCrcParts = 32;
-
 __global__ void __launch_bounds__(256) k_dec_crc(const int64_t *lens, const int64_t *off,
                                                  const uint8_t *out, uint32_t *crcs) {
   __shared__ uint32_t tbl[256];
@@ -1773,8 +1760,8 @@ __global__ void __launch_bounds__(256) k_dec_crc(const int64_t *lens, const int6
   __shared__ uint32_t part[2][8];
   const int k = blockIdx.y;
   const int64_t n = lens[k];
-  const int64_t nch = (n + 4095) / 4096;
-  const int64_t per = (nch + kCrcParts - 1) / kCrcParts;
+  const int64_t nch = (n + kCrcChunk - 1) / kCrcChunk;
+  const int64_t per = (nch + gridDim.x - 1) / gridDim.x;
   const int64_t b0 = (int64_t)blockIdx.x * per * 4096;
   const int64_t b1 = b0 + per * 4096 < n ? b0 + per * 4096 : n;
   if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -2108,7 +2095,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const uint32_t *wd = w.words.get<uint32_t>();
     const int64_t *dcand = w.cand.get<int64_t>();
     DecTab *dtab = w.tab.get<DecTab>();
-    const dim3 cgrid((kMaxChunks + kSymWarps - 1) / kSymWarps, nc);
+    const dim3 cgrid(chunk_grid(csize(order[0])), nc);
     k_dec_head<<<nc, kHeadThreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>());
     BZ_LAUNCH_CHECK();
     // few blocks: group starts by jump tables
@@ -2176,7 +2163,10 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const int32_t *didx = w.idx.get<int32_t>();
     const DecBlock *ddb = w.db.get<DecBlock>();
     BZ_CUDA(cudaMemcpyAsync(w.idx.p, acc.data(), 4 * na, cudaMemcpyHostToDevice, st));
-    const dim3 lgrid(kLfChunks, na);
+    int max_m = 0;
+    for (const int q : acc) max_m = std::max(max_m, hdb[q].m);
+    const ColumnGrids grids = column_grids(max_m);
+    const dim3 lgrid(grids.lf, na);
     k_dec_lf_hist<<<lgrid, 256, 0, st>>>(didx, ddb, L, w.hist.get<int32_t>(), cap);
     BZ_LAUNCH_CHECK();
     WalkCtl *dctl = w.ctl.get<WalkCtl>();
@@ -2185,18 +2175,18 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     k_dec_lf_rank<<<lgrid, 256, 0, st>>>(didx, ddb, L, w.hist.get<int32_t>(),
                                          w.tt.get<uint32_t>(), cap);
     BZ_LAUNCH_CHECK();
-    k_dec_walk<<<dim3((kMaxWalkers + 127) / 128, na), 128, 0, st>>>(
+    k_dec_walk<<<dim3(grids.walk, na), kWalkThreads, 0, st>>>(
         didx, ddb, w.tt.get<uint32_t>(), dctl, w.pool.get<uint8_t>(), cap);
     BZ_LAUNCH_CHECK();
     BZ_CUDA(cudaMemsetAsync(w.bad.p, 0, 4, st));
     k_dec_chain<<<na, kChainThreads, kChainSmem, st>>>(didx, ddb, dctl, w.bad.get<int>());
     BZ_LAUNCH_CHECK();
-    k_dec_gather<<<dim3((kMaxWalkChunks + kGatherChunks - 1) / kGatherChunks, na), 256, 0, st>>>(
+    k_dec_gather<<<dim3(grids.gather, na), 256, 0, st>>>(
         didx, ddb, dctl, w.pool.get<uint8_t>(), L, cap);
     BZ_LAUNCH_CHECK();
-    k_dec_repeat<<<dim3(16, na), 256, 0, st>>>(didx, ddb, w.ctl.get<WalkCtl>(), L, cap);
+    k_dec_repeat<<<dim3(grids.repeat, na), 256, 0, st>>>(didx, ddb, w.ctl.get<WalkCtl>(), L, cap);
     BZ_LAUNCH_CHECK();
-    const dim3 ugrid(kUnTiles, na);
+    const dim3 ugrid(grids.unrle, na);
     k_dec_unrle1_count<<<ugrid, 256, 0, st>>>(didx, ddb, L, cap, w.maps.get<RunMap>());
     BZ_LAUNCH_CHECK();
     k_dec_unrle1_scan<<<na, 256, 0, st>>>(didx, ddb, w.maps.get<RunMap>(), w.lens.get<int64_t>());
@@ -2223,7 +2213,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
                                               w.off.get<int64_t>(), w.out[slot].get<uint8_t>());
     BZ_LAUNCH_CHECK();
     BZ_CUDA(cudaMemsetAsync(w.crc.p, 0xFF, 4 * na, st));
-    k_dec_crc<<<dim3(kCrcParts, na), 256, 0, st>>>(w.lens.get<int64_t>(), w.off.get<int64_t>(),
+    k_dec_crc<<<dim3(crc_grid(*std::max_element(lens.begin(), lens.end())), na), 256, 0, st>>>(w.lens.get<int64_t>(), w.off.get<int64_t>(),
                                                    w.out[slot].get<uint8_t>(),
                                                    w.crc.get<uint32_t>());
     BZ_LAUNCH_CHECK();

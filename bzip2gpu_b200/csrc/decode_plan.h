@@ -1,0 +1,64 @@
+// Launch shapes of the decoder, from a batch's own blocks (host code without
+// CUDA; csrc/decode.cu has the kernels).
+#pragma once
+
+#include <stdint.h>
+
+#include <algorithm>
+
+namespace bz2g {
+
+constexpr int kDecMaxSel = 18002;
+// Per-block capacity of the last column (the reference's 900,000-byte raw
+// blocks can exceed 900,000 RLE1 bytes by up to a quarter).
+constexpr int kDecCap = 1200000;
+constexpr int kDecGroupSyms = 50;
+constexpr int kChunkGroups = 32;  // groups per warp of k_dec_syms and k_dec_emit
+constexpr int kMaxChunks = (kDecMaxSel + kChunkGroups - 1) / kChunkGroups;
+constexpr int kSymWarps = 4;
+constexpr int kLfChunk = 4096;    // last-column bytes per CTA of k_dec_lf_hist, _rank
+constexpr int kWalkThreads = 128;
+constexpr int kWalkChunk = 64;    // bytes per pool chunk of the walks
+constexpr int kGatherChunks = 128;  // pool chunks per CTA of k_dec_gather
+constexpr int kUnTile = 8192;     // RLE1 bytes per CTA of k_dec_unrle1_count, _write
+constexpr int kCrcParts = 32;     // CTAs that share a block's CRC, at most
+constexpr int kCrcChunk = 4096;   // output bytes they take at a time
+
+inline int dec_ceil(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
+
+// Walkers of the inverse BWT: one per walk_step(m) positions, and origPtr's.
+constexpr int walk_step(int m) { return m > kDecCap / 2 ? 128 : 64; }
+constexpr int walker_count(int m, int orig) {
+  return (m + walk_step(m) - 1) / walk_step(m) + (orig % walk_step(m) != 0);
+}
+
+// CTAs per block of k_dec_syms and k_dec_emit (whose warps take further chunks
+// a grid apart, so this is no bound): a code has at least a bit, and
+// `max_bits` is the most bits between two block candidates.
+inline int chunk_grid(int64_t max_bits) {
+  const int64_t groups = std::min<int64_t>(kDecMaxSel, max_bits / kDecGroupSyms + 1);
+  return dec_ceil(dec_ceil(groups, kChunkGroups), kSymWarps);
+}
+
+// CTAs per block of the stages after the entropy decode, for blocks of at most
+// m last-column bytes.  Grids for the largest block the format allows cost
+// more than the work for short ones: 5 MB in blocks of 1,000 bytes took 6.6 ms,
+// of which 4 launched CTAs that returned at once.
+struct ColumnGrids {
+  int lf, walk, gather, repeat, unrle;
+};
+inline ColumnGrids column_grids(int m) {
+  // (128 bytes a walker give fewer walkers than 64 for a shorter block)
+  const int walkers = dec_ceil(std::min(m, kDecCap / 2), 64) + 1;
+  const int most = std::max(walkers, dec_ceil(m, 128) + 1);
+  return {dec_ceil(m, kLfChunk), dec_ceil(most, kWalkThreads),
+          dec_ceil(most + m / kWalkChunk + 1, kGatherChunks), std::min(16, dec_ceil(m, 4096)),
+          dec_ceil(m, kUnTile)};
+}
+
+// CTAs per block of k_dec_crc, for blocks of at most n output bytes.
+inline int crc_grid(int64_t n) {
+  return (int)std::min<int64_t>(kCrcParts, std::max<int64_t>(1, dec_ceil(n, kCrcChunk)));
+}
+
+}  // namespace bz2g
