@@ -14,9 +14,9 @@
 //      h -> 2h) keys them (head << kb) | ISA[(i + h) mod m] and re-sorts them
 //      stably; the k-th of them in sorted order goes to the k-th active SA
 //      position (groups are contiguous, so this sorts within each group).
-//      Groups of up to kGroupMax rotations need no radix sort: a block whose
-//      active groups are all that short sorts them one by one in shared memory
-//      (k_bwt_groups), in the same rounds.
+//      Short groups need no radix sort: a block whose active groups hold at
+//      most kGroupMax rotations, and kGroupMean on average, sorts them one by
+//      one in shared memory (k_bwt_groups), in the same rounds.
 //   4. A block stops when no rotation is active, when a round splits no group
 //      (the rest are equal rotations, already index-ascending), or when the
 //      prefix length reaches m.
@@ -892,9 +892,16 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, int kb, const int3
 // takes the groups that start in a unit of `step` items of a block's active
 // list, and holds kTile, so a step is what the block's longest group leaves of
 // that (2048 for every block took a CTA for half of what it can hold).  Longer
-// groups would leave steps that mostly reload what other CTAs hold.
-constexpr int kMinStep = 512;
+// groups would leave steps that mostly reload what other CTAs hold, and every
+// doubling of a group is a merge more, where the radix passes cost the same
+// for any group.  Measured, 16 blocks of a repeat that doubles until the end,
+// by groups / by radix sort: groups of 3,500 26.3 / 16.0 ms, 1,800 24.5 / 16.0,
+// 1,280 21.6 / 16.1, 990 18.5 / 16.0, 750 17.9 / 16.0, 500 15.5 / 16.1.  Text has a
+// few long groups among very short ones, which the mean tells apart: with
+// kGroupMax at 1,024 and no mean 512 MiB of it take 15.2 instead of 14.5 ms.
+constexpr int kMinStep = 2048;
 constexpr int kGroupMax = kTile - kMinStep;
+constexpr int kGroupMean = 512;
 __device__ __forceinline__ int group_step(int gmax) { return (kTile - gmax) & ~31; }
 
 // Lists a block's tiles, or its units when it is sorted group by group.  The
@@ -940,7 +947,7 @@ __global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefi
       const int len = d.act_len[b];
       d.sort_len[b] = len;
       if (len > 0) {
-        if (packed && !d.loc[b] && d.gmax[b] <= kGroupMax) {
+        if (packed && !d.loc[b] && d.gmax[b] <= kGroupMax && len <= kGroupMean * d.ngroups[b]) {
           d.loc[b] = 1;
           d.loc_cur[b] = keys_now(d) ^ 1;
         }
