@@ -1248,14 +1248,16 @@ __global__ void __launch_bounds__(256) k_bwt_round_keys(SlabDev d, int h, int pa
   const uint64_t mask = (1ull << kb) - 1;
   for (int e = threadIdx.x; e < valid; e += blockDim.x) {
     if (packed) {
-      const uint64_t item = K[e];
+      uint64_t item = K[e];
       int i2 = (int)(item & mask) + h;
       if (i2 >= m) i2 -= m;
-      const uint32_t r = (uint32_t)IS[i2];
-      K[e] = item | ((uint64_t)r << kb);
-      // the first pass's digit, the low bits of the rank
-      if (!loc && wide) next_digits<9>(d)[off + lt + e] = r & 511u;
-      if (!loc && !wide) next_digits<8>(d)[off + lt + e] = (uint8_t)r;
+      item |= (uint64_t)(uint32_t)IS[i2] << kb;
+      K[e] = item;
+      // the first pass's digit: the bits from kb on, the rank's low ones and,
+      // where kb is less than a digit, the head's
+      const uint32_t low = (uint32_t)(item >> kb);
+      if (!loc && wide) next_digits<9>(d)[off + lt + e] = low & 511u;
+      if (!loc && !wide) next_digits<8>(d)[off + lt + e] = (uint8_t)low;
     } else {
       int i2 = (int)V[e] + h;
       if (i2 >= m) i2 -= m;
