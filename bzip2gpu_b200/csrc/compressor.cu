@@ -10,23 +10,22 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <condition_variable>
 #include <cstring>
 #include <exception>
 #include <mutex>
+#include <numeric>
 #include <thread>
 
 #include "engine.h"
 #include "selector.h"
+#include "slabs.h"
 
 namespace bz2g {
 
 static_assert(kMaxRounds == sizeof(StageTimes::round_ms) / sizeof(double),
               "per-round statistics size");
-
-// Fewest blocks worth a slab of their own, and blocks per slab of host input.
-constexpr int kMinSlabBlocks = 16;
-constexpr int kHostSlabBlocks = 128;
 
 struct Compressor::Worker {
   Workspace *ws = nullptr;
@@ -289,21 +288,14 @@ void Compressor::run(const uint8_t *const *ptrs, const int *lens, int nblocks, i
                      bool on_device, ByteSink &out, StageTimes *times, bool part,
                      int64_t *part_bits, uint32_t *part_crc) {
   std::lock_guard<std::mutex> call_lock(call_mu_);
-  // Blocks per slab.  A call that fits the workers' slabs once is split evenly
-  // over the workers, so that their stages (and, from host memory, the copies)
-  // overlap, down to kMinSlabBlocks blocks: below that the launches of another
-  // slab cost more than they overlap.  Host input takes slabs of about
-  // kHostSlabBlocks, so that the first kernels need not wait for a quarter of
-  // the input.  Measured, one slab of up to 384 blocks / split: 256 MiB 12.4 /
-  // 11.4 ms on the device, 17.1 / 13.3 ms from the host; 32 MiB 2.63 / 2.52
-  // and 3.24 / 2.98 ms; 8 MiB (10 blocks) 1.77 / 1.88 ms; 1 GiB 42.1 / 41.7
-  // and 48.2 / 46.2 ms.  Larger calls keep slab_blocks.
+  // Blocks per slab: a call that fits the workers' slabs once is split evenly
+  // (slabs.h), larger calls keep slab_blocks.
   int per_slab = cfg_.slab_blocks;
   {
     const int nw = (int)workers_.size();
     if (nblocks <= nw * (int64_t)cfg_.slab_blocks) {
-      const int rounds = on_device ? 1 : std::max(1, (int)(nblocks / (nw * kHostSlabBlocks)));
-      const int slabs = std::max(1, std::min(nw * rounds, nblocks / kMinSlabBlocks));
+      const int slabs =
+          slab_count(nblocks, std::accumulate(lens, lens + nblocks, int64_t(0)), nw, on_device);
       per_slab = std::min(per_slab, std::max(1, (nblocks + slabs - 1) / slabs));
     }
     // room for min(nblocks, slab_blocks) blocks, whatever per_slab is, so that
@@ -617,14 +609,12 @@ void Compressor::compress_batch(const Item *items, int count, bool on_device, By
                    [&](int a, int b) { return blks[a].len > blks[b].len; });
   // slabs over the queue: a slab takes up to the tuned block count for its
   // longest (first) block, fewer where the workspace's capacities end, and no
-  // more than a worker's share of the bytes, down to the bytes of kMinSlabBlocks
-  // full blocks (as in run()).  128 inputs, 120 MB: one slab 9.9 ms, split over
-  // the workers 9.2 ms; 43 inputs, 8 MB: 1.72 and 1.65 ms, but 1.78 and 3.96 ms
-  // in the first call after the program has page-locked memory
+  // more than a worker's share of the bytes (as in run(); the blocks may be
+  // short, so their number does not count).  128 inputs, 120 MB: one slab 9.9
+  // ms, split over the workers 9.2 ms
   reserve(nb);
-  const int64_t least = kMinSlabBlocks * std::max<int64_t>(cfg_.max_block_bytes, 1);
   const int64_t share = std::max<int64_t>(
-      1, ntot / std::max<int64_t>(1, std::min<int64_t>((int64_t)workers_.size(), ntot / least)));
+      1, ntot / slab_count(INT_MAX, ntot, (int)workers_.size(), true));
   const Workspace &ws0 = *workers_[0]->ws;
   std::vector<int> slab_at{0};
   {

@@ -1,0 +1,42 @@
+// How a call's blocks are cut into slabs (host code without CUDA;
+// csrc/compressor.cu drives them).
+#pragma once
+
+#include <stdint.h>
+
+#include <algorithm>
+
+namespace bz2g {
+
+// Fewest blocks of a slab: with fewer the launches of another slab cost more
+// than they overlap.
+constexpr int kMinSlabBlocks = 16;
+// Bytes of a call from which it takes a second slab, and per slab beyond that.
+// Every slab at work has a host thread, and where the program keeps the cores
+// busy (OpenMP's threads spin for some ms after a parallel loop) a thread
+// beyond the caller's costs about 1.1 ms, whatever the slab.  So a call is cut
+// only where even then it takes no longer than as one slab did before there
+// were several, sooner for host input, whose copies overlap too.  In ms, one
+// slab then / cut on an idle host / on a busy one: 30 MB on the device 3.1 /
+// 1.8 / 2.9 (two slabs), 110 MB 6.5 / 4.1 / 6.1 (three); 45 MB from the host
+// 4.5 / 2.8 / 4.1 (two), 110 MB 8.5 / 5.1 / 7.2 (four).  Cut by 16 blocks
+// alone, 6.4 MB in blocks of 100,000 took 2.1 / 1.3 / 4.2, now 1.2 on both.
+constexpr int64_t kTwoSlabBytes = 32 * 900000;
+constexpr int64_t kDeviceSlabBytes = 32 * 900000;
+constexpr int64_t kHostSlabBytes = 21 * 900000;
+// Blocks per slab of host input, from four slabs on.
+constexpr int kHostSlabBlocks = 128;
+
+// Slabs of a call that fits the workers' slabs once: split evenly over the
+// workers, so that their stages (and, from host memory, the copies) overlap.
+// Host input takes several per worker once they hold kHostSlabBlocks, so that
+// the first kernels need not wait for a quarter of the input.
+inline int slab_count(int nblocks, int64_t bytes, int workers, bool on_device) {
+  const int rounds = on_device ? 1 : std::max(1, nblocks / (workers * kHostSlabBlocks));
+  const int64_t each = on_device ? kDeviceSlabBytes : kHostSlabBytes;
+  const int64_t by_bytes = bytes < kTwoSlabBytes ? 1 : std::max<int64_t>(2, bytes / each);
+  const int64_t most = std::min<int64_t>(nblocks / kMinSlabBlocks, by_bytes);
+  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)workers * rounds, most));
+}
+
+}  // namespace bz2g
