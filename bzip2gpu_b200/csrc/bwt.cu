@@ -14,9 +14,9 @@
 //      h -> 2h) keys them (head << kb) | ISA[(i + h) mod m] and re-sorts them
 //      stably; the k-th of them in sorted order goes to the k-th active SA
 //      position (groups are contiguous, so this sorts within each group).
-//      Short groups need no radix sort: a block whose active groups hold at
-//      most kGroupMax rotations, and kGroupMean on average, sorts them one by
-//      one in shared memory (k_bwt_groups), in the same rounds.
+//      Short groups need no radix sort: a block whose active groups are all
+//      short (sorts_groups) sorts them one by one in shared memory
+//      (k_bwt_groups), in the same rounds.
 //   4. A block stops when no rotation is active, when a round splits no group
 //      (the rest are equal rotations, already index-ascending), or when the
 //      prefix length reaches m.
@@ -888,20 +888,32 @@ __global__ void __launch_bounds__(256) k_bwt_apply(SlabDev d, int kb, const int3
   }
 }
 
-// Groups of at most kGroupMax rotations are sorted in shared memory: a CTA
+// Groups of at most kGroupMax rotations can be sorted in shared memory: a CTA
 // takes the groups that start in a unit of `step` items of a block's active
 // list, and holds kTile, so a step is what the block's longest group leaves of
 // that (2048 for every block took a CTA for half of what it can hold).  Longer
-// groups would leave steps that mostly reload what other CTAs hold, and every
+// groups leave steps that mostly reload what other CTAs hold, and every
 // doubling of a group is a merge more, where the radix passes cost the same
-// for any group.  Measured, 16 blocks of a repeat that doubles until the end,
-// by groups / by radix sort: groups of 3,500 26.3 / 16.0 ms, 1,800 24.5 / 16.0,
-// 1,280 21.6 / 16.1, 990 18.5 / 16.0, 750 17.9 / 16.0, 500 15.5 / 16.1.  Text has a
-// few long groups among very short ones, which the mean tells apart: with
-// kGroupMax at 1,024 and no mean 512 MiB of it take 15.2 instead of 14.5 ms.
-constexpr int kMinStep = 2048;
+// for any group, and their launches the same for any number of rotations.
+// So groups of more than kGroupLong, or kGroupMean on average, are sorted here
+// only while the slab's blocks on the radix path have few rotations in all.
+// Measured, repeats that double until the end, by groups / by radix sort, ms:
+//   groups of    3,500        1,800        1,280        750          500
+//   1 block      3.6 / 3.8    2.9 / 3.8    2.9 / 3.8    2.6 / 3.8
+//   2 blocks     5.2 / 4.2    4.4 / 4.3    4.2 / 4.3    3.8 / 4.3
+//   4 blocks     8.0 / 6.1    7.4 / 6.1    6.4 / 6.1    5.7 / 6.1
+//   16 blocks    26.3 / 16.0  24.5 / 16.0  21.6 / 16.1  17.9 / 16.0  15.5 / 16.1
+// Text has a few long groups among very short ones, which the mean tells apart:
+// with kGroupMax at 1,024 and no mean 512 MiB of it take 15.2 instead of 14.5.
+constexpr int kMinStep = 512;
 constexpr int kGroupMax = kTile - kMinStep;
+constexpr int kGroupLong = 2048;
 constexpr int kGroupMean = 512;
+__device__ __forceinline__ bool sorts_groups(int gmax, int active, int groups, int radix_active) {
+  if (gmax > kGroupMax) return false;
+  if (gmax <= kGroupLong && active <= kGroupMean * groups) return true;
+  return radix_active <= (gmax > kGroupLong ? 1 << 20 : gmax > kGroupLong / 2 ? 2 << 20 : 6 << 20);
+}
 __device__ __forceinline__ int group_step(int gmax) { return (kTile - gmax) & ~31; }
 
 // Lists a block's tiles, or its units when it is sorted group by group.  The
@@ -935,6 +947,10 @@ __device__ __forceinline__ void write_lists(const TileRuns &r, int nb) {
 // those whose groups are all short.
 __global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefix_len, int packed) {
   __shared__ TileRuns runs;
+  // active rotations of the blocks that were on the radix path in this round
+  // (those sorted by groups add theirs below)
+  const int radix_active = d.sort_ctl[6];
+  __syncthreads();
   for (int b0 = 0; b0 < d.nblocks; b0 += 1024) {
     const int b = b0 + threadIdx.x;
     runs.n[threadIdx.x] = 0;
@@ -947,7 +963,7 @@ __global__ void __launch_bounds__(1024) k_bwt_tile_list(SlabDev d, int64_t prefi
       const int len = d.act_len[b];
       d.sort_len[b] = len;
       if (len > 0) {
-        if (packed && !d.loc[b] && d.gmax[b] <= kGroupMax && len <= kGroupMean * d.ngroups[b]) {
+        if (packed && !d.loc[b] && sorts_groups(d.gmax[b], len, d.ngroups[b], radix_active)) {
           d.loc[b] = 1;
           d.loc_cur[b] = keys_now(d) ^ 1;
         }

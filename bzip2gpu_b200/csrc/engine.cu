@@ -121,7 +121,7 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     dev.tile_c = (int32_t *)alloc(T * 4);
     dev.tile_d = (int32_t *)alloc(T * 4);
     dev.tile_list = (int32_t *)alloc(T * 4);
-    dev.loc_list = (int32_t *)alloc(2 * T * 4);
+    dev.loc_list = (int32_t *)alloc(8 * T * 4);
     dev.vt_list = (int32_t *)alloc(T * 4);
     dev.vg_list = (int32_t *)alloc(((int64_t)mgt + 1) * 4);
     dev.warp_last = (int32_t *)alloc(((int64_t)mt + 1) * (kTileThreads / 32) * 4);

@@ -103,7 +103,7 @@ struct SlabDev {
   // buffer; loc_act, loc_heads, loc_sing: the running round's active
   // rotations, groups and singletons; gmax: the largest active group after a
   // round; loc_step: items per work unit; loc_list: the units, by their first
-  // item / 32 [2 * ntiles].
+  // item / 32 [8 * ntiles].
   int32_t *loc, *loc_cur, *loc_act, *loc_heads, *loc_sing, *gmax, *loc_step, *loc_list;
   // The tiles that hold data, listed in block order (a block's workspace is
   // sized for its worst-case RLE1 output, so most of its tiles can be empty):

@@ -1,7 +1,8 @@
 """Which blocks sort their groups in shared memory: those whose active groups
-are short, at most 2,048 rotations and 512 on average; the others go on by
-radix sort.  Read off the count of radix scatter launches (the first sort has
-four), with the stream compared with the oracle's."""
+are short (at most 2,048 rotations and 512 on average), and of the others those
+that fit (3,584) while the slab holds few of their rotations; the rest goes on
+by radix sort.  Read off the count of radix scatter launches (the first sort
+has four), with the stream compared with the oracle's."""
 import numpy as np
 import pytest
 
@@ -11,14 +12,15 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 
-def _repeat(period, copies):
-    """Groups of `copies` rotations that stay together for many rounds."""
+def _repeat(copies, length=899_000):
+    """A block with groups of `copies` rotations that stay together for many rounds."""
+    period = length // copies
     unit = np.random.default_rng(period).integers(0, 256, period).astype(np.uint8)
     return np.concatenate([np.tile(unit, copies), np.array([7, 9], np.uint8)])
 
 
-def _few_long(k, n):
-    """One group of k rotations among n groups of 3."""
+def _few_long(k, n=3000):
+    """A block with one group of k rotations among n groups of 3."""
     rng = np.random.default_rng(k)
     heads = [np.array([250, 251, 252, 253], np.uint8)] * k
     for q in range(n):
@@ -27,18 +29,23 @@ def _few_long(k, n):
                            for i in rng.permutation(len(heads))])
 
 
-@pytest.mark.parametrize("make,args,radix", [
-    (_repeat, (1500, 2), False), (_repeat, (100, 400), False), (_repeat, (100, 500), False),
-    (_repeat, (100, 540), True), (_repeat, (100, 1000), True), (_repeat, (50, 3500), True),
-    (_few_long, (1900, 3000), False), (_few_long, (2040, 3000), False),
-    (_few_long, (2060, 3000), True), (_few_long, (3500, 3000), True)])
-def test_radix_sort_where_groups_are_long(torch_cuda, make, args, radix):
-    a = make(*args)
+@pytest.mark.parametrize("make,k,blocks,radix", [
+    (_repeat, 2, 2, False), (_repeat, 400, 8, False), (_repeat, 500, 8, False),
+    (_repeat, 540, 8, True), (_repeat, 540, 6, False), (_repeat, 1000, 8, True),
+    (_repeat, 1100, 3, True), (_repeat, 1100, 2, False), (_repeat, 2000, 3, True),
+    (_repeat, 2100, 2, True), (_repeat, 2100, 1, False), (_repeat, 3500, 2, True),
+    (_repeat, 3584, 1, False), (_repeat, 3700, 1, True),
+    (_few_long, 1900, 8, False), (_few_long, 2060, 8, False), (_few_long, 3700, 1, True)])
+def test_radix_sort_where_groups_are_long(torch_cuda, make, k, blocks, radix):
+    one = make(k)
+    a = np.tile(one, blocks)
     B.set_timing(True)
     try:
-        got = B.compress(a, 9)
+        got = B.compress(a, 9, one.size)
         scatters = B.last_stats()["scatter_launches"]
     finally:
         B.set_timing(False)
-    assert got == oracle.compress(a, 9)
+    # the blocks are alike: the oracle codes one
+    part, bits, fold, _ = oracle.compress_part(one, one.size)
+    assert got == oracle.assemble([part] * blocks, [bits] * blocks, [fold] * blocks, [1] * blocks)
     assert (scatters > 4) == radix, scatters
