@@ -18,12 +18,13 @@ constexpr int kMinSlabBlocks = 16;
 // only where even then it takes no longer than as one slab did before there
 // were several, sooner for host input, whose copies overlap too.  In ms, one
 // slab then / cut on an idle host / on a busy one: 30 MB on the device 3.1 /
-// 1.8 / 2.9 (two slabs), 110 MB 6.5 / 4.1 / 6.1 (three); 45 MB from the host
-// 4.5 / 2.8 / 4.1 (two), 110 MB 8.5 / 5.1 / 7.2 (four).  Cut by 16 blocks
-// alone, 6.4 MB in blocks of 100,000 took 2.1 / 1.3 / 4.2, now 1.2 on both.
+// 1.8 / 2.9 (two slabs), 110 MB 6.6 / 4.2 / 6.2 (three); 45 MB from the host
+// 4.6 / 2.8 / 4.1 (two), 110 MB 8.6 / 5.2 / 7.2 (four), but 60 MB 5.4 / 3.2 /
+// 5.7 with three.  Cut by 16 blocks alone, 6.4 MB in blocks of 100,000 took
+// 2.1 / 1.4 / 4.4, now 1.2 on both.
 constexpr int64_t kTwoSlabBytes = 32 * 900000;
 constexpr int64_t kDeviceSlabBytes = 32 * 900000;
-constexpr int64_t kHostSlabBytes = 21 * 900000;
+constexpr int64_t kHostSlabBytes = 26 * 900000;
 // Blocks per slab of host input, from four slabs on.
 constexpr int kHostSlabBlocks = 128;
 

@@ -32,7 +32,7 @@ def test_full_blocks(counts):
     rows = [(-(-s * MB // 900_000), s * MB, 4, 1) for s in sizes]
     assert counts(rows) == [1, 1, 1, 2, 2, 2, 3, 4, 4, 4]
     # host input is cut sooner, and takes several slabs per worker later
-    rows = [(-(-s * MB // 900_000), s * MB, 4, 0) for s in (28, 29, 56, 57, 75, 76)]
+    rows = [(-(-s * MB // 900_000), s * MB, 4, 0) for s in (28, 29, 70, 71, 93, 94)]
     assert counts(rows) == [1, 2, 2, 3, 3, 4]
     assert counts([(n, n * 900_000, 4, 0) for n in (128, 512, 1023, 1024, 1536)]) == [4, 4, 4, 8, 12]
 
