@@ -339,32 +339,16 @@ void Compressor::run(const uint8_t *const *ptrs, const int *lens, int nblocks, i
   }
   const int B = per_slab;
   // slabs: up to B blocks, fewer where long blocks would overflow a workspace
-  std::vector<int> slab_at{0};
-  {
-    int64_t raw = 0, elems = 0;
-    int rt = 0, tiles = 0, gt = 0, cnt = 0;
-    for (int b = 0; b < nblocks; b++) {
-      const BlockNeeds q = block_needs(lens[b], cfg_.m_cap);
-      BZ_REQUIRE(q.raw <= ws0.max_raw && q.raw_tiles <= ws0.max_raw_tiles &&
-                     q.elems <= ws0.max_elems && q.tiles <= ws0.max_tiles &&
-                     q.group_tiles <= ws0.max_group_tiles,
-                 kErrArg, "block larger than a slab");
-      if (cnt == B || raw + q.raw > ws0.max_raw || rt + q.raw_tiles > ws0.max_raw_tiles ||
-          elems + q.elems > ws0.max_elems || tiles + q.tiles > ws0.max_tiles ||
-          gt + q.group_tiles > ws0.max_group_tiles) {
-        slab_at.push_back(b);
-        raw = elems = 0;
-        rt = tiles = gt = cnt = 0;
-      }
-      raw += q.raw;
-      elems += q.elems;
-      rt += q.raw_tiles;
-      tiles += q.tiles;
-      gt += q.group_tiles;
-      cnt++;
-    }
-    if (nblocks > 0) slab_at.push_back(nblocks);
+  auto needs = [&](int b) { return block_needs(lens[b], cfg_.m_cap); };
+  const BlockNeeds room = ws0.room();
+  for (int b = 0; b < nblocks; b++) {
+    const BlockNeeds q = needs(b);
+    BZ_REQUIRE(q.raw <= room.raw && q.raw_tiles <= room.raw_tiles && q.elems <= room.elems &&
+                   q.tiles <= room.tiles && q.group_tiles <= room.group_tiles,
+               kErrArg, "block larger than a slab");
   }
+  const std::vector<int> slab_at =
+      cut_queue(nblocks, room, INT64_MAX, needs, [&](int) { return B; });
   const int nslabs = (int)slab_at.size() - 1;
 
   std::mutex mu;
@@ -613,32 +597,13 @@ void Compressor::compress_batch(const Item *items, int count, bool on_device, By
   // short, so their number does not count).  128 inputs, 120 MB: one slab 9.9
   // ms, split over the workers 9.2 ms
   reserve(nb);
-  const int64_t share = std::max<int64_t>(
-      1, ntot / slab_count(INT_MAX, ntot, (int)workers_.size(), true));
+  auto needs = [&](int q) { return block_needs(blks[order[q]].len, 0); };
   const Workspace &ws0 = *workers_[0]->ws;
-  std::vector<int> slab_at{0};
-  {
-    int64_t raw = 0, elems = 0;
-    int rt = 0, tiles = 0, gt = 0, cnt = 0, cap = 0;
-    for (int q = 0; q < nb; q++) {
-      const BlockNeeds bn = block_needs(blks[order[q]].len, 0);
-      if (cnt > 0 && (cnt == cap || raw >= share || raw + bn.raw > ws0.max_raw || elems + bn.elems > ws0.max_elems ||
-                      rt + bn.raw_tiles > ws0.max_raw_tiles || tiles + bn.tiles > ws0.max_tiles ||
-                      gt + bn.group_tiles > ws0.max_group_tiles)) {
-        slab_at.push_back(q);
-        raw = elems = 0;
-        rt = tiles = gt = cnt = 0;
-      }
-      if (cnt == 0) cap = std::min(tune_for(blks[order[q]].len).slab_blocks, ws0.max_blocks);
-      raw += bn.raw;
-      elems += bn.elems;
-      rt += bn.raw_tiles;
-      tiles += bn.tiles;
-      gt += bn.group_tiles;
-      cnt++;
-    }
-    if (nb > 0) slab_at.push_back(nb);
-  }
+  const int64_t share =
+      queue_share(nb, slab_count(INT_MAX, ntot, (int)workers_.size(), true), needs);
+  const std::vector<int> slab_at = cut_queue(nb, ws0.room(), share, needs, [&](int q) {
+    return std::min(tune_for(blks[order[q]].len).slab_blocks, ws0.max_blocks);
+  });
   const int nslabs = (int)slab_at.size() - 1;
   // worker streams: the tuned count for the byte-weighted median block length
   int tuned_workers = (int)workers_.size();

@@ -20,16 +20,13 @@
 #include <vector>
 
 #include "common.cuh"
+#include "slabs.h"
 
 namespace bz2g {
 
 // Per-slab plan, built on the host from the raw block lengths.
 // Workspace a block of L raw bytes takes in a slab.  m_cap > 0 bounds its
 // RLE1 bytes (the bzip2 split's blocks: many raw bytes, bounded RLE1 output).
-struct BlockNeeds {
-  int64_t raw, elems;
-  int raw_tiles, tiles, group_tiles;
-};
 BlockNeeds block_needs(int64_t L, int64_t m_cap);
 
 struct SlabPlan {
@@ -171,6 +168,10 @@ class Workspace {
   // Upload a plan (async on `st`; the plan's host vectors must stay alive until
   // the stream reaches this point, so they are copied into pinned staging).
   void upload_plan(const SlabPlan &p, cudaStream_t st);
+  // What a slab can hold.
+  BlockNeeds room() const {
+    return {max_raw, max_elems, max_raw_tiles, max_tiles, max_group_tiles};
+  }
   SlabDev dev;
   int max_blocks;
   int64_t max_raw, max_elems, out_words;

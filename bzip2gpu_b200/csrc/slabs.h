@@ -5,8 +5,16 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <vector>
 
 namespace bz2g {
+
+// Workspace a block takes in a slab (raw: its bytes rounded up to 16), and
+// what a slab has.
+struct BlockNeeds {
+  int64_t raw, elems;
+  int raw_tiles, tiles, group_tiles;
+};
 
 // Fewest blocks of a slab: with fewer the launches of another slab cost more
 // than they overlap.
@@ -38,6 +46,42 @@ inline int slab_count(int nblocks, int64_t bytes, int workers, bool on_device) {
   const int64_t by_bytes = bytes < kTwoSlabBytes ? 1 : std::max<int64_t>(2, bytes / each);
   const int64_t most = std::min<int64_t>(nblocks / kMinSlabBlocks, by_bytes);
   return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)workers * rounds, most));
+}
+
+// First block of each slab, and the end, for a queue of n blocks.  A slab is
+// closed when it holds cap(its first block) blocks or `share` bytes, or when
+// the next block finds no room.
+template <typename Needs, typename Cap>
+std::vector<int> cut_queue(int n, const BlockNeeds &room, int64_t share, Needs needs, Cap cap) {
+  std::vector<int> at{0};
+  BlockNeeds sum{};
+  int cnt = 0, most = 0;
+  for (int q = 0; q < n; q++) {
+    const BlockNeeds b = needs(q);
+    if (cnt > 0 && (cnt == most || sum.raw >= share || sum.raw + b.raw > room.raw ||
+                    sum.elems + b.elems > room.elems || sum.tiles + b.tiles > room.tiles ||
+                    sum.raw_tiles + b.raw_tiles > room.raw_tiles ||
+                    sum.group_tiles + b.group_tiles > room.group_tiles)) {
+      at.push_back(q);
+      sum = BlockNeeds{};
+      cnt = 0;
+    }
+    if (cnt++ == 0) most = cap(q);
+    sum = {sum.raw + b.raw, sum.elems + b.elems, sum.raw_tiles + b.raw_tiles, sum.tiles + b.tiles,
+           sum.group_tiles + b.group_tiles};
+  }
+  if (n > 0) at.push_back(n);
+  return at;
+}
+
+// The bytes at which a queue's slabs are closed so that it makes `slabs` of
+// them: counted as the slabs count them, or a queue of short blocks would be
+// closed before its last ones.
+template <typename Needs>
+int64_t queue_share(int n, int slabs, Needs needs) {
+  int64_t sum = 0;
+  for (int q = 0; q < n; q++) sum += needs(q).raw;
+  return std::max<int64_t>(1, (sum + slabs - 1) / slabs);
 }
 
 }  // namespace bz2g

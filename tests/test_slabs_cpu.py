@@ -9,16 +9,21 @@ MB = 1_000_000
 
 
 @pytest.fixture(scope="module")
-def counts(tmp_path_factory):
+def program(tmp_path_factory):
     exe = tmp_path_factory.mktemp("slabs") / "slabs"
     subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'bzip2gpu_b200' / 'csrc'}",
                     str(ROOT / "tests" / "cpp" / "slabs.cpp"), "-o", str(exe)], check=True)
 
-    def run(rows):
-        r = subprocess.run([str(exe)], input="\n".join(" ".join(map(str, x)) for x in rows),
+    def run(rows, *args):
+        r = subprocess.run([str(exe), *args], input="\n".join(" ".join(map(str, x)) for x in rows),
                            check=True, capture_output=True, text=True)
-        return [int(x) for x in r.stdout.split()]
+        return [[int(x) for x in ln.split()] for ln in r.stdout.splitlines()]
     return run
+
+
+@pytest.fixture(scope="module")
+def counts(program):
+    return lambda rows: [x[0] for x in program(rows)]
 
 
 def test_short_blocks_do_not_cut_a_small_call(counts):
@@ -44,3 +49,17 @@ def test_few_long_blocks_stay_together(counts):
 
 def test_workers_bound_the_count(counts):
     assert counts([(384, 345 * MB, w, 1) for w in (1, 2, 3, 4)]) == [1, 2, 3, 4]
+
+
+@pytest.mark.parametrize("n,length", [(500, 300), (200, 1001), (1000, 1001), (1000, 1), (7, 16)])
+@pytest.mark.parametrize("slabs", [1, 2, 3, 4])
+def test_a_queue_makes_the_slabs_it_is_meant_to(program, n, length, slabs):
+    # lengths that are no multiples of 16 take more room than they have bytes
+    sizes = program([(n, length, slabs, 1024)], "queue")[0]
+    assert sum(sizes) == n and len(sizes) == slabs
+    assert max(sizes) - min(sizes) <= slabs
+
+
+def test_a_slab_takes_at_most_its_blocks(program):
+    assert program([(1000, 500, 1, 384), (5, 16, 4, 1), (0, 16, 4, 1)], "queue") == [
+        [384, 384, 232], [1, 1, 1, 1, 1], []]
