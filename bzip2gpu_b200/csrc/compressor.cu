@@ -101,16 +101,11 @@ Compressor::Compressor(const CompressorConfig &cfg) : cfg_(cfg) {
   BZ_CUDA(cudaGetDevice(&device_));
   if (cfg_.slab_blocks < 1) cfg_.slab_blocks = 1;
   if (cfg_.workers < 1) cfg_.workers = 1;
-  // The workers' streams in order of priority: a slab's kernels fill the GPU,
-  // so slabs side by side would all finish at the end and leave their copies to
-  // the host for then; in order of priority they finish one after another.
-  // 256 MiB from the host 13.6 -> 12.8 ms, 512 MiB on the device 21.4 -> 20.6.
-  int least = 0, greatest = 0;
-  BZ_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
   for (int i = 0; i < cfg_.workers; i++) {
     auto w = std::make_unique<Worker>();
-    BZ_CUDA(cudaStreamCreateWithPriority(&w->st, cudaStreamNonBlocking,
-                                         std::min(least, greatest + i)));
+    // (the default priority, which is the lowest: the program's own kernels must
+    // not wait behind the workers')
+    BZ_CUDA(cudaStreamCreateWithFlags(&w->st, cudaStreamNonBlocking));
     for (auto &e : w->ev) BZ_CUDA(cudaEventCreate(&e));
     for (auto &e : w->kt_ev) BZ_CUDA(cudaEventCreate(&e));
     for (auto &e : w->rt_ev) BZ_CUDA(cudaEventCreate(&e));
