@@ -693,7 +693,6 @@ __global__ void __launch_bounds__(32 * NW)
 // instructions per position and table, a hundred times what the chain of
 // k_dec_groups needs, but nothing of it waits: 0.1 ms and 0.3 ms for one block,
 // where k_dec_groups takes 3.4 ms.  Positions are relative to the block's magic.
-constexpr int kJumpTile = 4096;
 constexpr int kJumpHalo = 1024;
 constexpr int kJumpAll = kJumpTile + kJumpHalo;
 constexpr int kJumpPer = kJumpAll / 256;             // positions per thread
@@ -728,26 +727,31 @@ __global__ void __launch_bounds__(256) k_dec_lens(const DecTab *tabs, uint8_t *l
   }
 }
 
-// jt0: first tile of each block among all blocks' (jt0[nc]: their number).
+// A CTA per tile: jt0 holds the first tile of each of the nc blocks (jt0[nc]:
+// their number).
 // jumps: per tile, per table, kJumpTile advances, twice the bits (table bytes;
 // kDeadJump: none).
 __global__ void __launch_bounds__(256) k_dec_jumps(const uint32_t *words, int64_t nwords,
                                                    const int64_t *cand, const DecTab *tabs,
                                                    const uint8_t *lens, const int32_t *jt0,
-                                                   uint16_t *jumps) {
+                                                   int nc, uint16_t *jumps) {
   extern __shared__ __align__(16) uint8_t jsm[];
   uint16_t *A = reinterpret_cast<uint16_t *>(jsm), *B = A + kJumpSlots, *C = B + kJumpSlots;
   uint8_t *llen = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(C + kJumpSlots) + 15) & ~(uintptr_t)15);
   __shared__ uint32_t bits[kJumpAll / 32 + 2];
   __shared__ uint32_t lj[kDecMaxCode + 4];
-  const int bi = blockIdx.y;
-  const int tile = jt0[bi] + blockIdx.x;
-  if (tile >= jt0[bi + 1]) return;
+  const int tile = blockIdx.x;
+  int bi = 0;  // jt0[bi] <= tile < jt0[end]
+  for (int end = nc; end - bi > 1;) {
+    const int mid = (bi + end) >> 1;
+    if (jt0[mid] <= tile) bi = mid;
+    else end = mid;
+  }
   const DecTab &tab = tabs[bi];
   if (tab.status != kDecOk) return;
   const int tid = threadIdx.x;
-  const int64_t p0 = cand[bi] + (int64_t)blockIdx.x * kJumpTile;
+  const int64_t p0 = cand[bi] + (int64_t)(tile - jt0[bi]) * kJumpTile;
   for (int q = tid; q < kJumpAll / 32 + 2; q += 256) bits[q] = bits_at(words, nwords, p0 + 32 * q);
   if (tid < 34) {  // positions past the halo, and the two states, in all buffers
     const uint32_t q = kJumpAll + tid;
@@ -2099,28 +2103,24 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     k_dec_head<<<nc, kHeadThreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>());
     BZ_LAUNCH_CHECK();
     // few blocks: group starts by jump tables
-    std::vector<int32_t> jt0(nc + 1, 0);
-    int jmax = 0;
-    int64_t jbits = 0;
-    for (int q = 0; q < nc; q++) {
-      const int nt = (int)std::min<int64_t>(csize(q) / kJumpTile + 1, 1 << 20);
-      jbits += (int64_t)nt * kJumpTile;
-      jmax = std::max(jmax, nt);
-      jt0[q + 1] = (int32_t)std::min<int64_t>((int64_t)jt0[q] + nt, 1 << 30);
-    }
+    std::vector<int64_t> bits(nc);
+    for (int q = 0; q < nc; q++) bits[q] = csize(q);
+    const std::vector<int32_t> jt0 = jump_tiles(bits);
+    const int64_t jbits = (int64_t)jt0[nc] * kJumpTile;
     const size_t jbytes = (size_t)jbits * kDecMaxGroups * 2;
     const bool few = jbits <= kJumpMaxBits;
-    if ((starts == Starts::kByRule ? few : starts == Starts::kJumps) && jmax <= 65535 && (jbytes <= w.jumps.cap || jbytes <= freeb / 4)) {
+    if ((starts == Starts::kByRule ? few : starts == Starts::kJumps) &&
+        (jbytes <= w.jumps.cap || jbytes <= freeb / 4)) {
       w.jumps.reserve(jbytes);
       w.jt0.reserve(4 * (size_t)(nc + 1));
       w.lutlen.reserve((size_t)nc * kLensBytes);
       BZ_CUDA(cudaMemcpyAsync(w.jt0.p, jt0.data(), 4 * (size_t)(nc + 1), cudaMemcpyHostToDevice, st));
       k_dec_lens<<<dim3(kDecMaxGroups, nc), 256, 0, st>>>(dtab, w.lutlen.get<uint8_t>());
       BZ_LAUNCH_CHECK();
-      k_dec_jumps<<<dim3(jmax, nc), 256, kJumpSmem, st>>>(wd, nwords, dcand, dtab,
-                                                          w.lutlen.get<uint8_t>(),
-                                                          w.jt0.get<int32_t>(),
-                                                          w.jumps.get<uint16_t>());
+      k_dec_jumps<<<jt0[nc], 256, kJumpSmem, st>>>(wd, nwords, dcand, dtab,
+                                                   w.lutlen.get<uint8_t>(),
+                                                   w.jt0.get<int32_t>(), nc,
+                                                   w.jumps.get<uint16_t>());
       BZ_LAUNCH_CHECK();
       k_dec_starts<<<nc, 256, kStartsSmem, st>>>(dtab, w.sel.get<uint8_t>(),
                                                  w.gstart.get<uint32_t>(), dcand,

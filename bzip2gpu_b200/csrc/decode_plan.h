@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <vector>
 
 namespace bz2g {
 
@@ -59,6 +60,23 @@ inline ColumnGrids column_grids(int m) {
 // CTAs per block of k_dec_crc, for blocks of at most n output bytes.
 inline int crc_grid(int64_t n) {
   return (int)std::min<int64_t>(kCrcParts, std::max<int64_t>(1, dec_ceil(n, kCrcChunk)));
+}
+
+// Tiles of the jumps over whole groups (k_dec_jumps): kJumpTile bit positions
+// of a block per CTA, blocks one after another.
+constexpr int kJumpTile = 4096;
+// No block is longer: header with symbol map, selectors of at most 6 bits, six
+// tables of 258 lengths of at most 63 steps, 50 codes of at most 20 bits per
+// group.  (Bytes that follow a stream's last block count as its own until then.)
+constexpr int64_t kMaxBlockBits = 105 + 16 + 256 + 18 + 6 * kDecMaxSel + 6 * (5 + 258 * 127) +
+                                  (int64_t)kDecMaxSel * kDecGroupSyms * 20;
+
+// First tile of each block, and their number, for blocks of the given bits.
+inline std::vector<int32_t> jump_tiles(const std::vector<int64_t> &bits) {
+  std::vector<int32_t> first(bits.size() + 1, 0);
+  for (size_t q = 0; q < bits.size(); q++)
+    first[q + 1] = first[q] + (int32_t)(std::min(bits[q], kMaxBlockBits) / kJumpTile) + 1;
+  return first;
 }
 
 }  // namespace bz2g

@@ -2,6 +2,7 @@
 //   grids M...      column_grids of each M
 //   chunks BITS...  chunk_grid
 //   crc N...        crc_grid
+//   tiles BITS...   jump_tiles of blocks of these bits
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -11,6 +12,13 @@
 using namespace bz2g;
 
 int main(int argc, char **argv) {
+  if (!std::strcmp(argv[1], "tiles")) {
+    std::vector<int64_t> bits;
+    for (int i = 2; i < argc; i++) bits.push_back(std::atoll(argv[i]));
+    for (const int32_t t : jump_tiles(bits)) std::printf("%d ", t);
+    std::printf("\n");
+    return 0;
+  }
   for (int i = 2; i < argc; i++) {
     const long long v = std::atoll(argv[i]);
     if (!std::strcmp(argv[1], "grids")) {

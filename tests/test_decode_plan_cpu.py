@@ -46,3 +46,13 @@ def test_short_blocks_take_few_ctas(plan):
 def test_chunk_and_crc_grids(plan):
     assert plan("chunks", 1, 160, 50 * 32 * 4, 50 * 18002, 1 << 40) == [[1], [1], [2], [141], [141]]
     assert plan("crc", 0, 1, 4096, 4097, 31 * 4096, 45_900_000) == [[1], [1], [1], [2], [31], [32]]
+
+
+def test_jump_tiles_are_those_of_the_blocks(plan):
+    assert plan("tiles", 1, 4095, 4096, 8192) == [[0, 1, 2, 4, 7]]
+    # many short blocks and a long one, and garbage after the last block that
+    # counts as its own: a CTA per tile, where a rectangle of the longest block's
+    # tiles for every block was 4,096 x 24,415; a block has at most 18,307,033 bits
+    short = [2400] * 4095
+    assert plan("tiles", *short, 1_400_000)[0][-1] == 4095 + 342
+    assert plan("tiles", *short, 100_000_000)[0][-1] == 4095 + 18_307_033 // 4096 + 1
