@@ -704,12 +704,8 @@ constexpr int kLensBytes = kDecMaxGroups << kLenBits;
 constexpr size_t kJumpSmem = (size_t)3 * kJumpSlots * 2 + (1 << kLenBits) + 64;
 constexpr int kStartStages = 4;  // tiles in flight: 48 KB each
 constexpr size_t kStartStage = (size_t)kDecMaxGroups * kJumpTile * 2;
+static_assert(kStartStage == kJumpTileBytes, "a tile's jumps");
 constexpr size_t kStartsSmem = kStartStages * kStartStage;
-// Compressed bits of a batch up to which the jumps are used: their work grows
-// with the bits of all blocks (about 17 us per 1.4 Mbit block), while
-// k_dec_groups takes the time of its longest block (3.4 ms for such a block)
-// until the blocks fill the GPU.
-constexpr int64_t kJumpMaxBits = 200 << 20;
 
 // Code length (0: longer than kLenBits, or none) by the next kLenBits bits.
 // grid: (table, block)
@@ -727,8 +723,8 @@ __global__ void __launch_bounds__(256) k_dec_lens(const DecTab *tabs, uint8_t *l
   }
 }
 
-// A CTA per tile: jt0 holds the first tile of each of the nc blocks (jt0[nc]:
-// their number).
+// A CTA per tile: jt0 holds the first tile of each of the nc blocks, and the
+// last one's end.
 // jumps: per tile, per table, kJumpTile advances, twice the bits (table bytes;
 // kDeadJump: none).
 __global__ void __launch_bounds__(256) k_dec_jumps(const uint32_t *words, int64_t nwords,
@@ -741,7 +737,7 @@ __global__ void __launch_bounds__(256) k_dec_jumps(const uint32_t *words, int64_
       (reinterpret_cast<uintptr_t>(C + kJumpSlots) + 15) & ~(uintptr_t)15);
   __shared__ uint32_t bits[kJumpAll / 32 + 2];
   __shared__ uint32_t lj[kDecMaxCode + 4];
-  const int tile = blockIdx.x;
+  const int tile = jt0[0] + blockIdx.x;
   int bi = 0;  // jt0[bi] <= tile < jt0[end]
   for (int end = nc; end - bi > 1;) {
     const int mid = (bi + end) >> 1;
@@ -793,7 +789,7 @@ __global__ void __launch_bounds__(256) k_dec_jumps(const uint32_t *words, int64_
     square(C, A);  // 8
     square(A, C);  // 16, kept
     square(C, A);  // 32
-    uint16_t *out = jumps + ((size_t)tile * kDecMaxGroups + t) * kJumpTile;
+    uint16_t *out = jumps + ((size_t)blockIdx.x * kDecMaxGroups + t) * kJumpTile;
 #pragma unroll
     for (int j = 0; j < kJumpTile / 256; j++) {
       const uint32_t v = B[C[cur[j]]];  // 50
@@ -815,7 +811,7 @@ __global__ void __launch_bounds__(256) k_dec_starts(DecTab *tabs, const uint8_t 
   DecTab &tab = tabs[bi];
   if (tab.status != kDecOk) return;
   const int ng = tab.ng, nsel = tab.nsel;
-  const int t0 = jt0[bi], nt = jt0[bi + 1] - t0;
+  const int t0 = jt0[bi] - jt0[0], nt = jt0[bi + 1] - jt0[bi];
   for (int q = tid; q < nsel; q += 256) sel[q] = selbuf[(size_t)bi * kDecMaxSel + q];
   uint32_t *gs = gstart + (size_t)bi * kDecMaxSel;
   const uint32_t first = (uint32_t)(tab.pay - cand[bi]);
@@ -2086,46 +2082,56 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const int nc = (int)std::min<size_t>(batch, cands.size() - ci);
     BZ_CUDA(cudaMemcpyAsync(w.cand.p, cands.data() + ci, 8 * nc, cudaMemcpyHostToDevice, st));
     // A launch lasts as long as its slowest blocks: start the largest ones
-    // first (compressed size = distance to the next candidate).
+    // first.
+    std::vector<int64_t> bits(nc);  // to the next block or end-of-stream magic
+    auto eos = std::upper_bound(eoss.begin(), eoss.end(), cands[ci]);
+    for (int q = 0; q < nc; q++) {
+      const size_t k = ci + (size_t)q;
+      while (eos != eoss.end() && *eos < cands[k]) ++eos;
+      bits[q] = std::min(k + 1 < cands.size() ? cands[k + 1] : nbits,
+                         eos != eoss.end() ? *eos : nbits) -
+                cands[k];
+    }
     order.resize(nc);
     for (int q = 0; q < nc; q++) order[q] = q;
-    auto csize = [&](int q) {
-      const size_t k = ci + (size_t)q;
-      return (k + 1 < cands.size() ? cands[k + 1] : nbits) - cands[k];
-    };
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return csize(a) > csize(b); });
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bits[a] > bits[b]; });
     BZ_CUDA(cudaMemcpyAsync(w.order.p, order.data(), 4 * nc, cudaMemcpyHostToDevice, st));
     const uint32_t *wd = w.words.get<uint32_t>();
     const int64_t *dcand = w.cand.get<int64_t>();
     DecTab *dtab = w.tab.get<DecTab>();
-    const dim3 cgrid(chunk_grid(csize(order[0])), nc);
+    const dim3 cgrid(chunk_grid(bits[order[0]]), nc);
     k_dec_head<<<nc, kHeadThreads, 0, st>>>(wd, nwords, dcand, dtab, w.sel.get<uint8_t>());
     BZ_LAUNCH_CHECK();
-    // few blocks: group starts by jump tables
-    std::vector<int64_t> bits(nc);
-    for (int q = 0; q < nc; q++) bits[q] = csize(q);
+    // group starts by jumps where that is the shorter way; k_dec_groups walks the
+    // blocks that have none yet
     const std::vector<int32_t> jt0 = jump_tiles(bits);
-    const int64_t jbits = (int64_t)jt0[nc] * kJumpTile;
-    const size_t jbytes = (size_t)jbits * kDecMaxGroups * 2;
-    const bool few = jbits <= kJumpMaxBits;
-    if ((starts == Starts::kByRule ? few : starts == Starts::kJumps) &&
-        (jbytes <= w.jumps.cap || jbytes <= freeb / 4)) {
-      w.jumps.reserve(jbytes);
+    const int64_t room = std::max<int64_t>(w.jumps.cap, freeb / 4) / kJumpTileBytes;
+    const std::vector<int> pieces = jump_pieces(jt0, std::min<int64_t>(room, kJumpMaxTiles));
+    if (!pieces.empty() && (starts == Starts::kJumps ||
+                            (starts == Starts::kByRule && jumps_pay(jt0, (int)pieces.size() - 1)))) {
+      int64_t most = 0;
+      for (size_t k = 0; k + 1 < pieces.size(); k++)
+        most = std::max<int64_t>(most, jt0[pieces[k + 1]] - jt0[pieces[k]]);
+      w.jumps.reserve((size_t)(most * kJumpTileBytes));
       w.jt0.reserve(4 * (size_t)(nc + 1));
       w.lutlen.reserve((size_t)nc * kLensBytes);
       BZ_CUDA(cudaMemcpyAsync(w.jt0.p, jt0.data(), 4 * (size_t)(nc + 1), cudaMemcpyHostToDevice, st));
-      k_dec_lens<<<dim3(kDecMaxGroups, nc), 256, 0, st>>>(dtab, w.lutlen.get<uint8_t>());
+      uint8_t *dlens = w.lutlen.get<uint8_t>();
+      k_dec_lens<<<dim3(kDecMaxGroups, nc), 256, 0, st>>>(dtab, dlens);
       BZ_LAUNCH_CHECK();
-      k_dec_jumps<<<jt0[nc], 256, kJumpSmem, st>>>(wd, nwords, dcand, dtab,
-                                                   w.lutlen.get<uint8_t>(),
-                                                   w.jt0.get<int32_t>(), nc,
-                                                   w.jumps.get<uint16_t>());
-      BZ_LAUNCH_CHECK();
-      k_dec_starts<<<nc, 256, kStartsSmem, st>>>(dtab, w.sel.get<uint8_t>(),
-                                                 w.gstart.get<uint32_t>(), dcand,
-                                                 w.jt0.get<int32_t>(), w.jumps.get<uint16_t>());
-      BZ_LAUNCH_CHECK();
+      for (size_t k = 0; k + 1 < pieces.size(); k++) {
+        const int q = pieces[k], nq = pieces[k + 1] - q;
+        const int32_t *djt0 = w.jt0.get<int32_t>() + q;
+        k_dec_jumps<<<jt0[q + nq] - jt0[q], 256, kJumpSmem, st>>>(
+            wd, nwords, dcand + q, dtab + q, dlens + (size_t)q * kLensBytes, djt0, nq,
+            w.jumps.get<uint16_t>());
+        BZ_LAUNCH_CHECK();
+        k_dec_starts<<<nq, 256, kStartsSmem, st>>>(
+            dtab + q, w.sel.get<uint8_t>() + (size_t)q * kDecMaxSel,
+            w.gstart.get<uint32_t>() + (size_t)q * kDecMaxSel, dcand + q, djt0,
+            w.jumps.get<uint16_t>());
+        BZ_LAUNCH_CHECK();
+      }
     }
     int gthreads = 0;
     const GroupsKernel groups = groups_kernel(nc, w.sms, starts, &gthreads);

@@ -79,4 +79,45 @@ inline std::vector<int32_t> jump_tiles(const std::vector<int64_t> &bits) {
   return first;
 }
 
+// Jumps or chains (k_dec_groups) for a batch.  Jumps cost work with the bits
+// of all blocks, chains the time of the longest block until the blocks fill
+// the GPU, and tables for every block; so the total over the longest block
+// decides, whatever their size, and blocks of few tiles take jumps.  Whole
+// decodes by jumps / chains, ms:
+//   blocks            8            40           100          140          300
+//   text, 900,000     1.6 / 4.4    3.3 / 5.4    6.8 / 7.5    9.3 / 9.2    19 / 15
+//   text, 100,000     0.74 / 1.0   0.99 / 1.4   1.4 / 1.5    1.9 / 1.7    2.9 / 2.3
+//   noise, 900,000    4.1 / 13.2   10.8 / 16.1  22.5 / 20.6
+//   noise, 100,000    1.0 / 2.0    1.8 / 2.3    3.2 / 2.9    4.0 / 3.2    8.0 / 5.0
+// The lines cross at about 130 blocks of text and 80 of noise, which cannot be
+// told apart by their bits; 1,000 blocks of 5,000 bytes take 1.1 / 1.6.
+// Jumps of more tiles than their scratch holds run in pieces of whole blocks;
+// each piece takes the chain of jumps through its longest block anew.  Only
+// noise has such blocks in numbers for which it pays (two pieces: 40 blocks
+// 11.2 / 14.9, 60 blocks 16.1 / 15.8).
+constexpr int kJumpRatio = 125;
+constexpr int kJumpRatioPieces = 55;
+constexpr int kJumpBlock = 3;
+constexpr int kJumpMaxTiles = 51200;  // a piece's: 2.5 GB of scratch
+constexpr int64_t kJumpTileBytes = 6 * 2 * kJumpTile;  // two bytes per table and position
+
+// Blocks at which the pieces begin, and the end; empty when a block alone has
+// more tiles than the scratch.
+inline std::vector<int> jump_pieces(const std::vector<int32_t> &first, int64_t room_tiles) {
+  std::vector<int> at{0};
+  for (int q = 0; q + 1 < (int)first.size(); q++) {
+    if (first[q + 1] - first[q] > room_tiles) return {};
+    if (first[q + 1] - first[at.back()] > room_tiles) at.push_back(q);
+  }
+  at.push_back((int)first.size() - 1);
+  return at;
+}
+
+inline bool jumps_pay(const std::vector<int32_t> &first, int pieces) {
+  const int64_t n = (int64_t)first.size() - 1;
+  int64_t longest = 1;
+  for (int64_t q = 0; q < n; q++) longest = std::max<int64_t>(longest, first[q + 1] - first[q]);
+  return first.back() <= (pieces > 1 ? kJumpRatioPieces : kJumpRatio) * longest + kJumpBlock * n;
+}
+
 }  // namespace bz2g

@@ -3,6 +3,7 @@
 //   chunks BITS...  chunk_grid
 //   crc N...        crc_grid
 //   tiles BITS...   jump_tiles of blocks of these bits
+//   jumps ROOM BITS...  the pieces they run in, then whether they pay
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -12,6 +13,15 @@
 using namespace bz2g;
 
 int main(int argc, char **argv) {
+  if (!std::strcmp(argv[1], "jumps")) {
+    std::vector<int64_t> bits;
+    for (int i = 3; i < argc; i++) bits.push_back(std::atoll(argv[i]));
+    const std::vector<int32_t> first = jump_tiles(bits);
+    const std::vector<int> at = jump_pieces(first, std::atoll(argv[2]));
+    for (const int q : at) std::printf("%d ", q);
+    std::printf("\n%d\n", !at.empty() && jumps_pay(first, (int)at.size() - 1));
+    return 0;
+  }
   if (!std::strcmp(argv[1], "tiles")) {
     std::vector<int64_t> bits;
     for (int i = 2; i < argc; i++) bits.push_back(std::atoll(argv[i]));

@@ -56,3 +56,31 @@ def test_jump_tiles_are_those_of_the_blocks(plan):
     short = [2400] * 4095
     assert plan("tiles", *short, 1_400_000)[0][-1] == 4095 + 342
     assert plan("tiles", *short, 100_000_000)[0][-1] == 4095 + 18_307_033 // 4096 + 1
+
+
+TEXT, SHORT, NOISE = 1_400_000, 155_000, 7_250_000
+
+
+@pytest.mark.parametrize("bits", [TEXT, SHORT, NOISE, 40_000])
+def test_the_blocks_in_all_decide_whatever_their_size(plan, bits):
+    # up to 125 times the longest block, and 3 tiles a block
+    tiles = bits // 4096 + 1
+    most = 125 * tiles // (tiles - 3)
+    assert plan("jumps", 1 << 30, *[bits] * most)[1] == [1]
+    assert plan("jumps", 1 << 30, *[bits] * (most + 1))[1] == [0]
+
+
+def test_short_blocks_take_jumps(plan):
+    assert plan("jumps", 1 << 30, *[2400] * 4096)[1] == [1]
+    assert plan("jumps", 1 << 30, *[10_000] * 4000)[1] == [1]
+    assert plan("jumps", 1 << 30, *[14_000] * 2000, TEXT)[1] == [1]  # beside a long one
+
+
+def test_jumps_run_in_pieces_of_whole_blocks(plan):
+    # 51,200 tiles a piece: 28 blocks of 1,771 tiles
+    assert plan("jumps", 51200, *[NOISE] * 28) == [[0, 28], [1]]
+    assert plan("jumps", 51200, *[NOISE] * 40) == [[0, 28, 40], [1]]
+    assert plan("jumps", 51200, *[NOISE] * 57) == [[0, 28, 56, 57], [0]]
+    assert plan("jumps", 51200, *[TEXT] * 150)[1] == [0]
+    assert plan("jumps", 1770, NOISE) == [[], [0]] and plan("jumps", 1771, NOISE) == [[0, 1], [1]]
+    assert plan("jumps", 3, 1, 4096, 4096, 1) == [[0, 2, 4], [1]]

@@ -183,3 +183,11 @@ def test_malformed_streams_are_errors(path, name):
     with pytest.raises(B.Bz2gError):
         B.decompress(s[: len(s) * 2 // 3])
     assert len(B.decompress(s)) > 0  # and the next call is right again
+
+
+@pytest.mark.gpu
+def test_more_tiles_than_a_piece_of_jumps(path):
+    # 240 Mbit: two pieces of jumps
+    d = B.gen_uniform(30_000_000, 6, device=True)
+    s = B.compress_device(d, 9)
+    assert B.decompress(s) == d.cpu().numpy().tobytes()
