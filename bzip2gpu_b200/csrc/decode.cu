@@ -39,6 +39,7 @@
 #include "compressor.h"
 #include "crc.cuh"
 #include "decode_plan.h"
+#include "grow_buf.h"
 
 namespace bz2g {
 
@@ -1808,24 +1809,20 @@ __global__ void __launch_bounds__(256) k_dec_crc(const int64_t *lens, const int6
   if (threadIdx.x == 0) atomicXor(&crcs[k], gf_mul(acc, xpow8((uint64_t)(n - b1))));
 }
 
-// Device buffer that only grows (contents are not kept).
-struct DevBuf {
-  void *p = nullptr;
-  size_t cap = 0;
-  template <typename T>
-  T *get() const {
-    return static_cast<T *>(p);
+struct DevMem {
+  static void *alloc(size_t bytes) {
+    void *p = nullptr;
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    BZ_CUDA(e);
+    return p;
   }
-  void reserve(size_t bytes) {
-    bytes = std::max<size_t>(bytes, 16);
-    if (bytes <= cap) return;
-    if (p) BZ_CUDA(cudaFree(p));
-    p = nullptr;
-    cap = 0;
-    BZ_CUDA(cudaMalloc(&p, bytes));
-    cap = bytes;
-  }
+  static void free(void *p) { BZ_CUDA(cudaFree(p)); }  // waits for kernels that use it
 };
+using DevBuf = GrowBuf<DevMem>;
 
 // Where decoded bytes go, batch by batch, in stream order.
 struct DecSink {
@@ -1914,9 +1911,18 @@ struct DecWork {
     BZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dec_groups<4>, 128, 0));
     resident = std::max(1, sms * per_sm);
   }
+  // The jumps' scratch (up to 2.5 GB) is the one that a call can do without:
+  // it is given up where any other is refused.
+  void reserve(DevBuf &b, size_t bytes) {
+    BZ_REQUIRE(reserve_or_free(b, bytes, jumps), kErrCuda,
+               "decoder: device allocation of " + std::to_string(bytes) + " bytes failed");
+  }
+  // What a batch's size counts on: all that is kept and grows with it.
   size_t held() const {
     size_t s = 0;
-    for (const DevBuf *b : {&L, &hist, &tt, &sel, &tab, &gstart, &ctl, &pool, &out[0], &out[1]}) s += b->cap;
+    for (const DevBuf *b : {&L, &hist, &tt, &sel, &tab, &gstart, &ctl, &pool, &maps, &lutlen,
+                            &jumps, &out[0], &out[1]})
+      s += b->cap;
     return s;
   }
 };
@@ -1938,7 +1944,8 @@ DecWork &dec_work() {
 constexpr size_t kSlotBytes = (size_t)kDecCap * 5 + (size_t)kLfChunks * 256 * 4 + kDecMaxSel * 5 +
                               sizeof(DecTab) + sizeof(WalkCtl) + sizeof(DecBlock) +
                               (size_t)kMaxWalkChunks * kWalkChunk +
-                              sizeof(RunMap) * kUnTiles + 64;
+                              sizeof(RunMap) * kUnTiles + kLensBytes + 64;
+static_assert(kSlotBytes / 100000 == 84, "8.4 MB, as documented");
 constexpr int kMaxBatch = 4096;
 
 bool is_header(const uint8_t *h) {
@@ -1967,9 +1974,9 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
   const int64_t nbits = (int64_t)n * 8;
   // candidates
   const int ccap = (int)std::min<int64_t>((int64_t)n / 8 + 64, 1 << 26);
-  w.blk.reserve(8 * (size_t)ccap);
-  w.eos.reserve(8 * (size_t)ccap);
-  w.cnt.reserve(8);
+  w.reserve(w.blk, 8 * (size_t)ccap);
+  w.reserve(w.eos, 8 * (size_t)ccap);
+  w.reserve(w.cnt, 8);
   BZ_CUDA(cudaMemsetAsync(w.cnt.p, 0, 8, st));
   k_dec_magic<<<(unsigned)((nwords + 255) / 256), 256, 0, st>>>(
       w.words.get<uint32_t>(), nwords, nbits, w.blk.get<int64_t>(), w.cnt.get<int>(),
@@ -2001,23 +2008,23 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
   const Starts starts = starts_choice();
   const int batch = (int)std::min<size_t>(bmax, std::max<size_t>(cands.size(), 1));
   const int cap = kDecCap;
-  w.cand.reserve(8 * (size_t)batch);
-  w.order.reserve(4 * (size_t)batch);
-  w.db.reserve(sizeof(DecBlock) * (size_t)batch);
-  w.L.reserve((size_t)batch * cap);
-  w.hist.reserve((size_t)batch * kLfChunks * 256 * 4);
-  w.sel.reserve((size_t)batch * kDecMaxSel);
-  w.gstart.reserve((size_t)batch * kDecMaxSel * 4);
-  w.tab.reserve((size_t)batch * sizeof(DecTab));
-  w.idx.reserve(4 * (size_t)batch);
-  w.tt.reserve((size_t)batch * cap * 4);
-  w.lens.reserve(8 * (size_t)batch);
-  w.off.reserve(8 * (size_t)batch);
-  w.crc.reserve(4 * (size_t)batch);
-  w.ctl.reserve(sizeof(WalkCtl) * (size_t)batch);
-  w.pool.reserve((size_t)kMaxWalkChunks * kWalkChunk * (size_t)batch);
-  w.bad.reserve(16);
-  w.maps.reserve(sizeof(RunMap) * kUnTiles * (size_t)batch);
+  w.reserve(w.cand, 8 * (size_t)batch);
+  w.reserve(w.order, 4 * (size_t)batch);
+  w.reserve(w.db, sizeof(DecBlock) * (size_t)batch);
+  w.reserve(w.L, (size_t)batch * cap);
+  w.reserve(w.hist, (size_t)batch * kLfChunks * 256 * 4);
+  w.reserve(w.sel, (size_t)batch * kDecMaxSel);
+  w.reserve(w.gstart, (size_t)batch * kDecMaxSel * 4);
+  w.reserve(w.tab, (size_t)batch * sizeof(DecTab));
+  w.reserve(w.idx, 4 * (size_t)batch);
+  w.reserve(w.tt, (size_t)batch * cap * 4);
+  w.reserve(w.lens, 8 * (size_t)batch);
+  w.reserve(w.off, 8 * (size_t)batch);
+  w.reserve(w.crc, 4 * (size_t)batch);
+  w.reserve(w.ctl, sizeof(WalkCtl) * (size_t)batch);
+  w.reserve(w.pool, (size_t)kMaxWalkChunks * kWalkChunk * (size_t)batch);
+  w.reserve(w.bad, 16);
+  w.reserve(w.maps, sizeof(RunMap) * kUnTiles * (size_t)batch);
   if (w.h_crc_cap < (size_t)batch) {
     if (w.h_crc) BZ_CUDA(cudaFreeHost(w.h_crc));
     w.h_crc = nullptr;
@@ -2107,14 +2114,14 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
     const std::vector<int32_t> jt0 = jump_tiles(bits);
     const int64_t room = std::max<int64_t>(w.jumps.cap, freeb / 4) / kJumpTileBytes;
     const std::vector<int> pieces = jump_pieces(jt0, std::min<int64_t>(room, kJumpMaxTiles));
-    if (!pieces.empty() && (starts == Starts::kJumps ||
-                            (starts == Starts::kByRule && jumps_pay(jt0, (int)pieces.size() - 1)))) {
-      int64_t most = 0;
-      for (size_t k = 0; k + 1 < pieces.size(); k++)
-        most = std::max<int64_t>(most, jt0[pieces[k + 1]] - jt0[pieces[k]]);
-      w.jumps.reserve((size_t)(most * kJumpTileBytes));
-      w.jt0.reserve(4 * (size_t)(nc + 1));
-      w.lutlen.reserve((size_t)nc * kLensBytes);
+    int64_t most = 0;
+    for (size_t k = 0; k + 1 < pieces.size(); k++)
+      most = std::max<int64_t>(most, jt0[pieces[k + 1]] - jt0[pieces[k]]);
+    if (!pieces.empty() &&
+        (starts == Starts::kJumps ||
+         (starts == Starts::kByRule && jumps_pay(jt0, (int)pieces.size() - 1))) &&
+        w.jt0.try_reserve(4 * (size_t)(nc + 1)) && w.lutlen.try_reserve((size_t)nc * kLensBytes) &&
+        w.jumps.try_reserve((size_t)(most * kJumpTileBytes))) {
       BZ_CUDA(cudaMemcpyAsync(w.jt0.p, jt0.data(), 4 * (size_t)(nc + 1), cudaMemcpyHostToDevice, st));
       uint8_t *dlens = w.lutlen.get<uint8_t>();
       k_dec_lens<<<dim3(kDecMaxGroups, nc), 256, 0, st>>>(dtab, dlens);
@@ -2213,7 +2220,7 @@ void decode_words(DecWork &w, size_t n, DecSink &sink) {
       if ((size_t)tot + 16 > w.out[slot].cap) BZ_CUDA(cudaEventSynchronize(w.copied[slot]));
       BZ_CUDA(cudaStreamWaitEvent(st, w.copied[slot], 0));
     }
-    w.out[slot].reserve((size_t)tot + 16);
+    w.reserve(w.out[slot], (size_t)tot + 16);
     BZ_CUDA(cudaMemcpyAsync(w.off.p, offs.data(), 8 * na, cudaMemcpyHostToDevice, st));
     k_dec_unrle1_write<<<ugrid, 256, 0, st>>>(didx, ddb, L, cap, w.maps.get<RunMap>(),
                                               w.off.get<int64_t>(), w.out[slot].get<uint8_t>());
@@ -2244,7 +2251,7 @@ void decode_into_sink(const uint8_t *in, size_t n, DecSink &sink) {
   std::lock_guard<std::mutex> g(w.mu);
   w.init();
   const size_t nwords = (n + 3) / 4 + 2;
-  w.words.reserve(nwords * 4);
+  w.reserve(w.words, nwords * 4);
   const size_t body = n / 4 * 4;
   BZ_CUDA(cudaMemsetAsync(w.words.get<uint8_t>() + body, 0, nwords * 4 - body, w.st));
   BZ_CUDA(cudaMemcpyAsync(w.words.p, in, n, cudaMemcpyDefault, w.st));
