@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstring>
 #include <sstream>
+#include <utility>
 
 namespace bz2g {
 
@@ -83,119 +84,119 @@ void SlabPlan::build(const int *lens, int n, int cut, int64_t mcap) {
   gt_begin[n] = (int)gt_block.size();
 }
 
-void *Workspace::alloc(size_t bytes) {
-  void *p = nullptr;
-  BZ_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 256)));
-  allocs_.push_back(p);
-  return p;
-}
-
 Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     : max_blocks(mb), max_raw(mr), max_elems(me), max_tiles(mt), max_raw_tiles(mrt),
       max_group_tiles(mgt) {
   std::memset(&dev, 0, sizeof(dev));
+  // One allocation on the device and one page-locked one, shared out: the calls
+  // for single stages make a workspace each, and one by one its 76 arrays cost
+  // more than the stage (CRC of 20,000 bytes 1.0 ms, of 900,000 8.2; so 0.6, 0.7).
+  size_t bytes = 0;
+  std::vector<std::pair<void **, size_t>> parts;
+  auto part = [&](auto *&p, size_t n) {
+    parts.push_back({(void **)&p, bytes});
+    bytes += (std::max<size_t>(n, 1) + 511) / 512 * 512;
+  };
   try {
     const int64_t E = me + kTile;  // slack for vector loads past a block's end
-    dev.raw = (uint8_t *)alloc(mr + 64);
-    dev.rle1 = (uint8_t *)alloc(E);
-    dev.last = (uint8_t *)alloc(E);
-    dev.mtf = (uint8_t *)alloc(E);
-    dev.sa = (int32_t *)alloc(E * 4);
-    dev.isa = (int32_t *)alloc(E * 4);
-    dev.kpos[0] = (int32_t *)alloc(E * 4);
-    dev.kpos[1] = (int32_t *)alloc(E * 4);
-    dev.keys[0] = (uint64_t *)alloc(E * 8);
-    dev.keys[1] = (uint64_t *)alloc(E * 8);
-    dev.vals[0] = (uint32_t *)alloc(E * 4);
-    dev.vals[1] = (uint32_t *)alloc(E * 4);
-    dev.rle2 = (uint16_t *)alloc(E * 2);
-    dev.sel = (uint8_t *)alloc(E / 32 + 64);
-    dev.sel_mtf = (uint8_t *)alloc(E / 32 + 64);
-    dev.grp_bits = (uint32_t *)alloc((E / 32 + 64) * 4);
+    const int64_t B = mb + 1;
+    const int64_t G = mt / kScanTiles + B;  // groups: t / kScanTiles + b of a block's tiles t
+    // (these three are zeroed)
+    part(dev.err, 64);
+    part(dev.scan_count, G * 4);
+    part(dev.blk_count, B * 4);
+    const size_t zeroed = bytes;
+    part(dev.raw, mr + 64);
+    part(dev.rle1, E);
+    part(dev.last, E);
+    part(dev.mtf, E);
+    part(dev.sa, E * 4);
+    part(dev.isa, E * 4);
+    part(dev.kpos[0], E * 4);
+    part(dev.kpos[1], E * 4);
+    part(dev.keys[0], E * 8);
+    part(dev.keys[1], E * 8);
+    part(dev.vals[0], E * 4);
+    part(dev.vals[1], E * 4);
+    part(dev.rle2, E * 2);
+    part(dev.sel, E / 32 + 64);
+    part(dev.sel_mtf, E / 32 + 64);
+    part(dev.grp_bits, (E / 32 + 64) * 4);
     // payload: <= 17 bits per symbol; header: <= 6 bits per selector + tables
     out_words = E * kMaxCodeLen / 32 + (int64_t)mb * 8192 + 64;
-    dev.out = (uint32_t *)alloc(out_words * 4);
+    part(dev.out, out_words * 4);
     const int64_t T = std::max<int64_t>(mt, mrt) + 1;
-    dev.tile_a = (int32_t *)alloc(T * 4);
-    dev.tile_b = (int32_t *)alloc(T * 4);
-    dev.tile_c = (int32_t *)alloc(T * 4);
-    dev.tile_d = (int32_t *)alloc(T * 4);
-    dev.tile_list = (int32_t *)alloc(T * 4);
-    dev.loc_list = (int32_t *)alloc(8 * T * 4);
-    dev.vt_list = (int32_t *)alloc(T * 4);
-    dev.vg_list = (int32_t *)alloc(((int64_t)mgt + 1) * 4);
-    dev.warp_last = (int32_t *)alloc(((int64_t)mt + 1) * (kTileThreads / 32) * 4);
-    dev.warp_act = (int32_t *)alloc(((int64_t)mt + 1) * (kTileThreads / 32) * 4);
-    dev.head_bits = (uint32_t *)alloc(((int64_t)mt * (kTile / 32) + 1) * 4);
-    dev.tile_hist = (uint32_t *)alloc((int64_t)mt * kMaxRadix * 4);
-    dev.tile_last = (int32_t *)alloc((int64_t)mt * 256 * 4);
-    dev.gt_bits = (uint32_t *)alloc(((int64_t)mgt + 1) * 4);
-    const int64_t B = mb + 1;
-    dev.m = (int32_t *)alloc(B * 4);
-    dev.s = (int32_t *)alloc(B * 4);
-    dev.n_in_use = (int32_t *)alloc(B * 4);
-    dev.orig_ptr = (int32_t *)alloc(B * 4);
-    dev.n_groups = (int32_t *)alloc(B * 4);
-    dev.n_sel = (int32_t *)alloc(B * 4);
-    dev.crc = (uint32_t *)alloc(B * 4);
-    dev.crc_acc = (uint32_t *)alloc(B * 4);
-    dev.present = (uint32_t *)alloc(B * 8 * 4);
-    dev.freq = (int32_t *)alloc(B * kMaxAlpha * 4);
-    dev.len = (uint8_t *)alloc(B * kMaxGroups * kMaxAlpha);
-    dev.code = (int32_t *)alloc(B * kMaxGroups * kMaxAlpha * 4);
-    dev.len_code = (uint32_t *)alloc(B * kLenCode * 4);
-    dev.rfreq = (int32_t *)alloc(B * kMaxGroups * kMaxAlpha * 4);
-    dev.learned = (int32_t *)alloc(B * 4);
-    dev.rfreq_m = (int32_t *)alloc(B * kMaxGroups * kMaxAlpha * 4);
-    dev.len2 = (uint8_t *)alloc(B * kMaxGroups * kMaxAlpha);
-    dev.sel2 = (uint8_t *)alloc(E / 32 + 64);
-    dev.rfreq2 = (int32_t *)alloc(B * kMaxGroups * kMaxAlpha * 4);
-    dev.plain_left = (int32_t *)alloc(B * 4);
-    dev.err = (int32_t *)alloc(64);
-    BZ_CUDA(cudaMemset(dev.err, 0, 64));
-    dev.sort_len = (int32_t *)alloc(B * 4);
-    dev.done = (int32_t *)alloc(B * 4);
-    dev.ngroups = (int32_t *)alloc(B * 4);
-    dev.act_len = (int32_t *)alloc(B * 4);
+    part(dev.tile_a, T * 4);
+    part(dev.tile_b, T * 4);
+    part(dev.tile_c, T * 4);
+    part(dev.tile_d, T * 4);
+    part(dev.tile_list, T * 4);
+    part(dev.loc_list, 8 * T * 4);
+    part(dev.vt_list, T * 4);
+    part(dev.vg_list, ((int64_t)mgt + 1) * 4);
+    part(dev.warp_last, ((int64_t)mt + 1) * (kTileThreads / 32) * 4);
+    part(dev.warp_act, ((int64_t)mt + 1) * (kTileThreads / 32) * 4);
+    part(dev.head_bits, ((int64_t)mt * (kTile / 32) + 1) * 4);
+    part(dev.tile_hist, (int64_t)mt * kMaxRadix * 4);
+    part(dev.tile_last, (int64_t)mt * 256 * 4);
+    part(dev.gt_bits, ((int64_t)mgt + 1) * 4);
+    part(dev.m, B * 4);
+    part(dev.s, B * 4);
+    part(dev.n_in_use, B * 4);
+    part(dev.orig_ptr, B * 4);
+    part(dev.n_groups, B * 4);
+    part(dev.n_sel, B * 4);
+    part(dev.crc, B * 4);
+    part(dev.crc_acc, B * 4);
+    part(dev.present, B * 8 * 4);
+    part(dev.freq, B * kMaxAlpha * 4);
+    part(dev.len, B * kMaxGroups * kMaxAlpha);
+    part(dev.code, B * kMaxGroups * kMaxAlpha * 4);
+    part(dev.len_code, B * kLenCode * 4);
+    part(dev.rfreq, B * kMaxGroups * kMaxAlpha * 4);
+    part(dev.learned, B * 4);
+    part(dev.rfreq_m, B * kMaxGroups * kMaxAlpha * 4);
+    part(dev.len2, B * kMaxGroups * kMaxAlpha);
+    part(dev.sel2, E / 32 + 64);
+    part(dev.rfreq2, B * kMaxGroups * kMaxAlpha * 4);
+    part(dev.plain_left, B * 4);
+    part(dev.sort_len, B * 4);
+    part(dev.done, B * 4);
+    part(dev.ngroups, B * 4);
+    part(dev.act_len, B * 4);
     for (int32_t **a : {&dev.loc, &dev.loc_cur, &dev.loc_act, &dev.loc_heads, &dev.loc_sing,
                         &dev.gmax, &dev.loc_step})
-      *a = (int32_t *)alloc(B * 4);
-    dev.active_sum = (int64_t *)alloc(B * 8);
-    dev.pstat = (int32_t *)alloc(B * 8 * 4);
-    dev.hdr_bits = (int64_t *)alloc(B * 8);
-    dev.pay_bits = (int64_t *)alloc(B * 8);
-    dev.blk_start = (int64_t *)alloc(B * 8);
-    dev.sort_ctl = (int32_t *)alloc(64);
-    const int64_t G = mt / kScanTiles + B;  // groups: t / kScanTiles + b of a block's tiles t
-    dev.scan_base = (uint32_t *)alloc(G * kMaxRadix * 4);
-    dev.scan_count = (int32_t *)alloc(G * 4);
-    BZ_CUDA(cudaMemset(dev.scan_count, 0, G * 4));
-    dev.blk_count = (int32_t *)alloc(B * 4);
-    BZ_CUDA(cudaMemset(dev.blk_count, 0, B * 4));
-    dev.stream = (uint64_t *)alloc(64);
-    dev.kt_elems = (uint64_t *)alloc(8 * kMaxTimedLaunches);
+      part(*a, B * 4);
+    part(dev.active_sum, B * 8);
+    part(dev.pstat, B * 8 * 4);
+    part(dev.hdr_bits, B * 8);
+    part(dev.pay_bits, B * 8);
+    part(dev.blk_start, B * 8);
+    part(dev.sort_ctl, 64);
+    part(dev.scan_base, G * kMaxRadix * 4);
+    part(dev.stream, 64);
+    part(dev.kt_elems, 8 * kMaxTimedLaunches);
     // plan arrays: 3 int64 per block + ints
     pinned_plan_bytes = (size_t)B * 3 * 8 + ((size_t)B * 4 + mrt * 2 + mt + mgt * 2) * 4 + 1024;
-    plan_dev_ = alloc(pinned_plan_bytes);
-    BZ_CUDA(cudaMallocHost(&pinned_plan, pinned_plan_bytes));
-    BZ_CUDA(cudaMallocHost((void **)&dev.h_flags, 64));
-    BZ_CUDA(cudaMallocHost((void **)&dev.live, 8 * sizeof(int)));
+    part(plan_dev_, pinned_plan_bytes);
+    BZ_CUDA(cudaMalloc((void **)&device_, bytes));
+    for (const auto &q : parts) *q.first = device_ + q.second;
+    BZ_CUDA(cudaMemset(device_, 0, zeroed));
+    BZ_CUDA(cudaMallocHost((void **)&host_, 128 + pinned_plan_bytes));
+    dev.h_flags = reinterpret_cast<int32_t *>(host_);
+    dev.live = reinterpret_cast<int *>(host_ + 64);
+    pinned_plan = host_ + 128;
     dev.live[0] = dev.live[1] = dev.live[2] = -1;
   } catch (...) {
-    for (void *p : allocs_) cudaFree(p);
-    allocs_.clear();
-    if (pinned_plan) cudaFreeHost(pinned_plan);
-    if (dev.h_flags) cudaFreeHost(dev.h_flags);
-    if (dev.live) cudaFreeHost(dev.live);
+    if (device_) cudaFree(device_);
+    if (host_) cudaFreeHost(host_);
     throw;
   }
 }
 
 Workspace::~Workspace() {
-  for (void *p : allocs_) cudaFree(p);
-  if (pinned_plan) cudaFreeHost(pinned_plan);
-  if (dev.h_flags) cudaFreeHost(dev.h_flags);
-  if (dev.live) cudaFreeHost(dev.live);
+  if (device_) cudaFree(device_);
+  if (host_) cudaFreeHost(host_);
 }
 
 void Workspace::upload_plan(const SlabPlan &p, cudaStream_t st) {

@@ -180,9 +180,8 @@ class Workspace {
   size_t pinned_plan_bytes = 0;
 
  private:
-  std::vector<void *> allocs_;
-  void *plan_dev_ = nullptr;
-  void *alloc(size_t bytes);
+  uint8_t *device_ = nullptr, *host_ = nullptr;  // all arrays, in two allocations
+  uint8_t *plan_dev_ = nullptr;
 };
 
 // The listed tiles of the slab (built on the first call after m, or s, is
