@@ -857,6 +857,7 @@ int bz2g_selector_dataset(int count, const uint8_t *const *d_inputs, const size_
     int64_t *ctl = nullptr;
     BZ_CUDA(cudaMalloc((void **)&ctl, sizeof(int64_t) * (1 + cfg.slab_blocks)));
     BZ_CUDA(cudaMemset(ctl, 0, sizeof(int64_t) * (1 + cfg.slab_blocks)));
+    BZ_CUDA(cudaStreamSynchronize(nullptr));  // the worker's stream does not wait for it
     mlp::SelectorTap tap{d_group_syms, d_labels, cap, ctl, ctl + 1};
     cfg.tap = &tap;
     try {

@@ -101,11 +101,11 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     const int64_t E = me + kTile;  // slack for vector loads past a block's end
     const int64_t B = mb + 1;
     const int64_t G = mt / kScanTiles + B;  // groups: t / kScanTiles + b of a block's tiles t
-    // (these three are zeroed)
+    // (these three are zeroed by the first upload_plan)
     part(dev.err, 64);
     part(dev.scan_count, G * 4);
     part(dev.blk_count, B * 4);
-    const size_t zeroed = bytes;
+    to_zero_ = bytes;
     part(dev.raw, mr + 64);
     part(dev.rle1, E);
     part(dev.last, E);
@@ -181,7 +181,6 @@ Workspace::Workspace(int mb, int64_t mr, int64_t me, int mt, int mrt, int mgt)
     part(plan_dev_, pinned_plan_bytes);
     BZ_CUDA(cudaMalloc((void **)&device_, bytes));
     for (const auto &q : parts) *q.first = device_ + q.second;
-    BZ_CUDA(cudaMemset(device_, 0, zeroed));
     BZ_CUDA(cudaMallocHost((void **)&host_, 128 + pinned_plan_bytes));
     dev.h_flags = reinterpret_cast<int32_t *>(host_);
     dev.live = reinterpret_cast<int *>(host_ + 64);
@@ -200,6 +199,10 @@ Workspace::~Workspace() {
 }
 
 void Workspace::upload_plan(const SlabPlan &p, cudaStream_t st) {
+  // on the stream whose work counts on it: a memset on the default stream may
+  // still wait for the program's kernels there when that work runs
+  if (to_zero_) BZ_CUDA(cudaMemsetAsync(device_, 0, to_zero_, st));
+  to_zero_ = 0;
   dev.live[0] = dev.live[1] = dev.live[2] = -1;  // a new slab: its lists are built anew
   BZ_REQUIRE(p.nblocks <= max_blocks && p.raw_total <= max_raw && p.elem_total <= max_elems &&
                  (int)p.tile_block.size() <= max_tiles && (int)p.rt_block.size() <= max_raw_tiles &&

@@ -182,6 +182,7 @@ class Workspace {
  private:
   uint8_t *device_ = nullptr, *host_ = nullptr;  // all arrays, in two allocations
   uint8_t *plan_dev_ = nullptr;
+  size_t to_zero_ = 0;  // bytes at the start of device_ not zeroed yet
 };
 
 // The listed tiles of the slab (built on the first call after m, or s, is
