@@ -9,8 +9,8 @@
 //   2. k_dec_head / _groups / _syms / _mscan / _emit: header and tables, the
 //      bit position of every 50-symbol group (the one serial chain, hopped 8
 //      codes at a time; for few blocks a group at a time, from the jumps of
-//      k_dec_lens / _jumps / _starts), the groups' symbols and the inverse move-to-front in
-//      parallel over chunks of 32 groups.  Out: the BWT last column L.
+//      k_dec_lens / _jumps / _starts), the groups' symbols and the inverse
+//      move-to-front in parallel over chunks of 32 groups.  Out: the BWT last column L.
 //   3. k_dec_lf_hist / _scan / _rank: LF vector
 //      tt[C[L[i]] + rank(i)] = i << 8 | L[i] by a stable counting sort.
 //   4. k_dec_walk / k_dec_chain / k_dec_gather: per block, the chain from
@@ -333,7 +333,7 @@ __device__ int code_lengths(const uint32_t *words, int64_t nwords, int64_t &p, i
 // them, and the ones before a zero are its move-to-front index.  The index
 // sequence moves a six-entry list; each thread runs its share from the
 // identity list, a scan of those permutations gives every share's starting
-// list.  The delta-coded lengths are a serial chain (one thread).
+// list.  The delta-coded lengths are one warp's (code_lengths).
 __global__ void __launch_bounds__(kHeadThreads) k_dec_head(const uint32_t *words, int64_t nwords,
                                                            const int64_t *cand, DecTab *tabs,
                                                            uint8_t *selbuf) {
@@ -685,8 +685,9 @@ __global__ void __launch_bounds__(32 * NW)
   if (tid == 0) tab.ngv = g;
 }
 
-// Few blocks: the jump over a whole group (50 codes) from every bit position
-// with every table, then the chain of group starts is one lookup per group.
+// Few blocks (jumps_pay): the jump over a whole group (50 codes) from every bit
+// position with every table, then the chain of group starts is one lookup per
+// group.
 // k_dec_jumps covers kJumpTile positions of a block per CTA: code lengths of
 // the tile and a halo (50 codes take at most 1000 bits), the map squared five
 // times in shared memory, composed to 32 + 16 + 2 codes.  k_dec_starts streams

@@ -290,8 +290,7 @@ __device__ __forceinline__ void heap_push(uint64_t *heap, int z, uint64_t e) {
   }
 }
 
-// Merges the two lightest nodes while the heap has more than `down_to`
-// entries.  Node numbers count up from n_nodes.
+// The node that joins p1 and p2, as a heap entry.
 __device__ __forceinline__ uint64_t merged(uint64_t p1, uint64_t p2, int node, int16_t *parent) {
   const uint32_t w1 = hw(p1), w2 = hw(p2);
   parent[(uint32_t)p1] = parent[(uint32_t)p2] = (int16_t)node;
@@ -301,6 +300,8 @@ __device__ __forceinline__ uint64_t merged(uint64_t p1, uint64_t p2, int node, i
   return ((uint64_t)wn << 32) | (uint32_t)node;
 }
 
+// Merges the two lightest nodes while the heap has more than `down_to`
+// entries.  Node numbers count up from n_nodes.
 template <int L>
 __device__ __forceinline__ void merge_down(uint64_t *heap, int16_t *parent, int down_to, int &n,
                                            int &n_nodes) {

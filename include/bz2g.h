@@ -124,9 +124,11 @@ int bz2g_set_batch_tuning(int n, const int *max_block_len, const int *slab_block
  * CUDA events around every stage of the following whole-stream calls.
  * bz2g_last_stats fills out[0..n) with, for the last whole-stream call on
  * this thread: blocks, sum n, sum m, sum A, sum s, sum groups, payload bits,
- * then device ms of RLE1+CRC, BWT, MTF, RLE2, Huffman, sizes, placement,
+ * then device ms of RLE1+CRC, BWT, MTF, RLE2, Huffman, sizes, placement (summed
+ * over the call's slabs, which run side by side and wait for one another),
  * then the radix-scatter kernel's timed launches, their summed device ms and
- * their algorithmic bytes (items read + written), then the blocks whose
+ * their algorithmic bytes (items read and written, and the next pass's digits
+ * written), then the blocks whose
  * tables came from the learned selector and the blocks with six tables;
  * returns the field count.
  * bz2g_launch_count: kernels launched by this library since it was loaded. */
